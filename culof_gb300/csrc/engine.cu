@@ -108,33 +108,11 @@ Engine::~Engine() {
     if (bgraph_exec_) cudaGraphExecDestroy(bgraph_exec_);
     for (auto& e : events_)
         if (e) cudaEventDestroy(e);
-    for (cudaStream_t st : {high_stream_, side_stream_})
-        if (st) {
-            cudaSetDevice(device_);
-            cudaStreamSynchronize(st);
-            cudaStreamDestroy(st);
-        }
-    for (cudaEvent_t e : {fork_ev_, high_join_, side_join_})
-        if (e) cudaEventDestroy(e);
     if (own_stream_) {
         cudaSetDevice(device_);
         cudaStreamSynchronize(own_stream_);
         cudaStreamDestroy(own_stream_);
     }
-}
-
-void Engine::make_fork_streams() {
-    if (side_stream_) return;
-    // non-blocking (they must not wait for the legacy default stream); the
-    // high one of the greatest priority, the side one of the least, so that
-    // of two kernels that become ready together the high one's CTAs are
-    // dispatched first
-    int least = 0, greatest = 0;
-    CG_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
-    CG_CUDA(cudaStreamCreateWithPriority(&high_stream_, cudaStreamNonBlocking, greatest));
-    CG_CUDA(cudaStreamCreateWithPriority(&side_stream_, cudaStreamNonBlocking, least));
-    for (cudaEvent_t* e : {&fork_ev_, &high_join_, &side_join_})
-        CG_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
 }
 
 // pipeline.cu:99-110: CULOF_TILE_ROWS overrides; otherwise a 2 GiB cap on
@@ -227,7 +205,7 @@ int64_t Engine::knn_core(const float* d_x, int64_t n, int d, int k, bool normali
     float* norms = norms_.as<float>(n);
     unsigned int* maxn = max_norm_.as<unsigned int>(1);
     CG_CUDA(cudaMemsetAsync(status_ptr(), 0, sizeof(int), stream_));
-    stat_total_blocks_ = 0;
+    stat_total_pairs_ = 0.0;
     for (bool& m : marked_) m = false;
     mark(0);
     center(d_x, n, d, normalize, xc, partial, mean, inv, stream_);
@@ -334,14 +312,13 @@ void Engine::stage_times(float* ms, int cap) {
 
 void Engine::pair_stats(double* evaluated, double* total) {
     unsigned long long ev = 0;
-    if (stat_total_blocks_ > 0) {
-        CG_CUDA(cudaMemcpyAsync(&ev, pair_stats_.get(2 * sizeof(unsigned long long)), sizeof(ev),
-                                cudaMemcpyDeviceToHost, stream_));
+    if (stat_total_pairs_ > 0.0) {
+        CG_CUDA(cudaMemcpyAsync(&ev, pair_stats_.get(sizeof(ev)), sizeof(ev), cudaMemcpyDeviceToHost, stream_));
         CG_CUDA(cudaStreamSynchronize(stream_));
     }
-    // one block = 16 rows x 128 columns
-    if (evaluated) *evaluated = static_cast<double>(ev) * 16.0 * 128.0;
-    if (total) *total = static_cast<double>(stat_total_blocks_) * 16.0 * 128.0;
+    // one unit = a row against 64 columns
+    if (evaluated) *evaluated = static_cast<double>(ev) * 64.0;
+    if (total) *total = stat_total_pairs_;
 }
 
 void Engine::probe_bounded_wait(long long limit) {

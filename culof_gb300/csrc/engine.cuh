@@ -145,13 +145,6 @@ private:
     int device_;
     cudaStream_t own_stream_ = nullptr;
     cudaStream_t stream_ = nullptr;
-    // Two streams forked from the call's stream for work that runs side by
-    // side (the small-d sweep on the high one, the isolated rows' pass on
-    // the side one), with the events that fork them and join them back;
-    // created on first use.
-    cudaStream_t high_stream_ = nullptr, side_stream_ = nullptr;
-    cudaEvent_t fork_ev_ = nullptr, high_join_ = nullptr, side_join_ = nullptr;
-    void make_fork_streams();
     int path_ = kPathAuto;
     int last_path_ = kPathAuto;
 
@@ -177,13 +170,11 @@ private:
     unsigned long long bgraph_kernels_ = 0;
     // fast path workspaces
     DevBuf morton_, perm_, sort_tmp_, sort_hist_, cols_, rows_, tc_lists_, tiles_;
-    // the FP32 sweep's evaluated (warp x column tile) blocks; the total it
-    // would evaluate without pruning
-    DevBuf pair_stats_, boxes_, plist_, pcount_, order_;
-    // isolated rows of the small-d sweep: threshold, count, list and flags;
-    // dimension-major columns and quarter-tile boxes
-    DevBuf iso_, iso_cols_;
-    unsigned long long stat_total_blocks_ = 0;
+    // the small-d sweep's evaluated (row, 64 columns) units and the pairs it
+    // would evaluate without pruning; tile boxes; the tensor path's tile lists
+    DevBuf pair_stats_, boxes_, plist_, pcount_;
+    DevBuf iso_;  // rows that leave the small-d sweep for their own pass
+    double stat_total_pairs_ = 0.0;
     // Device status word of the current call: kernels set it (a bounded wait
     // that expired, an out-of-range neighbour index); host paths check it.
     DevBuf status_;

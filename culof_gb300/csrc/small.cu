@@ -1,0 +1,1242 @@
+// The small-d exact k-NN (d <= 8): one kernel that finds every row's k best
+// over all column tiles, pruning per row, and a pass of its own for isolated
+// rows.
+//
+// A CTA owns 64 or 128 consecutive rows of the spatial order (8 warps of 8 or
+// 16 rows) and streams column tiles of 128 points into shared memory (TMA bulk
+// copies, the last warp done with a stage refills it):
+//   1. the window: its own tile T and the neighbours T+-1, T+-2, which start
+//      every row's list and k-th distance;
+//   2. rows whose k-th distance stays far above the CTA's median (isolated
+//      points) are handed to the pass of their own: they would make the CTA
+//      visit tiles that none of its other rows needs;
+//   3. the other tiles that can hold a candidate under the k-th distances so
+//      far (bounding boxes), nearest centres first, so that the k-th
+//      distances shrink early.
+// Per tile and warp, one test per lane compares the boxes of the tile's two
+// 64-column halves with every row's own k-th distance (16 rows x 2 halves).
+// Only the (row, half) pairs that pass are evaluated, lane = column pair, with the exact direct-difference distance; keys within the row's
+// k-th distance are inserted into the row's sorted list (32 or 64 keys, one or
+// two registers per lane while it is worked on, in shared memory between).
+//
+// What bounds it, and why per row: at n = 200,000, d = 8, k = 20 (five
+// clusters and 1% outliers) 20% of the (128 rows, tile) blocks hold a candidate
+// for some row of the block, but only 4.7% of the (row, half) pairs hold one
+// for their row (145 halves per row). Evaluating whole blocks with packed FMAs,
+// as an earlier form did, took 5.94 ms (and 0.52 ms for its seeds, 0.16 ms to
+// merge its lists); this kernel takes 3.64 ms with lists and output included
+// (ncu, same input). It is bound by issue: 2.6e9 warp instructions, 62% of the
+// issue slots while an SM is busy, about 40% of them distances, 20% box tests,
+// the rest list insertions and the window.
+#include <cuda_bf16.h>
+
+#include <algorithm>
+
+#include "engine.cuh"
+#include "small.cuh"
+#include "warp_sort.cuh"
+
+namespace culof_gb300 {
+
+namespace {
+
+using namespace small;
+
+constexpr int kWindow = 5;           // tiles of the window: T, T+1, T-1, T+2, T-2
+constexpr int kSmStages = kWindow;  // column tiles in flight (the window is staged whole)
+constexpr unsigned kFullMask = 0xffffffffu;
+constexpr int kInsertMax = 12;  // more new keys than this are sorted and merged
+constexpr float kSparseRatio = 4.0f;  // a tile is sparse when its squared diagonal exceeds 4x the median tile's
+constexpr int kSparseWaves = 4;       // sparse tiles leave whole up to 4 row tiles per SM (see launch_small)
+constexpr float kDeferRatio = 4.0f;  // a row leaves when its squared k-th distance exceeds 4x the CTA's median
+
+__device__ __forceinline__ float inf_f() { return __int_as_float(0x7f800000); }
+
+// ---------------------------------------------------------------- tiles
+
+// One CTA of 128 threads per tile, one thread per column: coordinates,
+// indices, half boxes, the quarter boxes of the isolated rows' pass (bf16
+// rounded outward: 16 values per quarter, lower bounds then upper bounds) and
+// the tile's box.
+template <int DP>
+__global__ void __launch_bounds__(kCT) small_tile_kernel(const float* __restrict__ xc, int64_t n, int d,
+                                                         const unsigned* __restrict__ perm, float* __restrict__ tiles,
+                                                         float* __restrict__ boxes, __nv_bfloat16* __restrict__ qbox) {
+    __shared__ float wb[kQuarters][2][DP];
+    const int64_t t = blockIdx.x;
+    const int c = threadIdx.x, lane = c & 31, q = c >> 5;
+    float* tile = tiles + t * tile_floats(DP);
+    const int64_t p = t * kCT + c;
+    const bool valid = p < n;
+    const unsigned orig = valid ? perm[p] : kNoIndex;
+    float mine = 0.0f;  // lane f: lower bound of dimension f of this quarter; lane 8 + f: upper bound
+#pragma unroll
+    for (int f = 0; f < DP; ++f) {
+        const float v = (valid && f < d) ? xc[static_cast<int64_t>(orig) * d + f] : 0.0f;
+        tile[f * kCT + c] = (!valid && f == 0) ? __int_as_float(0x7fc00000) : v;
+        float lo = valid ? v : inf_f(), hi = valid ? v : -inf_f();
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            lo = fminf(lo, __shfl_xor_sync(kFullMask, lo, o));
+            hi = fmaxf(hi, __shfl_xor_sync(kFullMask, hi, o));
+        }
+        if (lane == f) mine = lo;
+        if (lane == 8 + f) mine = hi;
+        if (lane == 0) {
+            wb[q][0][f] = lo;
+            wb[q][1][f] = hi;
+        }
+    }
+    reinterpret_cast<unsigned*>(tile)[tile_index_off(DP) + c] = orig;
+    if (lane < 16)
+        qbox[16 * (t * kQuarters + q) + lane] = lane < 8 ? __float2bfloat16_rd(mine) : __float2bfloat16_ru(mine);
+    __syncthreads();
+    if (c < kHalves * DP) {
+        const int h = c / DP, f = c % DP;
+        tile[tile_box_off(DP) + (h * DP + f) * 2] = fminf(wb[2 * h][0][f], wb[2 * h + 1][0][f]);
+        tile[tile_box_off(DP) + (h * DP + f) * 2 + 1] = -fmaxf(wb[2 * h][1][f], wb[2 * h + 1][1][f]);
+    }
+    if (c < DP) {
+        boxes[t * 2 * DP + c] = fminf(fminf(wb[0][0][c], wb[1][0][c]), fminf(wb[2][0][c], wb[3][0][c]));
+        boxes[t * 2 * DP + DP + c] = fmaxf(fmaxf(wb[0][1][c], wb[1][1][c]), fmaxf(wb[2][1][c], wb[3][1][c]));
+    }
+}
+
+// ---------------------------------------------------------------- spatial order
+
+// Refines the Morton order: every chunk of 1024 sorted points becomes a
+// balanced k-d order (halved along the dimension of largest variance down to
+// 16 points), which makes tiles, halves and the 16-row groups more compact:
+// the sweep evaluates 138 instead of 192 halves per row (n = 200,000, d = 8,
+// k = 20; larger chunks gain little more). One CTA per chunk, one thread per
+// point; a point's sort key is its coordinate's order-preserving bits with
+// the low 10 replaced by its place in the chunk (the order is a heuristic, no
+// result depends on it).
+constexpr int kChunk = 1024;
+__global__ void __launch_bounds__(kChunk) refine_order_kernel(const float* __restrict__ xc, int64_t n, int d,
+                                                              unsigned* __restrict__ perm) {
+    __shared__ float xs[kMaxDP][kChunk];
+    __shared__ unsigned key_s[kChunk];
+    __shared__ float stat[kChunk / 32][kMaxDP][2];
+    __shared__ float cnt[kChunk / 32];
+    __shared__ unsigned orig[kChunk];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int64_t pos = static_cast<int64_t>(blockIdx.x) * kChunk + tid;
+    const bool valid = pos < n;
+    const unsigned o = valid ? perm[pos] : 0u;
+    orig[tid] = o;
+    for (int f = 0; f < d; ++f) xs[f][tid] = valid ? xc[static_cast<int64_t>(o) * d + f] : 0.0f;
+    __syncthreads();
+    // slot: which of the chunk's points is at this place; places >= m hold none
+    const int m = static_cast<int>(n - static_cast<int64_t>(blockIdx.x) * kChunk < kChunk
+                                       ? n - static_cast<int64_t>(blockIdx.x) * kChunk
+                                       : kChunk);
+    unsigned slot = tid;
+    for (int size = kChunk; size >= 32; size >>= 1) {
+        // the segment's dimension of largest variance
+        const bool in = static_cast<int>(slot) < m;
+        for (int f = 0; f < d; ++f) {
+            const float v = in ? xs[f][slot] : 0.0f;
+            float s1 = v, s2 = v * v;
+#pragma unroll
+            for (int st = 16; st > 0; st >>= 1) {
+                s1 += __shfl_xor_sync(kFullMask, s1, st);
+                s2 += __shfl_xor_sync(kFullMask, s2, st);
+            }
+            if (lane == 0) {
+                stat[warp][f][0] = s1;
+                stat[warp][f][1] = s2;
+            }
+        }
+        const unsigned here = __ballot_sync(kFullMask, in);
+        if (lane == 0) cnt[warp] = static_cast<float>(__popc(here));
+        __syncthreads();
+        const int w0 = tid / size * (size / 32), nw = size / 32;
+        float var = -1.0f;
+        if (lane < d) {
+            float s1 = 0.0f, s2 = 0.0f, c = 0.0f;
+            for (int w = 0; w < nw; ++w) {
+                s1 += stat[w0 + w][lane][0];
+                s2 += stat[w0 + w][lane][1];
+                c += cnt[w0 + w];
+            }
+            var = c > 0.0f ? s2 - s1 * s1 / c : 0.0f;
+        }
+        int dim = lane;
+#pragma unroll
+        for (int st = 4; st > 0; st >>= 1) {
+            const float ov = __shfl_xor_sync(kFullMask, var, st);
+            const int od = __shfl_xor_sync(kFullMask, dim, st);
+            if (ov > var || (ov == var && od < dim)) {
+                var = ov;
+                dim = od;
+            }
+        }
+        dim = __shfl_sync(kFullMask, dim, 0);
+        if (dim >= d) dim = 0;
+        // bitonic sort of the segment by that coordinate
+        const unsigned u = __float_as_uint(xs[dim][slot]);
+        unsigned key = in ? ((u & 0x80000000u ? ~u : u | 0x80000000u) & ~1023u) | slot : 0xFFFFFC00u | slot;
+        for (int sz = 2; sz <= size; sz <<= 1) {
+            const bool asc = (tid & sz) == 0 || sz == size;
+            for (int st = sz >> 1; st > 0; st >>= 1) {
+                unsigned ok;
+                if (st >= 32) {
+                    __syncthreads();
+                    key_s[tid] = key;
+                    __syncthreads();
+                    ok = key_s[tid ^ st];
+                } else {
+                    ok = __shfl_xor_sync(kFullMask, key, st);
+                }
+                const bool keep_min = ((tid & st) == 0) == asc;
+                key = keep_min ? min(key, ok) : max(key, ok);
+            }
+        }
+        slot = key & 1023u;
+        __syncthreads();  // stat is rewritten by the next level
+    }
+    if (valid) perm[pos] = orig[slot];
+}
+
+// Squared diagonal of a tile's box.
+__device__ __forceinline__ float box_extent(const float* __restrict__ b, int dp) {
+    float e = 0.0f;
+    for (int f = 0; f < dp; ++f) {
+        const float w = b[dp + f] - b[f];
+        e = fmaf(w, w, e);
+    }
+    return e;
+}
+
+// Launch order of the sweep's row tiles [t0, t0 + mt): widest boxes first
+// (their rows lie in sparse regions, have far neighbours and take the
+// longest), so that no long CTA starts last. The rank is counted against
+// every other tile (mt^2 comparisons).
+__global__ void __launch_bounds__(256) tile_order_kernel(const float* __restrict__ boxes, int dp, int t0, int mt,
+                                                         int* __restrict__ order) {
+    __shared__ float other[256];
+    const auto extent = [&](int t) { return box_extent(boxes + static_cast<int64_t>(t0 + t) * 2 * dp, dp); };
+    const int t = blockIdx.x * 256 + threadIdx.x;
+    const float mine = t < mt ? extent(t) : 0.0f;
+    int rank = 0;
+    for (int c0 = 0; c0 < mt; c0 += 256) {
+        __syncthreads();
+        if (c0 + static_cast<int>(threadIdx.x) < mt) other[threadIdx.x] = extent(c0 + threadIdx.x);
+        __syncthreads();
+        const int c1 = min(256, mt - c0);
+        for (int i = 0; i < c1; ++i) {
+            const float v = other[i];
+            rank += (v > mine || (v == mine && c0 + i < t)) ? 1 : 0;
+        }
+    }
+    if (t < mt) order[rank] = t;
+}
+
+// ---------------------------------------------------------------- row lists
+
+// A row's list: its 32 * KR best keys so far in ascending order, element
+// e = 32 j + lane in register b[j] while a warp works on it.
+
+// Merges up to 32 keys, one per lane (kKeyMax: none), into the list (about 250
+// issue slots).
+template <int KR>
+__device__ __forceinline__ void list_merge(uint64_t (&b)[KR], uint64_t key) {
+    const int lane = threadIdx.x & 31;
+    uint64_t x[1] = {key};
+    warp_bitonic_sort<1>(x);
+    if constexpr (KR == 1) {
+        b[0] = warp_merge_lowest32(b[0], x[0]);
+    } else {
+        // the 32 best of (second register, new keys), then both runs of 32
+        // merged into 64: elementwise minimum and maximum against the
+        // reversed run, each a bitonic sequence
+        const uint64_t c = warp_merge_lowest32(b[1], x[0]);
+        const uint64_t rc = __shfl_sync(kFullMask, c, 31 - lane);
+        uint64_t lo = b[0] < rc ? b[0] : rc, hi = b[0] < rc ? rc : b[0];
+#pragma unroll
+        for (int st = 16; st > 0; st >>= 1) {
+            const uint64_t ol = shfl_xor_u64(lo, st), oh = shfl_xor_u64(hi, st);
+            lo = (lane & st) == 0 ? (ol < lo ? ol : lo) : (ol > lo ? ol : lo);
+            hi = (lane & st) == 0 ? (oh < hi ? oh : hi) : (oh > hi ? oh : hi);
+        }
+        b[0] = lo;
+        b[1] = hi;
+    }
+}
+
+// Adds the keys of the lanes in m. A few keys go in one by one (a ballot
+// gives the place, a shuffle shifts the rest: about 20 issue slots each);
+// more are sorted across the warp and merged.
+template <int KR>
+__device__ __forceinline__ void list_add(uint64_t (&b)[KR], uint64_t key, unsigned m) {
+    const int lane = threadIdx.x & 31;
+    if (__popc(m) > kInsertMax) {
+        list_merge<KR>(b, (m >> lane) & 1u ? key : kKeyMax);
+        return;
+    }
+    while (m) {
+        const uint64_t kx = __shfl_sync(kFullMask, key, __ffs(m) - 1);
+        m &= m - 1;
+        if constexpr (KR == 2) {  // the largest of the first register moves to the second
+            uint64_t up = __shfl_up_sync(kFullMask, b[1], 1);
+            const uint64_t last = __shfl_sync(kFullMask, b[0], 31);
+            if (lane == 0) up = last;
+            // elements above kx shift up by one; kx lands behind the last one below it
+            b[1] = kx < b[1] ? (kx < up ? up : kx) : b[1];
+        }
+        uint64_t up = __shfl_up_sync(kFullMask, b[0], 1);
+        if (lane == 0) up = 0;
+        b[0] = kx < b[0] ? (kx < up ? up : kx) : b[0];
+    }
+}
+
+// The element of rank r (0-based) of 32 * G values, G per lane.
+template <int G>
+__device__ __forceinline__ unsigned warp_rank_value(unsigned (&v)[G], int r) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int size = 2; size <= 32 * G; size <<= 1) {
+#pragma unroll
+        for (int st = size >> 1; st > 0; st >>= 1) {
+            if (st == 32) {
+                const unsigned a = v[0], c = v[G - 1];
+                v[0] = min(a, c);
+                v[G - 1] = max(a, c);
+            } else {
+#pragma unroll
+                for (int j = 0; j < G; ++j) {
+                    const unsigned o = __shfl_xor_sync(kFullMask, v[j], st);
+                    const bool asc = ((j * 32 + lane) & size) == 0, lower = (lane & st) == 0;
+                    v[j] = lower == asc ? min(v[j], o) : max(v[j], o);
+                }
+            }
+        }
+    }
+    unsigned x = __shfl_sync(kFullMask, v[0], r & 31);
+    if (G == 2 && r >= 32) x = __shfl_sync(kFullMask, v[G - 1], r & 31);
+    return x;
+}
+
+// The bits of a list's k-th distance (all ones while it holds fewer than k
+// keys), and the distance (+inf then).
+template <int KR>
+__device__ __forceinline__ unsigned list_kth_bits(const uint64_t (&b)[KR], int k) {
+    return KR == 1 ? __shfl_sync(kFullMask, static_cast<unsigned>(b[0] >> 32), k - 1)
+                   : __shfl_sync(kFullMask, static_cast<unsigned>(b[KR - 1] >> 32), k - 33);
+}
+template <int KR>
+__device__ __forceinline__ float list_kth(const uint64_t (&b)[KR], int k) {
+    const unsigned h = list_kth_bits<KR>(b, k);
+    return h == 0xFFFFFFFFu ? inf_f() : __uint_as_float(h);
+}
+
+// Writes a finished row (whole warp) in the reference's slot order: the keys
+// below the k-th by ascending index, then the ties (already in index order).
+template <int KR>
+__device__ __forceinline__ void emit_row(const uint64_t (&b)[KR], int k, int64_t n, unsigned self,
+                                         int32_t* __restrict__ nbr_idx, float* __restrict__ nbr_d2,
+                                         float* __restrict__ kdist2) {
+    const int lane = threadIdx.x & 31;
+    const unsigned kbits = KR == 1 ? __shfl_sync(kFullMask, static_cast<unsigned>(b[0] >> 32), k - 1)
+                                   : __shfl_sync(kFullMask, static_cast<unsigned>(b[KR - 1] >> 32), k - 33);
+    int below = 0, slot[KR];
+    unsigned ix[KR];
+#pragma unroll
+    for (int j = 0; j < KR; ++j) {
+        below += __popc(__ballot_sync(kFullMask, key_bits(b[j]) < kbits));  // all within the first k
+        ix[j] = key_index(b[j]);
+        slot[j] = 0;
+    }
+    for (int q = 0; q < below; ++q) {
+        unsigned o = __shfl_sync(kFullMask, ix[0], q & 31);
+        if (KR == 2 && q >= 32) o = __shfl_sync(kFullMask, ix[KR - 1], q & 31);
+#pragma unroll
+        for (int j = 0; j < KR; ++j) slot[j] += o < ix[j] ? 1 : 0;
+    }
+#pragma unroll
+    for (int j = 0; j < KR; ++j) {
+        const int e = 32 * j + lane;
+        if (e < k) {
+            const int64_t o = static_cast<int64_t>(e < below ? slot[j] : e) * n + self;
+            nbr_idx[o] = static_cast<int32_t>(ix[j] & 0x7FFFFFFFu);
+            nbr_d2[o] = __uint_as_float(key_bits(b[j]));
+        }
+    }
+    if (lane == 0) kdist2[self] = __uint_as_float(kbits);
+}
+
+// ---------------------------------------------------------------- sweep
+
+// Row record in shared memory (floats): coordinates, each twice (one operand
+// of the packed f32x2 instructions), k-th distance, own index.
+__host__ __device__ constexpr int row_stride(int dp) { return 2 * dp + 4; }
+
+__device__ __forceinline__ uint64_t sub2(uint64_t a, uint64_t b) {
+    uint64_t d;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ uint64_t add2_rd(uint64_t a, uint64_t b) {
+    uint64_t d;
+    asm("add.rm.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+
+template <int DP, int KR, int RW, int W>
+struct SmallSmem {
+    static constexpr int kRows = W * RW;
+    alignas(16) float tiles[kSmStages][tile_floats(DP)];  // also the unsorted tile list while no copy is in flight
+    uint64_t list[kRows][32 * KR];
+    alignas(16) float row[kRows][row_stride(DP)];
+    uint64_t full_bar[kSmStages];
+    alignas(8) unsigned ent[kSegTiles];  // (before: each warp's keys while it works on the window)
+                                         // listed tiles in visiting order: gap bits (upper 16) and offset in the segment
+    unsigned hist[32];
+    float wbox[W][2][DP];
+    float cbox[2][DP];
+    float wkmax[8];       // largest k-th distance among each warp's rows
+    float kdv[kRows];     // the rows' k-th distances at the end of the window
+    float median;
+    int done[kSmStages], stage_tile[kSmStages], last_fill[kSmStages];
+    int next_e, count;
+    int left;  // rows that asked to leave
+    unsigned evaluated;
+};
+static_assert(kSegTiles * 4 <= kSmStages * tile_bytes(2), "the unsorted list fits in the stages");
+
+// A row record's packed coordinates.
+template <int DP>
+__device__ __forceinline__ void load_row(const float* rec, uint64_t (&a)[DP]) {
+#pragma unroll
+    for (int f = 0; f < DP; f += 2) {
+        const ulonglong2 v = reinterpret_cast<const ulonglong2*>(rec)[f / 2];
+        a[f] = v.x;
+        a[f + 1] = v.y;
+    }
+}
+// This lane's two columns of a half of a tile.
+template <int DP>
+__device__ __forceinline__ void load_columns(const float* tl, int h, uint64_t (&x)[DP]) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int f = 0; f < DP; ++f) x[f] = *reinterpret_cast<const uint64_t*>(tl + f * kCT + h * kHalf + 2 * lane);
+}
+// Exact distances (the oracle's chain: t = a - b, s = fma(t, t, s) over the
+// dimensions in order) from a row to two columns, packed.
+template <int DP>
+__device__ __forceinline__ uint64_t pair_dist(const uint64_t (&a)[DP], const uint64_t (&x)[DP]) {
+    uint64_t s = 0;
+#pragma unroll
+    for (int f = 0; f < DP; ++f) {
+        const uint64_t t = sub2(a[f], x[f]);
+        s = fma2(t, t, s);
+    }
+    return s;
+}
+
+// N floats (a multiple of 4) from a 16-byte boundary.
+template <int N>
+__device__ __forceinline__ void load4(const float* p, float (&v)[N]) {
+    static_assert(N % 4 == 0, "whole 16-byte words");
+#pragma unroll
+    for (int i = 0; i < N / 4; ++i) {
+        const float4 x = reinterpret_cast<const float4*>(p)[i];
+        v[4 * i] = x.x;
+        v[4 * i + 1] = x.y;
+        v[4 * i + 2] = x.z;
+        v[4 * i + 3] = x.w;
+    }
+}
+
+// Rows that left the sweep: their positions, their lists and how many.
+struct IsoRows {
+    int* count;
+    int* pos;
+    uint64_t* list;  // [slot][32 KR]
+};
+
+template <int DP, int KR, int G, int RW, int W>
+__global__ void __launch_bounds__(32 * W, (KR == 1 ? 24 : 16) / W)
+small_sweep_kernel(const float* __restrict__ tiles, const float* __restrict__ boxes, const unsigned* __restrict__ perm,
+                   int64_t n, int nt, int64_t row0, const int* __restrict__ order, int mt, int k, int defer_rows,
+                   int segment, IsoRows iso,
+                   int32_t* __restrict__ nbr_idx, float* __restrict__ nbr_d2, float* __restrict__ kdist2,
+                   int* __restrict__ status, unsigned long long* __restrict__ evaluated_total) {
+    using Smem = SmallSmem<DP, KR, RW, W>;
+    constexpr int kRows = Smem::kRows, kThreads = 32 * W;
+    constexpr int kKd = 2 * DP, kSelf = 2 * DP + 1;  // fields of a row record
+    constexpr unsigned kTileBytes = tile_bytes(DP);
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    Smem& sh = *reinterpret_cast<Smem*>(smem_raw);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    // first row position; the tiles' CTAs start in the given order
+    constexpr int kPerTile = kCT / kRows;
+    const int tile_i = static_cast<int>(blockIdx.x) / kPerTile;
+    const int64_t base = row0 + static_cast<int64_t>(order ? order[tile_i] : tile_i) * kCT +
+                         static_cast<int>(blockIdx.x) % kPerTile * kRows;
+    if (base >= n) return;
+    const int T = static_cast<int>(base / kCT);
+    const int r_in_tile = static_cast<int>(base % kCT);
+    const int wsize = nt < kWindow ? nt : kWindow;
+    // a warp's rows are spread over (up to) 64 consecutive ones, so that the
+    // CTA's warps have about the same work on every tile
+    constexpr int kGroup = kRows < kHalf ? kRows : kHalf, kGroupWarps = kGroup / RW;
+    const int rfirst = warp / kGroupWarps * kGroup + warp % kGroupWarps;
+    const auto row_of = [&](int i) { return rfirst + i * kGroupWarps; };
+
+    if (tid < kRows) {
+        const float* own = tiles + static_cast<int64_t>(T) * tile_floats(DP);
+        const unsigned self = reinterpret_cast<const unsigned*>(own)[tile_index_off(DP) + r_in_tile + tid];
+#pragma unroll
+        for (int f = 0; f < DP; ++f) {
+            const float v = self != kNoIndex ? own[f * kCT + r_in_tile + tid] : 0.0f;
+            sh.row[tid][2 * f] = v;
+            sh.row[tid][2 * f + 1] = v;
+        }
+        sh.row[tid][kKd] = self != kNoIndex ? inf_f() : -inf_f();  // -inf: takes no candidates
+        sh.row[tid][kSelf] = __uint_as_float(self);
+    }
+    for (int i = tid; i < kRows * 32 * KR; i += kThreads) (&sh.list[0][0])[i] = kKeyMax;
+    if (tid < kSmStages) {
+        sh.done[tid] = 0;
+        sh.last_fill[tid] = 0;
+    }
+    if (tid < 8) sh.wkmax[tid] = tid < W ? inf_f() : -inf_f();
+    if (tid == 0) {
+        sh.evaluated = 0;
+        for (int s = 0; s < kSmStages; ++s) mbar_init(&sh.full_bar[s], 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        sh.left = 0;
+    }
+    __syncthreads();
+    if (tid == 0) {
+        // the window's tiles, one per stage (bulk copies are issued by one
+        // thread: their operands live in registers uniform over the warp)
+        for (int st = 0; st < kSmStages; ++st) {
+            if (st < wsize) {
+                const int t = spiral_tile(T, st, nt);
+                mbar_expect_tx(&sh.full_bar[st], kTileBytes);
+                tma_load_1d(sh.tiles[st], tiles + static_cast<int64_t>(t) * tile_floats(DP), kTileBytes,
+                            &sh.full_bar[st]);
+            } else {
+                mbar_arrive_plain(&sh.full_bar[st]);
+            }
+        }
+    }
+    __syncwarp();
+    // the tiles outside the window form a ring of `rest` tiles from first_up
+    // on; entry u of the phases' concatenated segments starts half a segment
+    // below the window, so that the first segment lies around it
+    const int rest = nt - wsize;
+    const int first_up = T + wsize / 2 + 1;
+    int seg_at = 0;  // the current segment's first entry
+    const auto ring_tile = [&](int u) {
+        const int ring = (u + rest - min(rest, segment) / 2) % rest;
+        return (first_up + ring) % nt;
+    };
+
+    // this lane's test: row tr of the warp against half th of a tile, its
+    // coordinates as packed (-a, a)
+    const int tr = lane & (RW - 1), th = lane / RW;
+    const bool tester = th < kHalves;
+    uint64_t na[DP];
+#pragma unroll
+    for (int f = 0; f < DP; ++f) {
+        const float v = sh.row[row_of(tr)][2 * f];
+        na[f] = static_cast<uint64_t>(__float_as_uint(-v)) | (static_cast<uint64_t>(__float_as_uint(v)) << 32);
+    }
+
+    // The stage loader (one warp at a time): the next listed tile whose gap is
+    // within the CTA's largest k-th distance (stale values only prune less);
+    // a stage with no tile left gets a sentinel.
+    auto fill = [&](int stage, int fill_no) {
+        float kmax = lane < 8 ? sh.wkmax[lane] : -inf_f();
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) kmax = fmaxf(kmax, __shfl_xor_sync(kFullMask, kmax, o));
+        kmax = __shfl_sync(kFullMask, kmax, 0);
+        int found = -1;
+        int e0 = sh.next_e;
+        const int count = sh.count;
+        while (found < 0 && e0 < count) {
+            const int e = e0 + lane;
+            unsigned v = 0;
+            bool pass = false;
+            if (e < count) {
+                v = sh.ent[e];
+                pass = __uint_as_float(v & 0xFFFF0000u) <= kmax;
+            }
+            const unsigned mk = __ballot_sync(kFullMask, pass);
+            if (mk) {
+                const int o = __ffs(mk) - 1;
+                found = static_cast<int>(__shfl_sync(kFullMask, v, o) & 0xFFFFu);
+                e0 += o + 1;
+            } else {
+                e0 += 32;
+            }
+        }
+        if (lane == 0) {
+            sh.next_e = e0;
+            sh.last_fill[stage] = fill_no;
+            if (found >= 0) {
+                const int t = ring_tile(seg_at + found);
+                sh.stage_tile[stage] = t;
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                mbar_expect_tx(&sh.full_bar[stage], kTileBytes);
+                tma_load_1d(sh.tiles[stage], tiles + static_cast<int64_t>(t) * tile_floats(DP), kTileBytes,
+                            &sh.full_bar[stage]);
+            } else {
+                sh.stage_tile[stage] = -1;
+                mbar_arrive_plain(&sh.full_bar[stage]);
+            }
+        }
+        __syncwarp();
+    };
+
+    bool ok = true;
+    // The window: every row against all of its columns at once. The smallest
+    // value of each of 32 (64) groups of columns, one or two groups per lane,
+    // bounds the row's k-th distance by the k-th smallest of them; the columns
+    // within that bound (about 31 of 640 at k = 20) are gathered, sorted and
+    // merged. (Inserting the columns half by half into the list cost 2.5 times
+    // the instructions of this form.)
+    for (int st = 0; st < kSmStages; ++st) ok = ok && mbar_wait_warp(&sh.full_bar[st], 0);
+    if (ok) {
+#pragma unroll 1
+        for (int i = 0; i < RW; ++i) {
+            const int r = row_of(i);
+            if (sh.row[r][kKd] < 0.0f) continue;  // padding row
+            uint64_t ra[DP];
+            load_row<DP>(sh.row[r], ra);
+            unsigned v[4 * kWindow];  // distance bits; all ones: no candidate
+#pragma unroll
+            for (int q = 0; q < kWindow; ++q) {
+#pragma unroll
+                for (int h = 0; h < kHalves; ++h) {
+                    uint64_t x[DP];
+                    load_columns<DP>(sh.tiles[q], h, x);
+                    const uint64_t s2 = pair_dist<DP>(ra, x);
+                    v[4 * q + 2 * h] = static_cast<unsigned>(s2);
+                    v[4 * q + 2 * h + 1] = static_cast<unsigned>(s2 >> 32);
+                }
+                const int t = q < wsize ? spiral_tile(T, q, nt) : nt;
+                if (static_cast<int64_t>(t + 1) * kCT > n) {  // the last tile's padding, or no tile
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        if (static_cast<int64_t>(t) * kCT + (j >> 1) * kHalf + 2 * lane + (j & 1) >= n)
+                            v[4 * q + j] = 0xFFFFFFFFu;
+                }
+            }
+            const int own = r_in_tile + r;  // the row's own column
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if ((j >> 1) * kHalf + 2 * lane + (j & 1) == own) v[j] = 0xFFFFFFFFu;
+            constexpr int kSpan = 4 * kWindow / G;
+            unsigned g[G];
+#pragma unroll
+            for (int j = 0; j < G; ++j) {
+                g[j] = v[j * kSpan];
+#pragma unroll
+                for (int e = 1; e < kSpan; ++e) g[j] = min(g[j], v[j * kSpan + e]);
+            }
+            unsigned bound = warp_rank_value<G>(g, k - 1);
+            uint64_t b[KR];
+#pragma unroll
+            for (int j = 0; j < KR; ++j) b[j] = kKeyMax;
+            // gather the keys within the bound (kBuf at most; the rest, if
+            // any, by further rounds with the bound that the first ones give)
+            constexpr int kBuf = kSegTiles / 2 / W;
+            uint64_t* buf = reinterpret_cast<uint64_t*>(sh.ent) + warp * kBuf;
+            for (;;) {
+                int found = 0;
+#pragma unroll
+                for (int e = 0; e < 4 * kWindow; ++e) {
+                    const bool in = v[e] <= bound && v[e] != 0xFFFFFFFFu;
+                    const unsigned m = __ballot_sync(kFullMask, in);
+                    const int at = found + __popc(m & ((1u << lane) - 1u));
+                    if (in && at < kBuf) {
+                        buf[at] = make_key(v[e], reinterpret_cast<const unsigned*>(
+                                                     sh.tiles[e / 4])[tile_index_off(DP) + (e % 4 >> 1) * kHalf + 2 * lane + (e & 1)]);
+                        v[e] = 0xFFFFFFFFu;  // taken
+                    }
+                    found += __popc(m);
+                }
+                __syncwarp();
+                const int have = min(found, kBuf);
+#pragma unroll 1
+                for (int e0 = 0; e0 < have; e0 += 32)
+                    list_merge<KR>(b, e0 + lane < have ? buf[e0 + lane] : kKeyMax);
+                __syncwarp();
+                if (found <= kBuf) break;
+                const unsigned kb = list_kth_bits<KR>(b, k);
+                bound = kb < bound ? kb : bound;
+            }
+#pragma unroll
+            for (int j = 0; j < KR; ++j) sh.list[r][32 * j + lane] = b[j];
+            const float kd = list_kth<KR>(b, k);  // the whole warp
+            if (lane == 0) sh.row[r][kKd] = kd;
+            __syncwarp();
+        }
+    }
+    unsigned evaluated = 0;
+    int m = kSmStages;  // fill number over all phases; the window was 0 .. kSmStages - 1
+    // phase p > 0: segment p - 1 of the other tiles
+    const int phases = 1 + (rest + segment - 1) / segment;
+    if (__syncthreads_or(ok ? 0 : 1)) {
+        if (tid == 0) atomicExch(status, 1);
+        return;
+    }
+    for (int ph = 1; ph < phases; ++ph) {
+        {
+            // every row's k-th distance and the box of the rows that take part
+            const int mine = row_of(lane & (RW - 1));
+            const float kdr = lane < RW ? sh.row[mine][kKd] : -inf_f();
+            float wk = kdr;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) wk = fmaxf(wk, __shfl_xor_sync(kFullMask, wk, o));
+            if (ph == 1) {
+                if (defer_rows) {
+                    if (lane < RW) sh.kdv[mine] = kdr;
+                    __syncthreads();
+                    if (tid < kRows) {
+                        const float v = sh.kdv[tid];
+                        int rank = 0;
+                        for (int i = 0; i < kRows; ++i) {
+                            const float w = sh.kdv[i];
+                            rank += (w < v || (w == v && i < tid)) ? 1 : 0;
+                        }
+                        if (rank == kRows / 2) sh.median = v;
+                    }
+                    __syncthreads();
+                    const float med = sh.median;
+                    // a tile of a sparse region: all of its rows leave
+                    const bool sparse =
+                        defer_rows == 2 && tile_i < mt / 32 &&
+                        box_extent(boxes + static_cast<int64_t>(T) * 2 * DP, DP) >
+                            kSparseRatio * box_extent(boxes + static_cast<int64_t>(row0 / kCT + order[mt / 2]) * 2 * DP, DP);
+                    const bool far = lane < RW && kdr >= 0.0f && kdr < inf_f() &&
+                                     (sparse || (med > 0.0f && kdr > kDeferRatio * med));
+                    unsigned leave = __ballot_sync(kFullMask, far);
+                    // otherwise at most a quarter of the CTA's rows (the list's capacity)
+                    const int most = sparse ? kRows : kRows / 4;
+                    int first = 0;
+                    if (lane == 0 && leave) first = atomicAdd(&sh.left, __popc(leave));
+                    first = __shfl_sync(kFullMask, first, 0);
+                    while (leave && first < most) {
+                        const int i = row_of(__ffs(leave) - 1);
+                        leave &= leave - 1;
+                        ++first;
+                        int slot = 0;
+                        if (lane == 0) slot = atomicAdd(iso.count, 1);
+                        slot = __shfl_sync(kFullMask, slot, 0);
+                        if (lane == 0) {
+                            iso.pos[slot] = static_cast<int>(base + i);
+                            sh.row[i][kKd] = -inf_f();
+                            sh.row[i][kSelf] = __uint_as_float(kNoIndex);
+                        }
+#pragma unroll
+                        for (int j = 0; j < KR; ++j)
+                            iso.list[(static_cast<int64_t>(slot) * KR + j) * 32 + lane] = sh.list[i][32 * j + lane];
+                    }
+                    __syncwarp();
+                    wk = lane < RW ? sh.row[mine][kKd] : -inf_f();
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1) wk = fmaxf(wk, __shfl_xor_sync(kFullMask, wk, o));
+                }
+                const bool in = lane < RW && sh.row[mine][kKd] >= 0.0f;
+#pragma unroll
+                for (int f = 0; f < DP; ++f) {
+                    const float v = sh.row[mine][2 * f];
+                    float lo = in ? v : inf_f(), hi = in ? v : -inf_f();
+#pragma unroll
+                    for (int o = RW / 2; o > 0; o >>= 1) {
+                        lo = fminf(lo, __shfl_xor_sync(kFullMask, lo, o));
+                        hi = fmaxf(hi, __shfl_xor_sync(kFullMask, hi, o));
+                    }
+                    if (lane == 0) {
+                        sh.wbox[warp][0][f] = lo;
+                        sh.wbox[warp][1][f] = hi;
+                    }
+                }
+            }
+            if (lane == 0) sh.wkmax[warp] = wk;
+            if (tid < 32) sh.hist[tid] = 0;
+            __syncthreads();
+            if (ph == 1 && tid < DP) {
+                float lo = inf_f(), hi = -inf_f();
+                for (int w = 0; w < W; ++w) {
+                    lo = fminf(lo, sh.wbox[w][0][tid]);
+                    hi = fmaxf(hi, sh.wbox[w][1][tid]);
+                }
+                sh.cbox[0][tid] = lo;
+                sh.cbox[1][tid] = hi;
+            }
+            seg_at = (ph - 1) * segment;
+            const int len = min(segment, rest - seg_at);
+            if (tid == 0) {
+                sh.next_e = 0;
+                sh.count = 0;
+            }
+            __syncthreads();
+            float kmax = sh.wkmax[0];
+            for (int w = 1; w < W; ++w) kmax = fmaxf(kmax, sh.wkmax[w]);
+            // visiting order: the centres' squared distance in quarter octaves
+            // over kmax / 8, 32 classes
+            const int c0 = static_cast<int>(__float_as_uint(kmax * 0.125f) >> 21);
+            unsigned* raw = reinterpret_cast<unsigned*>(&sh.tiles[0][0]);
+            for (int i = tid; i < len; i += kThreads) {
+                float bx[2 * DP];
+                load4(boxes + static_cast<int64_t>(ring_tile(seg_at + i)) * 2 * DP, bx);
+                float g2 = 0.0f, cd = 0.0f;
+#pragma unroll
+                for (int f = 0; f < DP; ++f) {
+                    const float lo = bx[f], hi = bx[DP + f];
+                    const float gap = fmaxf(0.0f, fmaxf(__fsub_rd(lo, sh.cbox[1][f]), __fsub_rd(sh.cbox[0][f], hi)));
+                    g2 = __fadd_rd(g2, __fmul_rd(gap, gap));
+                    const float cc = 0.5f * ((lo + hi) - (sh.cbox[0][f] + sh.cbox[1][f]));
+                    cd = fmaf(cc, cc, cd);
+                }
+                const float g = __fmul_rd(g2, kPruneShrink);
+                unsigned v = 0xFFFFFFFFu;
+                if (g <= kmax) {
+                    int cls = static_cast<int>(__float_as_uint(cd) >> 21) - c0;
+                    cls = cls < 0 ? 0 : cls > 31 ? 31 : cls;
+                    atomicAdd(&sh.hist[cls], 1u);
+                    // class in the low bits of the gap's 16 (rounded down further)
+                    v = (__float_as_uint(g) & 0xFFFF0000u) | static_cast<unsigned>(cls);
+                }
+                raw[i] = v;
+            }
+            __syncthreads();
+            if (warp == 0) {
+                const unsigned c = sh.hist[lane];
+                unsigned x = c;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const unsigned y = __shfl_up_sync(kFullMask, x, o);
+                    if (lane >= o) x += y;
+                }
+                sh.hist[lane] = x - c;
+                if (lane == 31) sh.count = static_cast<int>(x);
+            }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // before copies into the stages again
+            __syncthreads();
+            for (int i = tid; i < len; i += kThreads) {
+                const unsigned v = raw[i];
+                if (v != 0xFFFFFFFFu)
+                    sh.ent[atomicAdd(&sh.hist[v & 31u], 1u)] = (v & 0xFFFF0000u) | static_cast<unsigned>(i);
+            }
+            __syncthreads();
+        }
+        if (warp == 0)
+            for (int st = 0; st < kSmStages; ++st) fill((m + st) % kSmStages, m + st);
+
+        for (;; ++m) {
+            const int stage = m % kSmStages;
+            if (!mbar_wait_warp(&sh.full_bar[stage], (m / kSmStages) & 1)) {
+                ok = false;
+                break;
+            }
+            if (sh.stage_tile[stage] < 0) break;  // the phase is done
+            const float* tl = sh.tiles[stage];
+            // which of the warp's rows can find a candidate in which half
+            bool pass = false;
+            if (tester) {
+                float hb[2 * DP];
+                load4(tl + tile_box_off(DP) + th * 2 * DP, hb);
+                float g2 = 0.0f;
+#pragma unroll
+                for (int f = 0; f < DP; ++f) {  // (lo - a, a - hi) rounded down
+                    const uint64_t lh = static_cast<uint64_t>(__float_as_uint(hb[2 * f])) |
+                                        (static_cast<uint64_t>(__float_as_uint(hb[2 * f + 1])) << 32);
+                    const uint64_t g = add2_rd(lh, na[f]);
+                    const float gap = fmaxf(fmaxf(lo_f(g), hi_f(g)), 0.0f);
+                    g2 = __fmaf_rd(gap, gap, g2);
+                }
+                pass = __fmul_rd(g2, kPruneShrink) <= sh.row[row_of(tr)][kKd];
+            }
+            const unsigned todo = __ballot_sync(kFullMask, pass);
+            bool changed = false;
+            if (todo) {
+                evaluated += __popc(todo);
+#pragma unroll 1
+                for (int h = 0; h < kHalves; ++h) {
+                    unsigned rows = (todo >> (h * RW)) & ((1u << RW) - 1u);
+                    if (!rows) continue;
+                    uint64_t x[DP];
+                    load_columns<DP>(tl, h, x);
+                    const uint2 ix = *reinterpret_cast<const uint2*>(tl + tile_index_off(DP) + h * kHalf + 2 * lane);
+                    do {  // two rows at a time: two independent distance chains
+                        const int r0 = row_of(__ffs(rows) - 1);
+                        rows &= rows - 1;
+                        const int r1 = rows ? row_of(__ffs(rows) - 1) : r0;
+                        rows &= rows - 1;
+                        uint64_t a0[DP], a1[DP];
+                        load_row<DP>(sh.row[r0], a0);
+                        load_row<DP>(sh.row[r1], a1);
+                        const uint64_t s0 = pair_dist<DP>(a0, x), s1 = pair_dist<DP>(a1, x);
+                        const float k0 = sh.row[r0][kKd], k1 = sh.row[r1][kKd];
+                        // not farther than the k-th distance (NaN distances
+                        // count as candidates, as their keys order last)
+                        if (!__any_sync(kFullMask, !(lo_f(s0) > k0) || !(hi_f(s0) > k0) || !(lo_f(s1) > k1) ||
+                                                       !(hi_f(s1) > k1)))
+                            continue;
+#pragma unroll 1
+                        for (int w = 0; w < 2; ++w) {
+                            if (w && r1 == r0) break;
+                            const int r = w ? r1 : r0;
+                            const uint64_t s2 = w ? s1 : s0;
+                            float kd = w ? k1 : k0;
+                            if (!__any_sync(kFullMask, !(lo_f(s2) > kd) || !(hi_f(s2) > kd))) continue;
+                            uint64_t b[KR];
+#pragma unroll
+                            for (int j = 0; j < KR; ++j) b[j] = sh.list[r][32 * j + lane];
+#pragma unroll 1
+                            for (int e = 0; e < 2; ++e) {
+                                const float d2 = e ? hi_f(s2) : lo_f(s2);
+                                const unsigned i = e ? ix.y : ix.x;
+                                const unsigned hits = __ballot_sync(kFullMask, !(d2 > kd) && i != kNoIndex);
+                                if (hits) {
+                                    list_add<KR>(b, make_key(__float_as_uint(d2), i), hits);
+                                    kd = list_kth<KR>(b, k);
+                                    changed = true;
+                                }
+                            }
+#pragma unroll
+                            for (int j = 0; j < KR; ++j) sh.list[r][32 * j + lane] = b[j];
+                            if (lane == 0) sh.row[r][kKd] = kd;
+                            __syncwarp();
+                        }
+                    } while (rows);
+                }
+            }
+            if (changed) {
+                float wk = lane < RW ? sh.row[row_of(lane & (RW - 1))][kKd] : -inf_f();
+#pragma unroll
+                for (int o = RW / 2; o > 0; o >>= 1) wk = fmaxf(wk, __shfl_xor_sync(kFullMask, wk, o));
+                if (lane == 0) sh.wkmax[warp] = wk;
+            }
+            // done with this stage; the last warp out refills it
+            __syncwarp();
+            int prev = 0;
+            if (lane == 0) {
+                __threadfence_block();
+                prev = atomicAdd(&sh.done[stage], 1);
+            }
+            prev = __shfl_sync(kFullMask, prev, 0);
+            if (prev == W - 1) {
+                if (lane == 0) sh.done[stage] = 0;
+                fill(stage, m + kSmStages);
+            }
+        }
+        if (__syncthreads_or(ok ? 0 : 1)) {
+            if (tid == 0) atomicExch(status, 1);
+            // wait (bounded) for this CTA's copies still in flight before exiting
+            if (tid < kSmStages && sh.last_fill[tid] >= 0)
+                mbar_wait(&sh.full_bar[tid], (sh.last_fill[tid] / kSmStages) & 1);
+            __syncthreads();
+            return;
+        }
+        m += kSmStages;  // every stage holds a sentinel: the next phase fills them anew
+    }
+    if (lane == 0 && evaluated) atomicAdd(&sh.evaluated, evaluated);
+    for (int i = 0; i < RW; ++i) {
+        const int r = row_of(i);
+        const unsigned self = __float_as_uint(sh.row[r][kSelf]);
+        if (self == kNoIndex) continue;  // padding, or the row's own pass writes it
+        uint64_t b[KR];
+#pragma unroll
+        for (int j = 0; j < KR; ++j) b[j] = sh.list[r][32 * j + lane];
+        emit_row<KR>(b, k, n, self, nbr_idx, nbr_d2, kdist2);
+    }
+    __syncthreads();
+    if (tid == 0 && evaluated_total) atomicAdd(evaluated_total, static_cast<unsigned long long>(sh.evaluated));
+}
+
+// ---------------------------------------------------------------- isolated rows
+
+// Gaps are kept as the upper 16 bits of their float32 bit pattern
+// (non-negative floats truncated: rounded down, so pruning stays
+// conservative); kGapSkip marks a quarter the pass never visits.
+constexpr uint16_t kGapSkip = 0xFFFFu;
+constexpr int kIsoMaxTiles = 8192;  // 4 gaps of 2 bytes per column tile in shared memory
+__device__ __forceinline__ uint16_t gap_bits_down(float g) { return static_cast<uint16_t>(__float_as_uint(g) >> 16); }
+// the smallest 16-bit pattern not below distance b (+inf: 0x7F80)
+__device__ __forceinline__ unsigned bound_bits_up(float b) { return (__float_as_uint(b) + 0xFFFFu) >> 16; }
+
+// One CTA (kIsoWarps warps) per listed row: its k best over the column tiles
+// outside the window, joined with its list from the sweep.
+//  1. The rounded-down gap between the point and every quarter's box
+//     (coalesced, into shared memory; the window's quarters are skipped).
+//  2. Warp w owns quarter w of every tile (the quarters near the point are
+//     spread over all warps) and visits its quarters in three rounds of
+//     growing gap: gaps up to 1/16 of the row's current bound, then 1/4,
+//     then the whole bound, so that the bound tightens on the nearest
+//     quarters before the far ones are tested; quarters within the bound
+//     are evaluated kIsoBatch at a time.
+//  3. The warps share the bound (the smallest of the k-th distances held) in
+//     shared memory and merge their lists at the end.
+constexpr int kIsoWarps = 4;
+constexpr int kIsoBatch = 4;
+template <int DP, int KR>
+__global__ void __launch_bounds__(32 * kIsoWarps, 6)
+small_iso_kernel(const float* __restrict__ tiles, const __nv_bfloat16* __restrict__ qbox,
+                 const unsigned* __restrict__ perm, int64_t n, int nt, int k, IsoRows iso,
+                 int32_t* __restrict__ nbr_idx, float* __restrict__ nbr_d2, float* __restrict__ kdist2) {
+    extern __shared__ __align__(16) uint16_t qgap_s[];  // 4 per tile
+    __shared__ uint64_t fin[kIsoWarps][32 * KR];
+    __shared__ unsigned bound_s;  // float bits of the row's smallest k-th distance so far
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int count = *iso.count;
+    const int nb = (nt + 31) / 32;
+    const int64_t nq = static_cast<int64_t>(nt) * kQuarters;
+    const int wsize = nt < kWindow ? nt : kWindow;
+    const int wlo = (wsize - 1) / 2, whi = wsize / 2;  // the window: offsets -wlo .. whi
+    for (int h = blockIdx.x; h < count; h += gridDim.x) {
+        const int64_t pos = iso.pos[h];
+        const int T = static_cast<int>(pos / kCT), r = static_cast<int>(pos % kCT);
+        const float* own = tiles + static_cast<int64_t>(T) * tile_floats(DP);
+        float a[DP];
+#pragma unroll
+        for (int f = 0; f < DP; ++f) a[f] = tile_coord<DP>(own, r, f);
+        uint64_t b[KR];  // warp 0 starts from the window's list
+#pragma unroll
+        for (int j = 0; j < KR; ++j) b[j] = iso.list[(static_cast<int64_t>(h) * KR + j) * 32 + lane];
+        const float kd0 = list_kth<KR>(b, k);
+        if (warp != 0) {
+#pragma unroll
+            for (int j = 0; j < KR; ++j) b[j] = kKeyMax;
+        }
+        if (threadIdx.x == 0) bound_s = __float_as_uint(kd0);
+#pragma unroll 4
+        for (int q = threadIdx.x; q < nq; q += 32 * kIsoWarps) {
+            const int t = q / kQuarters;
+            int off = t - T;  // offset from the row tile, in (-nt/2, nt/2]
+            if (off > nt / 2) off -= nt;
+            if (off <= -((nt + 1) / 2)) off += nt;
+            const uint4 lo4 = reinterpret_cast<const uint4*>(qbox)[2 * q];
+            const uint4 hi4 = reinterpret_cast<const uint4*>(qbox)[2 * q + 1];
+            const unsigned lw[4] = {lo4.x, lo4.y, lo4.z, lo4.w}, hw[4] = {hi4.x, hi4.y, hi4.z, hi4.w};
+            float g2 = 0.0f;
+#pragma unroll
+            for (int f = 0; f < DP; ++f) {  // bf16 to float is exact: the bits shifted up
+                const float lo = __uint_as_float((f & 1 ? lw[f >> 1] >> 16 : lw[f >> 1] & 0xFFFFu) << 16);
+                const float hi = __uint_as_float((f & 1 ? hw[f >> 1] >> 16 : hw[f >> 1] & 0xFFFFu) << 16);
+                const float gap = fmaxf(0.0f, fmaxf(__fsub_rd(lo, a[f]), __fsub_rd(a[f], hi)));
+                g2 = __fadd_rd(g2, __fmul_rd(gap, gap));
+            }
+            qgap_s[q] = (off >= -wlo && off <= whi) ? kGapSkip : gap_bits_down(__fmul_rd(g2, kPruneShrink));
+        }
+        __syncthreads();
+        float bound = kd0;
+        const auto shared_bound = [&]() {  // publish this warp's bound, take the CTA's
+            unsigned sb = 0;
+            if (lane == 0) sb = atomicMin(&bound_s, __float_as_uint(bound));
+            sb = __shfl_sync(kFullMask, sb, 0);
+            bound = fminf(bound, __uint_as_float(sb));
+        };
+        // up to kIsoBatch quarters against the point, all loads issued first;
+        // lane l takes column l of each
+        const auto eval = [&](int q0, int q1, int q2, int q3, int mq) {
+            const int qs[kIsoBatch] = {q0, mq > 1 ? q1 : q0, mq > 2 ? q2 : q0, mq > 3 ? q3 : q0};
+            float x[kIsoBatch][DP];
+            unsigned ix[kIsoBatch];
+#pragma unroll
+            for (int i = 0; i < kIsoBatch; ++i) {
+                const int qi = qs[i];
+                const float* tl = tiles + static_cast<int64_t>(qi / kQuarters) * tile_floats(DP);
+                const int c = (qi % kQuarters) * kQuarter + lane;
+#pragma unroll
+                for (int f = 0; f < DP; ++f) x[i][f] = tl[f * kCT + c];
+                ix[i] = reinterpret_cast<const unsigned*>(tl)[tile_index_off(DP) + c];
+            }
+            float d2[kIsoBatch];
+#pragma unroll
+            for (int i = 0; i < kIsoBatch; ++i) {
+                d2[i] = 0.0f;
+#pragma unroll
+                for (int f = 0; f < DP; ++f) {
+                    const float t = __fsub_rn(a[f], x[i][f]);
+                    d2[i] = __fmaf_rn(t, t, d2[i]);
+                }
+            }
+#pragma unroll 1
+            for (int i = 0; i < mq; ++i) {  // one copy of the list code
+                float di = d2[0];
+                unsigned ii = ix[0];
+#pragma unroll
+                for (int j = 1; j < kIsoBatch; ++j) {
+                    di = i == j ? d2[j] : di;
+                    ii = i == j ? ix[j] : ii;
+                }
+                const unsigned hits = __ballot_sync(kFullMask, !(di > bound) && ii != kNoIndex);
+                if (hits) {
+                    list_add<KR>(b, make_key(__float_as_uint(di), ii), hits);
+                    bound = fminf(bound, list_kth<KR>(b, k));
+                }
+            }
+        };
+        const auto bound_up = [&]() { return isinf(bound) ? 0xFFFEu : bound_bits_up(bound); };
+        // quarters waiting for evaluation, the latest first (warp-uniform)
+        int w0 = 0, w1 = 0, w2 = 0, w3 = 0, nbatch = 0;
+        unsigned lo_bits = 0;  // this round takes tiles whose gap lies in [lo_bits, hi_bits]
+        for (int round = 0; round < 3; ++round) {
+            shared_bound();
+            const float frac = round == 0 ? 0.0625f : round == 1 ? 0.25f : 1.0f;
+            unsigned hi_bits = bound_bits_up(bound * frac);
+            if (round == 2 || hi_bits > 0xFFFEu) hi_bits = 0xFFFEu;  // the last round takes every quarter left
+            if (hi_bits < lo_bits) continue;
+            for (int bi = 0; bi < nb; ++bi) {
+                const int t = 32 * bi + lane;
+                const unsigned g = t < nt ? qgap_s[kQuarters * t + warp] : kGapSkip;
+                unsigned todo = __ballot_sync(kFullMask, g >= lo_bits && g <= hi_bits && g <= bound_up());
+                while (todo) {
+                    const int src = __ffs(todo) - 1;
+                    todo &= todo - 1;
+                    if (__shfl_sync(kFullMask, g, src) > bound_up()) continue;  // a tighter bound prunes it
+                    const int qn = (32 * bi + src) * kQuarters + warp;
+                    w3 = w2;
+                    w2 = w1;
+                    w1 = w0;
+                    w0 = qn;
+                    if (++nbatch == kIsoBatch) {
+                        eval(w0, w1, w2, w3, nbatch);
+                        nbatch = 0;
+                        shared_bound();
+                    }
+                }
+            }
+            lo_bits = hi_bits + 1;
+        }
+        if (nbatch > 0) eval(w0, w1, w2, w3, nbatch);
+#pragma unroll
+        for (int j = 0; j < KR; ++j) fin[warp][32 * j + lane] = b[j];
+        __syncthreads();
+        if (warp == 0) {
+            for (int w = 1; w < kIsoWarps; ++w)
+#pragma unroll
+                for (int j = 0; j < KR; ++j) {
+                    const uint64_t key = fin[w][32 * j + lane];
+                    const unsigned have = __ballot_sync(kFullMask, key != kKeyMax);
+                    if (have) list_add<KR>(b, key, have);
+                }
+            emit_row<KR>(b, k, n, perm[pos], nbr_idx, nbr_d2, kdist2);
+        }
+        __syncthreads();
+    }
+}
+
+struct SmallArgs {
+    const float* tiles;
+    const float* boxes;
+    const __nv_bfloat16* qbox;
+    const unsigned* perm;
+    int64_t n;
+    int nt, t0, mt, k, sms, segment;
+    bool defer;
+    const int* order;
+    IsoRows iso;
+    int32_t* idx;
+    float* d2;
+    float* kd;
+    int* status;
+    unsigned long long* evaluated;
+    cudaStream_t s;
+};
+
+template <int DP, int KR, int G, int RW, int W>
+void launch_small(const SmallArgs& A) {
+    using Smem = SmallSmem<DP, KR, RW, W>;
+    set_max_dynamic_smem(reinterpret_cast<const void*>(small_sweep_kernel<DP, KR, G, RW, W>), static_cast<int>(sizeof(Smem)));
+    const unsigned grid = static_cast<unsigned>(static_cast<int64_t>(A.mt) * kCT / Smem::kRows);
+    small_sweep_kernel<DP, KR, G, RW, W><<<grid, 32 * W, sizeof(Smem), A.s>>>(
+        A.tiles, A.boxes, A.perm, A.n, A.nt, static_cast<int64_t>(A.t0) * kCT, A.order, A.mt, A.k,
+        !A.defer ? 0 : A.mt <= kSparseWaves * A.sms ? 2 : 1, A.segment, A.iso,
+        A.idx, A.d2, A.kd, A.status, A.evaluated);
+    CG_LAUNCH_CHECK();
+    if (!A.defer) return;
+    const size_t gap_bytes = sizeof(uint16_t) * kQuarters * static_cast<size_t>(A.nt);
+    constexpr size_t kDefaultDynamicSmem = 40 * 1024;
+    if (gap_bytes > kDefaultDynamicSmem)
+        set_max_dynamic_smem(reinterpret_cast<const void*>(small_iso_kernel<DP, KR>), 72 * 1024);
+    small_iso_kernel<DP, KR><<<6 * A.sms, 32 * kIsoWarps, gap_bytes, A.s>>>(A.tiles, A.qbox, A.perm, A.n, A.nt, A.k,
+                                                                           A.iso, A.idx, A.d2, A.kd);
+    CG_LAUNCH_CHECK();
+}
+
+template <int DP, int KR, int G>
+void dispatch_rows(const SmallArgs& A) {
+    // Rows per CTA: 128 (16 per warp: a test per lane, each tile staged for
+    // more rows) from 6 row tiles per SM up, else 64 (n = 200,000, d = 8,
+    // k = 20: 4.42 against 5.59 ms per fit_predict; n = 20,000: 0.76 against
+    // 0.61 ms, the larger CTAs leave SMs idle).
+    if (A.mt >= 6 * A.sms) launch_small<DP, KR, G, 16, 8>(A);
+    else launch_small<DP, KR, G, 8, 8>(A);
+}
+template <int DP>
+void dispatch_small(const SmallArgs& A) {
+    // one group of window columns per lane up to k = 24, two above (the bound
+    // from 32 groups takes in 43 columns at k = 24 and 110 at k = 32)
+    if (A.k <= 24) dispatch_rows<DP, 1, 1>(A);
+    else if (A.k <= 32) dispatch_rows<DP, 1, 2>(A);
+    else dispatch_rows<DP, 2, 2>(A);
+}
+
+constexpr int kOrderMaxTiles = 16384;
+int64_t iso_capacity(int mt) { return static_cast<int64_t>(mt) * kCT / 4 + static_cast<int64_t>(mt / 32) * kCT; }
+
+}  // namespace
+
+void small_refine_order(const float* xc, int64_t n, int d, unsigned* perm, cudaStream_t s) {
+    refine_order_kernel<<<static_cast<unsigned>(ceil_div(n, kChunk)), kChunk, 0, s>>>(xc, n, d, perm);
+    CG_LAUNCH_CHECK();
+}
+
+size_t small_tiles_floats(int dp, int nt) { return static_cast<size_t>(tile_floats(dp)) * nt; }
+
+void small_build_tiles(const float* xc, int64_t n, int d, const unsigned* perm, int nt, float* tiles, float* boxes,
+                       void* qbox, cudaStream_t s) {
+    __nv_bfloat16* qb = static_cast<__nv_bfloat16*>(qbox);
+    switch (padded_dims(d)) {
+        case 2: small_tile_kernel<2><<<nt, kCT, 0, s>>>(xc, n, d, perm, tiles, boxes, qb); break;
+        case 4: small_tile_kernel<4><<<nt, kCT, 0, s>>>(xc, n, d, perm, tiles, boxes, qb); break;
+        case 6: small_tile_kernel<6><<<nt, kCT, 0, s>>>(xc, n, d, perm, tiles, boxes, qb); break;
+        default: small_tile_kernel<8><<<nt, kCT, 0, s>>>(xc, n, d, perm, tiles, boxes, qb); break;
+    }
+    CG_LAUNCH_CHECK();
+}
+
+size_t small_iso_bytes(int mt, int k) {
+    const size_t cap = static_cast<size_t>(iso_capacity(mt));
+    return 256 + sizeof(uint64_t) * cap * 32 * (k <= 32 ? 1 : 2) + sizeof(int) * (cap + mt);
+}
+
+void small_knn(const float* tiles, const float* boxes, const void* qbox, const unsigned* perm, int64_t n, int d, int nt,
+               int t0, int mt, int k, int sms, bool defer_rows, int segment, void* iso, int32_t* nbr_idx, float* nbr_d2,
+               float* kdist2, int* status, unsigned long long* evaluated, cudaStream_t s) {
+    if (mt <= 0) return;
+    SmallArgs A{tiles, boxes, static_cast<const __nv_bfloat16*>(qbox), perm, n, nt, t0, mt, k, sms,
+                segment, defer_rows && nt > kWindow && nt <= kIsoMaxTiles, nullptr, {}, nbr_idx, nbr_d2, kdist2, status,
+                evaluated, s};
+    char* w = static_cast<char*>(iso);
+    A.iso.count = reinterpret_cast<int*>(w);
+    A.iso.list = reinterpret_cast<uint64_t*>(w + 256);
+    A.iso.pos = reinterpret_cast<int*>(w + 256 + sizeof(uint64_t) * static_cast<size_t>(iso_capacity(mt)) * 32 * (k <= 32 ? 1 : 2));
+    if (A.defer) CG_CUDA(cudaMemsetAsync(A.iso.count, 0, sizeof(int), s));
+    if (mt <= kOrderMaxTiles) {
+        int* order = A.iso.pos + iso_capacity(mt);
+        tile_order_kernel<<<static_cast<unsigned>(ceil_div(mt, 256)), 256, 0, s>>>(boxes, padded_dims(d), t0, mt, order);
+        CG_LAUNCH_CHECK();
+        A.order = order;
+    } else {
+        A.defer = false;
+    }
+    switch (padded_dims(d)) {
+        case 2: dispatch_small<2>(A); break;
+        case 4: dispatch_small<4>(A); break;
+        case 6: dispatch_small<6>(A); break;
+        default: dispatch_small<8>(A); break;
+    }
+}
+
+}  // namespace culof_gb300
