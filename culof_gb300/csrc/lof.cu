@@ -18,10 +18,20 @@ namespace {
 
 constexpr int kBlock = 256;
 
-// One thread per point; `rows` (nullable) lists the m points of a row block
-// (a shard of a row-sharded run), otherwise every point.
+// A CTA of 8 warps takes 32 points (lane = point): the warps compute the
+// points' slot terms side by side, 32 slots at a time, and warp 0 adds them in
+// slot order. One thread per point, its k terms one after another, was bound
+// by the latency of that chain (a gather, an FP64 square root or division and
+// an addition per slot: 32 + 21 us at n = 500, k = 20, and still 33 + 24 us at
+// n = 20,000). From about 100,000 points on both forms are bound by the FP64
+// units.
+// `rows` (nullable) lists the m points of a row block (a shard of a
+// row-sharded run), otherwise every point.
+constexpr int kTermSlots = 32;
+constexpr int kTermWarps = kBlock / 32;
+
 __device__ __forceinline__ int64_t block_row(const int32_t* rows, int64_t m, int64_t n, int* status) {
-    const int64_t r = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    const int64_t r = static_cast<int64_t>(blockIdx.x) * 32 + (threadIdx.x & 31);
     if (r >= m) return -1;
     const int64_t i = rows ? static_cast<int64_t>(rows[r]) : r;
     if (i < 0 || i >= n) {
@@ -31,44 +41,101 @@ __device__ __forceinline__ int64_t block_row(const int32_t* rows, int64_t m, int
     return i;
 }
 
-__global__ void lrd_kernel(const int32_t* __restrict__ nbr_idx, const float* __restrict__ nbr_d2,
-                           const float* __restrict__ kdist2, int64_t n, int k, const int32_t* __restrict__ rows,
-                           int64_t m, float* __restrict__ lrd, int* status) {
+__global__ void __launch_bounds__(kBlock) lrd_kernel(const int32_t* __restrict__ nbr_idx,
+                                                     const float* __restrict__ nbr_d2,
+                                                     const float* __restrict__ kdist2, int64_t n, int k,
+                                                     const int32_t* __restrict__ rows, int64_t m,
+                                                     float* __restrict__ lrd, int* status) {
+    __shared__ double term[kTermSlots][32];
+    __shared__ int bad[32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t i = block_row(rows, m, n, status);
-    if (i < 0) return;
-    if (status != nullptr && *status != 0) {
+    if (warp == 0) bad[lane] = status != nullptr && *status != 0 ? 1 : 0;
+    __syncthreads();
+    double sum = 0.0;
+    for (int c0 = 0; c0 < k; c0 += kTermSlots) {
+        const int c1 = k - c0 < kTermSlots ? k - c0 : kTermSlots;
+        for (int t = warp; t < c1; t += kTermWarps) {
+            double v = 0.0;
+            if (i >= 0) {
+                const int64_t o = static_cast<int64_t>(c0 + t) * n + i;
+                const int32_t j = nbr_idx[o];
+                if (j < 0 || j >= n) bad[lane] = 2;  // never for a valid k-NN graph; do not read out of range
+                else v = __dsqrt_rn(static_cast<double>(fmaxf(kdist2[j], nbr_d2[o])));
+            }
+            term[t][lane] = v;
+        }
+        __syncthreads();
+        if (warp == 0)
+            for (int t = 0; t < c1; ++t) sum = __dadd_rn(sum, term[t][lane]);
+        __syncthreads();
+    }
+    if (warp != 0 || i < 0) return;
+    if (bad[lane]) {
+        if (bad[lane] == 2 && status != nullptr) atomicExch(status, 2);
         lrd[i] = __int_as_float(0x7fc00000);
         return;
-    }
-    double sum = 0.0;
-    for (int t = 0; t < k; ++t) {
-        const int64_t o = static_cast<int64_t>(t) * n + i;
-        const int32_t j = nbr_idx[o];
-        if (j < 0 || j >= n) {  // never happens for a valid k-NN graph; do not read out of range
-            if (status != nullptr) atomicExch(status, 2);
-            lrd[i] = __int_as_float(0x7fc00000);
-            return;
-        }
-        sum = __dadd_rn(sum, __dsqrt_rn(static_cast<double>(fmaxf(kdist2[j], nbr_d2[o]))));
     }
     lrd[i] = __double2float_rn(__ddiv_rn(1.0, __dadd_rn(__ddiv_rn(sum, static_cast<double>(k)), 1e-10)));
 }
 
-__global__ void score_kernel(const int32_t* __restrict__ nbr_idx, const float* __restrict__ lrd,
-                             int64_t n, int k, const int32_t* __restrict__ rows, int64_t m,
-                             float* __restrict__ scores, float* __restrict__ nof, int* status) {
+// The slot terms are the correctly rounded quotients lrd_j / lrd_i, from one
+// reciprocal y = RN(1 / lrd_i) per point: q0 = RN(a y), r = a - q0 b, q =
+// RN(q0 + r y). For a, b with 24-bit significands this is RN(a / b): q0 is off
+// by at most 1.5 ulp, so r has at most 25 significant bits above ulp(q0)
+// ulp(b) and is exact, and q0 + r y before its rounding is off from a / b by
+// at most 2^-104 of it, while a / b, not a midpoint of two neighbouring
+// doubles (a 54-bit midpoint M times b has more than 24 bits), is at least
+// 2^-78 away from one. A reciprocal that is zero or not finite (lrd_i infinite,
+// zero or not a number) takes the division itself.
+__global__ void __launch_bounds__(kBlock) score_kernel(const int32_t* __restrict__ nbr_idx,
+                                                       const float* __restrict__ lrd, int64_t n, int k,
+                                                       const int32_t* __restrict__ rows, int64_t m,
+                                                       float* __restrict__ scores, float* __restrict__ nof,
+                                                       int* status) {
+    __shared__ double term[kTermSlots][32];
+    __shared__ double recip[32];
+    __shared__ int bad[32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t i = block_row(rows, m, n, status);
-    if (i < 0) return;
-    const double self = static_cast<double>(lrd[i]);
+    const double self = i >= 0 ? static_cast<double>(lrd[i]) : 1.0;
+    if (warp == 0) {
+        recip[lane] = __ddiv_rn(1.0, self);
+        bad[lane] = 0;
+    }
+    __syncthreads();
+    const double y = recip[lane];
+    const bool quick = fabs(y) < __longlong_as_double(0x7ff0000000000000ll) && y != 0.0;
     double sum = 0.0;
-    for (int t = 0; t < k; ++t) {
-        const int32_t j = nbr_idx[static_cast<int64_t>(t) * n + i];
-        if (j < 0 || j >= n) {
-            if (status != nullptr) atomicExch(status, 2);
-            sum = __longlong_as_double(0x7ff8000000000000ll);
-            break;
+    for (int c0 = 0; c0 < k; c0 += kTermSlots) {
+        const int c1 = k - c0 < kTermSlots ? k - c0 : kTermSlots;
+        for (int t = warp; t < c1; t += kTermWarps) {
+            double v = 0.0;
+            if (i >= 0) {
+                const int32_t j = nbr_idx[static_cast<int64_t>(c0 + t) * n + i];
+                if (j < 0 || j >= n) {
+                    bad[lane] = 1;
+                } else {
+                    const double a = static_cast<double>(lrd[j]);
+                    if (quick) {
+                        const double q0 = __dmul_rn(a, y);
+                        v = __fma_rn(__fma_rn(-q0, self, a), y, q0);
+                    } else {
+                        v = __ddiv_rn(a, self);
+                    }
+                }
+            }
+            term[t][lane] = v;
         }
-        sum = __dadd_rn(sum, __ddiv_rn(static_cast<double>(lrd[j]), self));
+        __syncthreads();
+        if (warp == 0)
+            for (int t = 0; t < c1; ++t) sum = __dadd_rn(sum, term[t][lane]);
+        __syncthreads();
+    }
+    if (warp != 0 || i < 0) return;
+    if (bad[lane]) {
+        if (status != nullptr) atomicExch(status, 2);
+        sum = __longlong_as_double(0x7ff8000000000000ll);
     }
     const float s = __double2float_rn(__ddiv_rn(sum, static_cast<double>(k)));
     scores[i] = s;
@@ -212,7 +279,7 @@ void compute_lrd(const int32_t* nbr_idx, const float* nbr_d2, const float* kdist
                  float* lrd, int* status, cudaStream_t s, const int32_t* rows, int64_t m) {
     if (!rows) m = n;
     if (m <= 0) return;
-    lrd_kernel<<<static_cast<unsigned>(ceil_div(m, kBlock)), kBlock, 0, s>>>(nbr_idx, nbr_d2, kdist2, n, k, rows, m,
+    lrd_kernel<<<static_cast<unsigned>(ceil_div(m, 32)), kBlock, 0, s>>>(nbr_idx, nbr_d2, kdist2, n, k, rows, m,
                                                                              lrd, status);
     CG_LAUNCH_CHECK();
 }
@@ -221,7 +288,7 @@ void compute_scores(const int32_t* nbr_idx, const float* lrd, int64_t n, int k, 
                     float* nof, int* status, cudaStream_t s, const int32_t* rows, int64_t m) {
     if (!rows) m = n;
     if (m <= 0) return;
-    score_kernel<<<static_cast<unsigned>(ceil_div(m, kBlock)), kBlock, 0, s>>>(nbr_idx, lrd, n, k, rows, m, scores,
+    score_kernel<<<static_cast<unsigned>(ceil_div(m, 32)), kBlock, 0, s>>>(nbr_idx, lrd, n, k, rows, m, scores,
                                                                                nof, status);
     CG_LAUNCH_CHECK();
 }
