@@ -209,8 +209,9 @@ int64_t Engine::knn_core(const float* d_x, int64_t n, int d, int k, bool normali
     for (bool& m : marked_) m = false;
     mark(0);
     center(d_x, n, d, normalize, xc, partial, mean, inv, stream_);
-    squared_norms(xc, n, d, norms, maxn, stream_);
     const int path = choose_path(n, d, k);
+    // only the filters of the wide and tensor sweeps read the norms
+    if (path == kPathTensor || (path == kPathFast && d > 8)) squared_norms(xc, n, d, norms, maxn, stream_);
     int64_t count = n;
     if (path != kPathGeneral) {
         last_path_ = path;
@@ -251,10 +252,11 @@ void Engine::lof_device(const float* d_x, int64_t n, int d, int k, bool normaliz
     mark(6);
 }
 
-void Engine::offset_device(const float* d_nof, int64_t n, double contamination, double* d_offset) {
+void Engine::offset_device(const float* d_nof, int64_t n, double contamination, double* d_offset,
+                           int64_t* d_labels) {
     validate_contamination(contamination);
     void* scratch = offset_scratch_.get(offset_scratch_bytes());
-    contamination_offset(d_nof, n, plan_offset(n, contamination), scratch, d_offset, stream_);
+    contamination_offset(d_nof, n, plan_offset(n, contamination), scratch, d_offset, d_labels, stream_);
 }
 
 void Engine::bf16_gram(const void* A, int64_t rows_a, const void* B, int64_t rows_b, int K, float* G) {
@@ -271,8 +273,7 @@ void Engine::fit_predict_device(const float* d_x, int64_t n, int d, int k, bool 
     float* nof = d_nof ? d_nof : nof_.as<float>(n);
     double* off = d_offset ? d_offset : offset_.as<double>(1);
     lof_device(d_x, n, d, k, normalize, scores, nof);
-    offset_device(nof, n, contamination, off);
-    if (d_labels) labels_from_offset(nof, n, off, d_labels, stream_);
+    offset_device(nof, n, contamination, off, d_labels);
     mark(7);
 }
 

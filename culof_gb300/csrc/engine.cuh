@@ -99,7 +99,9 @@ public:
     // LOF.fit + predict on the device; d_offset is a device double.
     void fit_predict_device(const float* d_x, int64_t n, int d, int k, bool normalize,
                             double contamination, float* d_nof, int64_t* d_labels, double* d_offset);
-    void offset_device(const float* d_nof, int64_t n, double contamination, double* d_offset);
+    // (and the labels, if d_labels is not null)
+    void offset_device(const float* d_nof, int64_t n, double contamination, double* d_offset,
+                       int64_t* d_labels = nullptr);
     void bf16_gram(const void* A, int64_t rows_a, const void* B, int64_t rows_b, int K, float* G);
     // Gradient of sum_i g_i score_i with respect to the points (FP64), the
     // neighbour sets of a forward k-NN (nbr_idx, k x n) held fixed; optional

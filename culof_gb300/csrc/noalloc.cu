@@ -122,7 +122,7 @@ extern "C" CULOF_API int culof_contamination_offset_noalloc(void* cuda_stream, c
         }
         validate_contamination(contamination);
         void* scratch = scratch_address();
-        contamination_offset(d_nof, n_points, plan_offset(n_points, contamination), scratch, d_offset,
+        contamination_offset(d_nof, n_points, plan_offset(n_points, contamination), scratch, d_offset, nullptr,
                              static_cast<cudaStream_t>(cuda_stream));
         set_last_error("");
         return CULOF_OK;

@@ -57,9 +57,8 @@ struct OffsetState {
     int pad2;
 };
 size_t offset_scratch_bytes();
+// The offset and, if labels is not null, the n labels.
 void contamination_offset(const float* nof, int64_t n, const OffsetPlan& plan, void* scratch,
-                          double* offset_out_dev, cudaStream_t s);
-void labels_from_offset(const float* nof, int64_t n, const double* offset_dev, int64_t* labels,
-                        cudaStream_t s);
+                          double* offset_out_dev, int64_t* labels, cudaStream_t s);
 
 }  // namespace culof_gb300
