@@ -243,10 +243,10 @@ __global__ void offset_next_kernel(const float* __restrict__ nof, int64_t n, Off
     }
 }
 
-__global__ void offset_finalize_kernel(int64_t lo, int use_upper, float w, OffsetState* __restrict__ st,
+__global__ void offset_finalize_kernel(int64_t n, int64_t lo, int use_upper, float w, OffsetState* __restrict__ st,
                                        double* __restrict__ out) {
     const float a = from_order_key(st->prefix);
-    const float b = (static_cast<int64_t>(st->count_le) >= lo + 2) ? a : from_order_key(st->min_gt);
+    const float b = (static_cast<int64_t>(st->count_le) >= lo + 2 || lo >= n - 1) ? a : from_order_key(st->min_gt);
     const float diff = __fsub_rn(b, a);
     const float r = use_upper ? __fsub_rn(b, __fmul_rn(diff, w)) : __fadd_rn(a, __fmul_rn(diff, w));
     st->a_key = st->prefix;
@@ -345,7 +345,7 @@ offset_cluster_kernel(const float* __restrict__ nof, int64_t n, int64_t lo, int 
     mn = 0xFFFFFFFFu;
     for (int r = 0; r < nctas; ++r) mn = min(mn, *cl.map_shared_rank(&mn_s, r));
     const float a = from_order_key(prefix);
-    const float b = (static_cast<int64_t>(below) + eq >= lo + 2) ? a : from_order_key(mn);
+    const float b = (static_cast<int64_t>(below) + eq >= lo + 2 || lo >= n - 1) ? a : from_order_key(mn);
     const float diff = __fsub_rn(b, a);
     const float res = use_upper ? __fsub_rn(b, __fmul_rn(diff, w)) : __fadd_rn(a, __fmul_rn(diff, w));
     if (rank == 0 && tid == 0) *out = static_cast<double>(res);
@@ -459,7 +459,7 @@ void contamination_offset(const float* nof, int64_t n, const OffsetPlan& plan, v
     }
     offset_next_kernel<<<g, kBlock, 0, s>>>(nof, n, st);
     CG_LAUNCH_CHECK();
-    offset_finalize_kernel<<<1, 1, 0, s>>>(plan.lo, plan.use_upper, plan.w, st, offset_out_dev);
+    offset_finalize_kernel<<<1, 1, 0, s>>>(n, plan.lo, plan.use_upper, plan.w, st, offset_out_dev);
     CG_LAUNCH_CHECK();
     if (labels == nullptr) return;
     labels_kernel<<<small_grid(n), kBlock, 0, s>>>(nof, n, offset_out_dev, labels);
