@@ -434,7 +434,7 @@ __noinline__ __device__ int approx_compact(TcSmem& sh, uint64_t* __restrict__ ls
             if (lane == 0) {
                 sh.cnt[r] = keep;
                 sh.sorted[r] = keep;
-                if (keep <= cap) sh.athr[r] = thr;
+                if (keep <= cap) sh.athr[r] = fminf(sh.athr[r], thr);
             }
             __syncwarp();
             return keep;
@@ -473,7 +473,7 @@ __noinline__ __device__ int approx_compact(TcSmem& sh, uint64_t* __restrict__ ls
         if (lane == 0) {
             sh.cnt[r] = keep;
             sh.sorted[r] = keep;
-            sh.athr[r] = thr;
+            sh.athr[r] = fminf(sh.athr[r], thr);
         }
     }
     __syncwarp();
@@ -584,6 +584,12 @@ __noinline__ __device__ void rescore_final(uint64_t* __restrict__ lst, int r, in
     }
 }
 
+// Column tiles of a CTA's share that are scanned for the rows' bounds.
+__device__ __forceinline__ int bound_tiles(int count) {
+    const int part = count * 3 / 8;
+    return count <= 128 ? count : part > 128 ? part : 128;
+}
+
 __global__ void __launch_bounds__(kTcThreads, 2)
 tc_sweep_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ CUtensorMap tmapb,
                 const float* __restrict__ xr,
@@ -606,7 +612,11 @@ tc_sweep_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
     const int lcount = plist ? pcount[T] : 0;
     const int count = plist ? (lcount > split ? (lcount - split + nsplit - 1) / nsplit : 0) : (q1 > q0 ? q1 - q0 : 0);
     const uint2* tlist = plist ? plist + static_cast<int64_t>(T) * nt : nullptr;
-    auto col_tile = [&](int j) -> int {
+    // tiles 0 .. scan - 1 are read twice: first for the rows' bounds (below)
+    const int scan = scale->all != 0.0f ? 0 : bound_tiles(count);
+    const int total = scan + count;
+    auto col_tile = [&](int jj) -> int {
+        const int j = jj < scan ? jj : jj - scan;
         return tlist ? static_cast<int>(tlist[split + nsplit * j].x) : spiral_tile(T, q0 + j, nt);
     };
     const int nkb = Kp / 64;
@@ -650,7 +660,7 @@ tc_sweep_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
             int issued = 0;
             mbar_expect_tx(&sh.afull, nkb * kBox);
             for (int kb = 0; kb < nkb; ++kb) tc::tma_load_2d(sh.a[kb], &tmap, 64 * kb, static_cast<int>(rbase), &sh.afull);
-            for (int j = 0; j < count; ++j) {
+            for (int j = 0; j < total; ++j) {
                 const int s = j & 1;
                 if (j >= kTcStages && !mbar_wait(&sh.empty[s], ((j >> 1) - 1) & 1)) {
                     tc_abort(sh, status);
@@ -674,7 +684,7 @@ tc_sweep_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
             constexpr uint32_t idesc = tc::f16_idesc(128, 128);
             bool ok = mbar_wait(&sh.afull, 0);
             if (!ok) tc_abort(sh, status);
-            for (int j = 0; ok && j < count; ++j) {
+            for (int j = 0; ok && j < total; ++j) {
                 const int s = j & 1, acc = j & 1;
                 if (tc_aborted(sh) || !mbar_wait(&sh.full[s], (j >> 1) & 1) ||
                     (j >= 2 && !mbar_wait(&sh.tempty[acc], ((j >> 1) - 1) & 1))) {
@@ -722,7 +732,7 @@ tc_sweep_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
         // never waits on global memory.
         auto tile_base = [&](int jj) -> int64_t { return static_cast<int64_t>(col_tile(jj)) * kCT; };
         float4 npre = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (count > 0) npre = __ldg(reinterpret_cast<const float4*>(cn + tile_base(0)) + lane);
+        if (total > 0) npre = __ldg(reinterpret_cast<const float4*>(cn + tile_base(0)) + lane);
         int qc = 0;
         int64_t cbase = 0;
         const float* nbj = nullptr;
@@ -804,19 +814,85 @@ tc_sweep_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
             }
             if (changed) tq = tau_pair(row_tau());
         };
-        for (int j = 0; j < count; ++j) {
-            const int acc = j & 1;
+        // The accumulator of tile j: its column norms staged (and the next
+        // tile's requested), its MMA waited for. False if a wait expired.
+        auto begin_tile = [&](int j) -> bool {
             cbase = tile_base(j);
             float* nbw = sh.nb[wq][j & 1];
             reinterpret_cast<float4*>(nbw)[lane] = npre;
-            if (j + 1 < count) npre = __ldg(reinterpret_cast<const float4*>(cn + tile_base(j + 1)) + lane);
+            if (j + 1 < total) npre = __ldg(reinterpret_cast<const float4*>(cn + tile_base(j + 1)) + lane);
             nbj = nbw;
             __syncwarp();
-            if (!mbar_wait_warp(&sh.tfull[acc], (j >> 1) & 1)) {
+            if (!mbar_wait_warp(&sh.tfull[j & 1], (j >> 1) & 1)) {
                 if (lane == 0) tc_abort(sh, status);
-                break;
+                return false;
             }
             tc::tc_fence_after();
+            return true;
+        };
+        auto end_tile = [&](int j) {  // the accumulator is free for the next tile but one
+            tc::tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&sh.tempty[j & 1]);
+        };
+        bool alive = true;
+        if (scan > 0) {
+            // Bounds first: the row's smallest f in each of 64 groups of the
+            // scanned columns. k groups with a value <= B are k columns with
+            // f <= B, so the k-th smallest of the minima bounds the row's k-th
+            // f, and the threshold over it (approx_thr) starts the lists.
+            float gm[64];
+#pragma unroll
+            for (int q = 0; q < 64; ++q) gm[q] = __int_as_float(0x7f800000);
+            for (int j = 0; j < scan; ++j) {
+                if (!begin_tile(j)) {
+                    alive = false;
+                    break;
+                }
+                const uint32_t taddr = lane_addr + static_cast<uint32_t>((j & 1) * 128);
+#pragma unroll 1
+                for (int ch = 0; ch < 4; ch += 2) {
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        uint32_t ga[32];
+                        tc::tmem_ld32_async(taddr + static_cast<uint32_t>(32 * (ch + h)), ga);
+                        tc::tmem_wait32(ga);
+                        const float4* nb4 = reinterpret_cast<const float4*>(nbj + 32 * (ch + h));
+#pragma unroll
+                        for (int q = 0; q < 8; ++q) {
+                            const float4 nb = nb4[q];
+                            const uint64_t f0 = fma2(pack2(__uint_as_float(ga[4 * q]), __uint_as_float(ga[4 * q + 1])),
+                                                     k2, pack2(nb.x, nb.y));
+                            const uint64_t f1 = fma2(
+                                pack2(__uint_as_float(ga[4 * q + 2]), __uint_as_float(ga[4 * q + 3])), k2, pack2(nb.z, nb.w));
+                            float* g = gm + 32 * h + 4 * q;
+                            g[0] = fminf(g[0], lo_f(f0));
+                            g[1] = fminf(g[1], hi_f(f0));
+                            g[2] = fminf(g[2], lo_f(f1));
+                            g[3] = fminf(g[3], hi_f(f1));
+                        }
+                    }
+                }
+                end_tile(j);
+            }
+            // the k-th smallest minimum, by bisection over the ordered bits
+            uint32_t at = 0;
+#pragma unroll 1
+            for (int bit = 31; bit >= 0; --bit) {
+                const uint32_t probe = at | ((1u << bit) - 1u);  // every value with this bit clear
+                int below = 0;
+#pragma unroll
+                for (int q = 0; q < 64; ++q) below += flip_bits(gm[q]) <= probe ? 1 : 0;
+                if (below < k) at |= 1u << bit;
+            }
+            const float B = unflip(at);
+            if (row_valid && B < __int_as_float(0x7f800000)) sh.athr[r] = approx_thr(B, c2, rb.c3, rb.c4);
+            tq = tau_pair(row_tau());
+            __syncwarp();
+        }
+        for (int j = scan; alive && j < total; ++j) {
+            const int acc = j & 1;
+            if (!begin_tile(j)) break;
             qc = 0;
             // one 32-column chunk at a time, one call site: double-buffering
             // the TMEM loads inlines the filter twice and costs more in code
@@ -831,10 +907,7 @@ tc_sweep_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
                 tc::tmem_wait32(ga);
                 process_chunk(ga, ch);
             }
-            // the accumulator is free for the next tile but one
-            tc::tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&sh.tempty[acc]);
+            end_tile(j);
             if (qc > 0 && tc_drain(sh, glist, wq, row0, qc, rbase, cbase, xr, ix, d, dr, k)) tq = tau_pair(row_tau());
         }
         // ---- final: exact k best of this split per row; share the k-th key.
