@@ -724,7 +724,13 @@ tc_sweep_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
             if (sh.mode[r] == kModeApprox) t = fminf(t, sh.athr[r]);
             return t;
         };
-        uint64_t tq = tau_pair(row_tau());
+        float tau = 0.0f;  // the row's threshold, and as a packed pair
+        uint64_t tq = 0;
+        auto set_tau = [&]() {
+            tau = row_tau();
+            tq = tau_pair(tau);
+        };
+        set_tau();
         const uint64_t k2 = dup2(sc.k2);
         const uint32_t lane_addr = tmem + (static_cast<uint32_t>(row0) << 16);
         // This tile's column norms are staged in a per-warp shared ring one
@@ -738,31 +744,30 @@ tc_sweep_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
         const float* nbj = nullptr;
         // filter one 32-column chunk held in registers; list / queue its candidates
         auto process_chunk = [&](const uint32_t (&gr)[32], int ch) {
-            uint64_t dl[16];
-            unsigned signs = 0;
+            // the chunk's smallest f decides whether anything passes
+            uint64_t f[16];
             const float4* nb4 = reinterpret_cast<const float4*>(nbj + 32 * ch);
+            float lo = __int_as_float(0x7f800000);
 #pragma unroll
             for (int q = 0; q < 8; ++q) {
                 const float4 nb = nb4[q];
-                const uint64_t f0 = fma2(pack2(__uint_as_float(gr[4 * q]), __uint_as_float(gr[4 * q + 1])), k2,
-                                         pack2(nb.x, nb.y));
-                const uint64_t f1 = fma2(pack2(__uint_as_float(gr[4 * q + 2]), __uint_as_float(gr[4 * q + 3])), k2,
-                                         pack2(nb.z, nb.w));
-                dl[2 * q] = sub2(f0, tq);
-                dl[2 * q + 1] = sub2(f1, tq);
-                signs |= static_cast<unsigned>(dl[2 * q]) | static_cast<unsigned>(dl[2 * q] >> 32) |
-                         static_cast<unsigned>(dl[2 * q + 1]) | static_cast<unsigned>(dl[2 * q + 1] >> 32);
+                f[2 * q] = fma2(pack2(__uint_as_float(gr[4 * q]), __uint_as_float(gr[4 * q + 1])), k2, pack2(nb.x, nb.y));
+                f[2 * q + 1] =
+                    fma2(pack2(__uint_as_float(gr[4 * q + 2]), __uint_as_float(gr[4 * q + 3])), k2, pack2(nb.z, nb.w));
+                lo = fminf(fminf(lo, lo_f(f[2 * q])), hi_f(f[2 * q]));
+                lo = fminf(fminf(lo, lo_f(f[2 * q + 1])), hi_f(f[2 * q + 1]));
             }
-            if (all) signs = row_valid ? 0x80000000u : 0u;
-            if (!__any_sync(0xffffffffu, static_cast<int>(signs) < 0)) return;
+            if (!__any_sync(0xffffffffu, lo <= tau || all)) return;
             unsigned pass = 0;
             if (all) {
                 pass = row_valid ? 0xFFFFFFFFu : 0u;
             } else {
+                // the sign of f - tq, tq the next float above the threshold
 #pragma unroll
-                for (int q = 0; q < 16; ++q) {
-                    pass |= (static_cast<unsigned>(dl[q]) >> 31) << (2 * q);
-                    pass |= static_cast<unsigned>(dl[q] >> 63) << (2 * q + 1);
+                for (int q = 15; q >= 0; --q) {
+                    const uint64_t dl = sub2(f[q], tq);
+                    pass = __funnelshift_l(static_cast<unsigned>(dl >> 32), pass, 1);
+                    pass = __funnelshift_l(static_cast<unsigned>(dl), pass, 1);
                 }
             }
             const bool exact_row = sh.mode[r] == kModeExact;
@@ -812,7 +817,7 @@ tc_sweep_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
                 changed |= tc_drain(sh, glist, wq, row0, qc, rbase, cbase, xr, ix, d, dr, k);
                 qc = 0;
             }
-            if (changed) tq = tau_pair(row_tau());
+            if (changed) set_tau();
         };
         // The accumulator of tile j: its column norms staged (and the next
         // tile's requested), its MMA waited for. False if a wait expired.
@@ -850,30 +855,31 @@ tc_sweep_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
                     break;
                 }
                 const uint32_t taddr = lane_addr + static_cast<uint32_t>((j & 1) * 128);
-#pragma unroll 1
-                for (int ch = 0; ch < 4; ch += 2) {
 #pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        uint32_t ga[32];
-                        tc::tmem_ld32_async(taddr + static_cast<uint32_t>(32 * (ch + h)), ga);
-                        tc::tmem_wait32(ga);
-                        const float4* nb4 = reinterpret_cast<const float4*>(nbj + 32 * (ch + h));
+                for (int ch = 0; ch < 4; ++ch) {
+                    uint32_t ga[32];
+                    tc::tmem_ld32_bits(taddr + static_cast<uint32_t>(32 * ch), ga);
+                    if (ch == 3) end_tile(j);
+                    const float4* nb4 = reinterpret_cast<const float4*>(nbj + 32 * ch);
 #pragma unroll
-                        for (int q = 0; q < 8; ++q) {
-                            const float4 nb = nb4[q];
-                            const uint64_t f0 = fma2(pack2(__uint_as_float(ga[4 * q]), __uint_as_float(ga[4 * q + 1])),
-                                                     k2, pack2(nb.x, nb.y));
-                            const uint64_t f1 = fma2(
-                                pack2(__uint_as_float(ga[4 * q + 2]), __uint_as_float(ga[4 * q + 3])), k2, pack2(nb.z, nb.w));
-                            float* g = gm + 32 * h + 4 * q;
-                            g[0] = fminf(g[0], lo_f(f0));
-                            g[1] = fminf(g[1], hi_f(f0));
-                            g[2] = fminf(g[2], lo_f(f1));
-                            g[3] = fminf(g[3], hi_f(f1));
+                    for (int q = 0; q < 8; q += 2) {
+                        // columns c and c + 4 share a group: one three-way minimum
+                        uint64_t f[4];
+#pragma unroll
+                        for (int e = 0; e < 2; ++e) {
+                            const float4 nb = nb4[q + e];
+                            const uint32_t* g4 = ga + 4 * (q + e);
+                            f[2 * e] = fma2(pack2(__uint_as_float(g4[0]), __uint_as_float(g4[1])), k2, pack2(nb.x, nb.y));
+                            f[2 * e + 1] =
+                                fma2(pack2(__uint_as_float(g4[2]), __uint_as_float(g4[3])), k2, pack2(nb.z, nb.w));
                         }
+                        float* g = gm + 16 * ch + 2 * q;
+                        g[0] = fminf(fminf(g[0], lo_f(f[0])), lo_f(f[2]));
+                        g[1] = fminf(fminf(g[1], hi_f(f[0])), hi_f(f[2]));
+                        g[2] = fminf(fminf(g[2], lo_f(f[1])), lo_f(f[3]));
+                        g[3] = fminf(fminf(g[3], hi_f(f[1])), hi_f(f[3]));
                     }
                 }
-                end_tile(j);
             }
             // the k-th smallest minimum, by bisection over the ordered bits
             uint32_t at = 0;
@@ -887,7 +893,7 @@ tc_sweep_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
             }
             const float B = unflip(at);
             if (row_valid && B < __int_as_float(0x7f800000)) sh.athr[r] = approx_thr(B, c2, rb.c3, rb.c4);
-            tq = tau_pair(row_tau());
+            set_tau();
             __syncwarp();
         }
         for (int j = scan; alive && j < total; ++j) {
@@ -903,12 +909,11 @@ tc_sweep_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
             uint32_t ga[32];
 #pragma unroll 1
             for (int ch = 0; ch < 4; ++ch) {
-                tc::tmem_ld32_async(taddr + static_cast<uint32_t>(32 * ch), ga);
-                tc::tmem_wait32(ga);
+                tc::tmem_ld32_bits(taddr + static_cast<uint32_t>(32 * ch), ga);
+                if (ch == 3) end_tile(j);  // released before its last columns are filtered
                 process_chunk(ga, ch);
             }
-            end_tile(j);
-            if (qc > 0 && tc_drain(sh, glist, wq, row0, qc, rbase, cbase, xr, ix, d, dr, k)) tq = tau_pair(row_tau());
+            if (qc > 0 && tc_drain(sh, glist, wq, row0, qc, rbase, cbase, xr, ix, d, dr, k)) set_tau();
         }
         // ---- final: exact k best of this split per row; share the k-th key.
         // The operand buffers are free once every epilogue warp has read its
