@@ -678,30 +678,40 @@ void Engine::knn_fast(const float* xc, const float* norms, int64_t n, int d, int
     const int mt = static_cast<int>(static_cast<int64_t>(nt) * (shard + 1) / num_shards) - t0;
     int sms = 152;
     CG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device_));
-    // The tensor sweep runs two CTAs per SM. Every split of a row tile starts
-    // from the loose seed threshold and pays the candidate surge that follows,
-    // so it takes few splits: one from two waves of row tiles up, otherwise
-    // enough for about 4 x SMs CTAs (two waves at two per SM), at most 3
-    // (measured on 20k-50k point clusters in 32-128 dimensions: 3.9-9.6 ms
-    // against 5.0-11.5 ms with 7).
+    // The tensor sweep: every split of a row tile scans for its own bounds and
+    // keeps its own lists (together about 64 tile visits), so it takes the
+    // split that needs the least rounds of CTAs times their length (n = 30,011,
+    // d = 100, k = 30: 1.42 ms per fit_predict with one split, 1.50 with two,
+    // 1.53 with three; n = 50,000, d = 32, k = 20, forward and backward: 4.18,
+    // 4.06, 4.08 ms).
     int nsplit = 1;
     if (nt > 1) {
         if (wide) {
             nsplit = choose_splits(mt, sms);
             if (nsplit > nt - 1) nsplit = nt - 1;
-        } else if (mt < 4 * sms) {
-            nsplit = mt > 0 ? (4 * sms + mt / 2) / mt : 1;
-            nsplit = nsplit < 1 ? 1 : nsplit > 3 ? 3 : nsplit;
-            if (nsplit > nt - 1) nsplit = nt - 1;
+        } else if (tensor) {
+            const int64_t slots = 2 * sms;  // CTAs at a time
+            int64_t best = -1;
+            // (past two rounds the list entries that every split repeats cost
+            // more than the last round's idle SMs: n = 200,000, d = 128, k = 50,
+            // 24.2 ms with one split, 31.0 with two)
+            for (int v = 1; v <= (mt >= 2 * slots ? 1 : tc_max_splits()) && v < nt; ++v) {
+                const int64_t cost = ceil_div(static_cast<int64_t>(mt) * v, slots) * (nt / v + 64);
+                if (best < 0 || cost < best) {
+                    best = cost;
+                    nsplit = v;
+                }
+            }
         }
     }
     if (const char* env = std::getenv("CULOF_SPLITS")) {  // tuning override (1..nt-1)
         const long v = std::atol(env);
         if (v >= 1 && nt > 1) nsplit = static_cast<int>(v < nt - 1 ? v : nt - 1);
+        if (tensor && nsplit > tc_max_splits()) nsplit = tc_max_splits();
     }
     // the small-d seed of the tensor path covers the first qs spiral positions
     // of every row tile, the sweep the rest (the other seeds cover tile T alone)
-    const int qs = small_tc ? (nt < kSeedWindow ? nt : kSeedWindow) : 1;
+    const int qs = small_tc ? (nt < kSeedWindow ? nt : kSeedWindow) : tensor ? 0 : 1;
     const bool sweep = nt > qs;
     if (sweep && nsplit > nt - qs) nsplit = nt - qs;  // no split without a column tile
 
@@ -779,15 +789,15 @@ void Engine::knn_fast(const float* xc, const float* norms, int64_t n, int d, int
 
     // 3. seed lists and the shared k-th keys
     char* rows = static_cast<char*>(rows_.get(padded * sizeof(uint64_t) * (k + 1) +
-                                              static_cast<size_t>(nsplit) * padded * k * sizeof(uint64_t) + 256));
+                                              (tensor ? 0 : static_cast<size_t>(nsplit) * padded * k * sizeof(uint64_t)) + 256));
     uint64_t* seed_keys = reinterpret_cast<uint64_t*>(rows);
     unsigned long long* kth_shared = reinterpret_cast<unsigned long long*>(seed_keys + padded * k);
     uint64_t* partial = reinterpret_cast<uint64_t*>(kth_shared + padded);
     int* status = status_ptr();
     const unsigned* maxn = reinterpret_cast<const unsigned*>(max_norm_.get(sizeof(unsigned)));
     mark(2);
-    if (tensor && !small_tc) tc_seed(tcb, t0, mt, d, k, seed_keys, kth_shared, s);
-    else if (wide) wide_seed(tiles, nt, t0, mt, d, k, seed_keys, kth_shared, s);
+    if (tensor && !small_tc) {  // no seed: the sweep covers every tile
+    } else if (wide) wide_seed(tiles, nt, t0, mt, d, k, seed_keys, kth_shared, s);
     else switch (dp) {
         case 2: seed_kernel<2><<<mt, kThreads, 0, s>>>(tiles, nt, t0, n, k, qs, seed_keys, kth_shared); break;
         case 4: seed_kernel<4><<<mt, kThreads, 0, s>>>(tiles, nt, t0, n, k, qs, seed_keys, kth_shared); break;
@@ -819,7 +829,10 @@ void Engine::knn_fast(const float* xc, const float* norms, int64_t n, int d, int
     // 4. sweep over the other tiles, split S ways
     if (sweep && mt > 0 && tensor) {
         uint64_t* lists = static_cast<uint64_t*>(tc_lists_.get(tc_list_bytes(mt, nsplit)));
-        tc_sweep(tcb, nt, t0, mt, nsplit, d, k, maxn, kth_shared, partial, lists, status, s, qs, plist, pcount);
+        tc_sweep(tcb, n, nt, t0, mt, nsplit, d, k, maxn, small_tc ? kth_shared : nullptr, small_tc ? seed_keys : nullptr,
+                 lists, status, nbr_idx, nbr_d2, kdist2, s, qs, plist, pcount);
+        mark(4);
+        return;
     } else if (nt > 1 && mt > 0 && wide) {
         wide_sweep(tiles, nt, t0, mt, nsplit, d, k, maxn, kth_shared, partial, s);
     }

@@ -63,15 +63,18 @@ size_t tc_buffer_bytes(int64_t padded, int d);
 // minmax: the per-dimension (min, max) keys of the spatial-order pass.
 TcBuffers tc_prepare(void* buf, const float* xc, const float* norms, int64_t n, int d, const unsigned* perm, int nt,
                      const unsigned* minmax, cudaStream_t s);
-void tc_seed(const TcBuffers& b, int t0, int mt, int d, int k, uint64_t* seed_keys, unsigned long long* kth_shared,
-             cudaStream_t s);
+int tc_max_splits();
 // Workspace of the per-row lists of one sweep launch batch.
 size_t tc_list_bytes(int nt, int nsplit);
-// qs: the seed window (spiral positions 0..qs-1 are the seed's); plist /
-// pcount (nullable): per row tile, the column tiles to visit in order (the
-// small-d prune lists); without them every tile past the window is visited.
-void tc_sweep(const TcBuffers& b, int nt, int t0, int mt, int nsplit, int d, int k, const unsigned* maxn,
-              unsigned long long* kth_shared, uint64_t* partial, uint64_t* lists, int* status, cudaStream_t s,
-              int qs = 1, const uint2* plist = nullptr, const int* pcount = nullptr);
+// The sweep and the rows' final results (k best of the seed's lists and the
+// sweep's, in the reference's slot order). qs: the seed window (spiral
+// positions 0..qs-1 are the seed's; 0: no seed, kth_seed and seed_keys null);
+// plist / pcount (nullable): per row tile,
+// the column tiles to visit in order (the small-d prune lists); without them
+// every tile past the window is visited.
+void tc_sweep(const TcBuffers& b, int64_t n, int nt, int t0, int mt, int nsplit, int d, int k, const unsigned* maxn,
+              const unsigned long long* kth_seed, const uint64_t* seed_keys, uint64_t* lists, int* status,
+              int32_t* nbr_idx, float* nbr_d2, float* kdist2, cudaStream_t s, int qs,
+              const uint2* plist = nullptr, const int* pcount = nullptr);
 
 }  // namespace culof_gb300

@@ -10,22 +10,32 @@
 //     streams 128-column tiles of the same array by TMA (two stages);
 //   * one warp issues the TMA loads, one issues tcgen05.mma (M = N = 128,
 //     K = 16 per instruction) into one of two TMEM accumulators, and four
-//     epilogue warps read the accumulator back (thread = row), evaluate
-//     f = |b|^2 - 2 a.b with packed fma.rn.f32x2 and compare it with the
-//     row's threshold tau (sign of a packed subtract);
-//   * a passing pair's (f, column) enters the row's list directly (the
-//     row's own thread appends it; no global memory is read). Lists are
-//     compacted by f: with fk the k-th smallest f in the list, every entry
-//     above a proven margin over fk (approx_thr) is strictly farther than
-//     k listed columns and is dropped, and the filter threshold tightens to
-//     that margin;
-//   * at the end each row's surviving entries (about k) are rescored exactly
-//     from FP32 row-major coordinates (the oracle's direct-difference chain;
-//     coalesced column loads, differences staged in the freed operand
-//     buffers) and reduced to the exact k best keys, which the merge of the
-//     FP32 sweeps combines with the seed list. A row whose list would
-//     overflow with entries inside the margin (heavy duplicates) switches to
-//     exact lists: its candidates are then rescored as they pass.
+//     epilogue warps read the accumulator back (thread = row) and evaluate
+//     f = |b|^2 - 2 a.b with packed fma.rn.f32x2;
+//   * first the rows' bounds: part of the column tiles only feed 64 group
+//     minima of f per row, whose k-th smallest bounds the row's k-th f. A list
+//     of k that starts empty takes about k ln(columns / k) entries before it
+//     has its final threshold (375 per row for n = 200,000, k = 50); started
+//     from the bound it takes a fraction of that;
+//   * then every tile: if a chunk's smallest f reaches the row's threshold tau,
+//     the passing pairs' (f, column) enter the row's list (the row's own
+//     thread appends them; no coordinates are read). Lists are compacted by
+//     f: with fk the k-th smallest f in the list, every entry above a proven
+//     margin over fk (approx_thr) is strictly farther than k listed columns
+//     and is dropped, and the filter threshold tightens to that margin;
+//   * a second kernel rescores each row's surviving entries (about k) exactly
+//     from FP32 row-major coordinates (the oracle's direct-difference chain)
+//     and writes the k best in the reference's slot order. A row whose list
+//     would overflow with entries inside the margin (heavy duplicates)
+//     switches to exact lists: its candidates are then rescored as they pass.
+//
+// What bounds it: the MMAs and their operand copies alone take 7.6 ms at
+// n = 200,000, d = 128 (72% of the measured f16 rate); reading the
+// accumulators back and testing them 10.2 ms, a quarter of that again for the
+// bounds, and the list entries of about one chunk in six the rest of 20.2 ms
+// (34.7 ms without the bounds and with the rescoring as the sweep's last
+// phase). n = 30,011, d = 100, k = 30: 2.61 -> 0.68 ms; n = 50,000, d = 32,
+// k = 20: 3.10 -> 1.43 ms.
 //
 // Exactness: the thresholds (row_bounds below) cover the f16 rounding of
 // both operands (relative 2^-11, absolute 2^-14 in scaled units for values
@@ -37,11 +47,13 @@
 // then rescored exactly.
 #include <cuda_fp16.h>
 
+#include <cmath>
 #include <cstdlib>
 
 #include "common.cuh"
 #include "engine.cuh"
 #include "fast.cuh"
+#include "row_list.cuh"
 #include "sweep_common.cuh"
 #include "tc.cuh"
 
@@ -51,13 +63,12 @@ namespace {
 
 using namespace sweep;
 
-constexpr int kTcStages = 2;
+constexpr int kStages = 2;                        // column tiles in flight (two CTAs share an SM)
 constexpr int kEpiWarps = 4;
-constexpr int kTcThreads = 32 * (2 + kEpiWarps);  // producer, MMA, 4 epilogue warps
-constexpr int kTcQueue = 32 + 32 * 32;            // a drain chunk + one 32-column chunk of every lane
+constexpr int kTcThreads = 32 * (2 + kEpiWarps);  // producer, MMA, epilogue warps
+constexpr int kTmemCols = 256;                    // two 128-column f32 accumulators
 constexpr int kTcM = 128;                         // list capacity per row (k <= 64)
 constexpr int kBox = 128 * 128;                   // bytes of one TMA box: 128 rows x 64 f16
-constexpr int kTmemCols = 256;                    // two 128-column f32 accumulators
 
 // Scale record on the device: sc = 2^S, k2 = -2 * 2^-2S (undoes the scale of
 // a Gram value and doubles it), eta = 2^-14 * 2^-S (absolute f16 rounding
@@ -133,61 +144,6 @@ __global__ void tc_build_kernel(const float* __restrict__ xc, const float* __res
     }
 }
 
-// Per row of tile T: the exact k best keys over the tile's own columns and
-// the row's starting shared k-th key (as the FP32 seed kernels).
-__global__ void __launch_bounds__(256) tc_seed_kernel(const float* __restrict__ xr, const unsigned* __restrict__ ix,
-                                                      int t0, int d, int dr, int k, uint64_t* __restrict__ seed_keys,
-                                                      unsigned long long* __restrict__ kth_shared) {
-    extern __shared__ float spts[];  // [kCT][dr + 1]
-    const int T = t0 + static_cast<int>(blockIdx.x);
-    const int ld = dr + 1;  // odd stride: lanes reading different points hit different banks
-    const int64_t base = static_cast<int64_t>(T) * kCT;
-    for (int i = threadIdx.x; i < kCT * dr; i += blockDim.x) {
-        const int c = i / dr, f = i % dr;
-        spts[c * ld + f] = xr[(base + c) * dr + f];
-    }
-    unsigned* idx = reinterpret_cast<unsigned*>(spts + kCT * ld);
-    for (int i = threadIdx.x; i < kCT; i += blockDim.x) idx[i] = ix[base + i];
-    __syncthreads();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    for (int r = warp; r < kRT; r += nw) {
-        const int64_t pos = base + r;
-        const bool row_valid = idx[r] != kNoIndex;
-        // the lane's four columns as four independent chains (each in the
-        // oracle's order), the row's coordinate loaded once per dimension
-        float s4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll 4
-        for (int f = 0; f < d; ++f) {
-            const float a = spts[r * ld + f];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const float t = __fsub_rn(a, spts[(j * 32 + lane) * ld + f]);
-                s4[j] = __fmaf_rn(t, t, s4[j]);
-            }
-        }
-        uint64_t v[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int c = j * 32 + lane;
-            v[j] = (row_valid && c != r && idx[c] != kNoIndex) ? make_key(__float_as_uint(s4[j]), idx[c]) : kKeyMax;
-        }
-        warp_bitonic_sort<4>(v);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int e = j * 32 + lane;
-            if (e < k) seed_keys[pos * k + e] = v[j];
-        }
-        const int owner = (k - 1) & 31, oreg = (k - 1) >> 5;
-        uint64_t kk = kKeyMax;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const uint64_t t = __shfl_sync(0xffffffffu, v[j], owner);
-            if (j == oreg) kk = t;
-        }
-        if (lane == 0) kth_shared[pos] = row_valid ? kk : kKeyMax;
-    }
-}
-
 // ---- thresholds ---------------------------------------------------------------
 // Per row a (float32 norm na, K = Kp terms, u = 2^-24, g the relative error of
 // the float32 norms, A >= |a|, B >= |b| for every column b), the f16 Gram value
@@ -242,12 +198,15 @@ __device__ RowBounds row_bounds(float na_f, float nmax_f, int K, float eta_f, in
     r.c4 = __double2float_ru(a / (1.0 - g) + m0);
     return r;
 }
-__device__ __forceinline__ float exact_c1(int K) {
-    return __double2float_ru((1.0 + 8.0 * kU) / (1.0 - (K + 2) * kU));
+// (host) a double rounded up to float, and the two constants of the thresholds
+float up_float(double x) {
+    const float f = static_cast<float>(x);
+    return static_cast<double>(f) < x ? std::nextafter(f, INFINITY) : f;
 }
-__device__ __forceinline__ float approx_c2(int K) {
+float exact_c1(int K) { return up_float((1.0 + 8.0 * kU) / (1.0 - (K + 2) * kU)); }
+float approx_c2(int K) {
     const double dl = (K + 3) * kU / (1.0 - (K + 3) * kU);
-    return __double2float_ru(2.0 * dl / (1.0 - dl) * (1.0 + 8.0 * kU));
+    return up_float(2.0 * dl / (1.0 - dl) * (1.0 + 8.0 * kU));
 }
 // Filter threshold of a row from its exact k-th key.
 __device__ __forceinline__ float exact_tau(uint64_t kth, float c1, float c0) {
@@ -293,29 +252,30 @@ constexpr int kModeExact = 1;
 // lets two CTAs share an SM, so two epilogue warps per SM sub-partition
 // hide each other's latencies.
 constexpr int kTcListRow = kTcM;
-constexpr size_t kTcListCta = static_cast<size_t>(kRT) * kTcListRow;  // keys per CTA
-constexpr int kTcMaxCtasPerLaunch = 4096;                             // bounds the list workspace (512 MiB)
+constexpr size_t kTcListTile = static_cast<size_t>(kRT) * kTcListRow;  // keys per row tile
+constexpr int kTcMaxTilesPerLaunch = 4096;                             // bounds the list workspace (512 MiB)
 
 struct TcSmem {
-    uint8_t a[2][kBox];             // row tile operand (K boxes 0..1)
-    uint8_t b[kTcStages][2][kBox];  // column tile operands
-    uint64_t kth[kRT];              // exact k-th key known for the row (only decreases)
-    float athr[kRT];                // approximate threshold of the row's list (+inf until k entries)
-    float row_norm[kRT];
+    uint8_t a[2][kBox];           // row tile operand (K boxes 0..1)
+    uint8_t b[kStages][2][kBox];  // column tile operands
+    uint64_t kth[kRT];            // exact k-th key known for the row (only decreases)
+    float athr[kRT];              // approximate threshold of the row's list (+inf until k entries)
+    float c0[kRT], c3[kRT], c4[kRT];  // RowBounds
     int cnt[kRT];
     int sorted[kRT];  // the row's list[0..sorted) is sorted (the last compaction's result)
     int mode[kRT];
-    uint16_t queue[kEpiWarps][kTcQueue];  // exact-mode candidates (row << 8 | column) of the current tile
-    float nb[kEpiWarps][2][kCT];          // column norms of the current and the next tile, per epilogue warp
-    uint64_t full[kTcStages], empty[kTcStages], tfull[2], tempty[2], afull, fin;
+    float nb[kEpiWarps][2][kCT];  // column norms of the current and the next tile, per epilogue warp
+    uint64_t full[kStages], empty[kStages], tfull[2], tempty[2], afull, fin;
     uint32_t tmem_base;
     int abort;
 };
 static_assert(2 * (sizeof(TcSmem) + 1024 + 1024) <= 233472, "two tensor-sweep CTAs must fit on an SM");
-// The final exact rescoring reuses the operand buffers (free once the last MMA
-// has completed): per epilogue warp, 32 candidates x (128 + 1) differences.
-constexpr int kScratchLd = 129;
-static_assert(kEpiWarps * 32 * kScratchLd * 4 <= 3 * 2 * kBox, "scratch fits in the operand buffers");
+
+// What a row leaves to the final kernel, beside its list.
+struct TcRow {
+    int cnt, mode;
+    float c3, c4;
+};
 
 __device__ void tc_abort(TcSmem& sh, int* status) {
     *reinterpret_cast<volatile int*>(&sh.abort) = 1;
@@ -483,14 +443,14 @@ __noinline__ __device__ int approx_compact(TcSmem& sh, uint64_t* __restrict__ ls
 // Row r leaves approximate mode (its list would overflow with entries within
 // the approximate margin, e.g. many duplicates): every entry is rescored
 // exactly (one lane per entry) and the list becomes an exact k-best list.
-__noinline__ __device__ void to_exact_mode(TcSmem& sh, uint64_t* __restrict__ lst, int r, int64_t rbase,
+__noinline__ __device__ void to_exact_mode(TcSmem& sh, uint64_t* __restrict__ lst, int r, int64_t pa,
                                            const float* __restrict__ xr, const unsigned* __restrict__ ix, int d,
                                            int dr, int k) {
     const int lane = threadIdx.x & 31;
     const int c = min(sh.cnt[r], kTcListRow);
     for (int e = lane; e < c; e += 32) {
         const int64_t pb = static_cast<int64_t>(key_index(lst[e]));
-        lst[e] = exact_key_lane(xr, ix, rbase + r, pb, d, dr);
+        lst[e] = pb != pa ? exact_key_lane(xr, ix, pa, pb, d, dr) : kKeyMax;  // not the row itself
     }
     __syncwarp();
     if (lane == 0) {
@@ -501,102 +461,55 @@ __noinline__ __device__ void to_exact_mode(TcSmem& sh, uint64_t* __restrict__ ls
     compact_exact(sh, lst, r, k);
 }
 
-// Rescore the warp's queued exact-mode pairs of column tile cbase exactly and
-// add the keys that beat their row's k-th key. True if a list was compacted.
-__noinline__ __device__ bool tc_drain(TcSmem& sh, uint64_t* __restrict__ glist, int wq, int row0, int qc,
-                                      int64_t rbase, int64_t cbase, const float* __restrict__ xr,
-                                      const unsigned* __restrict__ ix, int d, int dr, int k) {
+// Exact-mode rows of a chunk (whole warp; pass: this lane's row's candidate
+// columns, 0 for rows in approximate mode): per row, lane c rescores column
+// cbase + c exactly and the keys that beat the list's k-th key join it. True
+// if a list was compacted.
+__noinline__ __device__ bool exact_chunk(TcSmem& sh, uint64_t* __restrict__ glist, int list0, unsigned pass,
+                                         int64_t pa0, int64_t cbase, const float* __restrict__ xr,
+                                         const unsigned* __restrict__ ix, int d, int dr, int k) {
     const int lane = threadIdx.x & 31;
     bool compacted = false;
-    for (int base = 0; base < qc; base += 32) {
-        const int i = base + lane;
-        if (i < qc) {
-            const unsigned e = sh.queue[wq][i];
-            const int r = static_cast<int>(e >> 8), c = static_cast<int>(e & 0xFF);
-            const uint64_t key = exact_key_lane(xr, ix, rbase + r, cbase + c, d, dr);
-            if (key < sh.kth[r]) {
-                const int slot = atomicAdd(&sh.cnt[r], 1);
-                glist[static_cast<size_t>(r) * kTcListRow + slot] = key;
-            }
-        }
+    unsigned rows = __ballot_sync(0xffffffffu, pass != 0u);
+    while (rows) {
+        const int src = __ffs(rows) - 1;
+        rows &= rows - 1;
+        const unsigned cols = __shfl_sync(0xffffffffu, pass, src);
+        const int l = list0 + src;
+        uint64_t* lst = glist + static_cast<size_t>(l) * kTcListRow;
+        const uint64_t key = ((cols >> lane) & 1u) && cbase + lane != pa0 + src
+                                 ? exact_key_lane(xr, ix, pa0 + src, cbase + lane, d, dr)
+                                 : kKeyMax;
+        const unsigned m = __ballot_sync(0xffffffffu, key < sh.kth[l]);
+        if (!m) continue;
+        const int cnt = sh.cnt[l];
+        if ((m >> lane) & 1u) lst[cnt + __popc(m & ((1u << lane) - 1u))] = key;
         __syncwarp();
-        unsigned full = __ballot_sync(0xffffffffu,
-                                      sh.mode[row0 + lane] == kModeExact && sh.cnt[row0 + lane] > kTcListRow - 32);
-        compacted |= full != 0;
-        while (full) {
-            const int rr = row0 + __ffs(full) - 1;
-            full &= full - 1;
-            compact_exact(sh, glist + static_cast<size_t>(rr) * kTcListRow, rr, k);
+        if (lane == 0) sh.cnt[l] = cnt + __popc(m);
+        __syncwarp();
+        if (cnt + __popc(m) > kTcListRow - 32) {
+            compact_exact(sh, lst, l, k);
+            compacted = true;
         }
     }
     return compacted;
 }
 
-// Final exact rescoring of the first P approximate entries of row r (whole
-// warp): lane l loads dimensions 4l..4l+3 of each candidate column with one
-// coalesced 512-byte warp load per column, forms the differences t = a - b
-// and stages them in shared memory; lane i then runs candidate i's FMA chain
-// in dimension order (bit-identical to the oracle's formula).
-__noinline__ __device__ void rescore_final(uint64_t* __restrict__ lst, int r, int P, float* __restrict__ scratch,
-                                           int64_t rbase, const float* __restrict__ xr,
-                                           const unsigned* __restrict__ ix, int d, int dr) {
-    const int lane = threadIdx.x & 31;
-    const bool has = 4 * lane < dr;
-    const float4 a4 = has ? __ldg(reinterpret_cast<const float4*>(xr + (rbase + r) * dr) + lane)
-                          : make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int base = 0; base < P; base += 32) {
-        const int nb = min(32, P - base);
-        const uint32_t mypos = lane < nb ? key_index(lst[base + lane]) : 0u;
-        for (int i0 = 0; i0 < nb; i0 += 8) {
-            float4 b4[8];
-#pragma unroll
-            for (int q = 0; q < 8; ++q) {
-                const int i = i0 + q;
-                const uint32_t pb = __shfl_sync(0xffffffffu, mypos, i & 31);
-                b4[q] = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (i < nb && has) b4[q] = __ldg(reinterpret_cast<const float4*>(xr + static_cast<int64_t>(pb) * dr) + lane);
-            }
-#pragma unroll
-            for (int q = 0; q < 8; ++q) {
-                float* t = scratch + (i0 + q) * kScratchLd + 4 * lane;
-                if (i0 + q < nb && has) {
-                    t[0] = __fsub_rn(a4.x, b4[q].x);
-                    t[1] = __fsub_rn(a4.y, b4[q].y);
-                    t[2] = __fsub_rn(a4.z, b4[q].z);
-                    t[3] = __fsub_rn(a4.w, b4[q].w);
-                }
-            }
-        }
-        __syncwarp();
-        uint64_t key = kKeyMax;
-        if (lane < nb) {
-            const unsigned ib = __ldg(ix + mypos);
-            if (ib != kNoIndex) {
-                const float* t = scratch + lane * kScratchLd;
-                float s = 0.0f;
-                for (int f = 0; f < d; ++f) s = __fmaf_rn(t[f], t[f], s);
-                key = make_key(__float_as_uint(s), ib);
-            }
-        }
-        __syncwarp();
-        if (lane < nb) lst[base + lane] = key;
-        __syncwarp();
-    }
-}
-
-// Column tiles of a CTA's share that are scanned for the rows' bounds.
-__device__ __forceinline__ int bound_tiles(int count) {
-    const int part = count * 3 / 8;
-    return count <= 128 ? count : part > 128 ? part : 128;
-}
+// Column tiles of a CTA's share that are scanned for the rows' bounds: 128, or
+// a quarter if that is more. A longer scan costs more than the list entries it
+// saves, a shorter one less (fit_predict with a scan of 1/8, 1/4, 1/2 and all:
+// 1563 tiles, d = 128, k = 50: 24.2, 24.0, 25.0, 28.1 ms; 235 tiles, d = 100,
+// k = 30: 1.60, 1.51, 1.42, 1.43 ms; 157 tiles, d = 32, k = 20: 1.48, 1.38,
+// 1.29, 1.22 ms).
+__device__ __forceinline__ int bound_tiles(int count) { return min(count, max(128, count / 4)); }
 
 __global__ void __launch_bounds__(kTcThreads, 2)
 tc_sweep_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ CUtensorMap tmapb,
                 const float* __restrict__ xr,
                 const float* __restrict__ cn, const unsigned* __restrict__ ix, const TcScale* __restrict__ scale,
-                int nt, int T0, int ntb, int nsplit, int d, int dr, int Kp, int split_ops, int ksteps, int k,
-                const unsigned* __restrict__ max_norm_bits, unsigned long long* __restrict__ kth_shared,
-                uint64_t* __restrict__ partial, uint64_t* __restrict__ lists, int* __restrict__ status, int qs,
+                int nt, int T0, int ntb, int nsplit, int d, int dr, int Kp, int split_ops, int ksteps, int k, float c1,
+                float c2, const unsigned* __restrict__ max_norm_bits, const unsigned long long* __restrict__ kth_seed,
+                uint64_t* __restrict__ lists, TcRow* __restrict__ row_info, int* __restrict__ status, int qs,
                 const uint2* __restrict__ plist, const int* __restrict__ pcount) {
     extern __shared__ uint8_t tc_raw[];
     TcSmem& sh = *reinterpret_cast<TcSmem*>((reinterpret_cast<uintptr_t>(tc_raw) + 1023) & ~uintptr_t(1023));
@@ -612,8 +525,11 @@ tc_sweep_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
     const int lcount = plist ? pcount[T] : 0;
     const int count = plist ? (lcount > split ? (lcount - split + nsplit - 1) / nsplit : 0) : (q1 > q0 ? q1 - q0 : 0);
     const uint2* tlist = plist ? plist + static_cast<int64_t>(T) * nt : nullptr;
+    // without a seed window the row itself is among the columns: its list holds
+    // one entry more
+    const int kx = qs == 0 ? k + 1 : k;
     // tiles 0 .. scan - 1 are read twice: first for the rows' bounds (below)
-    const int scan = scale->all != 0.0f ? 0 : bound_tiles(count);
+    const int scan = scale->all != 0.0f || kx > 64 ? 0 : bound_tiles(count);
     const int total = scan + count;
     auto col_tile = [&](int jj) -> int {
         const int j = jj < scan ? jj : jj - scan;
@@ -622,10 +538,10 @@ tc_sweep_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
     const int nkb = Kp / 64;
     const float nmax = __uint_as_float(*max_norm_bits);
     const int64_t rbase = static_cast<int64_t>(T) * kRT;
-    uint64_t* glist = lists + static_cast<size_t>(blockIdx.x) * kTcListCta;
+    uint64_t* glist = lists + static_cast<size_t>(blockIdx.x) * kTcListTile;
 
     if (tid == 0) {
-        for (int s = 0; s < kTcStages; ++s) {
+        for (int s = 0; s < kStages; ++s) {
             mbar_init(&sh.full[s], 1);
             mbar_init(&sh.empty[s], 1);
         }
@@ -641,13 +557,16 @@ tc_sweep_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
     if (warp == 1) tc::tmem_alloc(&sh.tmem_base, kTmemCols);
     if (warp >= 2) {
         const int r = 32 * (warp & 3) + lane;
-        sh.kth[r] = kth_shared[rbase + r];
-        sh.row_norm[r] = cn[rbase + r];
+        sh.kth[r] = kth_seed ? kth_seed[rbase + r] : kKeyMax;
         sh.cnt[r] = 0;
         sh.sorted[r] = 0;
         sh.athr[r] = __int_as_float(0x7f800000);
         // with the filter disabled the f values carry no information: exact lists
         sh.mode[r] = scale->all != 0.0f ? kModeExact : kModeApprox;
+        const RowBounds rb = row_bounds(cn[rbase + r], nmax, Kp, scale->eta, split_ops ? d : 0, 16 * ksteps);
+        sh.c0[r] = rb.c0;
+        sh.c3[r] = rb.c3;
+        sh.c4[r] = rb.c4;
     }
     tc::tc_fence_before();
     __syncthreads();
@@ -661,8 +580,8 @@ tc_sweep_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
             mbar_expect_tx(&sh.afull, nkb * kBox);
             for (int kb = 0; kb < nkb; ++kb) tc::tma_load_2d(sh.a[kb], &tmap, 64 * kb, static_cast<int>(rbase), &sh.afull);
             for (int j = 0; j < total; ++j) {
-                const int s = j & 1;
-                if (j >= kTcStages && !mbar_wait(&sh.empty[s], ((j >> 1) - 1) & 1)) {
+                const int s = j % kStages;
+                if (j >= kStages && !mbar_wait(&sh.empty[s], (j / kStages - 1) & 1)) {
                     tc_abort(sh, status);
                     break;
                 }
@@ -674,8 +593,8 @@ tc_sweep_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
             }
             // no copy may still be landing in shared memory when the CTA exits
             if (!mbar_wait(&sh.afull, 0)) atomicExch(status, 1);
-            for (int j = issued - kTcStages; j < issued; ++j)
-                if (j >= 0 && !mbar_wait(&sh.full[j & 1], (j >> 1) & 1)) atomicExch(status, 1);
+            for (int j = issued - kStages; j < issued; ++j)
+                if (j >= 0 && !mbar_wait(&sh.full[j % kStages], (j / kStages) & 1)) atomicExch(status, 1);
         }
         __syncwarp();
     } else if (warp == 1) {
@@ -685,8 +604,8 @@ tc_sweep_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
             bool ok = mbar_wait(&sh.afull, 0);
             if (!ok) tc_abort(sh, status);
             for (int j = 0; ok && j < total; ++j) {
-                const int s = j & 1, acc = j & 1;
-                if (tc_aborted(sh) || !mbar_wait(&sh.full[s], (j >> 1) & 1) ||
+                const int s = j % kStages, acc = j & 1;
+                if (tc_aborted(sh) || !mbar_wait(&sh.full[s], (j / kStages) & 1) ||
                     (j >= 2 && !mbar_wait(&sh.tempty[acc], ((j >> 1) - 1) & 1))) {
                     tc_abort(sh, status);
                     break;
@@ -699,8 +618,8 @@ tc_sweep_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
                     const uint64_t bd = tc::sw128_desc(smem_u32(sh.b[s][kb]) + 32 * sub);
                     tc::mma_f16kind(dt, ad, bd, idesc, kk > 0);
                 }
-                tc::mma_commit(&sh.empty[s]);
                 tc::mma_commit(&sh.tfull[acc]);
+                tc::mma_commit(&sh.empty[s]);
             }
             // every MMA issued has completed before TMEM is released
             tc::mma_commit(&sh.fin);
@@ -710,24 +629,23 @@ tc_sweep_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
     } else {
         // ---- epilogue: thread = row
         const int wq = warp - 2;
-        const int row0 = 32 * (warp & 3);
+        const int row0 = 32 * (warp & 3);  // the TMEM lanes this warp may read
         const int r = row0 + lane;
         uint64_t* const mylist = glist + static_cast<size_t>(r) * kTcListRow;
         const TcScale sc = *scale;
         const bool all = sc.all != 0.0f;
         const bool row_valid = __ldg(ix + rbase + r) != kNoIndex;
-        const RowBounds rb = row_bounds(sh.row_norm[r], nmax, Kp, sc.eta, split_ops ? d : 0, 16 * ksteps);
-        const float c1 = exact_c1(Kp), c2 = approx_c2(Kp);
-        auto row_tau = [&]() -> float {
-            if (!row_valid) return __int_as_float(0xff800000);
-            float t = exact_tau(sh.kth[r], c1, rb.c0);
-            if (sh.mode[r] == kModeApprox) t = fminf(t, sh.athr[r]);
-            return t;
-        };
-        float tau = 0.0f;  // the row's threshold, and as a packed pair
+        bool exact_any = all;  // some list of the warp is exact
+        bool exact_row = all;
+        int cnt = 0;  // entries of this thread's list while it is approximate (sh.cnt while compacting)
+        float tau = 0.0f;  // the list's threshold, and as a packed pair
         uint64_t tq = 0;
         auto set_tau = [&]() {
-            tau = row_tau();
+            tau = __int_as_float(0xff800000);
+            if (row_valid) {
+                tau = exact_tau(sh.kth[r], c1, sh.c0[r]);
+                if (!exact_row) tau = fminf(tau, sh.athr[r]);
+            }
             tq = tau_pair(tau);
         };
         set_tau();
@@ -736,96 +654,23 @@ tc_sweep_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
         // This tile's column norms are staged in a per-warp shared ring one
         // tile ahead (one coalesced 512-byte load per warp), so the filter
         // never waits on global memory.
-        auto tile_base = [&](int jj) -> int64_t { return static_cast<int64_t>(col_tile(jj)) * kCT; };
-        float4 npre = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (total > 0) npre = __ldg(reinterpret_cast<const float4*>(cn + tile_base(0)) + lane);
-        int qc = 0;
-        int64_t cbase = 0;
-        const float* nbj = nullptr;
-        // filter one 32-column chunk held in registers; list / queue its candidates
-        auto process_chunk = [&](const uint32_t (&gr)[32], int ch) {
-            // the chunk's smallest f decides whether anything passes
-            uint64_t f[16];
-            const float4* nb4 = reinterpret_cast<const float4*>(nbj + 32 * ch);
-            float lo = __int_as_float(0x7f800000);
-#pragma unroll
-            for (int q = 0; q < 8; ++q) {
-                const float4 nb = nb4[q];
-                f[2 * q] = fma2(pack2(__uint_as_float(gr[4 * q]), __uint_as_float(gr[4 * q + 1])), k2, pack2(nb.x, nb.y));
-                f[2 * q + 1] =
-                    fma2(pack2(__uint_as_float(gr[4 * q + 2]), __uint_as_float(gr[4 * q + 3])), k2, pack2(nb.z, nb.w));
-                lo = fminf(fminf(lo, lo_f(f[2 * q])), hi_f(f[2 * q]));
-                lo = fminf(fminf(lo, lo_f(f[2 * q + 1])), hi_f(f[2 * q + 1]));
-            }
-            if (!__any_sync(0xffffffffu, lo <= tau || all)) return;
-            unsigned pass = 0;
-            if (all) {
-                pass = row_valid ? 0xFFFFFFFFu : 0u;
-            } else {
-                // the sign of f - tq, tq the next float above the threshold
-#pragma unroll
-                for (int q = 15; q >= 0; --q) {
-                    const uint64_t dl = sub2(f[q], tq);
-                    pass = __funnelshift_l(static_cast<unsigned>(dl >> 32), pass, 1);
-                    pass = __funnelshift_l(static_cast<unsigned>(dl), pass, 1);
-                }
-            }
-            const bool exact_row = sh.mode[r] == kModeExact;
-            if (!exact_row && pass) {
-                // approximate keys straight into the row's own list (f
-                // recomputed exactly as the packed filter did)
-                int cnt = sh.cnt[r];
-                unsigned pp = pass;
-                while (pp) {
-                    const int b = __ffs(pp) - 1;
-                    pp &= pp - 1;
-                    const float f = __fmaf_rn(__uint_as_float(select32(gr, b)), sc.k2, nbj[32 * ch + b]);
-                    mylist[cnt++] = make_key(flip_bits(f), static_cast<uint32_t>(cbase + 32 * ch + b));
-                }
-                sh.cnt[r] = cnt;
-            }
-            if (__any_sync(0xffffffffu, exact_row && pass)) {
-                int tot;
-                int off = warp_prefix_offset(exact_row ? __popc(pass) : 0, tot);
-                if (exact_row) {
-                    unsigned pp = pass;
-                    while (pp) {
-                        const int b = __ffs(pp) - 1;
-                        pp &= pp - 1;
-                        sh.queue[wq][qc + off++] = static_cast<uint16_t>((r << 8) | (32 * ch + b));
-                    }
-                }
-                qc += tot;
-            }
-            __syncwarp();
-            // keep room for the next chunk: compact approximate lists with
-            // less than 32 free slots
-            unsigned full =
-                __ballot_sync(0xffffffffu, sh.mode[r] == kModeApprox && sh.cnt[r] > kTcListRow - 32);
-            bool changed = full != 0;
-            while (full) {
-                const int src = __ffs(full) - 1;
-                full &= full - 1;
-                const int rr = row0 + src;
-                uint64_t* lst = glist + static_cast<size_t>(rr) * kTcListRow;
-                const float c3 = __shfl_sync(0xffffffffu, rb.c3, src);
-                const float c4 = __shfl_sync(0xffffffffu, rb.c4, src);
-                if (approx_compact(sh, lst, rr, k, c2, c3, c4, kTcListRow - 32) > kTcListRow - 32)
-                    to_exact_mode(sh, lst, rr, rbase, xr, ix, d, dr, k);
-            }
-            if (qc >= 32) {
-                changed |= tc_drain(sh, glist, wq, row0, qc, rbase, cbase, xr, ix, d, dr, k);
-                qc = 0;
-            }
-            if (changed) set_tau();
+        auto tile_base = [&](int jj) -> int64_t {
+            return static_cast<int64_t>(col_tile(jj)) * kCT;
         };
+        auto tile_norms = [&](int jj) {
+            return __ldg(reinterpret_cast<const float4*>(cn + tile_base(jj)) + lane);
+        };
+        float4 npre = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (total > 0) npre = tile_norms(0);
+        int64_t cbase = 0;  // position of the tile's first column
+        const float* nbj = nullptr;
         // The accumulator of tile j: its column norms staged (and the next
         // tile's requested), its MMA waited for. False if a wait expired.
         auto begin_tile = [&](int j) -> bool {
             cbase = tile_base(j);
             float* nbw = sh.nb[wq][j & 1];
             reinterpret_cast<float4*>(nbw)[lane] = npre;
-            if (j + 1 < total) npre = __ldg(reinterpret_cast<const float4*>(cn + tile_base(j + 1)) + lane);
+            if (j + 1 < total) npre = tile_norms(j + 1);
             nbj = nbw;
             __syncwarp();
             if (!mbar_wait_warp(&sh.tfull[j & 1], (j >> 1) & 1)) {
@@ -840,12 +685,85 @@ tc_sweep_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
             __syncwarp();
             if (lane == 0) mbar_arrive(&sh.tempty[j & 1]);
         };
+        // filter one 32-column chunk held in registers; list its candidates
+        auto process_chunk = [&](const uint32_t (&gr)[32], int ch) {
+            // the chunk's smallest f decides whether anything passes
+            uint64_t f[16];
+            const float4* nb4 = reinterpret_cast<const float4*>(nbj + 32 * ch);
+            float lo[2] = {__int_as_float(0x7f800000), __int_as_float(0x7f800000)};
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                const float4 nb = nb4[q];
+                f[2 * q] = fma2(pack2(__uint_as_float(gr[4 * q]), __uint_as_float(gr[4 * q + 1])), k2, pack2(nb.x, nb.y));
+                f[2 * q + 1] =
+                    fma2(pack2(__uint_as_float(gr[4 * q + 2]), __uint_as_float(gr[4 * q + 3])), k2, pack2(nb.z, nb.w));
+                lo[0] = fminf(fminf(lo[0], lo_f(f[2 * q])), hi_f(f[2 * q]));
+                lo[1] = fminf(fminf(lo[1], lo_f(f[2 * q + 1])), hi_f(f[2 * q + 1]));
+            }
+            if (!__any_sync(0xffffffffu, fminf(lo[0], lo[1]) <= tau || all)) return;
+            unsigned pass = 0;
+            if (all) {
+                pass = row_valid ? 0xFFFFFFFFu : 0u;
+            } else {
+                // the signs of f - tq (tq the next float above the threshold),
+                // in four independent chains of shifts
+                unsigned part[4] = {0, 0, 0, 0};
+#pragma unroll
+                for (int q = 3; q >= 0; --q) {
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        const uint64_t dl = sub2(f[4 * c + q], tq);
+                        part[c] = __funnelshift_l(static_cast<unsigned>(dl >> 32), part[c], 1);
+                        part[c] = __funnelshift_l(static_cast<unsigned>(dl), part[c], 1);
+                    }
+                }
+                pass = part[0] | part[1] << 8 | part[2] << 16 | part[3] << 24;
+            }
+            if (!exact_row) {
+                // approximate keys straight into the thread's own list (f
+                // recomputed exactly as the packed filter did)
+                unsigned pp = pass;
+                while (pp) {
+                    const int b = __ffs(pp) - 1;
+                    pp &= pp - 1;
+                    const float fb = __fmaf_rn(__uint_as_float(select32(gr, b)), sc.k2, nbj[32 * ch + b]);
+                    mylist[cnt++] = make_key(flip_bits(fb), static_cast<uint32_t>(cbase + 32 * ch + b));
+                }
+            }
+            bool changed = false;
+            __syncwarp();
+            if (exact_any)
+                changed = exact_chunk(sh, glist, row0, exact_row ? pass : 0u, rbase + row0, cbase + 32 * ch, xr, ix, d,
+                                      dr, k);
+            // keep room for the next chunk: compact approximate lists with
+            // less than 32 free slots
+            unsigned full = __ballot_sync(0xffffffffu, !exact_row && cnt > kTcListRow - 32);
+            if (full) {
+                changed = true;
+                if (!exact_row) sh.cnt[r] = cnt;
+                __syncwarp();
+                while (full) {
+                    const int src = __ffs(full) - 1;
+                    full &= full - 1;
+                    uint64_t* lst = glist + static_cast<size_t>(row0 + src) * kTcListRow;
+                    if (approx_compact(sh, lst, row0 + src, kx, c2, sh.c3[row0 + src], sh.c4[row0 + src],
+                                       kTcListRow - 32) > kTcListRow - 32) {
+                        to_exact_mode(sh, lst, row0 + src, rbase + row0 + src, xr, ix, d, dr, k);
+                        exact_any = true;
+                    }
+                }
+                exact_row = sh.mode[r] == kModeExact;
+                cnt = sh.cnt[r];
+            }
+            if (changed) set_tau();
+        };
         bool alive = true;
         if (scan > 0) {
             // Bounds first: the row's smallest f in each of 64 groups of the
-            // scanned columns. k groups with a value <= B are k columns with
-            // f <= B, so the k-th smallest of the minima bounds the row's k-th
-            // f, and the threshold over it (approx_thr) starts the lists.
+            // scanned columns. k groups with a value <= B are k
+            // columns with f <= B, so the k-th smallest of the minima bounds
+            // the row's k-th f, and the threshold over it (approx_thr) starts
+            // the lists.
             float gm[64];
 #pragma unroll
             for (int q = 0; q < 64; ++q) gm[q] = __int_as_float(0x7f800000);
@@ -881,31 +799,26 @@ tc_sweep_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
                     }
                 }
             }
-            // the k-th smallest minimum, by bisection over the ordered bits
+            // the k-th smallest of the 64, by bisection over the ordered bits
             uint32_t at = 0;
 #pragma unroll 1
             for (int bit = 31; bit >= 0; --bit) {
-                const uint32_t probe = at | ((1u << bit) - 1u);  // every value with this bit clear
+                const float probe = unflip(at | ((1u << bit) - 1u));  // every value with this bit clear
                 int below = 0;
 #pragma unroll
-                for (int q = 0; q < 64; ++q) below += flip_bits(gm[q]) <= probe ? 1 : 0;
-                if (below < k) at |= 1u << bit;
+                for (int q = 0; q < 64; ++q) below += gm[q] <= probe ? 1 : 0;
+                // (a probe that is not a number lies outside the floats: all
+                // values are below a positive one, none below a negative one)
+                if (probe != probe) below = bit == 31 || (at >> 31) ? 64 : 0;
+                if (below < kx) at |= 1u << bit;
             }
             const float B = unflip(at);
-            if (row_valid && B < __int_as_float(0x7f800000)) sh.athr[r] = approx_thr(B, c2, rb.c3, rb.c4);
+            if (row_valid && B < __int_as_float(0x7f800000)) sh.athr[r] = approx_thr(B, c2, sh.c3[r], sh.c4[r]);
             set_tau();
-            __syncwarp();
         }
         for (int j = scan; alive && j < total; ++j) {
-            const int acc = j & 1;
             if (!begin_tile(j)) break;
-            qc = 0;
-            // one 32-column chunk at a time, one call site: double-buffering
-            // the TMEM loads inlines the filter twice and costs more in code
-            // size and registers (168 with spills against 128) than the
-            // overlap saves (factor-model sweep at n = 200k, d = 128, k = 50:
-            // 40.6 ms against 35.0 ms)
-            const uint32_t taddr = lane_addr + static_cast<uint32_t>(acc * 128);
+            const uint32_t taddr = lane_addr + static_cast<uint32_t>((j & 1) * 128);
             uint32_t ga[32];
 #pragma unroll 1
             for (int ch = 0; ch < 4; ++ch) {
@@ -913,35 +826,13 @@ tc_sweep_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
                 if (ch == 3) end_tile(j);  // released before its last columns are filtered
                 process_chunk(ga, ch);
             }
-            if (qc > 0 && tc_drain(sh, glist, wq, row0, qc, rbase, cbase, xr, ix, d, dr, k)) set_tau();
         }
-        // ---- final: exact k best of this split per row; share the k-th key.
-        // The operand buffers are free once every epilogue warp has read its
-        // last accumulator (the MMAs that read them have completed).
-        asm volatile("bar.sync 1, %0;" ::"r"(32 * kEpiWarps) : "memory");
-        float* scratch = reinterpret_cast<float*>(&sh.a[0][0]) + wq * 32 * kScratchLd;
-        for (int i = 0; i < 32; ++i) {
-            const int rr = row0 + i;
-            uint64_t* lst = glist + static_cast<size_t>(rr) * kTcListRow;
-            if (sh.mode[rr] == kModeApprox) {
-                const float c3 = __shfl_sync(0xffffffffu, rb.c3, i);
-                const float c4 = __shfl_sync(0xffffffffu, rb.c4, i);
-                const int P = approx_compact(sh, lst, rr, k, c2, c3, c4, kTcListRow);
-                rescore_final(lst, rr, P, scratch, rbase, xr, ix, d, dr);
-                if (lane == 0) {
-                    sh.mode[rr] = kModeExact;
-                    sh.sorted[rr] = 0;  // exact keys: the approximate order no longer holds
-                }
-                __syncwarp();
-            }
-            compact_exact(sh, lst, rr, k);
-            const int64_t pos = rbase + rr;
-            const int c = sh.cnt[rr];
-            uint64_t* out = partial + (static_cast<int64_t>(split) * nt * kRT + pos) * k;
-            for (int e = lane; e < k; e += 32) out[e] = e < c ? lst[e] : kKeyMax;
-            if (lane == 0 && sh.kth[rr] != kKeyMax)
-                atomicMin(&kth_shared[pos], static_cast<unsigned long long>(sh.kth[rr]));
-        }
+        TcRow info;
+        info.cnt = exact_row ? sh.cnt[r] : cnt;
+        info.mode = exact_row ? kModeExact : kModeApprox;
+        info.c3 = sh.c3[r];
+        info.c4 = sh.c4[r];
+        row_info[static_cast<size_t>(blockIdx.x) * kRT + r] = info;
     }
     tc::tc_fence_before();
     __syncthreads();
@@ -949,6 +840,109 @@ tc_sweep_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
         tc::tc_fence_after();
         tc::tmem_dealloc(tmem, kTmemCols);
     }
+}
+
+// ---- final: the rows' k best from their lists -------------------------------
+//
+// One warp per row. With fk the k-th smallest f (the row itself aside) over the lists of all splits,
+// the entries within approx_thr(fk) (about k + 2) are rescored exactly, lane =
+// candidate, and join the seed's list (if there is one), which is then written
+// in the reference's slot order. It is bound by its gathers (4 dr bytes per candidate from L2).
+// As the last phase of the sweep's four epilogue warps the same rescoring took
+// 1.2 million cycles per CTA (n = 200,000, d = 128, k = 50: 6 ms of 27, and
+// half of the sweep at n = 30,011); here a row's gathers hide behind those of
+// 31 other warps per SM.
+constexpr int kFinWarps = 8;
+constexpr int kMaxTcSplits = 4;
+
+template <int KR>
+__global__ void __launch_bounds__(32 * kFinWarps)
+tc_final_kernel(const float* __restrict__ xr, const unsigned* __restrict__ ix, int64_t n, int T0, int ntb, int nsplit,
+                int dr, int k, int kx, float c2, const uint64_t* __restrict__ lists, const TcRow* __restrict__ row_info,
+                const uint64_t* __restrict__ seed_keys, int32_t* __restrict__ nbr_idx, float* __restrict__ nbr_d2,
+                float* __restrict__ kdist2) {
+    __shared__ __align__(16) float row[kFinWarps][128];
+    __shared__ unsigned cand[kFinWarps][kMaxTcSplits * kTcListRow];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int local = blockIdx.x * kFinWarps + warp;  // row of the launch batch
+    const int64_t pos = static_cast<int64_t>(T0) * kRT + local;
+    if (local >= ntb * kRT || pos >= n) return;
+    for (int f = lane; f < dr; f += 32) row[warp][f] = xr[pos * dr + f];
+    uint64_t b[KR];
+#pragma unroll
+    for (int j = 0; j < KR; ++j) b[j] = seed_keys && 32 * j + lane < k ? seed_keys[pos * k + 32 * j + lane] : kKeyMax;
+    // the approximate entries of all splits, 4 per lane and split
+    uint64_t v[kMaxTcSplits * 4];
+    int have = 0;
+    float c3 = 0.0f, c4 = 0.0f;
+#pragma unroll
+    for (int s = 0; s < kMaxTcSplits; ++s) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) v[4 * s + j] = kKeyMax;
+        if (s >= nsplit) continue;
+        const size_t at = static_cast<size_t>(s) * ntb * kRT + local;
+        const TcRow info = row_info[at];
+        c3 = info.c3;
+        c4 = info.c4;
+        const uint64_t* lst = lists + at * kTcListRow;
+        if (info.mode == kModeExact) {  // exact keys already
+            for (int e0 = 0; e0 < info.cnt; e0 += 32) list_merge<KR>(b, e0 + lane < info.cnt ? lst[e0 + lane] : kKeyMax);
+            continue;
+        }
+        have += info.cnt;
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (32 * j + lane < info.cnt) v[4 * s + j] = lst[32 * j + lane];
+    }
+    uint32_t keep = 0xFFFFFFFFu;  // ordered bits of the largest f that is kept
+    if (have > kx) {
+        uint32_t at = 0;
+#pragma unroll 1
+        for (int bit = 31; bit >= 0; --bit) {
+            const uint32_t probe = at | ((1u << bit) - 1u);
+            int below = 0;
+#pragma unroll
+            for (int j = 0; j < 4 * kMaxTcSplits; ++j) below += key_bits(v[j]) <= probe ? 1 : 0;
+            if (__reduce_add_sync(0xffffffffu, below) < kx) at |= 1u << bit;
+        }
+        keep = flip_bits(approx_thr(unflip(at), c2, c3, c4));
+    }
+    __syncwarp();
+    int P = 0;
+#pragma unroll
+    for (int j = 0; j < 4 * kMaxTcSplits; ++j) {
+        const bool in = v[j] != kKeyMax && key_bits(v[j]) <= keep && key_index(v[j]) != static_cast<uint32_t>(pos);
+        const unsigned m = __ballot_sync(0xffffffffu, in);
+        if (in) cand[warp][P + __popc(m & ((1u << lane) - 1u))] = key_index(v[j]);
+        P += __popc(m);
+    }
+    __syncwarp();
+    const float4* ra = reinterpret_cast<const float4*>(row[warp]);
+    for (int e0 = 0; e0 < P; e0 += 32) {
+        uint64_t key = kKeyMax;
+        if (e0 + lane < P) {
+            const int64_t pb = cand[warp][e0 + lane];
+            const float4* rb = reinterpret_cast<const float4*>(xr + pb * dr);
+            // the oracle's chain (padded dimensions are zero in both: fma(0, 0, s) = s)
+            float s = 0.0f;
+#pragma unroll 8
+            for (int f = 0; f < dr / 4; ++f) {
+                const float4 x = ra[f], y = __ldg(rb + f);
+                float t = __fsub_rn(x.x, y.x);
+                s = __fmaf_rn(t, t, s);
+                t = __fsub_rn(x.y, y.y);
+                s = __fmaf_rn(t, t, s);
+                t = __fsub_rn(x.z, y.z);
+                s = __fmaf_rn(t, t, s);
+                t = __fsub_rn(x.w, y.w);
+                s = __fmaf_rn(t, t, s);
+            }
+            const unsigned ib = __ldg(ix + pb);
+            if (ib != kNoIndex) key = make_key(__float_as_uint(s), ib);
+        }
+        list_merge<KR>(b, key);
+    }
+    emit_row<KR>(b, k, n, __ldg(ix + pos), nbr_idx, nbr_d2, kdist2);
 }
 
 }  // namespace
@@ -974,10 +968,14 @@ size_t tc_buffer_bytes(int64_t padded, int d) {
            up(sizeof(float) * padded) + up(sizeof(unsigned) * padded) + up(sizeof(TcScale));
 }
 
+int tc_max_splits() { return kMaxTcSplits; }
+
+static int64_t tc_list_tiles(int nt, int nsplit) {
+    const int64_t tiles = static_cast<int64_t>(nt) * nsplit;
+    return tiles > kTcMaxTilesPerLaunch ? kTcMaxTilesPerLaunch : tiles;
+}
 size_t tc_list_bytes(int nt, int nsplit) {
-    int64_t ctas = static_cast<int64_t>(nt) * nsplit;
-    if (ctas > kTcMaxCtasPerLaunch) ctas = kTcMaxCtasPerLaunch;
-    return sizeof(uint64_t) * kTcListCta * static_cast<size_t>(ctas);
+    return (sizeof(uint64_t) * kTcListTile + sizeof(TcRow) * kRT) * static_cast<size_t>(tc_list_tiles(nt, nsplit));
 }
 
 TcBuffers tc_prepare(void* buf, const float* xc, const float* norms, int64_t n, int d, const unsigned* perm, int nt,
@@ -1017,29 +1015,32 @@ TcBuffers tc_prepare(void* buf, const float* xc, const float* norms, int64_t n, 
     return b;
 }
 
-void tc_seed(const TcBuffers& b, int t0, int mt, int d, int k, uint64_t* seed_keys, unsigned long long* kth_shared,
-             cudaStream_t s) {
-    const size_t smem = sizeof(float) * (static_cast<size_t>(kCT) * (b.dr + 1) + kCT);
-    set_max_dynamic_smem(reinterpret_cast<const void*>(tc_seed_kernel), 100 * 1024);
-    tc_seed_kernel<<<mt, 256, smem, s>>>(b.xr, b.ix, t0, d, b.dr, k, seed_keys, kth_shared);
-    CG_LAUNCH_CHECK();
-}
-
-void tc_sweep(const TcBuffers& b, int nt, int t0, int mt, int nsplit, int d, int k, const unsigned* maxn,
-              unsigned long long* kth_shared, uint64_t* partial, uint64_t* lists, int* status, cudaStream_t s, int qs,
-              const uint2* plist, const int* pcount) {
+void tc_sweep(const TcBuffers& b, int64_t n, int nt, int t0, int mt, int nsplit, int d, int k, const unsigned* maxn,
+              const unsigned long long* kth_seed, const uint64_t* seed_keys, uint64_t* lists, int* status,
+              int32_t* nbr_idx, float* nbr_d2, float* kdist2, cudaStream_t s, int qs, const uint2* plist,
+              const int* pcount) {
     const size_t smem = sizeof(TcSmem) + 1024;
     set_max_dynamic_smem(reinterpret_cast<const void*>(tc_sweep_kernel), static_cast<int>(smem));
     const CUtensorMap map = tc::make_kmajor_map(b.xh, static_cast<int64_t>(nt) * kCT, b.Kp, true);
     const CUtensorMap mapb = tc::make_kmajor_map(b.xb, static_cast<int64_t>(nt) * kCT, b.Kp, true);
+    TcRow* info = reinterpret_cast<TcRow*>(lists + kTcListTile * static_cast<size_t>(tc_list_tiles(mt, nsplit)));
+    const float c1 = exact_c1(b.Kp), c2 = approx_c2(b.Kp);
+    const int kx = qs == 0 ? k + 1 : k;
     // row tiles in batches, so that the list workspace stays bounded
-    const int ntb_max = kTcMaxCtasPerLaunch / nsplit > 0 ? kTcMaxCtasPerLaunch / nsplit : 1;
+    const int ntb_max = kTcMaxTilesPerLaunch / nsplit;
     for (int T0 = t0; T0 < t0 + mt; T0 += ntb_max) {
         const int ntb = t0 + mt - T0 < ntb_max ? t0 + mt - T0 : ntb_max;
-        tc_sweep_kernel<<<ntb * nsplit, kTcThreads, smem, s>>>(map, mapb, b.xr, b.cn, b.ix,
-                                                               reinterpret_cast<const TcScale*>(b.scale), nt, T0, ntb,
-                                                               nsplit, d, b.dr, b.Kp, b.split, b.ksteps, k, maxn,
-                                                               kth_shared, partial, lists, status, qs, plist, pcount);
+        tc_sweep_kernel<<<ntb * nsplit, kTcThreads, smem, s>>>(
+            map, mapb, b.xr, b.cn, b.ix, reinterpret_cast<const TcScale*>(b.scale), nt, T0, ntb, nsplit, d, b.dr, b.Kp,
+            b.split, b.ksteps, k, c1, c2, maxn, kth_seed, lists, info, status, qs, plist, pcount);
+        CG_LAUNCH_CHECK();
+        const unsigned grid = static_cast<unsigned>(ntb) * kRT / kFinWarps;
+        if (k <= 32)
+            tc_final_kernel<1><<<grid, 32 * kFinWarps, 0, s>>>(b.xr, b.ix, n, T0, ntb, nsplit, b.dr, k, kx, c2, lists, info,
+                                                               seed_keys, nbr_idx, nbr_d2, kdist2);
+        else
+            tc_final_kernel<2><<<grid, 32 * kFinWarps, 0, s>>>(b.xr, b.ix, n, T0, ntb, nsplit, b.dr, k, kx, c2, lists, info,
+                                                               seed_keys, nbr_idx, nbr_d2, kdist2);
         CG_LAUNCH_CHECK();
     }
 }
