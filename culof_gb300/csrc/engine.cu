@@ -203,15 +203,15 @@ int64_t Engine::knn_core(const float* d_x, int64_t n, int d, int k, bool normali
     double* mean = mean_.as<double>(d);
     double* inv = inv_std_.as<double>(d);
     float* norms = norms_.as<float>(n);
-    unsigned int* maxn = max_norm_.as<unsigned int>(1);
-    CG_CUDA(cudaMemsetAsync(status_ptr(), 0, sizeof(int), stream_));
+    // status, counters, largest norm and feature ranges: one memset
+    CG_CUDA(cudaMemsetAsync(call_words(), 0, sizeof(unsigned) * kCallWords, stream_));
     stat_total_pairs_ = 0.0;
     for (bool& m : marked_) m = false;
     mark(0);
-    center(d_x, n, d, normalize, xc, partial, mean, inv, stream_);
     const int path = choose_path(n, d, k);
+    center(d_x, n, d, normalize, xc, partial, mean, inv, stream_, path != kPathGeneral ? range_words() : nullptr);
     // only the filters of the wide and tensor sweeps read the norms
-    if (path == kPathTensor || (path == kPathFast && d > 8)) squared_norms(xc, n, d, norms, maxn, stream_);
+    if (path == kPathTensor || (path == kPathFast && d > 8)) squared_norms(xc, n, d, norms, max_norm_word(), stream_);
     int64_t count = n;
     if (path != kPathGeneral) {
         last_path_ = path;
@@ -314,7 +314,7 @@ void Engine::stage_times(float* ms, int cap) {
 void Engine::pair_stats(double* evaluated, double* total) {
     unsigned long long ev = 0;
     if (stat_total_pairs_ > 0.0) {
-        CG_CUDA(cudaMemcpyAsync(&ev, pair_stats_.get(sizeof(ev)), sizeof(ev), cudaMemcpyDeviceToHost, stream_));
+        CG_CUDA(cudaMemcpyAsync(&ev, evaluated_word(), sizeof(ev), cudaMemcpyDeviceToHost, stream_));
         CG_CUDA(cudaStreamSynchronize(stream_));
     }
     // one unit = a row against 64 columns

@@ -150,7 +150,7 @@ private:
     int path_ = kPathAuto;
     int last_path_ = kPathAuto;
 
-    DevBuf x_, xc_, partial_, mean_, inv_std_, norms_, max_norm_;
+    DevBuf x_, xc_, partial_, mean_, inv_std_, norms_;
     DevBuf nbr_idx_, nbr_d2_, kdist2_, lrd_, scores_, nof_, labels_, offset_, offset_scratch_;
     DevBuf tile_, bw_;
     // batched path (batched.cu)
@@ -171,16 +171,24 @@ private:
     cudaStream_t bgraph_stream_ = nullptr;
     unsigned long long bgraph_kernels_ = 0;
     // fast path workspaces
-    DevBuf morton_, perm_, sort_tmp_, sort_hist_, cols_, rows_, tc_lists_, tiles_;
-    // the small-d sweep's evaluated (row, 64 columns) units and the pairs it
-    // would evaluate without pruning; tile boxes; the tensor path's tile lists
-    DevBuf pair_stats_, boxes_, plist_, pcount_;
+    DevBuf morton_, perm_, sort_tmp_, cols_, rows_, tc_lists_, tiles_;
+    // tile boxes; the tensor path's tile lists over d <= 8 points
+    DevBuf boxes_, plist_, pcount_;
     DevBuf iso_;  // rows that leave the small-d sweep for their own pass
-    double stat_total_pairs_ = 0.0;
-    // Device status word of the current call: kernels set it (a bounded wait
-    // that expired, an out-of-range neighbour index); host paths check it.
-    DevBuf status_;
-    int* status_ptr() { return status_.as<int>(1); }
+    double stat_total_pairs_ = 0.0;  // pairs the small-d sweep would evaluate without pruning
+    // Words that every k-NN call starts from zero: the device status word
+    // (kernels set it: a bounded wait that expired, an out-of-range neighbour
+    // index; host paths check it), the largest row norm, the small-d sweep's
+    // evaluated (row, 64 columns) units, its count of rows that left, and the
+    // features' ranges.
+    static constexpr int kCallWords = 8 + 2 * kMaxRangeDims;
+    DevBuf call_words_;
+    unsigned* call_words() { return call_words_.as<unsigned>(kCallWords); }
+    int* status_ptr() { return reinterpret_cast<int*>(call_words()); }
+    unsigned* max_norm_word() { return call_words() + 1; }
+    unsigned long long* evaluated_word() { return reinterpret_cast<unsigned long long*>(call_words() + 2); }
+    int* iso_count_word() { return reinterpret_cast<int*>(call_words() + 4); }
+    unsigned* range_words() { return call_words() + 8; }
 
 public:
     // Raises kKernelFault if a kernel of the last call reported an error

@@ -28,8 +28,10 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
+#include <utility>
 
 #include "common.cuh"
+#include "block.cuh"
 #include "engine.cuh"
 #include "fast.cuh"
 #include "small.cuh"
@@ -56,92 +58,60 @@ __device__ __forceinline__ uint64_t sub2(uint64_t a, uint64_t b) {
 
 // ---------------------------------------------------------------- spatial order
 
-__device__ __forceinline__ unsigned flip_float(float f) {
-    const unsigned u = __float_as_uint(f);
-    return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-}
-__device__ __forceinline__ float unflip_float(unsigned k) {
-    return __uint_as_float((k & 0x80000000u) ? (k & 0x7FFFFFFFu) : ~k);
-}
-
-// Per dimension f: mm[2f] = min key, mm[2f+1] = max key (flipped floats).
-// One coalesced pass over the n x d values: each thread stays on one
-// dimension (the block's active threads and its stride are multiples of d),
-// reduces in shared memory, and one thread per dimension and block updates
-// the global words. Requires d <= kMaxMinmaxDims.
-constexpr int kMaxMinmaxDims = 256;
-__global__ void minmax_kernel(const float* __restrict__ xc, int64_t n, int d, unsigned* __restrict__ mm) {
-    __shared__ unsigned slo[kMaxMinmaxDims], shi[kMaxMinmaxDims];
-    for (int f = threadIdx.x; f < d; f += blockDim.x) {
-        slo[f] = 0xFFFFFFFFu;
-        shi[f] = 0u;
-    }
-    __syncthreads();
-    const int per = static_cast<int>(blockDim.x) / d * d;  // active threads
-    if (static_cast<int>(threadIdx.x) < per) {
-        const int f = static_cast<int>(threadIdx.x) % d;
-        unsigned lo = 0xFFFFFFFFu, hi = 0u;
-        const int64_t total = n * d;
-        for (int64_t t = static_cast<int64_t>(blockIdx.x) * per + threadIdx.x; t < total;
-             t += static_cast<int64_t>(gridDim.x) * per) {
-            const unsigned k = flip_float(xc[t]);
-            lo = min(lo, k);
-            hi = max(hi, k);
-        }
-        atomicMin(&slo[f], lo);
-        atomicMax(&shi[f], hi);
-    }
-    __syncthreads();
-    for (int f = threadIdx.x; f < d; f += blockDim.x) {
-        atomicMin(&mm[2 * f], slo[f]);
-        atomicMax(&mm[2 * f + 1], shi[f]);
-    }
-}
-
-__global__ void minmax_init_kernel(unsigned* mm, int d) {
-    for (int f = threadIdx.x; f < d; f += blockDim.x) {
-        mm[2 * f] = 0xFFFFFFFFu;
-        mm[2 * f + 1] = 0u;
-    }
-}
-
-// The (up to) kMortonDims dimensions with the widest range, widest first
-// (ties by index); one thread.
-__global__ void select_dims_kernel(const unsigned* __restrict__ mm, int d, int* __restrict__ dims) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    const int m = d < kMortonDims ? d : kMortonDims;
-    for (int j = 0; j < m; ++j) {
-        int best = -1;
-        float best_span = -1.0f;
-        for (int f = 0; f < d; ++f) {
-            bool taken = false;
-            for (int q = 0; q < j; ++q) taken |= dims[q] == f;
-            if (taken) continue;
-            const float span = unflip_float(mm[2 * f + 1]) - unflip_float(mm[2 * f]);
-            if (span > best_span) {
-                best_span = span;
-                best = f;
-            }
-        }
-        dims[j] = best;
-    }
-}
-
-// 32-bit Morton key: 32/m bits for each of the m selected dimensions,
-// interleaved from the most significant bit, over the bounding box of the
-// centred data.
+// 32-bit Morton key: 32/m bits for each of the (up to) kMortonDims features of
+// the widest range, widest first (ties by index), interleaved from the most
+// significant bit, over the bounding box of the centred data (mm, see
+// center()). Every block picks the features itself, with one warp.
 __global__ void morton_kernel(const float* __restrict__ xc, int64_t n, int d, const unsigned* __restrict__ mm,
-                              const int* __restrict__ dims, unsigned* __restrict__ keys, unsigned* __restrict__ vals) {
+                              unsigned* __restrict__ keys, unsigned* __restrict__ vals) {
+    __shared__ int dims[kMortonDims];
+    __shared__ float dlo[kMortonDims], dspan[kMortonDims];
     const int md = d < kMortonDims ? d : kMortonDims;
     const int bits = (32 / md) < 30 ? (32 / md) : 30;
+    if (threadIdx.x < 32) {
+        const int lane = threadIdx.x;
+        float span[kMaxWideD / 32];
+#pragma unroll
+        for (int j = 0; j < kMaxWideD / 32; ++j) {
+            const int f = 32 * j + lane;
+            span[j] = f < d ? range_hi(mm, f) - range_lo(mm, f) : -1.0f;
+        }
+        for (int q = 0; q < md; ++q) {
+            float best = -1.0f;
+            int at = d;
+#pragma unroll
+            for (int j = 0; j < kMaxWideD / 32; ++j)
+                if (span[j] > best) {
+                    best = span[j];
+                    at = 32 * j + lane;
+                }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                const float ob = __shfl_xor_sync(0xffffffffu, best, o);
+                const int oa = __shfl_xor_sync(0xffffffffu, at, o);
+                if (ob > best || (ob == best && oa < at)) {
+                    best = ob;
+                    at = oa;
+                }
+            }
+            if (at >= d) at = q;  // (ranges that are not numbers: any feature)
+#pragma unroll
+            for (int j = 0; j < kMaxWideD / 32; ++j)
+                if (32 * j + lane == at) span[j] = -2.0f;
+            if (lane == 0) {
+                dims[q] = at;
+                dlo[q] = range_lo(mm, at);
+                dspan[q] = range_hi(mm, at) - range_lo(mm, at);
+            }
+        }
+    }
+    __syncthreads();
     for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
          i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
         unsigned q[kMortonDims];
         for (int j = 0; j < md; ++j) {
-            const int f = dims[j];
-            const float lo = unflip_float(mm[2 * f]), hi = unflip_float(mm[2 * f + 1]);
-            const float span = hi - lo;
-            float t = span > 0.0f ? (xc[i * d + f] - lo) / span : 0.0f;
+            const float span = dspan[j];
+            float t = span > 0.0f ? (xc[i * d + dims[j]] - dlo[j]) / span : 0.0f;
             t = fminf(fmaxf(t, 0.0f), 1.0f);
             const float scale = static_cast<float>((1u << bits) - 1u);
             q[j] = static_cast<unsigned>(t * scale + 0.5f);
@@ -173,11 +143,30 @@ __global__ void sort_upsweep_kernel(const unsigned* __restrict__ keys, int64_t n
     counts[static_cast<int64_t>(threadIdx.x) * nblocks + blockIdx.x] = hist[threadIdx.x];
 }
 
-// Exclusive scan of counts[256 * nblocks] in digit-major order (one block):
-// each thread scans kScanItems consecutive counts per step, the block scans
-// the threads' totals.
+// Exclusive scan of each digit's row counts[digit][0 .. nblocks) and the row's
+// total, one block per digit (the downsweep adds the lower digits' totals; one
+// block scanning all rows took 14 us at n = 200,000 and 38 us at a million).
+constexpr int kRowScanThreads = 256;
+__global__ void __launch_bounds__(kRowScanThreads) sort_rowscan_kernel(unsigned* __restrict__ counts, int nblocks,
+                                                                       unsigned* __restrict__ totals) {
+    __shared__ int warp_sums[kRowScanThreads / 32];
+    unsigned* row = counts + static_cast<int64_t>(blockIdx.x) * nblocks;
+    unsigned carry = 0;
+    for (int b0 = 0; b0 < nblocks; b0 += kRowScanThreads) {
+        const int b = b0 + static_cast<int>(threadIdx.x);
+        const int v = b < nblocks ? static_cast<int>(row[b]) : 0;
+        int total;
+        const int excl = block_exclusive_scan(v, warp_sums, total);
+        if (b < nblocks) row[b] = carry + static_cast<unsigned>(excl);
+        carry += static_cast<unsigned>(total);
+    }
+    if (threadIdx.x == 0) totals[blockIdx.x] = carry;
+}
+
+// Exclusive scan of an array in place (one block): each thread scans
+// kScanItems consecutive entries per step, the block scans the threads' totals.
 constexpr int kScanItems = 8;
-__global__ void sort_scan_kernel(unsigned* __restrict__ counts, int64_t len) {
+__global__ void scan_kernel(unsigned* __restrict__ counts, int64_t len) {
     __shared__ unsigned warp_tot[32];
     __shared__ unsigned carry;
     if (threadIdx.x == 0) carry = 0;
@@ -223,8 +212,15 @@ __global__ void sort_scan_kernel(unsigned* __restrict__ counts, int64_t len) {
 
 __global__ void sort_downsweep_kernel(const unsigned* __restrict__ keys_in, const unsigned* __restrict__ vals_in,
                                       unsigned* __restrict__ keys_out, unsigned* __restrict__ vals_out, int64_t n,
-                                      int shift, const unsigned* __restrict__ offsets, int nblocks) {
+                                      int shift, const unsigned* __restrict__ offsets,
+                                      const unsigned* __restrict__ totals, int nblocks) {
     __shared__ unsigned wcount[kWarps][256];
+    __shared__ unsigned first[256];  // first place of each digit
+    __shared__ int warp_sums[kWarps];
+    {
+        int all;
+        first[threadIdx.x] = static_cast<unsigned>(block_exclusive_scan(static_cast<int>(totals[threadIdx.x]), warp_sums, all));
+    }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int d = lane; d < 256; d += 32) wcount[warp][d] = 0;
     __syncwarp();
@@ -263,7 +259,8 @@ __global__ void sort_downsweep_kernel(const unsigned* __restrict__ keys_in, cons
         const int64_t i = base + it * 32 + lane;
         if (i < n) {
             const unsigned dg = (key[it] >> shift) & 0xFF;
-            const unsigned pos = offsets[static_cast<int64_t>(dg) * nblocks + blockIdx.x] + wcount[warp][dg] + rank[it];
+            const unsigned pos =
+                first[dg] + offsets[static_cast<int64_t>(dg) * nblocks + blockIdx.x] + wcount[warp][dg] + rank[it];
             keys_out[pos] = key[it];
             vals_out[pos] = val[it];
         }
@@ -626,32 +623,31 @@ void launch_merge(const uint64_t* seed_keys, const uint64_t* partial, const unsi
     CG_LAUNCH_CHECK();
 }
 
-size_t sort_pairs_counts(int64_t n) { return static_cast<size_t>(256) * static_cast<size_t>(ceil_div(n, kSortTile)); }
+size_t sort_pairs_counts(int64_t n) {
+    return static_cast<size_t>(256) * (static_cast<size_t>(ceil_div(n, kSortTile)) + 1);  // the rows, then their totals
+}
 
 unsigned* sort_pairs_stable(unsigned* keys, unsigned* vals, unsigned* keys_tmp, unsigned* vals_tmp, int64_t n,
                             int key_bits, unsigned* counts, cudaStream_t s, unsigned** vals_out) {
     const int nblocks = static_cast<int>(ceil_div(n, kSortTile));
+    unsigned* totals = counts + static_cast<int64_t>(256) * nblocks;
     unsigned *kin = keys, *vin = vals, *kout = keys_tmp, *vout = vals_tmp;
     for (int shift = 0; shift < key_bits; shift += 8) {
         sort_upsweep_kernel<<<nblocks, kSortThreads, 0, s>>>(kin, n, shift, counts, nblocks);
         CG_LAUNCH_CHECK();
-        sort_scan_kernel<<<1, 1024, 0, s>>>(counts, static_cast<int64_t>(256) * nblocks);
+        sort_rowscan_kernel<<<256, kRowScanThreads, 0, s>>>(counts, nblocks, totals);
         CG_LAUNCH_CHECK();
-        sort_downsweep_kernel<<<nblocks, kSortThreads, 0, s>>>(kin, vin, kout, vout, n, shift, counts, nblocks);
+        sort_downsweep_kernel<<<nblocks, kSortThreads, 0, s>>>(kin, vin, kout, vout, n, shift, counts, totals, nblocks);
         CG_LAUNCH_CHECK();
-        unsigned* t = kin;
-        kin = kout;
-        kout = t;
-        t = vin;
-        vin = vout;
-        vout = t;
+        std::swap(kin, kout);
+        std::swap(vin, vout);
     }
     *vals_out = vin;
     return kin;
 }
 
 void exclusive_scan_u32(unsigned* data, int64_t len, cudaStream_t s) {
-    sort_scan_kernel<<<1, 1024, 0, s>>>(data, len);
+    scan_kernel<<<1, 1024, 0, s>>>(data, len);
     CG_LAUNCH_CHECK();
 }
 
@@ -716,37 +712,14 @@ void Engine::knn_fast(const float* xc, const float* norms, int64_t n, int d, int
     if (sweep && nsplit > nt - qs) nsplit = nt - qs;  // no split without a column tile
 
     // 1. Morton keys of the centred coordinates, then a stable radix sort.
-    unsigned* mm = reinterpret_cast<unsigned*>(sort_hist_.get(2 * sizeof(unsigned) * d + sizeof(int) * kMortonDims));
-    int* dims = reinterpret_cast<int*>(mm + 2 * d);
+    const unsigned* mm = range_words();  // from the centring
     unsigned* keys = morton_.as<unsigned>(2 * static_cast<size_t>(n));
     unsigned* vals = perm_.as<unsigned>(2 * static_cast<size_t>(n));
-    minmax_init_kernel<<<1, 32, 0, s>>>(mm, d);
+    morton_kernel<<<grid_for(n, 256), 256, 0, s>>>(xc, n, d, mm, keys, vals);
     CG_LAUNCH_CHECK();
-    minmax_kernel<<<grid_for(n * d, 256), 256, 0, s>>>(xc, n, d, mm);
-    CG_LAUNCH_CHECK();
-    select_dims_kernel<<<1, 32, 0, s>>>(mm, d, dims);
-    CG_LAUNCH_CHECK();
-    morton_kernel<<<grid_for(n, 256), 256, 0, s>>>(xc, n, d, mm, dims, keys, vals);
-    CG_LAUNCH_CHECK();
-    const int nblocks = static_cast<int>(ceil_div(n, kSortTile));
-    unsigned* counts = sort_tmp_.as<unsigned>(static_cast<size_t>(256) * nblocks);
-    unsigned *kin = keys, *vin = vals, *kout = keys + n, *vout = vals + n;
-    for (int pass = 0; pass < 4; ++pass) {
-        const int shift = 8 * pass;
-        sort_upsweep_kernel<<<nblocks, kSortThreads, 0, s>>>(kin, n, shift, counts, nblocks);
-        CG_LAUNCH_CHECK();
-        sort_scan_kernel<<<1, 1024, 0, s>>>(counts, static_cast<int64_t>(256) * nblocks);
-        CG_LAUNCH_CHECK();
-        sort_downsweep_kernel<<<nblocks, kSortThreads, 0, s>>>(kin, vin, kout, vout, n, shift, counts, nblocks);
-        CG_LAUNCH_CHECK();
-        unsigned* t = kin;
-        kin = kout;
-        kout = t;
-        t = vin;
-        vin = vout;
-        vout = t;
-    }
-    const unsigned* perm = vin;  // after 4 passes: back in the first half
+    unsigned* vin = nullptr;  // after 4 passes: back in the first half
+    sort_pairs_stable(keys, vals, keys + n, vals + n, n, 32, sort_tmp_.as<unsigned>(sort_pairs_counts(n)), s, &vin);
+    const unsigned* perm = vin;
     if (small_fp32 || small_tc) small_refine_order(xc, n, d, vin, s);
     const int64_t pos0 = static_cast<int64_t>(t0) * kCT;
     const int64_t pos1 = std::min<int64_t>(n, static_cast<int64_t>(t0 + mt) * kCT);
@@ -771,8 +744,7 @@ void Engine::knn_fast(const float* xc, const float* norms, int64_t n, int d, int
         if (small_fp32) {
             mark(2);
             mark(3);
-            unsigned long long* ev = pair_stats_.as<unsigned long long>(1);
-            CG_CUDA(cudaMemsetAsync(ev, 0, sizeof(unsigned long long), s));
+            unsigned long long* ev = evaluated_word();
             // pairs past the window (tile T and its four Morton neighbours)
             const int window = nt < kSeedWindow ? nt : kSeedWindow;
             stat_total_pairs_ = static_cast<double>(mt) * (nt - window) * kRT * kCT;
@@ -780,7 +752,7 @@ void Engine::knn_fast(const float* xc, const float* norms, int64_t n, int d, int
             // inputs of many segments do (the same results)
             const char* env = std::getenv("CULOF_PRUNE_LISTS");
             small_knn(tiles, boxes, qbox, perm, n, d, nt, t0, mt, k, sms, iso_rows_enabled(n),
-                      env && env[0] == '0' ? 8 : kSegTiles, iso_.get(small_iso_bytes(mt, k)), nbr_idx, nbr_d2, kdist2,
+                      env && env[0] == '0' ? 8 : kSegTiles, iso_.get(small_iso_bytes(mt, k)), iso_count_word(), nbr_idx, nbr_d2, kdist2,
                       status_ptr(), ev, s);
             mark(4);
             return;
@@ -794,7 +766,7 @@ void Engine::knn_fast(const float* xc, const float* norms, int64_t n, int d, int
     unsigned long long* kth_shared = reinterpret_cast<unsigned long long*>(seed_keys + padded * k);
     uint64_t* partial = reinterpret_cast<uint64_t*>(kth_shared + padded);
     int* status = status_ptr();
-    const unsigned* maxn = reinterpret_cast<const unsigned*>(max_norm_.get(sizeof(unsigned)));
+    const unsigned* maxn = max_norm_word();
     mark(2);
     if (tensor && !small_tc) {  // no seed: the sweep covers every tile
     } else if (wide) wide_seed(tiles, nt, t0, mt, d, k, seed_keys, kth_shared, s);

@@ -12,15 +12,18 @@
 // means (and the centred floats) agree with it bit for bit; the partials give
 // n/kCenterChunk x d parallel work instead of d blocks.
 #include "common.cuh"
+#include "fp64.cuh"
 #include "prep.cuh"
 
 namespace culof_gb300 {
 
 namespace {
 
+constexpr int kApplyThreads = 256;
+
 __device__ __forceinline__ double center_term(double s, float x, double m, bool square) {
-    if (!square) return __dadd_rn(s, static_cast<double>(x));
-    const double v = __dsub_rn(static_cast<double>(x), m);
+    if (!square) return __dadd_rn(s, widen(x));
+    const double v = __dsub_rn(widen(x), m);
     return __dadd_rn(s, __dmul_rn(v, v));
 }
 
@@ -102,16 +105,54 @@ __global__ void center_finalize_kernel(const double* __restrict__ partial, int64
     }
 }
 
-__global__ void center_apply_kernel(const float* __restrict__ x, int64_t n, int d,
-                                    const double* __restrict__ mean,
-                                    const double* __restrict__ inv_std,
-                                    float* __restrict__ xc) {
+// A value times the feature's scale; without normalising the scale is 1 and
+// the product the value itself.
+__device__ __forceinline__ double scale_by(double v, double inv) { return inv == 1.0 ? v : __dmul_rn(v, inv); }
+
+// One pass over the n x d values: each thread stays on one feature (the
+// block's active threads and its stride are multiples of d). With mm, also
+// the features' ranges for the spatial order (range_put), reduced in shared
+// memory first.
+__global__ void __launch_bounds__(kApplyThreads)
+center_apply_kernel(const float* __restrict__ x, int64_t n, int d, const double* __restrict__ mean,
+                    const double* __restrict__ inv_std, float* __restrict__ xc, unsigned* __restrict__ mm) {
+    __shared__ unsigned slo[kMaxRangeDims], shi[kMaxRangeDims];
+    if (mm != nullptr) {
+        for (int f = threadIdx.x; f < d; f += blockDim.x) slo[f] = shi[f] = 0u;
+        __syncthreads();
+    }
     const int64_t total = n * d;
-    for (int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; t < total;
-         t += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-        const int f = static_cast<int>(t % d);
-        const double v = __dmul_rn(__dsub_rn(static_cast<double>(x[t]), mean[f]), inv_std[f]);
-        xc[t] = __double2float_rn(v);
+    if (d <= kApplyThreads) {
+        const int per = kApplyThreads / d * d;  // active threads
+        if (static_cast<int>(threadIdx.x) < per) {
+            const int f = static_cast<int>(threadIdx.x) % d;
+            const double m = mean[f], inv = inv_std[f];
+            unsigned lo = 0u, hi = 0u;
+            for (int64_t t = static_cast<int64_t>(blockIdx.x) * per + threadIdx.x; t < total;
+                 t += static_cast<int64_t>(gridDim.x) * per) {
+                const float v = narrow(scale_by(__dsub_rn(widen(x[t]), m), inv));
+                xc[t] = v;
+                lo = max(lo, ~range_key(v));
+                hi = max(hi, range_key(v));
+            }
+            if (mm != nullptr) {
+                atomicMax(&slo[f], lo);
+                atomicMax(&shi[f], hi);
+            }
+        }
+    } else {
+        for (int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; t < total;
+             t += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+            const int f = static_cast<int>(t % d);
+            xc[t] = narrow(scale_by(__dsub_rn(widen(x[t]), mean[f]), inv_std[f]));
+        }
+    }
+    if (mm != nullptr) {
+        __syncthreads();
+        for (int f = threadIdx.x; f < d; f += blockDim.x) {
+            atomicMax(&mm[2 * f], slo[f]);
+            atomicMax(&mm[2 * f + 1], shi[f]);
+        }
     }
 }
 
@@ -126,7 +167,8 @@ constexpr int kSmallRows = 8192;
 constexpr int kSmallThreads = 256;
 __global__ void __launch_bounds__(kSmallThreads)
 center_small_kernel(const float* __restrict__ x, int n, int d, int normalize, double* __restrict__ partial,
-                    double* __restrict__ mean, double* __restrict__ inv_std, float* __restrict__ xc) {
+                    double* __restrict__ mean, double* __restrict__ inv_std, float* __restrict__ xc,
+                    unsigned* __restrict__ mm) {
     extern __shared__ float col[];
     __shared__ double part[kSmallRows / kCenterChunk];
     __shared__ double stat[2];
@@ -170,9 +212,21 @@ center_small_kernel(const float* __restrict__ x, int n, int d, int normalize, do
         __syncthreads();
     }
     const double m = stat[0], v = stat[1];
-    for (int i = tid; i < n; i += kSmallThreads)
-        xc[static_cast<int64_t>(i) * d + f] = __double2float_rn(
-            __dmul_rn(__dsub_rn(static_cast<double>(col[i + i / kCenterChunk]), m), v));
+    unsigned lo = 0u, hi = 0u;
+    for (int i = tid; i < n; i += kSmallThreads) {
+        const float c = narrow(scale_by(__dsub_rn(widen(col[i + i / kCenterChunk]), m), v));
+        xc[static_cast<int64_t>(i) * d + f] = c;
+        lo = max(lo, ~range_key(c));
+        hi = max(hi, range_key(c));
+    }
+    if (mm != nullptr) {
+        lo = __reduce_max_sync(0xffffffffu, lo);
+        hi = __reduce_max_sync(0xffffffffu, hi);
+        if ((tid & 31) == 0) {
+            atomicMax(&mm[2 * f], lo);
+            atomicMax(&mm[2 * f + 1], hi);
+        }
+    }
 }
 
 // norms[i] = (float) sum_f (double) xc[i,f]^2 (feature order), and the
@@ -185,8 +239,8 @@ __global__ void norms_kernel(const float* __restrict__ xc, int64_t n, int d,
         const float* row = xc + i * d;
         double s = 0.0;
         for (int f = 0; f < d; ++f) {
-            const double v = static_cast<double>(row[f]);
-            s = __dadd_rn(s, __dmul_rn(v, v));
+            const double v = widen(row[f]);
+            s = __fma_rn(v, v, s);  // (the square of a float is exact in double)
         }
         const float nf = __double2float_rn(s);
         norms[i] = nf;
@@ -208,14 +262,15 @@ int grid_for(int64_t items, int block, int max_blocks = 152 * 16) {
 }  // namespace
 
 void center(const float* x, int64_t n, int d, bool normalize, float* xc, double* partial,
-            double* mean, double* inv_std, cudaStream_t s) {
+            double* mean, double* inv_std, cudaStream_t s, unsigned* mm) {
+    if (d > kMaxRangeDims) mm = nullptr;
     const int64_t chunks = ceil_div(n, kCenterChunk);
     const int64_t items = chunks * d;
     // up to 8,192 rows (the column's shared memory) and 131,072 values (a
     // column's strided reads cost whole sectors)
     if (n <= kSmallRows && n * d <= (1 << 17)) {
         center_small_kernel<<<d, kSmallThreads, sizeof(float) * static_cast<size_t>(n + chunks), s>>>(
-            x, static_cast<int>(n), d, normalize ? 1 : 0, partial, mean, inv_std, xc);
+            x, static_cast<int>(n), d, normalize ? 1 : 0, partial, mean, inv_std, xc, mm);
         CG_LAUNCH_CHECK();
         return;
     }
@@ -231,13 +286,12 @@ void center(const float* x, int64_t n, int d, bool normalize, float* xc, double*
         center_finalize_kernel<<<d, 256, 0, s>>>(partial, chunks, d, n, 1, mean, inv_std);
         CG_LAUNCH_CHECK();
     }
-    center_apply_kernel<<<grid_for(n * d, 256), 256, 0, s>>>(x, n, d, mean, inv_std, xc);
+    center_apply_kernel<<<grid_for(n * d, kApplyThreads, 152 * 8), kApplyThreads, 0, s>>>(x, n, d, mean, inv_std, xc, mm);
     CG_LAUNCH_CHECK();
 }
 
 void squared_norms(const float* xc, int64_t n, int d, float* norms, unsigned int* max_norm_bits,
                    cudaStream_t s) {
-    if (max_norm_bits != nullptr) CG_CUDA(cudaMemsetAsync(max_norm_bits, 0, sizeof(unsigned int), s));
     norms_kernel<<<grid_for(n, 256), 256, 0, s>>>(xc, n, d, norms, max_norm_bits);
     CG_LAUNCH_CHECK();
 }

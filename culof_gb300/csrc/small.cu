@@ -212,22 +212,29 @@ __device__ __forceinline__ float box_extent(const float* __restrict__ b, int dp)
 // every other tile (mt^2 comparisons).
 __global__ void __launch_bounds__(256) tile_order_kernel(const float* __restrict__ boxes, int dp, int t0, int mt,
                                                          int* __restrict__ order) {
+    // 32 tiles per block, eight threads per tile for an eighth of the others each
     __shared__ float other[256];
+    __shared__ int ranks[32];
     const auto extent = [&](int t) { return box_extent(boxes + static_cast<int64_t>(t0 + t) * 2 * dp, dp); };
-    const int t = blockIdx.x * 256 + threadIdx.x;
+    const int lane = threadIdx.x & 31, part = threadIdx.x >> 5;
+    const int t = blockIdx.x * 32 + lane;
     const float mine = t < mt ? extent(t) : 0.0f;
+    if (part == 0) ranks[lane] = 0;
     int rank = 0;
     for (int c0 = 0; c0 < mt; c0 += 256) {
         __syncthreads();
         if (c0 + static_cast<int>(threadIdx.x) < mt) other[threadIdx.x] = extent(c0 + threadIdx.x);
         __syncthreads();
-        const int c1 = min(256, mt - c0);
-        for (int i = 0; i < c1; ++i) {
+        const int c1 = min(32 * (part + 1), mt - c0);
+        for (int i = 32 * part; i < c1; ++i) {
             const float v = other[i];
             rank += (v > mine || (v == mine && c0 + i < t)) ? 1 : 0;
         }
     }
-    if (t < mt) order[rank] = t;
+    __syncthreads();
+    atomicAdd(&ranks[lane], rank);
+    __syncthreads();
+    if (part == 0 && t < mt) order[ranks[lane]] = t;
 }
 
 // ---------------------------------------------------------------- window
@@ -1101,24 +1108,23 @@ void small_build_tiles(const float* xc, int64_t n, int d, const unsigned* perm, 
 
 size_t small_iso_bytes(int mt, int k) {
     const size_t cap = static_cast<size_t>(iso_capacity(mt));
-    return 256 + sizeof(uint64_t) * cap * 32 * (k <= 32 ? 1 : 2) + sizeof(int) * (cap + mt);
+    return sizeof(uint64_t) * cap * 32 * (k <= 32 ? 1 : 2) + sizeof(int) * (cap + mt);
 }
 
 void small_knn(const float* tiles, const float* boxes, const void* qbox, const unsigned* perm, int64_t n, int d, int nt,
-               int t0, int mt, int k, int sms, bool defer_rows, int segment, void* iso, int32_t* nbr_idx, float* nbr_d2,
+               int t0, int mt, int k, int sms, bool defer_rows, int segment, void* iso, int* iso_count, int32_t* nbr_idx, float* nbr_d2,
                float* kdist2, int* status, unsigned long long* evaluated, cudaStream_t s) {
     if (mt <= 0) return;
     SmallArgs A{tiles, boxes, static_cast<const __nv_bfloat16*>(qbox), perm, n, nt, t0, mt, k, sms,
                 segment, defer_rows && nt > kWindow && nt <= kIsoMaxTiles, nullptr, {}, nbr_idx, nbr_d2, kdist2, status,
                 evaluated, s};
     char* w = static_cast<char*>(iso);
-    A.iso.count = reinterpret_cast<int*>(w);
-    A.iso.list = reinterpret_cast<uint64_t*>(w + 256);
-    A.iso.pos = reinterpret_cast<int*>(w + 256 + sizeof(uint64_t) * static_cast<size_t>(iso_capacity(mt)) * 32 * (k <= 32 ? 1 : 2));
-    if (A.defer) CG_CUDA(cudaMemsetAsync(A.iso.count, 0, sizeof(int), s));
+    A.iso.count = iso_count;
+    A.iso.list = reinterpret_cast<uint64_t*>(w);
+    A.iso.pos = reinterpret_cast<int*>(w + sizeof(uint64_t) * static_cast<size_t>(iso_capacity(mt)) * 32 * (k <= 32 ? 1 : 2));
     if (mt <= kOrderMaxTiles) {
         int* order = A.iso.pos + iso_capacity(mt);
-        tile_order_kernel<<<static_cast<unsigned>(ceil_div(mt, 256)), 256, 0, s>>>(boxes, padded_dims(d), t0, mt, order);
+        tile_order_kernel<<<static_cast<unsigned>(ceil_div(mt, 32)), 256, 0, s>>>(boxes, padded_dims(d), t0, mt, order);
         CG_LAUNCH_CHECK();
         A.order = order;
     } else {

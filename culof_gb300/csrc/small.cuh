@@ -63,10 +63,11 @@ void small_build_tiles(const float* xc, int64_t n, int d, const unsigned* perm, 
 size_t small_iso_bytes(int mt, int k);
 // Exact k-NN of the rows of row tiles [t0, t0 + mt), written in the
 // reference's slot order. evaluated (nullable) counts (row, half) pairs
-// past the seed window; iso is small_iso_bytes(mt, k) bytes; segment (at most
+// past the seed window; iso is small_iso_bytes(mt, k) bytes,
+// *iso_count zero; segment (at most
 // kSegTiles) column tiles are listed at a time.
 void small_knn(const float* tiles, const float* boxes, const void* qbox, const unsigned* perm, int64_t n, int d, int nt,
-               int t0, int mt, int k, int sms, bool defer_rows, int segment, void* iso, int32_t* nbr_idx, float* nbr_d2,
+               int t0, int mt, int k, int sms, bool defer_rows, int segment, void* iso, int* iso_count, int32_t* nbr_idx, float* nbr_d2,
                float* kdist2, int* status, unsigned long long* evaluated, cudaStream_t s);
 
 }  // namespace culof_gb300

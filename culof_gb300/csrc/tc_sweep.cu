@@ -53,6 +53,7 @@
 #include "common.cuh"
 #include "engine.cuh"
 #include "fast.cuh"
+#include "prep.cuh"
 #include "row_list.cuh"
 #include "sweep_common.cuh"
 #include "tc.cuh"
@@ -81,17 +82,18 @@ __device__ __forceinline__ float unflip(unsigned k) {
     return __uint_as_float((k & 0x80000000u) ? (k & 0x7FFFFFFFu) : ~k);
 }
 
-// One thread: the scale exponent from the per-dimension min/max keys of the
-// spatial-order pass.
+// One warp: the scale exponent from the features' ranges.
 __global__ void tc_scale_kernel(const unsigned* __restrict__ mm, int d, TcScale* __restrict__ out) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
     float mx = 0.0f;
     bool finite = true;
-    for (int f = 0; f < d; ++f) {
-        const float lo = unflip(mm[2 * f]), hi = unflip(mm[2 * f + 1]);
+    for (int f = threadIdx.x; f < d; f += 32) {
+        const float lo = range_lo(mm, f), hi = range_hi(mm, f);
         finite = finite && isfinite(lo) && isfinite(hi);
         mx = fmaxf(mx, fmaxf(fabsf(lo), fabsf(hi)));
     }
+    mx = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(mx)));
+    finite = __all_sync(0xffffffffu, finite);
+    if (threadIdx.x != 0) return;
     int S = 0;
     bool all = !finite;
     if (finite && mx > 0.0f) {
