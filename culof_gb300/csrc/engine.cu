@@ -129,17 +129,29 @@ int Engine::tile_rows_for(int64_t n) {
     return choose_tile_rows(n, usable < cap ? usable : cap);
 }
 
-// AUTO: the general tile + select path for n <= 4096 (a few kernels against
-// the fused paths' ~45; fit_predict on the device, d = 8, k = 20: n = 1000,
-// 0.18 ms against 0.38 ms; n = 4000, 0.39 against 0.58 ms; n = 8000, 1.02
-// against 0.62 ms) and beyond the fused paths' limits (d > 128 or k > 64);
-// otherwise the FP32 fused
-// sweep for d <= 8 and the tensor-core sweep for 8 < d <= 128 (the FP32 wide
-// sweep for d <= 16 below one wave of row tiles). All give the same bits.
+// AUTO, with the direct two-pass kernel (direct.cu) wherever it is fastest; all
+// give the same bits. lof_device on clusters, k = 20, one call, in us:
+//   d        n     direct  small-d   tensor   tile + select
+//   8     4000        128      278
+//   8     8000        329      327             (direct up to 7168 points)
+//  12     4000        180               204
+//  12     8000        480               261    (direct up to 4096 points)
+//  24     3000                          206             217
+//  24     2000                          194             146  (tensor from 2561)
+// 128     4000                          251             541
+// - n <= 4096 (2560 for d > 16): the general path, which takes the direct
+//   kernel for d <= 16 and k <= 64;
+// - d <= 8: the FP32 path (direct up to 7168 points, then the small-d sweep);
+//   8 < d <= 16 up to 7168 points: the FP32 path by the direct kernel too,
+//   which ties the tensor path there and keeps every stage in FP32;
+// - otherwise the tensor path up to d = 256, the general path beyond and for
+//   k > 64.
 // CULOF_GB300_PATH=general|fast|tensor overrides AUTO for a process.
-constexpr int64_t kSmallN = 4096;
-int Engine::choose_path(int64_t n, int d, int k) const {
+constexpr int64_t kSmallN = 4096, kSmallWideN = 2560, kDirectFastN = 7168;
+constexpr int64_t kDirectGeneralN = 8192;
+int Engine::choose_path(int64_t n, int d, int k, bool* direct) const {
     int p = path_;
+    *direct = false;
     if (p == kPathAuto) {
         if (const char* env = std::getenv("CULOF_GB300_PATH")) {
             if (env[0] == 'g') p = kPathGeneral;
@@ -148,25 +160,18 @@ int Engine::choose_path(int64_t n, int d, int k) const {
         }
     }
     const bool ok = fast_path_supported(n, d, k);
-    if (p == kPathGeneral) return kPathGeneral;
     if ((p == kPathFast || p == kPathTensor) && !ok)
         throw Error(kInvalidArgument, "fused path requested but unsupported for this n/d/k");
     if (p == kPathFast || p == kPathTensor) return p;
-    if (!ok || n <= kSmallN) return kPathGeneral;
-    // d <= 8: the FP32 small-d sweep at every k (fit_predict on clusters
-    // against the tensor sweep over the same seed window and prune lists:
-    // k = 64, n = 20k / 50k / 200k: 1.42 / 3.13 / 17.6 against 3.38 / 6.90 /
-    // 25.2 ms; k = 48, 200k: 16.3 against 18.8 ms)
-    if (d <= 8) return kPathFast;
-    // 8 < d <= 16 with fewer row tiles than SMs: the FP32 wide sweep ties the
-    // tensor path (n = 20k, d = 16: 1.91 against 1.87 ms); from there up the
-    // tensor path wins (n = 30k: 2.33 against 2.80 ms; 38k: 3.01 against
-    // 3.79 ms), and at every size for d > 16 (d = 24, n = 20k: 1.81 against
-    // 2.31 ms; d = 32, n = 10k: 1.15 against 1.45 ms)
-    int sms = 0;
-    CG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device_));
-    const int64_t nt = (n + 127) / 128;
-    if (d <= 16 && nt < static_cast<int64_t>(sms)) return kPathFast;
+    const bool direct_ok = direct_supported(n, d, k);
+    if (p == kPathGeneral || n <= (d > 16 ? kSmallWideN : kSmallN) || !tensor_supported(n, d, k)) {
+        *direct = direct_ok && n <= kDirectGeneralN;
+        return kPathGeneral;
+    }
+    if (d <= 8 || (d <= 16 && n <= kDirectFastN)) {
+        *direct = direct_ok && n <= kDirectFastN;
+        return kPathFast;
+    }
     return kPathTensor;
 }
 
@@ -208,13 +213,15 @@ int64_t Engine::knn_core(const float* d_x, int64_t n, int d, int k, bool normali
     stat_total_pairs_ = 0.0;
     for (bool& m : marked_) m = false;
     mark(0);
-    const int path = choose_path(n, d, k);
-    center(d_x, n, d, normalize, xc, partial, mean, inv, stream_, path != kPathGeneral ? range_words() : nullptr);
+    bool direct = false;
+    const int path = choose_path(n, d, k, &direct);
+    const bool fused = path != kPathGeneral && !direct;
+    center(d_x, n, d, normalize, xc, partial, mean, inv, stream_, fused ? range_words() : nullptr);
     // only the filters of the wide and tensor sweeps read the norms
-    if (path == kPathTensor || (path == kPathFast && d > 8)) squared_norms(xc, n, d, norms, max_norm_word(), stream_);
+    if (fused && (path == kPathTensor || d > 8)) squared_norms(xc, n, d, norms, max_norm_word(), stream_);
     int64_t count = n;
-    if (path != kPathGeneral) {
-        last_path_ = path;
+    last_path_ = path;
+    if (fused) {
         mark(1);
         knn_fast(xc, norms, n, d, k, path == kPathTensor, nbr_idx, nbr_d2, kdist2, shard, num_shards, rows);
         if (num_shards > 1) {  // whole row tiles of 128 points
@@ -223,13 +230,13 @@ int64_t Engine::knn_core(const float* d_x, int64_t n, int d, int k, bool normali
             count = std::min<int64_t>(n, t1 * 128) - std::min<int64_t>(n, t0 * 128);
         }
     } else {
-        last_path_ = kPathGeneral;
         mark(1);
         mark(2);
         mark(3);
-        // a shard of the general path: a block of original rows
+        // a shard of the general path (or of the direct kernel): a block of original rows
         const int64_t b = n * shard / num_shards, e = n * (shard + 1) / num_shards;
-        knn_general(xc, norms, n, d, k, nbr_idx, nbr_d2, kdist2, b, e);
+        if (direct) direct_knn(xc, n, d, b, e, k, nbr_idx, nbr_d2, kdist2, stream_);
+        else knn_general(xc, norms, n, d, k, nbr_idx, nbr_d2, kdist2, b, e);
         if (rows && e > b) iota_rows(rows, b, e - b, stream_);
         count = e - b;
         mark(4);

@@ -135,7 +135,7 @@ private:
     bool batch_same_plan(int num, const int64_t* offsets, const int* ks, int d, bool normalize) const;
     void batch_launch(const float* d_x, float* d_scores);
     void batch_autotune(const float* d_x, float* d_scores);
-    int choose_path(int64_t n, int d, int k) const;
+    int choose_path(int64_t n, int d, int k, bool* direct) const;
     void knn_general(const float* xc, const float* norms, int64_t n, int d, int k, int32_t* nbr_idx,
                      float* nbr_d2, float* kdist2, int64_t row_begin, int64_t row_end);
     void knn_fast(const float* xc, const float* norms, int64_t n, int d, int k, bool tensor, int32_t* nbr_idx,

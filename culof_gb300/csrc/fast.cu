@@ -70,9 +70,9 @@ __global__ void morton_kernel(const float* __restrict__ xc, int64_t n, int d, co
     const int bits = (32 / md) < 30 ? (32 / md) : 30;
     if (threadIdx.x < 32) {
         const int lane = threadIdx.x;
-        float span[kMaxWideD / 32];
+        float span[kMaxTensorD / 32];
 #pragma unroll
-        for (int j = 0; j < kMaxWideD / 32; ++j) {
+        for (int j = 0; j < kMaxTensorD / 32; ++j) {
             const int f = 32 * j + lane;
             span[j] = f < d ? range_hi(mm, f) - range_lo(mm, f) : -1.0f;
         }
@@ -80,7 +80,7 @@ __global__ void morton_kernel(const float* __restrict__ xc, int64_t n, int d, co
             float best = -1.0f;
             int at = d;
 #pragma unroll
-            for (int j = 0; j < kMaxWideD / 32; ++j)
+            for (int j = 0; j < kMaxTensorD / 32; ++j)
                 if (span[j] > best) {
                     best = span[j];
                     at = 32 * j + lane;
@@ -96,7 +96,7 @@ __global__ void morton_kernel(const float* __restrict__ xc, int64_t n, int d, co
             }
             if (at >= d) at = q;  // (ranges that are not numbers: any feature)
 #pragma unroll
-            for (int j = 0; j < kMaxWideD / 32; ++j)
+            for (int j = 0; j < kMaxTensorD / 32; ++j)
                 if (32 * j + lane == at) span[j] = -2.0f;
             if (lane == 0) {
                 dims[q] = at;
@@ -654,6 +654,10 @@ void exclusive_scan_u32(unsigned* data, int64_t len, cudaStream_t s) {
 bool fast_path_supported(int64_t n, int d, int k) {
     return d >= 1 && d <= kMaxWideD && k >= 1 && k <= kMaxK && n >= 2 && static_cast<int64_t>(k) < n &&
            n <= (static_cast<int64_t>(1) << 30);
+}
+
+bool tensor_supported(int64_t n, int d, int k) {
+    return d >= 1 && d <= kMaxTensorD && fast_path_supported(n, 1, k);
 }
 
 // Host orchestration of the fast path.

@@ -10,6 +10,12 @@ namespace culof_gb300 {
 // True when the fast path handles (n, d, k).
 bool fast_path_supported(int64_t n, int d, int k);
 
+// Small inputs (direct.cu): the k nearest of rows [row_begin, row_end) among
+// all n points by two passes over the columns.
+bool direct_supported(int64_t n, int d, int k);
+void direct_knn(const float* xc, int64_t n, int d, int64_t row_begin, int64_t row_end, int k, int32_t* idx, float* d2,
+                float* kd, cudaStream_t s);
+
 // The wide-point variant (8 < d <= 128), wide.cu.
 int wide_dims_padded(int d);
 size_t wide_tiles_floats(int d, int nt);
@@ -64,6 +70,9 @@ size_t tc_buffer_bytes(int64_t padded, int d);
 TcBuffers tc_prepare(void* buf, const float* xc, const float* norms, int64_t n, int d, const unsigned* perm, int nt,
                      const unsigned* minmax, cudaStream_t s);
 int tc_max_splits();
+constexpr int kMaxTensorD = 256;
+// True when the tensor path handles (n, d, k) (AUTO only above d = 128).
+bool tensor_supported(int64_t n, int d, int k);
 // Workspace of the per-row lists of one sweep launch batch.
 size_t tc_list_bytes(int nt, int nsplit);
 // The sweep and the rows' final results (k best of the seed's lists and the

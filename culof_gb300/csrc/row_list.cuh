@@ -69,6 +69,33 @@ __device__ __forceinline__ void list_add(uint64_t (&b)[KR], uint64_t key, unsign
     }
 }
 
+// The element of rank r (0-based) of 32 * G values, G per lane.
+template <int G>
+__device__ __forceinline__ unsigned warp_rank_value(unsigned (&v)[G], int r) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int size = 2; size <= 32 * G; size <<= 1) {
+#pragma unroll
+        for (int st = size >> 1; st > 0; st >>= 1) {
+            if (st == 32) {
+                const unsigned a = v[0], c = v[G - 1];
+                v[0] = min(a, c);
+                v[G - 1] = max(a, c);
+            } else {
+#pragma unroll
+                for (int j = 0; j < G; ++j) {
+                    const unsigned o = __shfl_xor_sync(kFullMask, v[j], st);
+                    const bool asc = ((j * 32 + lane) & size) == 0, lower = (lane & st) == 0;
+                    v[j] = lower == asc ? min(v[j], o) : max(v[j], o);
+                }
+            }
+        }
+    }
+    unsigned x = __shfl_sync(kFullMask, v[0], r & 31);
+    if (G == 2 && r >= 32) x = __shfl_sync(kFullMask, v[G - 1], r & 31);
+    return x;
+}
+
 // The bits of a list's k-th distance (all ones while it holds fewer than k
 // keys), and the distance (+inf then).
 template <int KR>

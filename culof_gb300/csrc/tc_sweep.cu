@@ -1,11 +1,11 @@
 // The fused distance + filtered exact select on the tensor cores
-// (8 < d <= 128): the same algorithm as the FP32 sweeps (fast.cu, wide.cu),
+// (8 < d <= 256): the same algorithm as the FP32 sweeps (fast.cu, wide.cu),
 // with the per-pair filter value taken from an FP16 Gram tile computed by
 // tcgen05.mma instead of an FP32 FMA chain.
 //
 //   * operands: the centred points in Morton order, scaled by a power of two
 //     2^S (so the largest coordinate lands in [2^14, 2^15)) and rounded to
-//     f16, row-major [padded][Kp] (Kp = 64 or 128, zero padded);
+//     f16, row-major [padded][Kp] (Kp = 64, 128, 192 or 256, zero padded);
 //   * a CTA owns a 128-row tile (its A operand stays in shared memory) and
 //     streams 128-column tiles of the same array by TMA (two stages);
 //   * one warp issues the TMA loads, one issues tcgen05.mma (M = N = 128,
@@ -257,21 +257,26 @@ constexpr int kTcListRow = kTcM;
 constexpr size_t kTcListTile = static_cast<size_t>(kRT) * kTcListRow;  // keys per row tile
 constexpr int kTcMaxTilesPerLaunch = 4096;                             // bounds the list workspace (512 MiB)
 
-struct TcSmem {
-    uint8_t a[2][kBox];           // row tile operand (K boxes 0..1)
-    uint8_t b[kStages][2][kBox];  // column tile operands
+struct TcRows {
     uint64_t kth[kRT];            // exact k-th key known for the row (only decreases)
     float athr[kRT];              // approximate threshold of the row's list (+inf until k entries)
     float c0[kRT], c3[kRT], c4[kRT];  // RowBounds
     int cnt[kRT];
     int sorted[kRT];  // the row's list[0..sorted) is sorted (the last compaction's result)
     int mode[kRT];
+    int abort;
+};
+// NB: operand boxes of 64 K values (2: d <= 128, two CTAs per SM; 4: d <= 256,
+// one).
+template <int NB>
+struct TcSmem : TcRows {
+    alignas(1024) uint8_t a[NB][kBox];  // row tile operand
+    uint8_t b[kStages][NB][kBox];       // column tile operands
     float nb[kEpiWarps][2][kCT];  // column norms of the current and the next tile, per epilogue warp
     uint64_t full[kStages], empty[kStages], tfull[2], tempty[2], afull, fin;
     uint32_t tmem_base;
-    int abort;
 };
-static_assert(2 * (sizeof(TcSmem) + 1024 + 1024) <= 233472, "two tensor-sweep CTAs must fit on an SM");
+static_assert(2 * (sizeof(TcSmem<2>) + 1024 + 1024) <= 233472, "two tensor-sweep CTAs must fit on an SM");
 
 // What a row leaves to the final kernel, beside its list.
 struct TcRow {
@@ -279,11 +284,11 @@ struct TcRow {
     float c3, c4;
 };
 
-__device__ void tc_abort(TcSmem& sh, int* status) {
+__device__ void tc_abort(TcRows& sh, int* status) {
     *reinterpret_cast<volatile int*>(&sh.abort) = 1;
     atomicExch(status, 1);
 }
-__device__ __forceinline__ bool tc_aborted(TcSmem& sh) { return *reinterpret_cast<volatile int*>(&sh.abort) != 0; }
+__device__ __forceinline__ bool tc_aborted(TcRows& sh) { return *reinterpret_cast<volatile int*>(&sh.abort) != 0; }
 
 // g[b] for a lane-dependent b, without local memory: a 5-level select tree.
 __device__ __forceinline__ uint32_t select32(const uint32_t (&g)[32], int b) {
@@ -327,7 +332,7 @@ static_assert(kListE == 4, "the compaction sorts 4 keys per lane");
 
 // Exact list of row r (whole warp): sort, drop duplicates, keep the k
 // smallest; tighten the row's exact k-th key.
-__noinline__ __device__ void compact_exact(TcSmem& sh, uint64_t* __restrict__ lst, int r, int k) {
+__noinline__ __device__ void compact_exact(TcRows& sh, uint64_t* __restrict__ lst, int r, int k) {
     const int lane = threadIdx.x & 31;
     const int c = min(sh.cnt[r], kTcListRow);
     {
@@ -374,7 +379,7 @@ __noinline__ __device__ void compact_exact(TcSmem& sh, uint64_t* __restrict__ ls
 // and keep the entries with f <= approx_thr(fk) (all of them while fewer than
 // k are known). Returns the number kept; if that exceeds `cap`, the list is
 // left untrimmed and the caller decides.
-__noinline__ __device__ int approx_compact(TcSmem& sh, uint64_t* __restrict__ lst, int r, int k, float c2, float c3,
+__noinline__ __device__ int approx_compact(TcRows& sh, uint64_t* __restrict__ lst, int r, int k, float c2, float c3,
                                            float c4, int cap) {
     const int lane = threadIdx.x & 31;
     const int c = min(sh.cnt[r], kTcListRow);
@@ -445,7 +450,7 @@ __noinline__ __device__ int approx_compact(TcSmem& sh, uint64_t* __restrict__ ls
 // Row r leaves approximate mode (its list would overflow with entries within
 // the approximate margin, e.g. many duplicates): every entry is rescored
 // exactly (one lane per entry) and the list becomes an exact k-best list.
-__noinline__ __device__ void to_exact_mode(TcSmem& sh, uint64_t* __restrict__ lst, int r, int64_t pa,
+__noinline__ __device__ void to_exact_mode(TcRows& sh, uint64_t* __restrict__ lst, int r, int64_t pa,
                                            const float* __restrict__ xr, const unsigned* __restrict__ ix, int d,
                                            int dr, int k) {
     const int lane = threadIdx.x & 31;
@@ -467,7 +472,7 @@ __noinline__ __device__ void to_exact_mode(TcSmem& sh, uint64_t* __restrict__ ls
 // columns, 0 for rows in approximate mode): per row, lane c rescores column
 // cbase + c exactly and the keys that beat the list's k-th key join it. True
 // if a list was compacted.
-__noinline__ __device__ bool exact_chunk(TcSmem& sh, uint64_t* __restrict__ glist, int list0, unsigned pass,
+__noinline__ __device__ bool exact_chunk(TcRows& sh, uint64_t* __restrict__ glist, int list0, unsigned pass,
                                          int64_t pa0, int64_t cbase, const float* __restrict__ xr,
                                          const unsigned* __restrict__ ix, int d, int dr, int k) {
     const int lane = threadIdx.x & 31;
@@ -505,7 +510,8 @@ __noinline__ __device__ bool exact_chunk(TcSmem& sh, uint64_t* __restrict__ glis
 // 1.29, 1.22 ms).
 __device__ __forceinline__ int bound_tiles(int count) { return min(count, max(128, count / 4)); }
 
-__global__ void __launch_bounds__(kTcThreads, 2)
+template <int NB>
+__global__ void __launch_bounds__(kTcThreads, NB == 2 ? 2 : 1)
 tc_sweep_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ CUtensorMap tmapb,
                 const float* __restrict__ xr,
                 const float* __restrict__ cn, const unsigned* __restrict__ ix, const TcScale* __restrict__ scale,
@@ -514,7 +520,7 @@ tc_sweep_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
                 uint64_t* __restrict__ lists, TcRow* __restrict__ row_info, int* __restrict__ status, int qs,
                 const uint2* __restrict__ plist, const int* __restrict__ pcount) {
     extern __shared__ uint8_t tc_raw[];
-    TcSmem& sh = *reinterpret_cast<TcSmem*>((reinterpret_cast<uintptr_t>(tc_raw) + 1023) & ~uintptr_t(1023));
+    TcSmem<NB>& sh = *reinterpret_cast<TcSmem<NB>*>((reinterpret_cast<uintptr_t>(tc_raw) + 1023) & ~uintptr_t(1023));
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int T = T0 + static_cast<int>(blockIdx.x) % ntb;
     const int split = static_cast<int>(blockIdx.x) / ntb;
@@ -863,7 +869,7 @@ tc_final_kernel(const float* __restrict__ xr, const unsigned* __restrict__ ix, i
                 int dr, int k, int kx, float c2, const uint64_t* __restrict__ lists, const TcRow* __restrict__ row_info,
                 const uint64_t* __restrict__ seed_keys, int32_t* __restrict__ nbr_idx, float* __restrict__ nbr_d2,
                 float* __restrict__ kdist2) {
-    __shared__ __align__(16) float row[kFinWarps][128];
+    __shared__ __align__(16) float row[kFinWarps][kMaxTensorD];
     __shared__ unsigned cand[kFinWarps][kMaxTcSplits * kTcListRow];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int local = blockIdx.x * kFinWarps + warp;  // row of the launch batch
@@ -958,7 +964,7 @@ static bool tc_use_split(int d) {
 }
 static int tc_kp(int d, bool split) {
     const int w = split ? 3 * d : d;
-    return w <= 64 ? 64 : 128;
+    return (w + 63) / 64 * 64;
 }
 
 size_t tc_buffer_bytes(int64_t padded, int d) {
@@ -988,7 +994,7 @@ TcBuffers tc_prepare(void* buf, const float* xc, const float* norms, int64_t n, 
     const bool split = tc_use_split(d);
     b.split = split ? 1 : 0;
     b.Kp = tc_kp(d, split);
-    b.ksteps = split ? (3 * d + 15) / 16 : b.Kp / 16;
+    b.ksteps = ((split ? 3 * d : d) + 15) / 16;
     b.dr = (d + 3) & ~3;
     char* p = static_cast<char*>(buf);
     b.xh = p;
@@ -1021,8 +1027,10 @@ void tc_sweep(const TcBuffers& b, int64_t n, int nt, int t0, int mt, int nsplit,
               const unsigned long long* kth_seed, const uint64_t* seed_keys, uint64_t* lists, int* status,
               int32_t* nbr_idx, float* nbr_d2, float* kdist2, cudaStream_t s, int qs, const uint2* plist,
               const int* pcount) {
-    const size_t smem = sizeof(TcSmem) + 1024;
-    set_max_dynamic_smem(reinterpret_cast<const void*>(tc_sweep_kernel), static_cast<int>(smem));
+    const bool wide = b.Kp > 128;
+    const size_t smem = (wide ? sizeof(TcSmem<4>) : sizeof(TcSmem<2>)) + 1024;
+    const auto kernel = wide ? tc_sweep_kernel<4> : tc_sweep_kernel<2>;
+    set_max_dynamic_smem(reinterpret_cast<const void*>(kernel), static_cast<int>(smem));
     const CUtensorMap map = tc::make_kmajor_map(b.xh, static_cast<int64_t>(nt) * kCT, b.Kp, true);
     const CUtensorMap mapb = tc::make_kmajor_map(b.xb, static_cast<int64_t>(nt) * kCT, b.Kp, true);
     TcRow* info = reinterpret_cast<TcRow*>(lists + kTcListTile * static_cast<size_t>(tc_list_tiles(mt, nsplit)));
@@ -1032,7 +1040,7 @@ void tc_sweep(const TcBuffers& b, int64_t n, int nt, int t0, int mt, int nsplit,
     const int ntb_max = kTcMaxTilesPerLaunch / nsplit;
     for (int T0 = t0; T0 < t0 + mt; T0 += ntb_max) {
         const int ntb = t0 + mt - T0 < ntb_max ? t0 + mt - T0 : ntb_max;
-        tc_sweep_kernel<<<ntb * nsplit, kTcThreads, smem, s>>>(
+        kernel<<<ntb * nsplit, kTcThreads, smem, s>>>(
             map, mapb, b.xr, b.cn, b.ix, reinterpret_cast<const TcScale*>(b.scale), nt, T0, ntb, nsplit, d, b.dr, b.Kp,
             b.split, b.ksteps, k, c1, c2, maxn, kth_seed, lists, info, status, qs, plist, pcount);
         CG_LAUNCH_CHECK();
