@@ -21,6 +21,7 @@
 #include "common.cuh"
 #include "engine.cuh"
 #include "fast.cuh"
+#include "fp64.cuh"
 #include "prep.cuh"
 
 namespace culof_gb300 {
@@ -46,64 +47,99 @@ __device__ __forceinline__ int64_t warp_id() { return (static_cast<int64_t>(bloc
 __device__ __forceinline__ int64_t warp_count() { return (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5; }
 
 // d2[e] (e = t * n + i, the layout of the k-NN slots) in FP64 from the raw
-// points: (x_i - x_j) * inv_std, the mean cancels. A warp per point, lanes
-// over dimensions.
-__global__ void bw_pair_kernel(const float* __restrict__ x, int64_t n, int d, int k, const int32_t* __restrict__ nbr,
-                               const double* __restrict__ inv, double* __restrict__ d2, int* __restrict__ status) {
-    const int lane = threadIdx.x & 31;
-    for (int64_t i = warp_id(); i < n; i += warp_count()) {
+// points: (x_i - x_j) * inv_std, the mean cancels. A thread per slot, features
+// in order (blockIdx.y = t, neighbouring threads neighbouring points): two FP64
+// instructions per feature and 32 slots (three when normalising). A warp per
+// point with its lanes over the features needed ten per slot for its shuffle
+// sum, and FP64 issues once per 64 cycles and scheduler: 626 us at n = 50,000,
+// d = 32, k = 20.
+__global__ void __launch_bounds__(256) bw_pair_kernel(const float* __restrict__ x, int64_t n, int d,
+                                                      const int32_t* __restrict__ nbr, const double* __restrict__ inv,
+                                                      int normalize, int aligned, double* __restrict__ d2,
+                                                      int* __restrict__ status) {
+    const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const int64_t e = static_cast<int64_t>(blockIdx.y) * n + i;
+    const int32_t j = nbr[e];
+    double s = 0.0;
+    if (j < 0 || j >= n) {
+        flag_bad(status);
+    } else {
         const float* xi = x + i * d;
-        for (int t = 0; t < k; ++t) {
-            const int64_t e = static_cast<int64_t>(t) * n + i;
-            const int32_t j = nbr[e];
-            double s = 0.0;
-            if (j < 0 || j >= n) {
-                if (lane == 0) flag_bad(status);
-            } else {
-                const float* xj = x + static_cast<int64_t>(j) * d;
-                for (int f = lane; f < d; f += 32) {
-                    const double u = __dmul_rn(__dsub_rn(static_cast<double>(xi[f]), static_cast<double>(xj[f])), inv[f]);
+        const float* xj = x + static_cast<int64_t>(j) * d;
+        if (aligned) {  // rows on 16-byte boundaries
+            for (int f = 0; f < d; f += 4) {
+                const float4 p = *reinterpret_cast<const float4*>(xi + f), q = *reinterpret_cast<const float4*>(xj + f);
+                const float pv[4] = {p.x, p.y, p.z, p.w}, qv[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    double u = __dsub_rn(widen(pv[c]), widen(qv[c]));
+                    if (normalize) u = __dmul_rn(u, inv[f + c]);
                     s = __fma_rn(u, u, s);
                 }
             }
-            s = warp_sum(s);
-            if (lane == 0) d2[e] = s;
+        } else {
+            for (int f = 0; f < d; ++f) {
+                double u = __dsub_rn(widen(xi[f]), widen(xj[f]));
+                if (normalize) u = __dmul_rn(u, inv[f]);
+                s = __fma_rn(u, u, s);
+            }
         }
     }
+    d2[e] = s;
 }
 
-// Per point: reach distances of its slots, lrd. A warp per point, lanes over slots.
-__global__ void bw_lrd_kernel(int64_t n, int k, const int32_t* __restrict__ nbr, const double* __restrict__ d2,
-                              double* __restrict__ reach, double* __restrict__ lrd) {
-    const int lane = threadIdx.x & 31;
-    for (int64_t i = warp_id(); i < n; i += warp_count()) {
-        double R = 0.0;
-        for (int t = lane; t < k; t += 32) {
-            const int64_t e = static_cast<int64_t>(t) * n + i;
-            const int64_t j = clampj(nbr[e], n);
-            const double kd = d2[static_cast<int64_t>(k - 1) * n + j];
-            const double r = __dsqrt_rn(fmax(kd, d2[e]));
-            reach[e] = r;
-            R = __dadd_rn(R, r);
+// Per point: reach distances of its slots, lrd. A CTA of 8 warps takes 32
+// points (lane = point), the warps compute the slots side by side, 32 at a
+// time, and warp 0 adds them in slot order.
+__global__ void __launch_bounds__(256) bw_lrd_kernel(int64_t n, int k, const int32_t* __restrict__ nbr,
+                                                     const double* __restrict__ d2, double* __restrict__ reach,
+                                                     double* __restrict__ lrd) {
+    __shared__ double term[32][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t i = static_cast<int64_t>(blockIdx.x) * 32 + lane;
+    double R = 0.0;
+    for (int c0 = 0; c0 < k; c0 += 32) {
+        const int c1 = k - c0 < 32 ? k - c0 : 32;
+        for (int t = warp; t < c1; t += 8) {
+            double r = 0.0;
+            if (i < n) {
+                const int64_t e = static_cast<int64_t>(c0 + t) * n + i;
+                const int64_t j = clampj(nbr[e], n);
+                r = __dsqrt_rn(fmax(d2[static_cast<int64_t>(k - 1) * n + j], d2[e]));
+                reach[e] = r;
+            }
+            term[t][lane] = r;
         }
-        R = warp_sum(R);
-        if (lane == 0) lrd[i] = __ddiv_rn(1.0, __dadd_rn(__ddiv_rn(R, static_cast<double>(k)), 1e-10));
+        __syncthreads();
+        if (warp == 0)
+            for (int t = 0; t < c1; ++t) R = __dadd_rn(R, term[t][lane]);
+        __syncthreads();
     }
+    if (warp == 0 && i < n) lrd[i] = __ddiv_rn(1.0, __dadd_rn(__ddiv_rn(R, static_cast<double>(k)), 1e-10));
 }
 
-// Per point: S_i = sum_j lrd_j and the score. A warp per point.
+// Per point (a thread): S_i = sum_j lrd_j, the score, and w_i = g_i / (k lrd_i),
+// what the point adds to dL/dlrd of each of its neighbours.
 __global__ void bw_score_kernel(int64_t n, int k, const int32_t* __restrict__ nbr, const double* __restrict__ lrd,
-                                double* __restrict__ S, double* __restrict__ score) {
-    const int lane = threadIdx.x & 31;
-    for (int64_t i = warp_id(); i < n; i += warp_count()) {
-        double s = 0.0;
-        for (int t = lane; t < k; t += 32) s = __dadd_rn(s, lrd[clampj(nbr[static_cast<int64_t>(t) * n + i], n)]);
-        s = warp_sum(s);
-        if (lane == 0) {
-            S[i] = s;
-            if (score) score[i] = __ddiv_rn(s, __dmul_rn(static_cast<double>(k), lrd[i]));
-        }
+                                const double* __restrict__ g, double* __restrict__ S, double* __restrict__ w,
+                                double* __restrict__ score) {
+    const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    double s = 0.0;
+    for (int t0 = 0; t0 < k; t0 += 8) {  // eight gathers in flight
+        double v[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+            v[j] = t0 + j < k ? lrd[clampj(nbr[static_cast<int64_t>(t0 + j) * n + i], n)] : 0.0;
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+            if (t0 + j < k) s = __dadd_rn(s, v[j]);
     }
+    S[i] = s;
+    const double kl = __dmul_rn(static_cast<double>(k), lrd[i]);
+    w[i] = __ddiv_rn(g[i], kl);
+    if (score) score[i] = __ddiv_rn(s, kl);
 }
 
 // Transposed slot list: count slots per neighbour index (integer atomics,
@@ -119,47 +155,45 @@ __global__ void bw_rev_init_kernel(int64_t n, int64_t total, const int32_t* __re
     }
 }
 
-// dL/dlrd_m = -g_m S_m / (k lrd_m^2) + sum over reverse slots (i, t) of g_i / (k lrd_i).
-// (A warp per point, lanes over the reverse slots.)
-__global__ void bw_glrd_kernel(int64_t n, int k, const double* __restrict__ g, const double* __restrict__ lrd,
-                               const double* __restrict__ S, const unsigned* __restrict__ off,
-                               const unsigned* __restrict__ rev, double* __restrict__ glrd) {
-    const double dk = static_cast<double>(k);
+// Per point, over its reverse slots (i, t): the sum of w_i. (A warp per point,
+// lanes over the reverse slots.)
+__global__ void bw_gather_kernel(int64_t n, const double* __restrict__ w, const unsigned* __restrict__ off,
+                                 const unsigned* __restrict__ rev, double* __restrict__ acc_out) {
     const int lane = threadIdx.x & 31;
+    const unsigned n32 = static_cast<unsigned>(n);
     for (int64_t m = warp_id(); m < n; m += warp_count()) {
         double acc = 0.0;
-        for (unsigned p = off[m] + lane; p < off[m + 1]; p += 32) {
-            const int64_t i = static_cast<int64_t>(rev[p]) % n;
-            acc = __dadd_rn(acc, __ddiv_rn(g[i], __dmul_rn(dk, lrd[i])));
-        }
+        for (unsigned p = off[m] + lane; p < off[m + 1]; p += 32) acc = __dadd_rn(acc, w[rev[p] % n32]);
         acc = warp_sum(acc);
-        if (lane == 0) {
-            const double lm = lrd[m];
-            glrd[m] = __dadd_rn(-__ddiv_rn(__dmul_rn(g[m], S[m]), __dmul_rn(dk, __dmul_rn(lm, lm))), acc);
-        }
+        if (lane == 0) acc_out[m] = acc;
     }
+}
+
+// Per point (a thread): dL/dlrd_m = -g_m S_m / (k lrd_m^2) + the reverse sum,
+// and gR_m = -dL/dlrd_m lrd_m^2 / k, the gradient of its reach distances' sum.
+__global__ void bw_point_kernel(int64_t n, int k, const double* __restrict__ g, const double* __restrict__ lrd,
+                                const double* __restrict__ S, const double* __restrict__ acc, double* __restrict__ gR) {
+    const int64_t m = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (m >= n) return;
+    const double dk = static_cast<double>(k), lm = lrd[m], l2 = __dmul_rn(lm, lm);
+    const double glrd = __dadd_rn(-__ddiv_rn(__dmul_rn(g[m], S[m]), __dmul_rn(dk, l2)), acc[m]);
+    gR[m] = -__ddiv_rn(__dmul_rn(glrd, l2), dk);
 }
 
 // Per slot: the reach-distance gradient c = dL/dR_i / (2 reach), routed to
 // d2_ij (gd2) or to kd2_j (gkd).
-__global__ void bw_route_kernel(int64_t n, int k, const int32_t* __restrict__ nbr, const double* __restrict__ d2,
-                                const double* __restrict__ reach, const double* __restrict__ lrd,
-                                const double* __restrict__ glrd, double* __restrict__ gd2, double* __restrict__ gkd) {
-    const int64_t total = n * k;
-    const double dk = static_cast<double>(k);
-    for (int64_t e = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; e < total;
-         e += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-        const int64_t i = e % n;
-        const int64_t j = clampj(nbr[e], n);
-        const double li = lrd[i];
-        const double gR = -__ddiv_rn(__dmul_rn(glrd[i], __dmul_rn(li, li)), dk);
-        const double r = reach[e];
-        const double c = r > 0.0 ? __ddiv_rn(gR, __dmul_rn(2.0, r)) : 0.0;
-        const double kd = d2[static_cast<int64_t>(k - 1) * n + j];
-        const bool via_d2 = d2[e] > kd;
-        gd2[e] = via_d2 ? c : 0.0;
-        gkd[e] = via_d2 ? 0.0 : c;
-    }
+__global__ void bw_route_kernel(int64_t n, const int32_t* __restrict__ nbr, const double* __restrict__ d2,
+                                const double* __restrict__ kd2, const double* __restrict__ reach, const double* __restrict__ gR,
+                                double* __restrict__ gd2, double* __restrict__ gkd) {
+    const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const int64_t e = static_cast<int64_t>(blockIdx.y) * n + i;
+    const int64_t j = clampj(nbr[e], n);
+    const double r = reach[e];
+    const double c = r > 0.0 ? __ddiv_rn(gR[i], __dmul_rn(2.0, r)) : 0.0;
+    const bool via_d2 = d2[e] > kd2[j];
+    gd2[e] = via_d2 ? c : 0.0;
+    gkd[e] = via_d2 ? 0.0 : c;
 }
 
 // Per point j: the k-distance gradient (sum over its reverse slots, fixed
@@ -179,41 +213,43 @@ __global__ void bw_kd_kernel(int64_t n, int k, const unsigned* __restrict__ off,
     }
 }
 
-// Gradient with respect to the normalised coordinates, one warp per point
-// (lanes over dimensions): sum_t 2 gd2 (xc_i - xc_j) over its own slots minus
-// the same over its reverse slots.
+// Gradient with respect to the normalised coordinates, one warp per point:
+// over its own and its reverse slots, the sum of gd2 (x_i - x_other), times
+// 2 inv at the end. Lanes take the features; with d <= 16 the warp works on 32
+// / DL slots side by side (DL = d rounded up to a power of two, at most 32) and
+// adds the groups' sums in a fixed order. Two FP64 instructions per slot and
+// lane, with the slot's scaling left to the end and the floats widened by
+// integers (six before, 723 us at n = 50,000, d = 32, k = 20).
+template <int DL>
 __global__ void bw_gx_kernel(const float* __restrict__ x, int64_t n, int d, int k, const int32_t* __restrict__ nbr,
                              const double* __restrict__ inv, const double* __restrict__ gd2,
                              const unsigned* __restrict__ off, const unsigned* __restrict__ rev,
                              double* __restrict__ gxc) {
-    const int lane = threadIdx.x & 31;
-    const int64_t warps = static_cast<int64_t>(gridDim.x) * (blockDim.x >> 5);
-    for (int64_t i = static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5); i < n; i += warps) {
-        const float* xi = x + i * d;
-        for (int f0 = 0; f0 < d; f0 += 32) {
-            const int f = f0 + lane;
+    constexpr int kGroups = 32 / DL;
+    const int lane = threadIdx.x & 31, fl = lane % DL, grp = lane / DL;
+    const unsigned n32 = static_cast<unsigned>(n);
+    for (int64_t i = warp_id(); i < n; i += warp_count()) {
+        const unsigned r0 = off[i], r1 = off[i + 1];
+        for (int f0 = 0; f0 < d; f0 += DL) {
+            const int f = f0 + fl;
             const bool on = f < d;
-            const double xif = on ? static_cast<double>(xi[f]) : 0.0;
-            const double iv = on ? inv[f] : 0.0;
+            const double xif = on ? widen(x[i * d + f]) : 0.0;
             double acc = 0.0;
-            for (int t = 0; t < k; ++t) {
+#pragma unroll 4
+            for (int t = grp; t < k; t += kGroups) {
                 const int64_t e = static_cast<int64_t>(t) * n + i;
-                const double g2 = __dmul_rn(2.0, gd2[e]);
-                if (on) {
-                    const double diff = __dmul_rn(__dsub_rn(xif, static_cast<double>(x[clampj(nbr[e], n) * d + f])), iv);
-                    acc = __fma_rn(g2, diff, acc);
-                }
+                const double g = gd2[e];
+                if (on) acc = __fma_rn(g, __dsub_rn(xif, widen(x[clampj(nbr[e], n) * d + f])), acc);
             }
-            for (unsigned p = off[i]; p < off[i + 1]; ++p) {
+#pragma unroll 4
+            for (unsigned p = r0 + grp; p < r1; p += kGroups) {
                 const unsigned e = rev[p];
-                const int64_t m = static_cast<int64_t>(e) % n;
-                const double g2 = __dmul_rn(2.0, gd2[e]);
-                if (on) {
-                    const double diff = __dmul_rn(__dsub_rn(static_cast<double>(x[m * d + f]), xif), iv);
-                    acc = __fma_rn(-g2, diff, acc);
-                }
+                const double g = gd2[e];
+                if (on) acc = __fma_rn(g, __dsub_rn(xif, widen(x[static_cast<int64_t>(e % n32) * d + f])), acc);
             }
-            if (on) gxc[i * d + f] = acc;
+#pragma unroll
+            for (int o = DL; o < 32; o <<= 1) acc = __dadd_rn(acc, __shfl_xor_sync(0xffffffffu, acc, o));
+            if (on && grp == 0) gxc[i * d + f] = __dmul_rn(acc, __dmul_rn(2.0, inv[f]));
         }
     }
 }
@@ -331,17 +367,16 @@ void Engine::lof_backward_device(const float* d_x, int64_t n, int d, int k, bool
     cudaStream_t s = stream_;
     const int64_t total = n * k;
     const size_t nk = static_cast<size_t>(total);
-    // statistics of the forward centring (same kernels, same order)
-    float* xc = xc_.as<float>(static_cast<size_t>(n) * d);
+    // statistics of the forward centring (same kernels, same order; no points)
     double* partial = partial_.as<double>(center_partial_count(n, d));
     double* mean = mean_.as<double>(d);
     double* inv = inv_std_.as<double>(d);
     CG_CUDA(cudaMemsetAsync(status_ptr(), 0, sizeof(int), s));
-    center(d_x, n, d, normalize, xc, partial, mean, inv, s);
+    center(d_x, n, d, normalize, nullptr, partial, mean, inv, s);
 
     // workspace: FP64 slot arrays, per-point arrays, the transposed slot list
     const size_t chunks_d = center_partial_count(n, d);
-    char* w = static_cast<char*>(bw_.get(sizeof(double) * (4 * nk + 4 * static_cast<size_t>(n) +
+    char* w = static_cast<char*>(bw_.get(sizeof(double) * (4 * nk + 5 * static_cast<size_t>(n) +
                                                           2 * chunks_d + 2 * static_cast<size_t>(d) +
                                                           static_cast<size_t>(n) * d) +
                                          sizeof(unsigned) * (4 * nk + static_cast<size_t>(n) + 1 +
@@ -358,7 +393,8 @@ void Engine::lof_backward_device(const float* d_x, int64_t n, int d, int k, bool
     double* gkd = reinterpret_cast<double*>(take(sizeof(double) * nk));
     double* lrd = reinterpret_cast<double*>(take(sizeof(double) * n));
     double* S = reinterpret_cast<double*>(take(sizeof(double) * n));
-    double* glrd = reinterpret_cast<double*>(take(sizeof(double) * n));
+    double* w_pt = reinterpret_cast<double*>(take(sizeof(double) * n));
+    double* gR = reinterpret_cast<double*>(take(sizeof(double) * n));
     double* gxc = reinterpret_cast<double*>(take(sizeof(double) * n * d));
     double* pa = reinterpret_cast<double*>(take(sizeof(double) * chunks_d));
     double* pb = reinterpret_cast<double*>(take(sizeof(double) * chunks_d));
@@ -373,12 +409,20 @@ void Engine::lof_backward_device(const float* d_x, int64_t n, int d, int k, bool
     unsigned* counts = reinterpret_cast<unsigned*>(take(sizeof(unsigned) * sort_pairs_counts(total)));
     int* status = status_ptr();
     double* score = scores_out;
+    const int aligned = (d & 3) == 0 && (reinterpret_cast<uintptr_t>(d_x) & 15) == 0 ? 1 : 0;
 
-    bw_pair_kernel<<<grid_of(n * 32), 256, 0, s>>>(d_x, n, d, k, nbr_idx, inv, d2, status);
+    const dim3 slots(static_cast<unsigned>(ceil_div(n, 256)), static_cast<unsigned>(k));
+    const unsigned points = static_cast<unsigned>(ceil_div(n, 256));
+    // (blockIdx.y takes at most 65535 slots)
+    for (int t0 = 0; t0 < k; t0 += 65535) {
+        const dim3 g(slots.x, static_cast<unsigned>(k - t0 < 65535 ? k - t0 : 65535));
+        bw_pair_kernel<<<g, 256, 0, s>>>(d_x, n, d, nbr_idx + static_cast<int64_t>(t0) * n, inv, normalize ? 1 : 0,
+                                         aligned, d2 + static_cast<int64_t>(t0) * n, status);
+        CG_LAUNCH_CHECK();
+    }
+    bw_lrd_kernel<<<static_cast<unsigned>(ceil_div(n, 32)), 256, 0, s>>>(n, k, nbr_idx, d2, reach, lrd);
     CG_LAUNCH_CHECK();
-    bw_lrd_kernel<<<grid_of(n * 32), 256, 0, s>>>(n, k, nbr_idx, d2, reach, lrd);
-    CG_LAUNCH_CHECK();
-    bw_score_kernel<<<grid_of(n * 32), 256, 0, s>>>(n, k, nbr_idx, lrd, S, score);
+    bw_score_kernel<<<points, 256, 0, s>>>(n, k, nbr_idx, lrd, grad_scores, S, w_pt, score);
     CG_LAUNCH_CHECK();
     // transposed slots: offsets from the per-index counts, slots in (t, i)
     // enumeration order within each index (stable sort)
@@ -391,13 +435,22 @@ void Engine::lof_backward_device(const float* d_x, int64_t n, int d, int k, bool
     unsigned* rev = nullptr;
     sort_pairs_stable(keys, vals, keys2, vals2, total, bits, counts, s, &rev);
 
-    bw_glrd_kernel<<<grid_of(n * 32), 256, 0, s>>>(n, k, grad_scores, lrd, S, off, rev, glrd);
+    bw_gather_kernel<<<grid_of(n * 32), 256, 0, s>>>(n, w_pt, off, rev, gR);
     CG_LAUNCH_CHECK();
-    bw_route_kernel<<<grid_of(total), 256, 0, s>>>(n, k, nbr_idx, d2, reach, lrd, glrd, gd2, gkd);
+    bw_point_kernel<<<points, 256, 0, s>>>(n, k, grad_scores, lrd, S, gR, gR);
     CG_LAUNCH_CHECK();
+    for (int t0 = 0; t0 < k; t0 += 65535) {
+        const dim3 g(slots.x, static_cast<unsigned>(k - t0 < 65535 ? k - t0 : 65535));
+        const int64_t at = static_cast<int64_t>(t0) * n;
+        bw_route_kernel<<<g, 256, 0, s>>>(n, nbr_idx + at, d2 + at, d2 + static_cast<int64_t>(k - 1) * n, reach + at, gR,
+                                          gd2 + at, gkd + at);
+        CG_LAUNCH_CHECK();
+    }
     bw_kd_kernel<<<grid_of(n * 32), 256, 0, s>>>(n, k, off, rev, gkd, gd2);
     CG_LAUNCH_CHECK();
-    bw_gx_kernel<<<grid_of(n * 32), 256, 0, s>>>(d_x, n, d, k, nbr_idx, inv, gd2, off, rev, gxc);
+    const auto gx = d <= 1 ? bw_gx_kernel<1> : d <= 2 ? bw_gx_kernel<2> : d <= 4 ? bw_gx_kernel<4> : d <= 8
+                        ? bw_gx_kernel<8> : d <= 16 ? bw_gx_kernel<16> : bw_gx_kernel<32>;
+    gx<<<grid_of(n * 32), 256, 0, s>>>(d_x, n, d, k, nbr_idx, inv, gd2, off, rev, gxc);
     CG_LAUNCH_CHECK();
     // the centring statistics' partials of (x - mean)^2 are still in `partial`
     // when normalising (the second pass of center())

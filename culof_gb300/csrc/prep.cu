@@ -169,7 +169,8 @@ __global__ void __launch_bounds__(kSmallThreads)
 center_small_kernel(const float* __restrict__ x, int n, int d, int normalize, double* __restrict__ partial,
                     double* __restrict__ mean, double* __restrict__ inv_std, float* __restrict__ xc,
                     unsigned* __restrict__ mm) {
-    extern __shared__ float col[];
+    extern __shared__ double sq[];  // squares (when normalising), padded as the column
+    float* col = reinterpret_cast<float*>(sq + (normalize ? n + n / kCenterChunk + 1 : 0));
     __shared__ double part[kSmallRows / kCenterChunk];
     __shared__ double stat[2];
     const int f = blockIdx.x, tid = threadIdx.x;
@@ -178,20 +179,28 @@ center_small_kernel(const float* __restrict__ x, int n, int d, int normalize, do
     const int chunks = (n + kCenterChunk - 1) / kCenterChunk;
     const double dn = static_cast<double>(n);
     for (int pass = 0; pass <= normalize; ++pass) {
+        if (pass) {  // every thread: the squares, so that the chains below only add
+            for (int i = tid; i < n; i += kSmallThreads) {
+                const int at = i + i / kCenterChunk;
+                const double v = __dsub_rn(widen(col[at]), stat[0]);
+                sq[at] = __dmul_rn(v, v);
+            }
+            __syncthreads();
+        }
         if (tid < chunks) {
             const int begin = tid * kCenterChunk, len = min(kCenterChunk, n - begin);
             const float* c = col + begin + tid;
-            const double m = pass ? stat[0] : 0.0;
+            const double* q = sq + begin + tid;
             double s = 0.0;
             int i = 0;
             for (; i + 16 <= len; i += 16) {
-                float v[16];
+                double v[16];
 #pragma unroll
-                for (int j = 0; j < 16; ++j) v[j] = c[i + j];
+                for (int j = 0; j < 16; ++j) v[j] = pass ? q[i + j] : widen(c[i + j]);
 #pragma unroll
-                for (int j = 0; j < 16; ++j) s = center_term(s, v[j], m, pass != 0);
+                for (int j = 0; j < 16; ++j) s = __dadd_rn(s, v[j]);
             }
-            for (; i < len; ++i) s = center_term(s, c[i], m, pass != 0);
+            for (; i < len; ++i) s = __dadd_rn(s, pass ? q[i] : widen(c[i]));
             part[tid] = s;
             partial[static_cast<int64_t>(tid) * d + f] = s;
         }
@@ -211,6 +220,7 @@ center_small_kernel(const float* __restrict__ x, int n, int d, int normalize, do
         }
         __syncthreads();
     }
+    if (xc == nullptr) return;
     const double m = stat[0], v = stat[1];
     unsigned lo = 0u, hi = 0u;
     for (int i = tid; i < n; i += kSmallThreads) {
@@ -269,7 +279,11 @@ void center(const float* x, int64_t n, int d, bool normalize, float* xc, double*
     // up to 8,192 rows (the column's shared memory) and 131,072 values (a
     // column's strided reads cost whole sectors)
     if (n <= kSmallRows && n * d <= (1 << 17)) {
-        center_small_kernel<<<d, kSmallThreads, sizeof(float) * static_cast<size_t>(n + chunks), s>>>(
+        const size_t places = static_cast<size_t>(n) + n / kCenterChunk + 1;
+        const size_t smem = places * (sizeof(float) + (normalize ? sizeof(double) : 0));
+        set_max_dynamic_smem(reinterpret_cast<const void*>(center_small_kernel),
+                             static_cast<int>((kSmallRows + kSmallRows / kCenterChunk + 1) * (sizeof(float) + sizeof(double))));
+        center_small_kernel<<<d, kSmallThreads, smem, s>>>(
             x, static_cast<int>(n), d, normalize ? 1 : 0, partial, mean, inv_std, xc, mm);
         CG_LAUNCH_CHECK();
         return;
@@ -286,6 +300,7 @@ void center(const float* x, int64_t n, int d, bool normalize, float* xc, double*
         center_finalize_kernel<<<d, 256, 0, s>>>(partial, chunks, d, n, 1, mean, inv_std);
         CG_LAUNCH_CHECK();
     }
+    if (xc == nullptr) return;
     center_apply_kernel<<<grid_for(n * d, kApplyThreads, 152 * 8), kApplyThreads, 0, s>>>(x, n, d, mean, inv_std, xc, mm);
     CG_LAUNCH_CHECK();
 }
