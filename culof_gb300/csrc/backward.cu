@@ -142,16 +142,24 @@ __global__ void bw_score_kernel(int64_t n, int k, const int32_t* __restrict__ nb
     if (score) score[i] = __ddiv_rn(s, kl);
 }
 
-// Transposed slot list: count slots per neighbour index (integer atomics,
-// order-free), keys/values for the stable sort.
+// Transposed slot list: keys and values for the stable sort, then each
+// index's first place in the sorted keys (off[n] = total).
 __global__ void bw_rev_init_kernel(int64_t n, int64_t total, const int32_t* __restrict__ nbr, unsigned* __restrict__ keys,
-                                   unsigned* __restrict__ vals, unsigned* __restrict__ counts) {
+                                   unsigned* __restrict__ vals) {
     for (int64_t e = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; e < total;
          e += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-        const unsigned j = static_cast<unsigned>(clampj(nbr[e], n));
-        keys[e] = j;
+        keys[e] = static_cast<unsigned>(clampj(nbr[e], n));
         vals[e] = static_cast<unsigned>(e);
-        atomicAdd(&counts[j], 1u);
+    }
+}
+__global__ void bw_rev_offsets_kernel(int64_t n, int64_t total, const unsigned* __restrict__ keys,
+                                      unsigned* __restrict__ off) {
+    for (int64_t p = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; p <= total;
+         p += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+        // indices past the previous key, up to this one (the end: up to n)
+        int64_t j = p > 0 ? static_cast<int64_t>(keys[p - 1]) + 1 : 0;
+        const int64_t last = p < total ? static_cast<int64_t>(keys[p]) : n;
+        for (; j <= last; ++j) off[j] = static_cast<unsigned>(p);
     }
 }
 
@@ -424,16 +432,16 @@ void Engine::lof_backward_device(const float* d_x, int64_t n, int d, int k, bool
     CG_LAUNCH_CHECK();
     bw_score_kernel<<<points, 256, 0, s>>>(n, k, nbr_idx, lrd, grad_scores, S, w_pt, score);
     CG_LAUNCH_CHECK();
-    // transposed slots: offsets from the per-index counts, slots in (t, i)
-    // enumeration order within each index (stable sort)
-    CG_CUDA(cudaMemsetAsync(off, 0, sizeof(unsigned) * (n + 1), s));
-    bw_rev_init_kernel<<<grid_of(total), 256, 0, s>>>(n, total, nbr_idx, keys, vals, off);
+    // transposed slots: in (t, i) enumeration order within each index (stable
+    // sort)
+    bw_rev_init_kernel<<<grid_of(total), 256, 0, s>>>(n, total, nbr_idx, keys, vals);
     CG_LAUNCH_CHECK();
-    exclusive_scan_u32(off, n + 1, s);
     int bits = 8;
     while (bits < 32 && (static_cast<int64_t>(1) << bits) < n) bits += 8;
     unsigned* rev = nullptr;
-    sort_pairs_stable(keys, vals, keys2, vals2, total, bits, counts, s, &rev);
+    const unsigned* sorted = sort_pairs_stable(keys, vals, keys2, vals2, total, bits, counts, s, &rev);
+    bw_rev_offsets_kernel<<<grid_of(total + 1), 256, 0, s>>>(n, total, sorted, off);
+    CG_LAUNCH_CHECK();
 
     bw_gather_kernel<<<grid_of(n * 32), 256, 0, s>>>(n, w_pt, off, rev, gR);
     CG_LAUNCH_CHECK();

@@ -30,7 +30,9 @@
 #include "common.cuh"
 #include "engine.cuh"
 #include "fast.cuh"
+#include "fp64.cuh"
 #include "sweep_common.cuh"
+#include "sweep_rows.cuh"
 
 namespace culof_gb300 {
 
@@ -126,11 +128,17 @@ __global__ void bm_minmax_kernel(const float* __restrict__ xc, const int64_t* __
     }
     __syncthreads();
     const int64_t b = off[p], e = off[p + 1];
-    for (int64_t t = threadIdx.x; t < (e - b) * d; t += blockDim.x) {
-        const int f = static_cast<int>(t % d);
-        const unsigned k = flip_f(xc[b * d + t]);
-        atomicMin(&lo[f], k);
-        atomicMax(&hi[f], k);
+    const int per = static_cast<int>(blockDim.x) / d * d;  // each thread stays on one feature
+    if (static_cast<int>(threadIdx.x) < per) {
+        const int f = static_cast<int>(threadIdx.x) % d;
+        unsigned mn = 0xFFFFFFFFu, mx = 0u;
+        for (int64_t t = threadIdx.x; t < (e - b) * d; t += per) {
+            const unsigned k = flip_f(xc[b * d + t]);
+            mn = min(mn, k);
+            mx = max(mx, k);
+        }
+        atomicMin(&lo[f], mn);
+        atomicMax(&hi[f], mx);
     }
     __syncthreads();
     for (int f = threadIdx.x; f < d; f += blockDim.x) {
@@ -204,6 +212,83 @@ __global__ void bm_gather_kernel(const float* __restrict__ xc, int64_t ntot, int
         xs[t] = xc[static_cast<int64_t>(src) * d + f];
         if (f == 0) lidx[i] = static_cast<unsigned>(src - off[pid[src]]);
     }
+}
+
+// One CTA of 128 threads per (problem, tile of 128 sorted points): the column
+// tile of the row-pruned sweep (small.cuh's layout) and its box.
+template <int DP>
+__global__ void __launch_bounds__(kCT) bm_tile_kernel(const float* __restrict__ xc, int d,
+                                                      const unsigned* __restrict__ perm, const int64_t* __restrict__ off,
+                                                      const int* __restrict__ tpid, const int64_t* __restrict__ toff,
+                                                      float* __restrict__ tiles, float* __restrict__ boxes) {
+    __shared__ float wb[kCT / 32][2][DP];
+    const int64_t g = blockIdx.x;
+    const int c = threadIdx.x, lane = c & 31, q = c >> 5;
+    const int p = tpid[g];
+    const int64_t pos = off[p] + (g - toff[p]) * kCT + c;
+    const bool valid = pos < off[p + 1];
+    const unsigned src = valid ? perm[pos] : 0u;
+    float* tile = tiles + g * small::tile_floats(DP);
+#pragma unroll
+    for (int f = 0; f < DP; ++f) {
+        const float v = (valid && f < d) ? xc[static_cast<int64_t>(src) * d + f] : 0.0f;
+        tile[f * kCT + c] = (!valid && f == 0) ? __int_as_float(0x7fc00000) : v;
+        float lo = valid ? v : __int_as_float(0x7f800000), hi = valid ? v : __int_as_float(0xff800000);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+            hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+        }
+        if (lane == 0) {
+            wb[q][0][f] = lo;
+            wb[q][1][f] = hi;
+        }
+    }
+    reinterpret_cast<unsigned*>(tile)[small::tile_index_off(DP) + c] =
+        valid ? static_cast<unsigned>(src - off[p]) : kNoIndex;
+    __syncthreads();
+    if (c < small::kHalves * DP) {
+        const int h = c / DP, f = c % DP;
+        tile[small::tile_box_off(DP) + (h * DP + f) * 2] = fminf(wb[2 * h][0][f], wb[2 * h + 1][0][f]);
+        tile[small::tile_box_off(DP) + (h * DP + f) * 2 + 1] = -fmaxf(wb[2 * h][1][f], wb[2 * h + 1][1][f]);
+    }
+    if (c < DP) {
+        boxes[g * 2 * DP + c] = fminf(fminf(wb[0][0][c], wb[1][0][c]), fminf(wb[2][0][c], wb[3][0][c]));
+        boxes[g * 2 * DP + DP + c] = fmaxf(fmaxf(wb[0][1][c], wb[1][1][c]), fmaxf(wb[2][1][c], wb[3][1][c]));
+    }
+}
+
+// Batches of up to 16 features: one CTA per 64 rows of a problem, the
+// row-pruned sweep over the problem's own tiles (sweep_rows.cuh). In the
+// evaluated workload (256 problems, d = 16, three clusters and 2% outliers
+// each) the boxes rule out the other clusters' tiles, two thirds of all pairs.
+template <int DP, int KR, int G>
+__global__ void __launch_bounds__(kThreads, DP <= 8 && KR == 1 ? 3 : 2)
+batched_sweep_kernel(const float* __restrict__ tiles, const float* __restrict__ boxes, const int64_t* __restrict__ off,
+                     const int* __restrict__ ks, const int64_t* __restrict__ nkoff, const int64_t* __restrict__ toff,
+                     const uint2* __restrict__ items, int32_t* __restrict__ nbr_idx, float* __restrict__ nbr_d2,
+                     float* __restrict__ kdist2, int* __restrict__ status) {
+    constexpr int kRowsPer = 8;
+    using Smem = small::SmallSmem<DP, KR, kRowsPer, kWarps>;
+    extern __shared__ __align__(128) unsigned char bsw_raw[];
+    Smem& sh = *reinterpret_cast<Smem*>(bsw_raw);
+    constexpr int kPerTile = kCT / Smem::kRows;
+    const uint2 it = items[blockIdx.x / kPerTile];
+    const int p = static_cast<int>(it.x);
+    small::SweepRows P{};
+    P.n = off[p + 1] - off[p];
+    P.base = static_cast<int64_t>(it.y) * kCT + static_cast<int>(blockIdx.x) % kPerTile * Smem::kRows;
+    if (P.base >= P.n) return;
+    P.nt = static_cast<int>((P.n + kCT - 1) / kCT);
+    P.tiles = tiles + toff[p] * small::tile_floats(DP);
+    P.boxes = boxes + toff[p] * 2 * DP;
+    P.k = ks[p];
+    P.segment = small::kSegTiles;
+    P.nbr_idx = nbr_idx + nkoff[p];
+    P.nbr_d2 = nbr_d2 + nkoff[p];
+    P.kdist2 = kdist2 + off[p];
+    P.status = status;
+    small::sweep_rows<DP, KR, G, kRowsPer, kWarps, false>(sh, P);
 }
 
 // One warp per (problem, tile of 128 sorted points): the tile's bounding box,
@@ -547,7 +632,7 @@ __global__ void bl_lrd_kernel(int64_t ntot, const int* __restrict__ pid, const i
         const int64_t o = static_cast<int64_t>(t) * n + i;
         const int32_t j = ni[o];
         const float kj = (j >= 0 && j < n) ? kdist2[base + j] : __int_as_float(0x7fc00000);
-        sum = __dadd_rn(sum, __dsqrt_rn(static_cast<double>(fmaxf(kj, nd[o]))));
+        sum = __dadd_rn(sum, __dsqrt_rn(widen(fmaxf(kj, nd[o]))));
     }
     lrd[g] = __double2float_rn(__ddiv_rn(1.0, __dadd_rn(__ddiv_rn(sum, static_cast<double>(k)), 1e-10)));
 }
@@ -563,12 +648,21 @@ __global__ void bl_score_kernel(int64_t ntot, const int* __restrict__ pid, const
     const int64_t n = off[p + 1] - base, i = g - base;
     const int k = ks[p];
     const int32_t* ni = nbr_idx + nkoff[p];
-    const double self = static_cast<double>(lrd[g]);
+    // the quotients from one reciprocal (lof.cu: score_kernel has the proof)
+    const double self = widen(lrd[g]), y = __ddiv_rn(1.0, self);
+    const bool quick = fabs(y) < __longlong_as_double(0x7ff0000000000000ll) && y != 0.0;
     double sum = 0.0;
     for (int t = 0; t < k; ++t) {
         const int32_t j = ni[static_cast<int64_t>(t) * n + i];
-        const double lj = (j >= 0 && j < n) ? static_cast<double>(lrd[base + j]) : __longlong_as_double(0x7ff8000000000000ll);
-        sum = __dadd_rn(sum, __ddiv_rn(lj, self));
+        const double lj = (j >= 0 && j < n) ? widen(lrd[base + j]) : __longlong_as_double(0x7ff8000000000000ll);
+        double q;
+        if (quick) {
+            const double q0 = __dmul_rn(lj, y);
+            q = __fma_rn(__fma_rn(-q0, self, lj), y, q0);
+        } else {
+            q = __ddiv_rn(lj, self);
+        }
+        sum = __dadd_rn(sum, q);
     }
     scores[g] = __double2float_rn(__ddiv_rn(sum, static_cast<double>(k)));
 }
@@ -600,6 +694,34 @@ void launch_knn(int dp, bool cp2, int grid, const BatchDev& b, cudaStream_t s) {
         case 64: launch_knn_t<64, 1>(grid, b, s); break;
         default: throw Error(kInternal, "bad padded dimension");
     }
+}
+
+constexpr int kSweepMaxD = 16;  // more features take batched_knn_kernel
+int sweep_dp(int d) { return d <= 4 ? 4 : d <= 8 ? 8 : d <= 12 ? 12 : 16; }
+
+// The items of one list form, [first, first + count). one_cta: shared memory
+// padded so that a single CTA fits on an SM.
+template <int DP, int KR, int G>
+void launch_sweep(const BatchDev& b, int first, int count, bool one_cta, int* status, cudaStream_t s) {
+    if (count == 0) return;
+    size_t smem = sizeof(small::SmallSmem<DP, KR, 8, kWarps>);
+    set_max_dynamic_smem(reinterpret_cast<const void*>(batched_sweep_kernel<DP, KR, G>), 227 * 1024);
+    if (one_cta) smem = std::max<size_t>(smem, 120 * 1024);
+    batched_sweep_kernel<DP, KR, G><<<static_cast<unsigned>(count) * 2, kThreads, smem, s>>>(
+        b.tiles, b.tbox, b.off, b.ks, b.nkoff, b.toff, b.items + first, b.nbr, b.d2, b.kd, status);
+    CG_LAUNCH_CHECK();
+}
+template <int DP>
+void launch_sweeps(const BatchDev& b, bool one_cta, int* status, cudaStream_t s) {
+    launch_sweep<DP, 2, 2>(b, 0, b.group[0], one_cta, status, s);
+    launch_sweep<DP, 1, 2>(b, b.group[0], b.group[1], one_cta, status, s);
+    launch_sweep<DP, 1, 1>(b, b.group[0] + b.group[1], b.group[2], one_cta, status, s);
+}
+template <int DP>
+void launch_tiles(const BatchDev& b, const unsigned* perm, cudaStream_t s) {
+    bm_tile_kernel<DP><<<static_cast<unsigned>(b.ntiles), kCT, 0, s>>>(b.xc, b.d, perm, b.off, b.tpid, b.toff, b.tiles,
+                                                                       b.tbox);
+    CG_LAUNCH_CHECK();
 }
 
 template <int DP>
@@ -669,6 +791,17 @@ void Engine::batch_plan(int num, const int64_t* offsets, const int* ks, int d, b
     // largest problems first: their items are the longest, the tail stays short
     std::stable_sort(items.begin(), items.end(),
                      [](const std::pair<int64_t, uint2>& a, const std::pair<int64_t, uint2>& b) { return a.first > b.first; });
+    // the sweep's list forms (k > 32, k > 24, the rest) are launched one after
+    // another, each largest problems first
+    const auto form = [&](const std::pair<int64_t, uint2>& it) {
+        const int k = ks[it.second.x];
+        return k > 32 ? 0 : k > 24 ? 1 : 2;
+    };
+    if (d <= kSweepMaxD)
+        std::stable_sort(items.begin(), items.end(),
+                         [&](const std::pair<int64_t, uint2>& a, const std::pair<int64_t, uint2>& b) { return form(a) < form(b); });
+    for (int& g : bdev_.group) g = 0;
+    for (const auto& it : items) ++bdev_.group[form(it)];
     P.items.resize(items.size());
     for (size_t i = 0; i < items.size(); ++i) P.items[i] = items[i].second;
     P.ntot = offsets[num];
@@ -706,14 +839,17 @@ void Engine::batch_plan(int num, const int64_t* offsets, const int* ks, int d, b
     b.kd = bkd_.as<float>(P.ntot);
     b.lrd = blrd_.as<float>(P.ntot);
     b.counter = bcounter_.as<unsigned>(1);
-    b.xs = bxs_.as<float>(static_cast<size_t>(P.ntot) * d);
+    const bool sweep = d <= kSweepMaxD;
+    const int width = sweep ? sweep_dp(d) : d;  // of a box
+    b.xs = sweep ? nullptr : bxs_.as<float>(static_cast<size_t>(P.ntot) * d);
+    if (sweep) b.tiles = btiles_.as<float>(static_cast<size_t>(b.ntiles) * small::tile_floats(width));
     b.lidx = blidx_.as<unsigned>(P.ntot);
     b.pmm = bpmm_.as<float>(static_cast<size_t>(num) * d * 2);
     b.pdims = bpdims_.as<int>(static_cast<size_t>(num) * kMortonDimsB);
     b.skeys = bskeys_.as<unsigned>(2 * static_cast<size_t>(P.ntot));
     b.svals = bsvals_.as<unsigned>(2 * static_cast<size_t>(P.ntot));
     b.scounts = bscounts_.as<unsigned>(sort_pairs_counts(P.ntot));
-    b.tbox = btbox_.as<float>(static_cast<size_t>(b.ntiles) * 2 * d);
+    b.tbox = btbox_.as<float>(static_cast<size_t>(b.ntiles) * 2 * width);
     pid_kernel<<<num < 4096 ? num : 4096, 256, 0, s>>>(b.off, num, b.pid);
     CG_LAUNCH_CHECK();
     CG_CUDA(cudaStreamSynchronize(s));
@@ -759,13 +895,24 @@ void Engine::batch_launch(const float* d_x, float* d_scores) {
     while (pbits < 32 && (static_cast<int64_t>(1) << pbits) < P.num) pbits += 8;
     unsigned* perm = nullptr;
     sort_pairs_stable(ks1, vs, kother, vother, P.ntot, pbits, b.scounts, s, &perm);
-    bm_gather_kernel<<<grid_cap(P.ntot * d), 256, 0, s>>>(b.xc, P.ntot, d, perm, b.pid, b.off, b.xs, b.lidx);
-    CG_LAUNCH_CHECK();
-    bm_tilebox_kernel<<<static_cast<unsigned>(ceil_div(b.ntiles, 8)), 256, 0, s>>>(b.xs, b.off, d, b.tpid, b.toff,
-                                                                                   b.ntiles, b.tbox);
-    CG_LAUNCH_CHECK();
-    CG_CUDA(cudaMemsetAsync(b.counter, 0, sizeof(unsigned), s));
-    launch_knn(dp_for(d), btune_packed_, btune_grid_, b, s);
+    if (d <= kSweepMaxD) {
+        const bool one_cta = btune_grid_ == bsms_;
+        CG_CUDA(cudaMemsetAsync(status_ptr(), 0, sizeof(int), s));
+        switch (sweep_dp(d)) {
+            case 4: launch_tiles<4>(b, perm, s); launch_sweeps<4>(b, one_cta, status_ptr(), s); break;
+            case 8: launch_tiles<8>(b, perm, s); launch_sweeps<8>(b, one_cta, status_ptr(), s); break;
+            case 12: launch_tiles<12>(b, perm, s); launch_sweeps<12>(b, one_cta, status_ptr(), s); break;
+            default: launch_tiles<16>(b, perm, s); launch_sweeps<16>(b, one_cta, status_ptr(), s); break;
+        }
+    } else {
+        bm_gather_kernel<<<grid_cap(P.ntot * d), 256, 0, s>>>(b.xc, P.ntot, d, perm, b.pid, b.off, b.xs, b.lidx);
+        CG_LAUNCH_CHECK();
+        bm_tilebox_kernel<<<static_cast<unsigned>(ceil_div(b.ntiles, 8)), 256, 0, s>>>(b.xs, b.off, d, b.tpid, b.toff,
+                                                                                       b.ntiles, b.tbox);
+        CG_LAUNCH_CHECK();
+        CG_CUDA(cudaMemsetAsync(b.counter, 0, sizeof(unsigned), s));
+        launch_knn(dp_for(d), btune_packed_, btune_grid_, b, s);
+    }
     bl_lrd_kernel<<<static_cast<unsigned>(ceil_div(P.ntot, 256)), 256, 0, s>>>(P.ntot, b.pid, b.off, b.ks, b.nkoff,
                                                                                b.nbr, b.d2, b.kd, b.lrd);
     CG_LAUNCH_CHECK();
@@ -783,13 +930,16 @@ void Engine::batch_autotune(const float* d_x, float* d_scores) {
     int max_per_sm = static_cast<int>(227 * 1024 / (smem + 1024));
     if (max_per_sm < 1) max_per_sm = 1;
     if (max_per_sm > 2) max_per_sm = 2;
+    const bool sweep = bplan_.d <= kSweepMaxD;  // one CTA per SM, or (2) as many as fit
+    if (sweep) max_per_sm = 2;
+    bsms_ = sms;
     cudaEvent_t e0, e1;
     CG_CUDA(cudaEventCreate(&e0));
     CG_CUDA(cudaEventCreate(&e1));
     float best = 1e30f;
     for (float& t : btune_ms_) t = -1.0f;
     for (int per = 1; per <= max_per_sm; ++per) {
-        for (int packed = 0; packed <= (dp <= 16 ? 1 : 0); ++packed) {
+        for (int packed = 0; packed <= (!sweep && dp <= 16 ? 1 : 0); ++packed) {
             btune_grid_ = per * sms;
             btune_packed_ = packed != 0;
             batch_launch(d_x, d_scores);  // warm (first use configures the kernel)

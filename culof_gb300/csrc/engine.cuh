@@ -65,6 +65,8 @@ struct BatchDev {
     int64_t* toff = nullptr;
     int64_t ntiles = 0;
     float* tbox = nullptr;
+    float* tiles = nullptr;       // column tiles of the sweep (d <= 16)
+    int group[3] = {0, 0, 0};     // items of each list form
 };
 
 enum Path : int { kPathAuto = 0, kPathFast = 1, kPathGeneral = 2, kPathTensor = 3 };
@@ -116,7 +118,8 @@ public:
     void set_graphs(bool on) { use_graphs_ = on; }
     // The batched autotuner's measurements for the current layout (times of
     // the whole batched call): ms4[2 (c - 1) + (p - 1)] for the k-NN kernel at
-    // c CTAs per SM and p column pairs per lane (-1: not tried), and its
+    // c CTAs per SM (the sweep of up to 16 features: 1, or 2 for as many as fit)
+    // and p column pairs per lane (-1: not tried), and its
     // choice (0 before the first batched call).
     void batched_tuning(float* ms4, int* per_sm, int* pairs_per_lane) const;
     // Pairs the last FP32 small-d sweep evaluated and the pairs of an
@@ -159,10 +162,10 @@ private:
     DevBuf bplan_off_, bplan_nkoff_, bplan_coff_, bplan_ks_, bplan_items_, bplan_cp_;
     DevBuf bpid_, bxc_, bpartial_, bmean_, binv_, bnbr_, bd2_, bkd_, blrd_, bcounter_;
     DevBuf bxs_, blidx_, bpmm_, bpdims_, bskeys_, bsvals_, bscounts_;
-    DevBuf bplan_toff_, bplan_tpid_, btbox_;
+    DevBuf bplan_toff_, bplan_tpid_, btbox_, btiles_;
     bool use_graphs_ = true;
     bool btuned_ = false, btune_packed_ = true, bbest_packed_ = true;
-    int btune_grid_ = 152, bbest_grid_ = 152;
+    int btune_grid_ = 152, bbest_grid_ = 152, bsms_ = 152;
     float btune_ms_[4] = {-1.0f, -1.0f, -1.0f, -1.0f};  // (CTAs per SM 1..2) x (column pairs 1..2)
     cudaGraphExec_t bgraph_exec_ = nullptr;
     bool bgraph_valid_ = false;

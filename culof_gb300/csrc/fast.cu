@@ -163,53 +163,6 @@ __global__ void __launch_bounds__(kRowScanThreads) sort_rowscan_kernel(unsigned*
     if (threadIdx.x == 0) totals[blockIdx.x] = carry;
 }
 
-// Exclusive scan of an array in place (one block): each thread scans
-// kScanItems consecutive entries per step, the block scans the threads' totals.
-constexpr int kScanItems = 8;
-__global__ void scan_kernel(unsigned* __restrict__ counts, int64_t len) {
-    __shared__ unsigned warp_tot[32];
-    __shared__ unsigned carry;
-    if (threadIdx.x == 0) carry = 0;
-    __syncthreads();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int64_t step = static_cast<int64_t>(blockDim.x) * kScanItems;
-    for (int64_t base = 0; base < len; base += step) {
-        const int64_t i0 = base + static_cast<int64_t>(threadIdx.x) * kScanItems;
-        unsigned v[kScanItems];
-        unsigned tsum = 0;
-#pragma unroll
-        for (int j = 0; j < kScanItems; ++j) {
-            v[j] = i0 + j < len ? counts[i0 + j] : 0u;
-            tsum += v[j];
-        }
-        unsigned x = tsum;
-        for (int o = 1; o < 32; o <<= 1) {
-            const unsigned y = __shfl_up_sync(0xffffffffu, x, o);
-            if (lane >= o) x += y;
-        }
-        if (lane == 31) warp_tot[warp] = x;
-        __syncthreads();
-        if (warp == 0) {
-            unsigned w = lane < (int)(blockDim.x >> 5) ? warp_tot[lane] : 0u;
-            for (int o = 1; o < 32; o <<= 1) {
-                const unsigned y = __shfl_up_sync(0xffffffffu, w, o);
-                if (lane >= o) w += y;
-            }
-            warp_tot[lane] = w;
-        }
-        __syncthreads();
-        unsigned run = (warp > 0 ? warp_tot[warp - 1] : 0u) + carry + x - tsum;
-#pragma unroll
-        for (int j = 0; j < kScanItems; ++j) {
-            if (i0 + j < len) counts[i0 + j] = run;
-            run += v[j];
-        }
-        __syncthreads();
-        if (threadIdx.x == blockDim.x - 1) carry = run;
-        __syncthreads();
-    }
-}
-
 __global__ void sort_downsweep_kernel(const unsigned* __restrict__ keys_in, const unsigned* __restrict__ vals_in,
                                       unsigned* __restrict__ keys_out, unsigned* __restrict__ vals_out, int64_t n,
                                       int shift, const unsigned* __restrict__ offsets,
@@ -337,7 +290,7 @@ __global__ void __launch_bounds__(256) prune_list_kernel(const float* __restrict
                 const float gap = fmaxf(0.0f, fmaxf(__fsub_rd(b[f], tbox[1][f]), __fsub_rd(tbox[0][f], b[DP + f])));
                 g2 = __fadd_rd(g2, __fmul_rd(gap, gap));
             }
-            pass = !(__fmul_rd(g2, kPruneShrink) > kmax);
+            pass = !(__fmul_rd(g2, prune_shrink<DP>()) > kmax);
         }
         const unsigned m = __ballot_sync(0xffffffffu, pass);
         if (lane == 0) wtot[warp] = __popc(m);
@@ -644,11 +597,6 @@ unsigned* sort_pairs_stable(unsigned* keys, unsigned* vals, unsigned* keys_tmp, 
     }
     *vals_out = vin;
     return kin;
-}
-
-void exclusive_scan_u32(unsigned* data, int64_t len, cudaStream_t s) {
-    scan_kernel<<<1, 1024, 0, s>>>(data, len);
-    CG_LAUNCH_CHECK();
 }
 
 bool fast_path_supported(int64_t n, int d, int k) {

@@ -35,8 +35,6 @@ void wide_sweep(const float* tiles, int nt, int t0, int mt, int nsplit, int d, i
 size_t sort_pairs_counts(int64_t n);
 unsigned* sort_pairs_stable(unsigned* keys, unsigned* vals, unsigned* keys_tmp, unsigned* vals_tmp, int64_t n,
                             int key_bits, unsigned* counts, cudaStream_t s, unsigned** vals_out);
-// In-place exclusive prefix sum (one block; for index-sized arrays).
-void exclusive_scan_u32(unsigned* data, int64_t len, cudaStream_t s);
 
 // Shared by the FP32 and tensor-core sweeps (fast.cu).
 int choose_splits(int nt, int sms);

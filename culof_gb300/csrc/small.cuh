@@ -38,10 +38,13 @@ __device__ __forceinline__ float tile_coord(const float* tile, int c, int f) {
 }
 
 // Pruning margin: the float32 direct-difference distance D of two points at
-// real squared distance T >= LB satisfies D >= T (1 - (d + 2) 2^-24) >
-// LB (1 - 2^-20) for d <= 8, so a box whose rounded-down gap times
-// (1 - 2^-20) exceeds a row's k-th distance holds no candidate for it.
-constexpr float kPruneShrink = 0.99999904632568359375f;  // 1 - 2^-20
+// real squared distance T >= LB satisfies D >= T (1 - (d + 2) 2^-24), so a box
+// whose rounded-down gap times the factor exceeds a row's k-th distance holds
+// no candidate for it: 1 - 2^-20 for d <= 8, 1 - 2^-17 for d <= 64.
+template <int DP>
+__device__ __forceinline__ constexpr float prune_shrink() {
+    return DP <= 8 ? 0.99999904632568359375f : 0.9999923706054688f;
+}
 
 constexpr int kSegTiles = 1024;  // column tiles a CTA lists at a time
 
