@@ -25,6 +25,8 @@
 // index), identical to the general path and the oracle; the filter only
 // decides which pairs get an exact evaluation, and its bound is proven
 // conservative (sweep_common.cuh: tau_from; tc_sweep.cu: row_bounds).
+#include <cooperative_groups.h>
+
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
@@ -539,6 +541,134 @@ merge_kernel(const uint64_t* __restrict__ seed_keys, const uint64_t* __restrict_
     if (lane == 0) kdist2[self] = __uint_as_float(kbits);
 }
 
+// The whole sort of a small input in one launch: a cluster of eight CTAs, each
+// with a contiguous eighth of the pairs, runs all passes with its digit counts
+// in (distributed) shared memory; the pairs go through global memory (L2)
+// between passes, ordered by the cluster barriers: bound by their latency and
+// the eight SMs' issue rate. Three launches per pass spent most of their time
+// starting and in the gaps; the order (keys, sort, refinement) of 8,000 points
+// at d=200 takes 45 us for 96, of 20,000 at d=8 87 for 125 (31 of it this
+// kernel), of 30,000 at d=100 68 for 105, of 50,000 at d=3 112 for 121 (66 of
+// it this kernel). At 65,536 pairs the two meet: that is the limit.
+constexpr int kCsThreads = 1024;
+constexpr int kCsWarps = kCsThreads / 32;
+constexpr int kCsCtas = 8;
+constexpr int kCsItems = 8;  // most pairs per thread
+constexpr int64_t kCsMax = static_cast<int64_t>(kCsCtas) * kCsThreads * kCsItems;
+
+struct ClusterSortSmem {
+    unsigned wcount[kCsWarps][256];
+    unsigned totals[2][256];  // this CTA's digit counts, by pass parity (other CTAs read them)
+    unsigned first[256];      // first place of the CTA's pairs of each digit
+    int warp_sums[8];
+};
+
+template <int IPT>
+__global__ void __launch_bounds__(kCsThreads)
+cluster_sort_kernel(unsigned* __restrict__ keys, unsigned* __restrict__ vals, unsigned* __restrict__ keys_tmp,
+                    unsigned* __restrict__ vals_tmp, int n, int key_bits) {
+    namespace cg = cooperative_groups;
+    extern __shared__ __align__(16) unsigned char cs_raw[];
+    ClusterSortSmem& sh = *reinterpret_cast<ClusterSortSmem*>(cs_raw);
+    cg::cluster_group cl = cg::this_cluster();
+    const int rank = static_cast<int>(cl.block_rank());
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const unsigned lt = (1u << lane) - 1u;
+    // warp w of CTA r owns pairs [(r kCsWarps + w) 32 IPT, ...), 32 at a time
+    const int base = (rank * kCsWarps + warp) * 32 * IPT + lane;
+    unsigned *kin = keys, *vin = vals, *kout = keys_tmp, *vout = vals_tmp;
+    for (int shift = 0, pass = 0; shift < key_bits; shift += 8, ++pass) {
+        for (int i = tid; i < kCsWarps * 256; i += kCsThreads) (&sh.wcount[0][0])[i] = 0;
+        unsigned key[IPT], val[IPT], place[IPT];
+#pragma unroll
+        for (int it = 0; it < IPT; ++it) {
+            const int i = base + it * 32;
+            key[it] = i < n ? __ldcg(kin + i) : 0u;
+            val[it] = i < n ? __ldcg(vin + i) : 0u;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int it = 0; it < IPT; ++it) {
+            const bool valid = base + it * 32 < n;
+            const unsigned dg = valid ? (key[it] >> shift) & 0xFFu : 256u;
+            const unsigned peers = __match_any_sync(0xffffffffu, dg);
+            const unsigned r = __popc(peers & lt);
+            const unsigned prior = valid ? sh.wcount[warp][dg] : 0u;
+            place[it] = prior + r;
+            __syncwarp();
+            if (valid && r == 0) sh.wcount[warp][dg] = prior + __popc(peers);
+            __syncwarp();
+        }
+        __syncthreads();
+        if (tid < 256) {  // exclusive prefix over the warps
+            unsigned run = 0;
+#pragma unroll 8
+            for (int w = 0; w < kCsWarps; ++w) {
+                const unsigned t = sh.wcount[w][tid];
+                sh.wcount[w][tid] = run;
+                run += t;
+            }
+            sh.totals[pass & 1][tid] = run;
+        }
+        cl.sync();
+        // places of the lower digits' pairs and of the same digit's in lower CTAs
+        unsigned all = 0, lower = 0;
+        if (tid < 256) {
+            for (int c = 0; c < kCsCtas; ++c) {
+                const unsigned t = *cl.map_shared_rank(&sh.totals[pass & 1][tid], c);
+                all += t;
+                lower += c < rank ? t : 0u;
+            }
+            const int incl = warp_inclusive_scan(static_cast<int>(all));
+            if (lane == 31) sh.warp_sums[warp] = incl;
+            sh.first[tid] = static_cast<unsigned>(incl) - all + lower;
+        }
+        __syncthreads();
+        if (tid < 256) {
+            unsigned before = 0;
+            for (int w = 0; w < warp; ++w) before += static_cast<unsigned>(sh.warp_sums[w]);
+            sh.first[tid] += before;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int it = 0; it < IPT; ++it) {
+            if (base + it * 32 < n) {
+                const unsigned dg = (key[it] >> shift) & 0xFFu;
+                const unsigned pos = sh.first[dg] + sh.wcount[warp][dg] + place[it];
+                __stcg(kout + pos, key[it]);
+                __stcg(vout + pos, val[it]);
+            }
+        }
+        cl.sync();  // the next pass reads what every CTA wrote
+        unsigned* t = kin;
+        kin = kout;
+        kout = t;
+        t = vin;
+        vin = vout;
+        vout = t;
+    }
+}
+
+template <int IPT>
+void launch_cluster_sort(unsigned* keys, unsigned* vals, unsigned* keys_tmp, unsigned* vals_tmp, int n, int key_bits,
+                         cudaStream_t s) {
+    set_max_dynamic_smem(reinterpret_cast<const void*>(cluster_sort_kernel<IPT>), sizeof(ClusterSortSmem));
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute attr{};
+    cfg.gridDim = dim3(kCsCtas);
+    cfg.blockDim = dim3(kCsThreads);
+    cfg.dynamicSmemBytes = sizeof(ClusterSortSmem);
+    cfg.stream = s;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = kCsCtas;
+    attr.val.clusterDim.y = 1;
+    attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    CG_CUDA(cudaLaunchKernelEx(&cfg, cluster_sort_kernel<IPT>, keys, vals, keys_tmp, vals_tmp, n, key_bits));
+    count_launch();
+}
+
 int grid_for(int64_t items, int block) {
     int64_t g = ceil_div(items, block);
     if (g > 152 * 8) g = 152 * 8;
@@ -584,6 +714,16 @@ unsigned* sort_pairs_stable(unsigned* keys, unsigned* vals, unsigned* keys_tmp, 
                             int key_bits, unsigned* counts, cudaStream_t s, unsigned** vals_out) {
     const int nblocks = static_cast<int>(ceil_div(n, kSortTile));
     unsigned* totals = counts + static_cast<int64_t>(256) * nblocks;
+    if (n <= kCsMax) {
+        const int ni = static_cast<int>(n), per = static_cast<int>(ceil_div(n, kCsCtas * kCsThreads));
+        if (per <= 1) launch_cluster_sort<1>(keys, vals, keys_tmp, vals_tmp, ni, key_bits, s);
+        else if (per <= 2) launch_cluster_sort<2>(keys, vals, keys_tmp, vals_tmp, ni, key_bits, s);
+        else if (per <= 4) launch_cluster_sort<4>(keys, vals, keys_tmp, vals_tmp, ni, key_bits, s);
+        else launch_cluster_sort<kCsItems>(keys, vals, keys_tmp, vals_tmp, ni, key_bits, s);
+        const bool back = (key_bits + 7) / 8 % 2 == 0;  // an even number of passes: in the first buffers
+        *vals_out = back ? vals : vals_tmp;
+        return back ? keys : keys_tmp;
+    }
     unsigned *kin = keys, *vin = vals, *kout = keys_tmp, *vout = vals_tmp;
     for (int shift = 0; shift < key_bits; shift += 8) {
         sort_upsweep_kernel<<<nblocks, kSortThreads, 0, s>>>(kin, n, shift, counts, nblocks);

@@ -65,3 +65,14 @@ def test_forced_fused_paths_still_refuse_more_than_128_features():
             ctx.set_path(path)
             with pytest.raises(ValueError):
                 ctx.lof(X, 10)
+
+
+@pytest.mark.parametrize("n", [7169, 8193, 16385, 32769, 65536, 65537])
+def test_spatial_order_sorts(n):
+    # the one-launch sort's pairs per thread and its limit, through the small-d
+    # path (every point is placed once: the k-NN graph is the oracle's)
+    X = synthetic.clusters_with_outliers(n, 3, seed=n)
+    with _culof.Context() as ctx:
+        ctx.set_path(_culof.PATH_FAST)
+        got = ctx.lof(X, 12)
+    np.testing.assert_array_equal(got.view(np.uint32), oracle.lof(X, 12).view(np.uint32))
