@@ -19,7 +19,7 @@ namespace culof_gb300 {
 
 namespace {
 
-constexpr int kApplyThreads = 256;
+constexpr int kApplyThreads = 1024;  // at most (center_apply_kernel)
 
 __device__ __forceinline__ double center_term(double s, float x, double m, bool square) {
     if (!square) return __dadd_rn(s, widen(x));
@@ -105,14 +105,19 @@ __global__ void center_finalize_kernel(const double* __restrict__ partial, int64
     }
 }
 
-// A value times the feature's scale; without normalising the scale is 1 and
-// the product the value itself.
-__device__ __forceinline__ double scale_by(double v, double inv) { return inv == 1.0 ? v : __dmul_rn(v, inv); }
-
 // One pass over the n x d values: each thread stays on one feature (the
-// block's active threads and its stride are multiples of d). With mm, also
-// the features' ranges for the spatial order (range_put), reduced in shared
-// memory first.
+// block's active threads and its stride are multiples of d) and has
+// kApplyLoads loads in flight. With mm, also the features' ranges for the
+// spatial order (range_put), reduced in shared memory first. One load at a
+// time, a comparison and a product per value that does not need them (an FP64
+// instruction each) and 256-thread blocks with two global atomics per feature
+// each took 158 us at n = 200,000, d = 128 (now 91, where the one FP64
+// instruction per value takes 44), 39 at n = 30,011, d = 100 (16) and 32 at
+// n = 8,000, d = 200 (13). Blocks of 1,024 threads mean fewer atomics; below
+// d = 32, where those are few, the 341 threads of a feature in one block's
+// shared atomics cost more (8 us for 5 at n = 50,021, d = 3): 256 threads.
+constexpr int kApplyLoads = 4;
+template <bool kScale>  // normalising (otherwise the scale is 1 and the product the value itself)
 __global__ void __launch_bounds__(kApplyThreads)
 center_apply_kernel(const float* __restrict__ x, int64_t n, int d, const double* __restrict__ mean,
                     const double* __restrict__ inv_std, float* __restrict__ xc, unsigned* __restrict__ mm) {
@@ -122,18 +127,29 @@ center_apply_kernel(const float* __restrict__ x, int64_t n, int d, const double*
         __syncthreads();
     }
     const int64_t total = n * d;
-    if (d <= kApplyThreads) {
-        const int per = kApplyThreads / d * d;  // active threads
+    if (d <= static_cast<int>(blockDim.x)) {
+        const int per = static_cast<int>(blockDim.x) / d * d;  // active threads
         if (static_cast<int>(threadIdx.x) < per) {
             const int f = static_cast<int>(threadIdx.x) % d;
             const double m = mean[f], inv = inv_std[f];
             unsigned lo = 0u, hi = 0u;
+            const int64_t stride = static_cast<int64_t>(gridDim.x) * per;
             for (int64_t t = static_cast<int64_t>(blockIdx.x) * per + threadIdx.x; t < total;
-                 t += static_cast<int64_t>(gridDim.x) * per) {
-                const float v = narrow(scale_by(__dsub_rn(widen(x[t]), m), inv));
-                xc[t] = v;
-                lo = max(lo, ~range_key(v));
-                hi = max(hi, range_key(v));
+                 t += stride * kApplyLoads) {
+                float v[kApplyLoads];
+#pragma unroll
+                for (int j = 0; j < kApplyLoads; ++j)
+                    if (t + j * stride < total) v[j] = x[t + j * stride];
+#pragma unroll
+                for (int j = 0; j < kApplyLoads; ++j) {
+                    if (t + j * stride >= total) break;
+                    double w = __dsub_rn(widen(v[j]), m);
+                    if (kScale) w = __dmul_rn(w, inv);
+                    const float c = narrow(w);
+                    xc[t + j * stride] = c;
+                    lo = max(lo, ~range_key(c));
+                    hi = max(hi, range_key(c));
+                }
             }
             if (mm != nullptr) {
                 atomicMax(&slo[f], lo);
@@ -144,14 +160,17 @@ center_apply_kernel(const float* __restrict__ x, int64_t n, int d, const double*
         for (int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; t < total;
              t += static_cast<int64_t>(gridDim.x) * blockDim.x) {
             const int f = static_cast<int>(t % d);
-            xc[t] = narrow(scale_by(__dsub_rn(widen(x[t]), mean[f]), inv_std[f]));
+            double w = __dsub_rn(widen(x[t]), mean[f]);
+            if (kScale) w = __dmul_rn(w, inv_std[f]);
+            xc[t] = narrow(w);
         }
     }
     if (mm != nullptr) {
         __syncthreads();
         for (int f = threadIdx.x; f < d; f += blockDim.x) {
-            atomicMax(&mm[2 * f], slo[f]);
-            atomicMax(&mm[2 * f + 1], shi[f]);
+            // (ranges only grow: most blocks find theirs covered and write nothing)
+            if (__ldcg(&mm[2 * f]) < slo[f]) atomicMax(&mm[2 * f], slo[f]);
+            if (__ldcg(&mm[2 * f + 1]) < shi[f]) atomicMax(&mm[2 * f + 1], shi[f]);
         }
     }
 }
@@ -224,7 +243,9 @@ center_small_kernel(const float* __restrict__ x, int n, int d, int normalize, do
     const double m = stat[0], v = stat[1];
     unsigned lo = 0u, hi = 0u;
     for (int i = tid; i < n; i += kSmallThreads) {
-        const float c = narrow(scale_by(__dsub_rn(widen(col[i + i / kCenterChunk]), m), v));
+        double w = __dsub_rn(widen(col[i + i / kCenterChunk]), m);
+        if (normalize) w = __dmul_rn(w, v);
+        const float c = narrow(w);
         xc[static_cast<int64_t>(i) * d + f] = c;
         lo = max(lo, ~range_key(c));
         hi = max(hi, range_key(c));
@@ -240,7 +261,11 @@ center_small_kernel(const float* __restrict__ x, int n, int d, int normalize, do
 }
 
 // norms[i] = (float) sum_f (double) xc[i,f]^2 (feature order), and the
-// maximum norm (non-negative float bits order like the values).
+// maximum norm (non-negative float bits order like the values). Bound by the
+// chain of d multiply-adds per row: blocks of 64 rows reach every SM from
+// 10,000 rows on, and a row's loads are 16 bytes wide (d a multiple of 4),
+// because each touches 32 lines: 47 us at n = 200,000, d = 128 and 20 at
+// n = 8,000, d = 200, where blocks of 256 rows and single loads took 101 and 29.
 __global__ void norms_kernel(const float* __restrict__ xc, int64_t n, int d,
                              float* __restrict__ norms, unsigned int* __restrict__ max_norm_bits) {
     unsigned int local_max = 0u;
@@ -248,9 +273,23 @@ __global__ void norms_kernel(const float* __restrict__ xc, int64_t n, int d,
          i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
         const float* row = xc + i * d;
         double s = 0.0;
-        for (int f = 0; f < d; ++f) {
+        int f = 0;
+        if ((d & 3) == 0) {
+            const float4* r4 = reinterpret_cast<const float4*>(row);
+            for (; f + 16 <= d; f += 16) {
+                float4 u[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) u[j] = r4[f / 4 + j];
+#pragma unroll
+                for (int j = 0; j < 16; ++j) {
+                    const double v = widen(reinterpret_cast<const float*>(u)[j]);
+                    s = __fma_rn(v, v, s);  // (the square of a float is exact in double)
+                }
+            }
+        }
+        for (; f < d; ++f) {
             const double v = widen(row[f]);
-            s = __fma_rn(v, v, s);  // (the square of a float is exact in double)
+            s = __fma_rn(v, v, s);
         }
         const float nf = __double2float_rn(s);
         norms[i] = nf;
@@ -301,13 +340,16 @@ void center(const float* x, int64_t n, int d, bool normalize, float* xc, double*
         CG_LAUNCH_CHECK();
     }
     if (xc == nullptr) return;
-    center_apply_kernel<<<grid_for(n * d, kApplyThreads, 152 * 8), kApplyThreads, 0, s>>>(x, n, d, mean, inv_std, xc, mm);
+    const int ablock = d < 32 ? 256 : kApplyThreads;
+    const int agrid = grid_for(n * d, ablock * kApplyLoads, 152 * 2048 / ablock);
+    if (normalize) center_apply_kernel<true><<<agrid, ablock, 0, s>>>(x, n, d, mean, inv_std, xc, mm);
+    else center_apply_kernel<false><<<agrid, ablock, 0, s>>>(x, n, d, mean, inv_std, xc, mm);
     CG_LAUNCH_CHECK();
 }
 
 void squared_norms(const float* xc, int64_t n, int d, float* norms, unsigned int* max_norm_bits,
                    cudaStream_t s) {
-    norms_kernel<<<grid_for(n, 256), 256, 0, s>>>(xc, n, d, norms, max_norm_bits);
+    norms_kernel<<<grid_for(n, 64, 152 * 32), 64, 0, s>>>(xc, n, d, norms, max_norm_bits);
     CG_LAUNCH_CHECK();
 }
 
