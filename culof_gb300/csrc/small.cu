@@ -107,12 +107,18 @@ __global__ void __launch_bounds__(kCT) small_tile_kernel(const float* __restrict
 // point; a point's sort key is its coordinate's order-preserving bits with
 // the low 10 replaced by its place in the chunk (the order is a heuristic, no
 // result depends on it).
+// Bound by the instructions and barriers of the sorts. Chunks of 512 take half
+// the time (18 us for 34 at n = 20,000, d = 8) and cost the sweep more (277 us
+// for 253; 3,759 for 3,599 at n = 200,000). The V sums of a level by V
+// reductions of their own took 40 and 66 us, together 34 and 59.
 constexpr int kChunk = 1024;
+template <int DP>
 __global__ void __launch_bounds__(kChunk) refine_order_kernel(const float* __restrict__ xc, int64_t n, int d,
                                                               unsigned* __restrict__ perm) {
-    __shared__ float xs[kMaxDP][kChunk];
+    constexpr int V = DP <= 2 ? 4 : DP <= 4 ? 8 : 16;  // sums and sums of squares, padded
+    __shared__ float xs[DP][kChunk];
     __shared__ unsigned key_s[kChunk];
-    __shared__ float stat[kChunk / 32][kMaxDP][2];
+    __shared__ float stat[kChunk / 32][V];
     __shared__ float cnt[kChunk / 32];
     __shared__ unsigned orig[kChunk];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -130,29 +136,37 @@ __global__ void __launch_bounds__(kChunk) refine_order_kernel(const float* __res
     for (int size = kChunk; size >= 32; size >>= 1) {
         // the segment's dimension of largest variance
         const bool in = static_cast<int>(slot) < m;
-        for (int f = 0; f < d; ++f) {
-            const float v = in ? xs[f][slot] : 0.0f;
-            float s1 = v, s2 = v * v;
+        float v[V];
 #pragma unroll
-            for (int st = 16; st > 0; st >>= 1) {
-                s1 += __shfl_xor_sync(kFullMask, s1, st);
-                s2 += __shfl_xor_sync(kFullMask, s2, st);
-            }
-            if (lane == 0) {
-                stat[warp][f][0] = s1;
-                stat[warp][f][1] = s2;
+        for (int f = 0; f < V / 2; ++f) {
+            const float x = in && f < d ? xs[f < DP ? f : 0][slot] : 0.0f;
+            v[2 * f] = x;
+            v[2 * f + 1] = x * x;
+        }
+        // the warp's V sums, halving the number of values with each exchange:
+        // sum lane / (32 / V) ends up in every lane
+#pragma unroll
+        for (int h = V / 2, st = 16; h > 0; h >>= 1, st >>= 1) {
+            const bool up = (lane & st) != 0;
+#pragma unroll
+            for (int j = 0; j < h; ++j) {
+                const float give = up ? v[j] : v[j + h], keep = up ? v[j + h] : v[j];
+                v[j] = keep + __shfl_xor_sync(kFullMask, give, st);
             }
         }
+#pragma unroll
+        for (int st = 16 / V; st > 0; st >>= 1) v[0] += __shfl_xor_sync(kFullMask, v[0], st);
+        if (lane % (32 / V) == 0) stat[warp][lane / (32 / V)] = v[0];
         const unsigned here = __ballot_sync(kFullMask, in);
         if (lane == 0) cnt[warp] = static_cast<float>(__popc(here));
         __syncthreads();
         const int w0 = tid / size * (size / 32), nw = size / 32;
         float var = -1.0f;
-        if (lane < d) {
+        if (lane < d) {  // (d <= DP <= V / 2)
             float s1 = 0.0f, s2 = 0.0f, c = 0.0f;
             for (int w = 0; w < nw; ++w) {
-                s1 += stat[w0 + w][lane][0];
-                s2 += stat[w0 + w][lane][1];
+                s1 += stat[w0 + w][2 * lane];
+                s2 += stat[w0 + w][2 * lane + 1];
                 c += cnt[w0 + w];
             }
             var = c > 0.0f ? s2 - s1 * s1 / c : 0.0f;
@@ -493,7 +507,13 @@ int64_t iso_capacity(int mt) { return static_cast<int64_t>(mt) * kCT / 4 + stati
 }  // namespace
 
 void small_refine_order(const float* xc, int64_t n, int d, unsigned* perm, cudaStream_t s) {
-    refine_order_kernel<<<static_cast<unsigned>(ceil_div(n, kChunk)), kChunk, 0, s>>>(xc, n, d, perm);
+    const unsigned grid = static_cast<unsigned>(ceil_div(n, kChunk));
+    switch (padded_dims(d)) {
+        case 2: refine_order_kernel<2><<<grid, kChunk, 0, s>>>(xc, n, d, perm); break;
+        case 4: refine_order_kernel<4><<<grid, kChunk, 0, s>>>(xc, n, d, perm); break;
+        case 6: refine_order_kernel<6><<<grid, kChunk, 0, s>>>(xc, n, d, perm); break;
+        default: refine_order_kernel<8><<<grid, kChunk, 0, s>>>(xc, n, d, perm); break;
+    }
     CG_LAUNCH_CHECK();
 }
 
