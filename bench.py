@@ -12,14 +12,15 @@ offset and the labels.
 * e2e: the same metric through culof_context_fit_predict with pinned host
   buffers: host->device copy of X, the pipeline and the device->host copy of
   nof + labels + offset, every step (wall time of the synchronous call).
-* roofline: the distance sweep kernel (the dominant kernel): the algorithmic
-  work, 2d FLOP for each of the n (n - 640) pairs outside the rows' seed
-  windows (the own tile and its four nearest Morton neighbour tiles, which
-  the seed kernel covers; one evaluation per pair), over its event time,
-  against the measured FP32 FMA peak. The kernel skips column tiles that a bounding-box test proves
-  farther than every k-th neighbour; the pairs it actually evaluated, the
-  pruned fraction and its FLOP rate on the evaluated pairs are reported
-  beside it (executed_tflops, executed_frac).
+* roofline: the sweep stage (small_sweep_kernel, the dominant kernel, and
+  the pass over the rows that leave it): the algorithmic work, 2d FLOP for
+  each of the n (n - 640) pairs outside the rows' windows (the own tile and
+  its four nearest Morton neighbour tiles, which the kernel always
+  evaluates; one evaluation per pair), over its event time, against the
+  measured FP32 FMA peak. The kernel skips, row by row, the 64-column halves
+  that a bounding-box test proves farther than the row's k-th neighbour; the
+  pairs it actually evaluated, the pruned fraction and its FLOP rate on the
+  evaluated pairs are reported beside it (executed_tflops, executed_frac).
 * cpu_baseline: one whole fit_predict of the same workload (centre, exact
   k-NN of all n rows, LRD, scores, offset, labels) by the CPU oracle, a C
   restatement of the same exact algorithm, on all host threads.
@@ -57,7 +58,7 @@ L2_FLUSH_BYTES = 256 << 20
 
 PATH_NAMES = ["auto", "fast", "general", "tensor"]
 
-# DRAM traffic of one sweep_kernel launch, measured by one ncu capture of this
+# DRAM traffic of one small_sweep_kernel launch, measured by one ncu capture of this
 # very workload (dram__bytes_read.sum + dram__bytes_write.sum); other
 # workloads report null.
 MEASURED_SWEEP_TRAFFIC = {
@@ -405,17 +406,17 @@ def run_ours(args):
 
     stages = {name: statistics.mean(v) for name, v in stage_acc.items()}
     fp32_peak = max(_culof.probe_fp32_tflops(True), _culof.probe_fp32_tflops(False))
-    # the sweep evaluates every pair outside the rows' seed window: the own
-    # 128-point tile (tensor and wide paths), or the own tile and its four
-    # nearest Morton neighbour tiles (small-d path, d <= 8)
+    # the sweep's share: every pair outside the rows' window, the own 128-point
+    # tile (tensor and wide paths), or the own tile and its four nearest Morton
+    # neighbour tiles (small-d path, d <= 8)
     nt = (n + 127) // 128
     window = min(nt, 5) if (ctx.last_path() == _culof.PATH_FAST and d <= 8) else 1
     sweep_pairs = float(n) * float(n - min(n, 128 * window)) if nt > window else 0.0
     sweep_ms = stages.get("sweep")
     roofline = None
     if sweep_ms and sweep_pairs > 0 and ctx.last_path() == _culof.PATH_TENSOR:
-        # the f16 Gram of every pair on the tensor cores (K = d padded to 64/128)
-        kp = 64 if d <= 64 else 128
+        # the f16 Gram of every pair on the tensor cores (K = d padded to a multiple of 64)
+        kp = (d + 63) // 64 * 64
         peak, peak_src = tensor_peak()
         achieved = 2.0 * kp * sweep_pairs / (sweep_ms * 1e-3) / 1e12
         roofline = {
@@ -432,7 +433,7 @@ def run_ours(args):
             "sweep_share_of_step": sweep_ms / mean_ms,
         }
     elif sweep_ms and sweep_pairs > 0 and ctx.last_path() == _culof.PATH_FAST:
-        # algorithmic work: 2d FLOP for every pair past the row's seed window
+        # algorithmic work: 2d FLOP for every pair past the row's window
         # (one evaluation per pair); the kernel itself evaluates only the
         # pairs of column tiles a bounding-box test cannot rule out, and its
         # efficiency on those is reported beside it
@@ -441,7 +442,7 @@ def run_ours(args):
         traffic, traffic_src = MEASURED_SWEEP_TRAFFIC.get((args.workload, n, d, k), (None, None))
         roofline = {
             "bound": "fp32",
-            "kernel": "sweep_kernel (fused distance + filtered exact select)",
+            "kernel": "small_sweep_kernel (exact distances with per-row pruning + exact select)",
             "achieved": achieved,
             "peak": fp32_peak,
             "unit": "TFLOP/s",

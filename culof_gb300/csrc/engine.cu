@@ -130,25 +130,34 @@ int Engine::tile_rows_for(int64_t n) {
 }
 
 // AUTO, with the direct two-pass kernel (direct.cu) wherever it is fastest; all
-// give the same bits. lof_device on clusters, k = 20, one call, in us:
-//   d        n     direct  small-d   tensor   tile + select
-//   8     4000        128      278
-//   8     8000        329      327             (direct up to 7168 points)
-//  12     4000        180               204
-//  12     8000        480               261    (direct up to 4096 points)
-//  24     3000                          206             217
-//  24     2000                          194             146  (tensor from 2561)
-// 128     4000                          251             541
-// - n <= 4096 (2560 for d > 16): the general path, which takes the direct
-//   kernel for d <= 16 and k <= 64;
-// - d <= 8: the FP32 path (direct up to 7168 points, then the small-d sweep);
-//   8 < d <= 16 up to 7168 points: the FP32 path by the direct kernel too,
-//   which ties the tensor path there and keeps every stage in FP32;
+// give the same bits. k-NN on clusters (d = 128: factor model), one call, in us:
+//   d     n   k   direct  small-d   tensor   tile + select
+//   3   7168  20     155      226
+//   8   7168  20     242      273             (at 8000 direct 329, small-d 267)
+//  12   4096  20     179               157
+//  12   7168  20     376               194
+//  16   3000  20     178               148             203
+//  16   5000  20     363               168
+//  16   7000  64     548              1300
+//  24   2560  20                       143             180
+//  24   3000  64                       776             237
+//  43   3000  20                       602             264
+// 128   3000  20                       168             384
+// - n <= 4096: the general path, which takes the direct kernel for d <= 16 and
+//   k <= 64. From 2561 points the tensor path for split f16 operands (16 < d
+//   <= 42) and k <= 48: with single operands its time depends on the data's
+//   spread (43 and 128 features above), and past k = 48 its lists have little
+//   room for the filter's margin. Also for d > 128, where the tile costs most
+//   (factor model, d = 200, n = 3,000: 180 us for 430).
+// - d <= 8: the FP32 path (direct up to 7168 points, then the small-d sweep).
+// - 8 < d <= 16: the direct kernel as far as it wins, 7168 points past k = 48
+//   and 4096 for d > 12 else; for d <= 12 up to 6144, where the tensor path
+//   would be faster from about 4000 on: this range is documented as FP32.
 // - otherwise the tensor path up to d = 256, the general path beyond and for
 //   k > 64.
 // CULOF_GB300_PATH=general|fast|tensor overrides AUTO for a process.
-constexpr int64_t kSmallN = 4096, kSmallWideN = 2560, kDirectFastN = 7168;
-constexpr int64_t kDirectGeneralN = 8192;
+constexpr int64_t kSmallN = 4096, kSmallSplitN = 2560, kDirectFastN = 7168, kDirectMidN = 6144;
+constexpr int kRoomyK = 48;
 int Engine::choose_path(int64_t n, int d, int k, bool* direct) const {
     int p = path_;
     *direct = false;
@@ -162,14 +171,17 @@ int Engine::choose_path(int64_t n, int d, int k, bool* direct) const {
     const bool ok = fast_path_supported(n, d, k);
     if ((p == kPathFast || p == kPathTensor) && !ok)
         throw Error(kInvalidArgument, "fused path requested but unsupported for this n/d/k");
-    if (p == kPathFast || p == kPathTensor) return p;
+    if (p != kPathAuto) return p;  // a path asked for by name runs its own kernels
     const bool direct_ok = direct_supported(n, d, k);
-    if (p == kPathGeneral || n <= (d > 16 ? kSmallWideN : kSmallN) || !tensor_supported(n, d, k)) {
-        *direct = direct_ok && n <= kDirectGeneralN;
+    const bool tensor_early = (d > 16 && d <= kTcSplitD && k <= kRoomyK) || d > 128;
+    const int64_t small = tensor_early ? kSmallSplitN : kSmallN;
+    if (n <= small || !tensor_supported(n, d, k)) {
+        *direct = direct_ok && n <= kSmallN;
         return kPathGeneral;
     }
-    if (d <= 8 || (d <= 16 && n <= kDirectFastN)) {
-        *direct = direct_ok && n <= kDirectFastN;
+    const int64_t fp32 = d <= 8 || k > kRoomyK ? kDirectFastN : d <= 12 ? kDirectMidN : kSmallN;
+    if (d <= 8 || (d <= 16 && n <= fp32)) {
+        *direct = direct_ok && n <= fp32;
         return kPathFast;
     }
     return kPathTensor;

@@ -46,8 +46,6 @@ namespace {
 
 using namespace small;
 
-constexpr int kPairs = kCT / 2;
-constexpr int kRowsPerLane = 4;
 constexpr int kSeedWindow = 5;  // tiles of the seed: T, T+1, T-1, T+2, T-2
 constexpr int kMaxWideD = 128;
 constexpr int kMortonDims = 8;  // Morton key over (up to) the 8 widest dimensions
@@ -779,12 +777,15 @@ void Engine::knn_fast(const float* xc, const float* norms, int64_t n, int d, int
             if (nsplit > nt - 1) nsplit = nt - 1;
         } else if (tensor) {
             const int64_t slots = 2 * sms;  // CTAs at a time
+            // (k > 56 leaves a list little room for the filter's margin: most
+            // rows rescore candidates exactly, and every split pays that anew)
+            const int64_t own = k > 56 ? 256 : 64;
             int64_t best = -1;
             // (past two rounds the list entries that every split repeats cost
             // more than the last round's idle SMs: n = 200,000, d = 128, k = 50,
             // 24.2 ms with one split, 31.0 with two)
             for (int v = 1; v <= (mt >= 2 * slots ? 1 : tc_max_splits()) && v < nt; ++v) {
-                const int64_t cost = ceil_div(static_cast<int64_t>(mt) * v, slots) * (nt / v + 64);
+                const int64_t cost = ceil_div(static_cast<int64_t>(mt) * v, slots) * (nt / v + own);
                 if (best < 0 || cost < best) {
                     best = cost;
                     nsplit = v;

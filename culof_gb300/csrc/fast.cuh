@@ -58,6 +58,7 @@ struct TcBuffers {
     float* cn;
     unsigned* ix;
     void* scale;
+    float* rn;  // residual norms of the operand rows (single operands)
     int Kp;
     int dr;
     int split;
@@ -69,6 +70,7 @@ TcBuffers tc_prepare(void* buf, const float* xc, const float* norms, int64_t n, 
                      const unsigned* minmax, cudaStream_t s);
 int tc_max_splits();
 constexpr int kMaxTensorD = 256;
+constexpr int kTcSplitD = 42;  // split operands up to here (3d <= 128)
 // True when the tensor path handles (n, d, k) (AUTO only above d = 128).
 bool tensor_supported(int64_t n, int d, int k);
 // Workspace of the per-row lists of one sweep launch batch.

@@ -73,9 +73,11 @@ constexpr int kBox = 128 * 128;                   // bytes of one TMA box: 128 r
 
 // Scale record on the device: sc = 2^S, k2 = -2 * 2^-2S (undoes the scale of
 // a Gram value and doubles it), eta = 2^-14 * 2^-S (absolute f16 rounding
-// bound in unscaled units), all = 1 when the filter is disabled.
+// bound in unscaled units), all = 1 when the filter is disabled, resmax the
+// largest residual norm (tc_resid_kernel).
 struct TcScale {
     float sc, k2, eta, all;
+    unsigned resmax;  // float bits
 };
 
 __device__ __forceinline__ float unflip(unsigned k) {
@@ -106,6 +108,7 @@ __global__ void tc_scale_kernel(const unsigned* __restrict__ mm, int d, TcScale*
     r.k2 = -ldexpf(1.0f, 1 - 2 * S);
     r.eta = ldexpf(1.0f, -14 - S);
     r.all = all ? 1.0f : 0.0f;
+    r.resmax = 0u;
     *out = r;
 }
 
@@ -146,15 +149,50 @@ __global__ void tc_build_kernel(const float* __restrict__ xc, const float* __res
     }
 }
 
+// Residual norms of the single f16 operands: rn[p] >= |a - f16(a)| (unscaled;
+// an operand below the f16 normal range may be flushed, so its residual is the
+// larger of the value and its rounding error), and the largest of them. A
+// warp per row; every rounding upwards. Bound by reading the coordinates. The
+// worst case over all values, 2^-11 |a|, is about two and a half times the
+// measured norm, and the filter's margin follows it (row_bounds): with it
+// clusters of d = 64, n = 20,000, k = 20 take 3.1 ms for 6.7.
+__global__ void __launch_bounds__(256) tc_resid_kernel(const float* __restrict__ xr, int64_t padded, int d, int dr,
+                                                       TcScale* __restrict__ scale, float* __restrict__ rn) {
+    const int lane = threadIdx.x & 31;
+    const float sc = scale->sc;
+    float most = 0.0f;
+    const int64_t step = static_cast<int64_t>(gridDim.x) * 8;
+    for (int64_t p = static_cast<int64_t>(blockIdx.x) * 8 + (threadIdx.x >> 5); p < padded; p += step) {
+        float s = 0.0f;
+        for (int f = lane; f < d; f += 32) {
+            const float xs = xr[p * dr + f] * sc;
+            const float hi = __half2float(__float2half_rn(xs));
+            float r = fabsf(__fsub_rn(xs, hi));
+            if (fabsf(hi) < 6.103515625e-05f) r = fmaxf(r, fabsf(xs));  // 2^-14
+            s = __fmaf_ru(r, r, s);
+        }
+#pragma unroll
+        for (int st = 16; st > 0; st >>= 1) s = __fadd_ru(s, __shfl_xor_sync(0xffffffffu, s, st));
+        const float v = __fdiv_ru(__fsqrt_ru(s), sc);
+        if (lane == 0) rn[p] = v;
+        most = fmaxf(most, v);
+    }
+    __shared__ unsigned top;
+    if (threadIdx.x == 0) top = 0u;
+    __syncthreads();
+    if (lane == 0) atomicMax(&top, __float_as_uint(most));
+    __syncthreads();
+    if (threadIdx.x == 0 && __ldcg(&scale->resmax) < top) atomicMax(&scale->resmax, top);
+}
+
 // ---- thresholds ---------------------------------------------------------------
 // Per row a (float32 norm na, K = Kp terms, u = 2^-24, g the relative error of
-// the float32 norms, A >= |a|, B >= |b| for every column b), the f16 Gram value
-// G of a column b and its filter value f = fl(Nb - 2 G) satisfy
-//   |G - a.b| <= E = (2 uh + uh^2) A B + eta (1 + uh) sqrt(K) (A + B) + K eta^2
-//                    + K ua ((1 + uh) A + sqrt(K) eta) ((1 + uh) B + sqrt(K) eta)
+// the float32 norms, A >= |a|, B >= |b| for every column b, ra >= |a - f16(a)|,
+// rb >= |b - f16(b)| for every column b), the f16 Gram value G of a column b
+// and its filter value f = fl(Nb - 2 G) satisfy
+//   |G - a.b| <= E = ra B + (A + ra) rb + K ua (A + ra) (B + rb)
 //   |f - (|b|^2 - 2 a.b)| <= m0 = g / (1 - g) Nmax + 2 E + u (Nmax + 2 (A B + E))
-// (uh = 2^-11 the f16 rounding, eta the absolute f16 error, ua = 2^-20 per
-// accumulated term of the tensor core). Two consequences, each evaluated with
+// (ua = 2^-20 per accumulated term of the tensor core). Two consequences, each evaluated with
 // upward rounding:
 //  * exact threshold: a column whose exact float32 distance is <= D has
 //    f <= D c1 + c0 (c1 = (1 + 8u) / (1 - (K + 2) u),
@@ -165,7 +203,8 @@ __global__ void tc_build_kernel(const float* __restrict__ xc, const float* __res
 //    (+ slack) is strictly farther than every column c with f_c <= fk, so once
 //    k columns with f <= fk are known, b can never be among the k nearest.
 // With split operands (x = hi + r exactly, lo = f16(r), |r| <= uh |x|,
-// |lo - r| <= uh |r| + eta) the summed products hi.hi + lo.hi + hi.lo miss
+// |lo - r| <= uh |r| + eta, uh = 2^-11 the f16 rounding, eta the absolute f16
+// error) the summed products hi.hi + lo.hi + hi.lo miss
 // a.b by at most
 //   E = (3 uh^2 + 3 uh^3) A B + eta (1 + uh) sqrt(d) (A + B) + 2 d eta^2
 //       + Ka ua (1 + 3 uh) ((1 + uh) A + sqrt(Ka) eta) ((1 + uh) B + sqrt(Ka) eta)
@@ -175,7 +214,8 @@ struct RowBounds {
 };
 constexpr double kU = 5.9604644775390625e-08;  // 2^-24
 
-__device__ RowBounds row_bounds(float na_f, float nmax_f, int K, float eta_f, int split_d, int kacc) {
+__device__ RowBounds row_bounds(float na_f, float nmax_f, int K, float ra_f, float rb_f, float eta_f, int split_d,
+                                int kacc) {
     const double uh = 4.8828125e-04;        // 2^-11
     const double ua = 9.5367431640625e-07;  // 2^-20
     const double g = (K + 1) * kU / (1.0 - (K + 1) * kU);
@@ -188,9 +228,8 @@ __device__ RowBounds row_bounds(float na_f, float nmax_f, int K, float eta_f, in
             2.0 * split_d * eta * eta +
             kacc * ua * (1.0 + 3.0 * uh) * ((1.0 + uh) * A + sa * eta) * ((1.0 + uh) * B + sa * eta);
     } else {
-        const double sk = sqrt(static_cast<double>(K));
-        E = (2.0 * uh + uh * uh) * A * B + eta * (1.0 + uh) * sk * (A + B) + K * eta * eta +
-            K * ua * ((1.0 + uh) * A + sk * eta) * ((1.0 + uh) * B + sk * eta);
+        const double ra = static_cast<double>(ra_f), rb = static_cast<double>(rb_f);
+        E = ra * B + (A + ra) * rb + K * ua * (A + ra) * (B + rb);
     }
     const double m0 = g / (1.0 - g) * m + 2.0 * E + kU * (m + 2.0 * (A * B + E));
     const double slack = 8.0 * kU * (a + m + 2.0 * A * B) + 1e-30;
@@ -307,21 +346,20 @@ __device__ __forceinline__ uint32_t select32(const uint32_t (&g)[32], int b) {
 // Exact key of (row position pa, column position pb), one lane: the oracle's
 // direct-difference chain over row-major FP32 coordinates.
 __device__ __forceinline__ uint64_t exact_key_lane(const float* __restrict__ xr, const unsigned* __restrict__ ix,
-                                                   int64_t pa, int64_t pb, int d, int dr) {
+                                                   int64_t pa, int64_t pb, int dr) {
     const unsigned ib = __ldg(ix + pb);
     if (ib == kNoIndex) return kKeyMax;
     const float4* va = reinterpret_cast<const float4*>(xr + pa * dr);
     const float4* vb = reinterpret_cast<const float4*>(xr + pb * dr);
     float s = 0.0f;
-    for (int f4 = 0; 4 * f4 < d; ++f4) {
+#pragma unroll 4
+    for (int f4 = 0; 4 * f4 < dr; ++f4) {  // (the zero padding past d adds fma(0, 0, s) = s)
         const float4 x = __ldg(va + f4), y = __ldg(vb + f4);
         const float xa[4] = {x.x, x.y, x.z, x.w}, yb[4] = {y.x, y.y, y.z, y.w};
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-            if (4 * f4 + q < d) {
-                const float t = __fsub_rn(xa[q], yb[q]);
-                s = __fmaf_rn(t, t, s);
-            }
+            const float t = __fsub_rn(xa[q], yb[q]);
+            s = __fmaf_rn(t, t, s);
         }
     }
     return make_key(__float_as_uint(s), ib);
@@ -451,13 +489,13 @@ __noinline__ __device__ int approx_compact(TcRows& sh, uint64_t* __restrict__ ls
 // the approximate margin, e.g. many duplicates): every entry is rescored
 // exactly (one lane per entry) and the list becomes an exact k-best list.
 __noinline__ __device__ void to_exact_mode(TcRows& sh, uint64_t* __restrict__ lst, int r, int64_t pa,
-                                           const float* __restrict__ xr, const unsigned* __restrict__ ix, int d,
-                                           int dr, int k) {
+                                           const float* __restrict__ xr, const unsigned* __restrict__ ix, int dr,
+                                           int k) {
     const int lane = threadIdx.x & 31;
     const int c = min(sh.cnt[r], kTcListRow);
     for (int e = lane; e < c; e += 32) {
         const int64_t pb = static_cast<int64_t>(key_index(lst[e]));
-        lst[e] = pb != pa ? exact_key_lane(xr, ix, pa, pb, d, dr) : kKeyMax;  // not the row itself
+        lst[e] = pb != pa ? exact_key_lane(xr, ix, pa, pb, dr) : kKeyMax;  // not the row itself
     }
     __syncwarp();
     if (lane == 0) {
@@ -468,35 +506,75 @@ __noinline__ __device__ void to_exact_mode(TcRows& sh, uint64_t* __restrict__ ls
     compact_exact(sh, lst, r, k);
 }
 
+// Candidates of exact-mode rows waiting to be rescored: one per lane, the
+// first `n` lanes (n the same in all).
+struct ExactPending {
+    int n = 0;
+    int row = 0;      // row of the tile
+    int64_t col = 0;  // column position
+};
+
+// Rescores the pending pairs (whole warp, a lane per pair) and appends the keys
+// that beat their row's k-th key. True if a list was compacted.
+__noinline__ __device__ bool exact_flush(TcRows& sh, uint64_t* __restrict__ glist, const ExactPending& p, int64_t rbase,
+                                         const float* __restrict__ xr, const unsigned* __restrict__ ix, int dr, int k) {
+    const int lane = threadIdx.x & 31;
+    uint64_t key = kKeyMax;
+    if (lane < p.n) key = exact_key_lane(xr, ix, rbase + p.row, p.col, dr);
+    const bool in = lane < p.n && key < sh.kth[p.row];
+    const unsigned peers = __match_any_sync(0xffffffffu, in ? p.row : -1 - lane);
+    const int rank = __popc(peers & ((1u << lane) - 1u));
+    int cnt = 0;
+    if (in) {
+        cnt = sh.cnt[p.row];
+        glist[static_cast<size_t>(p.row) * kTcListRow + cnt + rank] = key;
+    }
+    __syncwarp();
+    if (in && rank == 0) sh.cnt[p.row] = cnt + __popc(peers);
+    __syncwarp();
+    // room for the next 32 of a row
+    unsigned full = __ballot_sync(0xffffffffu, in && rank == 0 && cnt + __popc(peers) > kTcListRow - 32);
+    const bool compacted = full != 0;
+    while (full) {
+        const int r = __shfl_sync(0xffffffffu, p.row, __ffs(full) - 1);
+        full &= full - 1;
+        compact_exact(sh, glist + static_cast<size_t>(r) * kTcListRow, r, k);
+    }
+    return compacted;
+}
+
 // Exact-mode rows of a chunk (whole warp; pass: this lane's row's candidate
-// columns, 0 for rows in approximate mode): per row, lane c rescores column
-// cbase + c exactly and the keys that beat the list's k-th key join it. True
-// if a list was compacted.
-__noinline__ __device__ bool exact_chunk(TcRows& sh, uint64_t* __restrict__ glist, int list0, unsigned pass,
-                                         int64_t pa0, int64_t cbase, const float* __restrict__ xr,
-                                         const unsigned* __restrict__ ix, int d, int dr, int k) {
+// columns, 0 for rows in approximate mode): the chunk's pairs join the pending
+// ones, 32 at a time are rescored. A row at a time, its candidates over the
+// lanes, leaves most lanes idle where the filter's margin is wide but passes a
+// few columns per chunk (clusters, d = 64, n = 20,000, k = 20: 9.3 ms, this
+// way 6.7).
+// True if a list was compacted.
+__noinline__ __device__ bool exact_chunk(TcRows& sh, uint64_t* __restrict__ glist, int row0, unsigned pass,
+                                         ExactPending& p, int64_t rbase, int64_t cbase, const float* __restrict__ xr,
+                                         const unsigned* __restrict__ ix, int dr, int k) {
     const int lane = threadIdx.x & 31;
     bool compacted = false;
-    unsigned rows = __ballot_sync(0xffffffffu, pass != 0u);
-    while (rows) {
-        const int src = __ffs(rows) - 1;
-        rows &= rows - 1;
-        const unsigned cols = __shfl_sync(0xffffffffu, pass, src);
-        const int l = list0 + src;
-        uint64_t* lst = glist + static_cast<size_t>(l) * kTcListRow;
-        const uint64_t key = ((cols >> lane) & 1u) && cbase + lane != pa0 + src
-                                 ? exact_key_lane(xr, ix, pa0 + src, cbase + lane, d, dr)
-                                 : kKeyMax;
-        const unsigned m = __ballot_sync(0xffffffffu, key < sh.kth[l]);
-        if (!m) continue;
-        const int cnt = sh.cnt[l];
-        if ((m >> lane) & 1u) lst[cnt + __popc(m & ((1u << lane) - 1u))] = key;
-        __syncwarp();
-        if (lane == 0) sh.cnt[l] = cnt + __popc(m);
-        __syncwarp();
-        if (cnt + __popc(m) > kTcListRow - 32) {
-            compact_exact(sh, lst, l, k);
-            compacted = true;
+    const int64_t own = rbase + row0 + lane - cbase;  // not the row itself
+    if (own >= 0 && own < 32) pass &= ~(1u << static_cast<int>(own));
+    while (__any_sync(0xffffffffu, pass != 0u)) {
+        // every row with candidates left gives one to the next free lanes
+        const unsigned rows = __ballot_sync(0xffffffffu, pass != 0u);
+        const int give = __popc(rows), room = 32 - p.n, take = give < room ? give : room;
+        const int mine = __popc(rows & ((1u << lane) - 1u));  // my place among the givers
+        const int b = pass != 0u ? __ffs(pass) - 1 : 0;
+        const int want = lane - p.n;  // which giver this lane takes
+        const int src = want >= 0 && want < take ? static_cast<int>(__fns(rows, 0, want + 1)) : 0;
+        const int gb = __shfl_sync(0xffffffffu, b, src);
+        if (want >= 0 && want < take) {
+            p.row = row0 + src;
+            p.col = cbase + gb;
+        }
+        if (pass != 0u && mine < take) pass &= pass - 1;
+        p.n += take;
+        if (p.n == 32) {
+            compacted |= exact_flush(sh, glist, p, rbase, xr, ix, dr, k);
+            p.n = 0;
         }
     }
     return compacted;
@@ -508,14 +586,17 @@ __noinline__ __device__ bool exact_chunk(TcRows& sh, uint64_t* __restrict__ glis
 // 1563 tiles, d = 128, k = 50: 24.2, 24.0, 25.0, 28.1 ms; 235 tiles, d = 100,
 // k = 30: 1.60, 1.51, 1.42, 1.43 ms; 157 tiles, d = 32, k = 20: 1.48, 1.38,
 // 1.29, 1.22 ms).
+// (k = 64, d = 24, n = 20,000: 2.8 ms in two halves, 3.2 without a scan; the
+// lists of k = 50 are as fast either way, 0.9 ms)
+constexpr int kHalvesK = 56;
 __device__ __forceinline__ int bound_tiles(int count) { return min(count, max(128, count / 4)); }
 
 template <int NB>
 __global__ void __launch_bounds__(kTcThreads, NB == 2 ? 2 : 1)
 tc_sweep_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ CUtensorMap tmapb,
                 const float* __restrict__ xr,
-                const float* __restrict__ cn, const unsigned* __restrict__ ix, const TcScale* __restrict__ scale,
-                int nt, int T0, int ntb, int nsplit, int d, int dr, int Kp, int split_ops, int ksteps, int k, float c1,
+                const float* __restrict__ cn, const float* __restrict__ rn, const unsigned* __restrict__ ix,
+                const TcScale* __restrict__ scale, int nt, int T0, int ntb, int nsplit, int d, int dr, int Kp, int split_ops, int ksteps, int k, float c1,
                 float c2, const unsigned* __restrict__ max_norm_bits, const unsigned long long* __restrict__ kth_seed,
                 uint64_t* __restrict__ lists, TcRow* __restrict__ row_info, int* __restrict__ status, int qs,
                 const uint2* __restrict__ plist, const int* __restrict__ pcount) {
@@ -537,10 +618,13 @@ tc_sweep_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
     // one entry more
     const int kx = qs == 0 ? k + 1 : k;
     // tiles 0 .. scan - 1 are read twice: first for the rows' bounds (below)
-    const int scan = scale->all != 0.0f || kx > 64 ? 0 : bound_tiles(count);
+    const int scan = scale->all != 0.0f ? 0 : bound_tiles(count);
     const int total = scan + count;
+    const int halves = kx > kHalvesK && scan > 1 ? 2 : 1;
     auto col_tile = [&](int jj) -> int {
-        const int j = jj < scan ? jj : jj - scan;
+        // (two halves: the even tiles, then the odd)
+        const int even = (scan + 1) / 2;
+        const int j = jj >= scan ? jj - scan : halves == 1 ? jj : jj < even ? 2 * jj : 2 * (jj - even) + 1;
         return tlist ? static_cast<int>(tlist[split + nsplit * j].x) : spiral_tile(T, q0 + j, nt);
     };
     const int nkb = Kp / 64;
@@ -571,7 +655,8 @@ tc_sweep_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
         sh.athr[r] = __int_as_float(0x7f800000);
         // with the filter disabled the f values carry no information: exact lists
         sh.mode[r] = scale->all != 0.0f ? kModeExact : kModeApprox;
-        const RowBounds rb = row_bounds(cn[rbase + r], nmax, Kp, scale->eta, split_ops ? d : 0, 16 * ksteps);
+        const RowBounds rb = row_bounds(cn[rbase + r], nmax, Kp, split_ops ? 0.0f : rn[rbase + r],
+                                        __uint_as_float(scale->resmax), scale->eta, split_ops ? d : 0, 16 * ksteps);
         sh.c0[r] = rb.c0;
         sh.c3[r] = rb.c3;
         sh.c4[r] = rb.c4;
@@ -645,6 +730,7 @@ tc_sweep_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
         const bool row_valid = __ldg(ix + rbase + r) != kNoIndex;
         bool exact_any = all;  // some list of the warp is exact
         bool exact_row = all;
+        ExactPending pending;
         int cnt = 0;  // entries of this thread's list while it is approximate (sh.cnt while compacting)
         float tau = 0.0f;  // the list's threshold, and as a packed pair
         uint64_t tq = 0;
@@ -741,7 +827,7 @@ tc_sweep_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
             bool changed = false;
             __syncwarp();
             if (exact_any)
-                changed = exact_chunk(sh, glist, row0, exact_row ? pass : 0u, rbase + row0, cbase + 32 * ch, xr, ix, d,
+                changed = exact_chunk(sh, glist, row0, exact_row ? pass : 0u, pending, rbase, cbase + 32 * ch, xr, ix,
                                       dr, k);
             // keep room for the next chunk: compact approximate lists with
             // less than 32 free slots
@@ -756,7 +842,7 @@ tc_sweep_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
                     uint64_t* lst = glist + static_cast<size_t>(row0 + src) * kTcListRow;
                     if (approx_compact(sh, lst, row0 + src, kx, c2, sh.c3[row0 + src], sh.c4[row0 + src],
                                        kTcListRow - 32) > kTcListRow - 32) {
-                        to_exact_mode(sh, lst, row0 + src, rbase + row0 + src, xr, ix, d, dr, k);
+                        to_exact_mode(sh, lst, row0 + src, rbase + row0 + src, xr, ix, dr, k);
                         exact_any = true;
                     }
                 }
@@ -768,59 +854,69 @@ tc_sweep_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
         bool alive = true;
         if (scan > 0) {
             // Bounds first: the row's smallest f in each of 64 groups of the
-            // scanned columns. k groups with a value <= B are k
-            // columns with f <= B, so the k-th smallest of the minima bounds
-            // the row's k-th f, and the threshold over it (approx_thr) starts
-            // the lists.
+            // scanned columns. k groups with a value <= B are k columns with
+            // f <= B, so the k-th smallest of the minima bounds the row's k-th
+            // f, and the threshold over it (approx_thr) starts the lists.
+            // Above kHalvesK in two halves of the scan, half of the k from
+            // each: the k-th smallest of 64 minima has about -64 ln(1 - k / 64)
+            // scanned columns below it (102 at k = 51, all at 64), the halves
+            // together -128 ln(1 - k / 128) (65 and 89).
             float gm[64];
+            float B = __int_as_float(0xff800000);
+#pragma unroll 1
+            for (int part = 0; part < halves && alive; ++part) {
+                const int need = halves == 1 ? kx : part == 0 ? (kx + 1) / 2 : kx / 2;
 #pragma unroll
-            for (int q = 0; q < 64; ++q) gm[q] = __int_as_float(0x7f800000);
-            for (int j = 0; j < scan; ++j) {
-                if (!begin_tile(j)) {
-                    alive = false;
-                    break;
-                }
-                const uint32_t taddr = lane_addr + static_cast<uint32_t>((j & 1) * 128);
+                for (int q = 0; q < 64; ++q) gm[q] = __int_as_float(0x7f800000);
+                const int j1 = part == halves - 1 ? scan : (scan + 1) / 2;
+                for (int j = part == 0 ? 0 : (scan + 1) / 2; j < j1; ++j) {
+                    if (!begin_tile(j)) {
+                        alive = false;
+                        break;
+                    }
+                    const uint32_t taddr = lane_addr + static_cast<uint32_t>((j & 1) * 128);
 #pragma unroll
-                for (int ch = 0; ch < 4; ++ch) {
-                    uint32_t ga[32];
-                    tc::tmem_ld32_bits(taddr + static_cast<uint32_t>(32 * ch), ga);
-                    if (ch == 3) end_tile(j);
-                    const float4* nb4 = reinterpret_cast<const float4*>(nbj + 32 * ch);
+                    for (int ch = 0; ch < 4; ++ch) {
+                        uint32_t ga[32];
+                        tc::tmem_ld32_bits(taddr + static_cast<uint32_t>(32 * ch), ga);
+                        if (ch == 3) end_tile(j);
+                        const float4* nb4 = reinterpret_cast<const float4*>(nbj + 32 * ch);
 #pragma unroll
-                    for (int q = 0; q < 8; q += 2) {
-                        // columns c and c + 4 share a group: one three-way minimum
-                        uint64_t f[4];
+                        for (int q = 0; q < 8; q += 2) {
+                            // columns c and c + 4 share a group: one three-way minimum
+                            uint64_t f[4];
 #pragma unroll
-                        for (int e = 0; e < 2; ++e) {
-                            const float4 nb = nb4[q + e];
-                            const uint32_t* g4 = ga + 4 * (q + e);
-                            f[2 * e] = fma2(pack2(__uint_as_float(g4[0]), __uint_as_float(g4[1])), k2, pack2(nb.x, nb.y));
-                            f[2 * e + 1] =
-                                fma2(pack2(__uint_as_float(g4[2]), __uint_as_float(g4[3])), k2, pack2(nb.z, nb.w));
+                            for (int e = 0; e < 2; ++e) {
+                                const float4 nb = nb4[q + e];
+                                const uint32_t* g4 = ga + 4 * (q + e);
+                                f[2 * e] = fma2(pack2(__uint_as_float(g4[0]), __uint_as_float(g4[1])), k2, pack2(nb.x, nb.y));
+                                f[2 * e + 1] =
+                                    fma2(pack2(__uint_as_float(g4[2]), __uint_as_float(g4[3])), k2, pack2(nb.z, nb.w));
+                            }
+                            float* g = gm + 16 * ch + 2 * q;
+                            g[0] = fminf(fminf(g[0], lo_f(f[0])), lo_f(f[2]));
+                            g[1] = fminf(fminf(g[1], hi_f(f[0])), hi_f(f[2]));
+                            g[2] = fminf(fminf(g[2], lo_f(f[1])), lo_f(f[3]));
+                            g[3] = fminf(fminf(g[3], hi_f(f[1])), hi_f(f[3]));
                         }
-                        float* g = gm + 16 * ch + 2 * q;
-                        g[0] = fminf(fminf(g[0], lo_f(f[0])), lo_f(f[2]));
-                        g[1] = fminf(fminf(g[1], hi_f(f[0])), hi_f(f[2]));
-                        g[2] = fminf(fminf(g[2], lo_f(f[1])), lo_f(f[3]));
-                        g[3] = fminf(fminf(g[3], hi_f(f[1])), hi_f(f[3]));
                     }
                 }
-            }
-            // the k-th smallest of the 64, by bisection over the ordered bits
-            uint32_t at = 0;
+                // the need-th smallest of the 64, by bisection over the ordered bits
+                uint32_t at = 0;
 #pragma unroll 1
-            for (int bit = 31; bit >= 0; --bit) {
-                const float probe = unflip(at | ((1u << bit) - 1u));  // every value with this bit clear
-                int below = 0;
+                for (int bit = 31; bit >= 0; --bit) {
+                    const float probe = unflip(at | ((1u << bit) - 1u));  // every value with this bit clear
+                    int below = 0;
 #pragma unroll
-                for (int q = 0; q < 64; ++q) below += gm[q] <= probe ? 1 : 0;
-                // (a probe that is not a number lies outside the floats: all
-                // values are below a positive one, none below a negative one)
-                if (probe != probe) below = bit == 31 || (at >> 31) ? 64 : 0;
-                if (below < kx) at |= 1u << bit;
+                    for (int q = 0; q < 64; ++q) below += gm[q] <= probe ? 1 : 0;
+                    // (a probe that is not a number lies outside the floats: all
+                    // values are below a positive one, none below a negative one)
+                    if (probe != probe) below = bit == 31 || (at >> 31) ? 64 : 0;
+                    if (below < need) at |= 1u << bit;
+                }
+                const float bound = need <= 64 ? unflip(at) : __int_as_float(0x7f800000);
+                B = bound == bound ? fmaxf(B, bound) : __int_as_float(0x7f800000);
             }
-            const float B = unflip(at);
             if (row_valid && B < __int_as_float(0x7f800000)) sh.athr[r] = approx_thr(B, c2, sh.c3[r], sh.c4[r]);
             set_tau();
         }
@@ -835,6 +931,7 @@ tc_sweep_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
                 process_chunk(ga, ch);
             }
         }
+        if (pending.n > 0) exact_flush(sh, glist, pending, rbase, xr, ix, dr, k);
         TcRow info;
         info.cnt = exact_row ? sh.cnt[r] : cnt;
         info.mode = exact_row ? kModeExact : kModeApprox;
@@ -960,7 +1057,7 @@ tc_final_kernel(const float* __restrict__ xr, const unsigned* __restrict__ ix, i
 static bool tc_use_split(int d) {
     const char* env = std::getenv("CULOF_TC_SPLIT");
     if (env && env[0] == '0') return false;
-    return 3 * d <= 128;
+    return d <= kTcSplitD;
 }
 static int tc_kp(int d, bool split) {
     const int w = split ? 3 * d : d;
@@ -973,7 +1070,7 @@ size_t tc_buffer_bytes(int64_t padded, int d) {
     const int dr = (d + 3) & ~3;
     const auto up = [](size_t x) { return (x + 255) & ~static_cast<size_t>(255); };
     return up(sizeof(__half) * padded * Kp) * (split ? 2 : 1) + up(sizeof(float) * padded * dr) +
-           up(sizeof(float) * padded) + up(sizeof(unsigned) * padded) + up(sizeof(TcScale));
+           2 * up(sizeof(float) * padded) + up(sizeof(unsigned) * padded) + up(sizeof(TcScale));
 }
 
 int tc_max_splits() { return kMaxTcSplits; }
@@ -1008,6 +1105,8 @@ TcBuffers tc_prepare(void* buf, const float* xc, const float* norms, int64_t n, 
     p += up(sizeof(float) * padded * b.dr);
     b.cn = reinterpret_cast<float*>(p);
     p += up(sizeof(float) * padded);
+    b.rn = reinterpret_cast<float*>(p);
+    p += up(sizeof(float) * padded);
     b.ix = reinterpret_cast<unsigned*>(p);
     p += up(sizeof(unsigned) * padded);
     b.scale = p;
@@ -1020,6 +1119,13 @@ TcBuffers tc_prepare(void* buf, const float* xc, const float* norms, int64_t n, 
                                                              static_cast<__half*>(b.xh), static_cast<__half*>(b.xb),
                                                              b.xr, b.cn, b.ix);
     CG_LAUNCH_CHECK();
+    if (!split) {
+        g = ceil_div(padded, 8);
+        if (g > 152 * 8) g = 152 * 8;
+        tc_resid_kernel<<<static_cast<unsigned>(g), 256, 0, s>>>(b.xr, padded, d, b.dr, reinterpret_cast<TcScale*>(b.scale),
+                                                                 b.rn);
+        CG_LAUNCH_CHECK();
+    }
     return b;
 }
 
@@ -1041,7 +1147,7 @@ void tc_sweep(const TcBuffers& b, int64_t n, int nt, int t0, int mt, int nsplit,
     for (int T0 = t0; T0 < t0 + mt; T0 += ntb_max) {
         const int ntb = t0 + mt - T0 < ntb_max ? t0 + mt - T0 : ntb_max;
         kernel<<<ntb * nsplit, kTcThreads, smem, s>>>(
-            map, mapb, b.xr, b.cn, b.ix, reinterpret_cast<const TcScale*>(b.scale), nt, T0, ntb, nsplit, d, b.dr, b.Kp,
+            map, mapb, b.xr, b.cn, b.rn, b.ix, reinterpret_cast<const TcScale*>(b.scale), nt, T0, ntb, nsplit, d, b.dr, b.Kp,
             b.split, b.ksteps, k, c1, c2, maxn, kth_seed, lists, info, status, qs, plist, pcount);
         CG_LAUNCH_CHECK();
         const unsigned grid = static_cast<unsigned>(ntb) * kRT / kFinWarps;

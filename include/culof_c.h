@@ -37,10 +37,15 @@ extern "C" {
 #define CULOF_ERR_KERNEL 5 /* a kernel reported an error status word (e.g. a bounded wait expired) */
 
 /* Path selection for culof_context_set_path. */
-#define CULOF_PATH_AUTO 0    /* GENERAL for n <= 4096; FAST for d <= 8; TENSOR above; GENERAL past the fused limits */
-#define CULOF_PATH_FAST 1    /* fused FP32 distance + filtered select (d <= 128, k <= 64) */
+/* AUTO: GENERAL for n <= 4096 (2560 for d > 16), past k = 64 or past d = 256;
+ * FAST for d <= 8, and for d <= 16 up to n = 7168; TENSOR otherwise. Inputs
+ * of up to 7168 points and 16 features (k <= 64) then run one direct kernel
+ * instead of the FAST or GENERAL path's own. */
+#define CULOF_PATH_AUTO 0
+#define CULOF_PATH_FAST 1    /* fused FP32 distance + select (d <= 128, k <= 64)          */
 #define CULOF_PATH_GENERAL 2 /* exact distance tile + radix select (any d, any k)        */
-#define CULOF_PATH_TENSOR 3  /* f16 tensor-core filter + exact rescoring (d <= 128, k <= 64) */
+#define CULOF_PATH_TENSOR 3  /* f16 tensor-core filter + exact rescoring (d <= 128 when
+                              * asked for; AUTO uses it up to d = 256; k <= 64)       */
 
 typedef struct culof_context culof_context;
 
@@ -106,8 +111,9 @@ CULOF_API int culof_context_fit_predict_device(culof_context* ctx, const float* 
 
 /* Per-stage timing with CUDA events on the context stream (off by default).
  * culof_context_stage_times writes milliseconds of the last call for up to
- * cap stages (0 centre+norms, 1 spatial order+tiles, 2 seed, 3 sweep or tile
- * select, 4 merge, 5 lrd+score, 6 offset+labels; -1 = did not run) and
+ * cap stages (0 centre+norms, 1 spatial order+tiles, 2 seed, 3 sweep, direct
+ * kernel or tile select, 4 merge, 5 lrd+score, 6 offset+labels; -1 = did not
+ * run; seed and merge are empty but for the wide FP32 sweep) and
  * synchronises the stream. No reference counterpart: measurement support. */
 CULOF_API int culof_context_set_timing(culof_context* ctx, int on);
 CULOF_API int culof_context_stage_times(culof_context* ctx, float* ms, int cap);
@@ -116,9 +122,10 @@ CULOF_API int culof_context_stage_times(culof_context* ctx, float* ms, int cap);
  * counterpart: measurement support. */
 CULOF_API unsigned long long culof_kernel_launch_count(void);
 /* Row x column pairs the last small-d FP32 sweep of this context evaluated
- * (tiles that a bounding-box test proves farther than every k-th neighbour
- * are skipped) and the pairs it would evaluate without that test (every
- * column tile past the seed's own and four neighbour tiles); both 0 after
+ * past the rows' windows (64-column halves that a bounding-box test proves
+ * farther than a row's k-th neighbour are skipped, row by row) and the pairs
+ * it would evaluate without that test (every column tile past the window, the
+ * row tile's own and its four neighbour tiles); both 0 after
  * other paths. Synchronises the context stream. */
 CULOF_API int culof_context_pair_stats(culof_context* ctx, double* evaluated_pairs, double* total_pairs);
 
@@ -229,8 +236,9 @@ CULOF_API int culof_context_set_graphs(culof_context* ctx, int on);
 /* The batched autotuner's record for the context's current batch layout
  * (measurement support; no reference counterpart): ms4[2 (c - 1) + (p - 1)]
  * is the whole batched call's time in milliseconds with the k-NN kernel at
- * c CTAs per SM and p column pairs per lane (-1 if that variant was not
- * tried: two CTAs need the shared memory, two pairs d <= 16), and *ctas_per_sm /
+ * c CTAs per SM (up to 16 features: 2 = as many as fit) and p column pairs per
+ * lane (-1 if that variant was not tried: two CTAs need the shared memory, two
+ * pairs are not tried), and *ctas_per_sm /
  * *pairs_per_lane the chosen variant (0 before the first batched call). */
 CULOF_API int culof_context_batched_tuning(culof_context* ctx, float* ms4, int* ctas_per_sm, int* pairs_per_lane);
 

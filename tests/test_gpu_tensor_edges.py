@@ -38,3 +38,32 @@ def test_tensor_path_bit_exact(monkeypatch, n, d, k, splits):
     np.testing.assert_array_equal(kd.cpu().numpy().view(np.uint32), o_kd.view(np.uint32))
     np.testing.assert_array_equal(idx.cpu().numpy(), o_idx)
     np.testing.assert_array_equal(d2.cpu().numpy().view(np.uint32), o_d2.view(np.uint32))
+
+
+def _check_tensor(X, k, path):
+    n, d = X.shape
+    with _culof.Context() as ctx:
+        ctx.set_path(path)
+        dx = torch.from_numpy(X).cuda()
+        idx = torch.zeros((k, n), dtype=torch.int32, device="cuda")
+        d2 = torch.zeros((k, n), device="cuda")
+        kd = torch.zeros(n, device="cuda")
+        ctx.knn_device(dx.data_ptr(), n, d, k, False, idx.data_ptr(), d2.data_ptr(), kd.data_ptr())
+        ctx.synchronize()
+        assert ctx.last_path() == _culof.PATH_TENSOR
+    Xc, _, _ = oracle.center(X)
+    o_idx, o_d2, o_kd = oracle.knn(Xc, k)
+    np.testing.assert_array_equal(kd.cpu().numpy().view(np.uint32), o_kd.view(np.uint32))
+    np.testing.assert_array_equal(idx.cpu().numpy(), o_idx)
+    np.testing.assert_array_equal(d2.cpu().numpy().view(np.uint32), o_d2.view(np.uint32))
+
+
+@pytest.mark.parametrize("n,d,k", [(2600, 24, 56), (4200, 40, 64), (4100, 43, 20), (5000, 64, 33), (4300, 100, 64),
+                                   (4200, 126, 57), (2600, 200, 20), (2700, 256, 64)])
+def test_lists_without_room_turn_exact(n, d, k):
+    # clusters far from the origin: a wide filter margin, most rows rescore
+    # their candidates exactly, 32 pending pairs at a time
+    X = synthetic.clusters_with_outliers(n, d, seed=n + k)
+    X[: n // 2] += np.float32(40.0)
+    X[20:30] = X[19]
+    _check_tensor(X, k, _culof.PATH_TENSOR if d <= 128 else _culof.PATH_AUTO)
