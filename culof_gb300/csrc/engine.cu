@@ -148,7 +148,8 @@ int Engine::tile_rows_for(int64_t n) {
 //   <= 42) and k <= 48: with single operands its time depends on the data's
 //   spread (43 and 128 features above), and past k = 48 its lists have little
 //   room for the filter's margin. Also for d > 128, where the tile costs most
-//   (factor model, d = 200, n = 3,000: 180 us for 430).
+//   (d = 200, n = 4,100, k = 20: factor model 205 us for 741, clusters 311 for
+//   721; the worst measured, clusters at k = 64: 2,182 for 727).
 // - d <= 8: the FP32 path (direct up to 7168 points, then the small-d sweep).
 // - 8 < d <= 16: the direct kernel as far as it wins, 7168 points past k = 48
 //   and 4096 for d > 12 else; for d <= 12 up to 6144, where the tensor path

@@ -177,6 +177,7 @@ private:
     DevBuf morton_, perm_, sort_tmp_, cols_, rows_, tc_lists_, tiles_;
     // tile boxes; the tensor path's tile lists over d <= 8 points
     DevBuf boxes_, plist_, pcount_;
+    DevBuf lost_;  // rows that the tensor path leaves to the distance tile (d > 128)
     DevBuf iso_;  // rows that leave the small-d sweep for their own pass
     double stat_total_pairs_ = 0.0;  // pairs the small-d sweep would evaluate without pruning
     // Words that every k-NN call starts from zero: the device status word
@@ -190,6 +191,7 @@ private:
     int* status_ptr() { return reinterpret_cast<int*>(call_words()); }
     unsigned* max_norm_word() { return call_words() + 1; }
     unsigned long long* evaluated_word() { return reinterpret_cast<unsigned long long*>(call_words() + 2); }
+    int* lost_count_word() { return reinterpret_cast<int*>(call_words() + 5); }
     int* iso_count_word() { return reinterpret_cast<int*>(call_words() + 4); }
     unsigned* range_words() { return call_words() + 8; }
 

@@ -80,10 +80,11 @@ size_t tc_list_bytes(int nt, int nsplit);
 // positions 0..qs-1 are the seed's; 0: no seed, kth_seed and seed_keys null);
 // plist / pcount (nullable): per row tile,
 // the column tiles to visit in order (the small-d prune lists); without them
-// every tile past the window is visited.
+// every tile past the window is visited. lost_rows / lost_count: d > 128, the
+// original indices of the rows that this path leaves to the general one.
 void tc_sweep(const TcBuffers& b, int64_t n, int nt, int t0, int mt, int nsplit, int d, int k, const unsigned* maxn,
               const unsigned long long* kth_seed, const uint64_t* seed_keys, uint64_t* lists, int* status,
-              int32_t* nbr_idx, float* nbr_d2, float* kdist2, cudaStream_t s, int qs,
+              int32_t* nbr_idx, float* nbr_d2, float* kdist2, cudaStream_t s, int qs, int32_t* lost_rows, int* lost_count,
               const uint2* plist = nullptr, const int* pcount = nullptr);
 
 }  // namespace culof_gb300

@@ -287,6 +287,12 @@ __device__ __forceinline__ uint32_t flip_bits(float f) {
 // exact lists hold the usual (distance bits << 32 | original index).
 constexpr int kModeApprox = 0;
 constexpr int kModeExact = 1;
+// More than 128 features: a row whose list overflows leaves the path, and the
+// distance tile and select of the general path take it afterwards. Rescoring
+// its candidates one by one reads two rows of coordinates per pair, which past
+// a tenth of the pairs costs more than the whole tile (clusters, d = 256, n =
+// 8,000, k = 20: 7.5 ms, this way 2.1; the tile and select of all rows 2.7).
+constexpr int kModeLost = 2;
 
 // Per-row lists live in global memory (L2-resident while their CTA runs):
 // kTcM keys per row, 128 rows per CTA. Keeping them out of shared memory
@@ -602,6 +608,7 @@ tc_sweep_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
                 const uint2* __restrict__ plist, const int* __restrict__ pcount) {
     extern __shared__ uint8_t tc_raw[];
     TcSmem<NB>& sh = *reinterpret_cast<TcSmem<NB>*>((reinterpret_cast<uintptr_t>(tc_raw) + 1023) & ~uintptr_t(1023));
+    constexpr bool kLose = NB > 2;  // overflowing rows leave (kModeLost)
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int T = T0 + static_cast<int>(blockIdx.x) % ntb;
     const int split = static_cast<int>(blockIdx.x) / ntb;
@@ -654,7 +661,7 @@ tc_sweep_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
         sh.sorted[r] = 0;
         sh.athr[r] = __int_as_float(0x7f800000);
         // with the filter disabled the f values carry no information: exact lists
-        sh.mode[r] = scale->all != 0.0f ? kModeExact : kModeApprox;
+        sh.mode[r] = scale->all == 0.0f ? kModeApprox : kLose ? kModeLost : kModeExact;
         const RowBounds rb = row_bounds(cn[rbase + r], nmax, Kp, split_ops ? 0.0f : rn[rbase + r],
                                         __uint_as_float(scale->resmax), scale->eta, split_ops ? d : 0, 16 * ksteps);
         sh.c0[r] = rb.c0;
@@ -726,17 +733,18 @@ tc_sweep_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
         const int r = row0 + lane;
         uint64_t* const mylist = glist + static_cast<size_t>(r) * kTcListRow;
         const TcScale sc = *scale;
-        const bool all = sc.all != 0.0f;
+        const bool all = !kLose && sc.all != 0.0f;
         const bool row_valid = __ldg(ix + rbase + r) != kNoIndex;
         bool exact_any = all;  // some list of the warp is exact
         bool exact_row = all;
+        bool lost = kLose && sc.all != 0.0f;
         ExactPending pending;
         int cnt = 0;  // entries of this thread's list while it is approximate (sh.cnt while compacting)
         float tau = 0.0f;  // the list's threshold, and as a packed pair
         uint64_t tq = 0;
         auto set_tau = [&]() {
             tau = __int_as_float(0xff800000);
-            if (row_valid) {
+            if (row_valid && !lost) {
                 tau = exact_tau(sh.kth[r], c1, sh.c0[r]);
                 if (!exact_row) tau = fminf(tau, sh.athr[r]);
             }
@@ -826,7 +834,7 @@ tc_sweep_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
             }
             bool changed = false;
             __syncwarp();
-            if (exact_any)
+            if (!kLose && exact_any)
                 changed = exact_chunk(sh, glist, row0, exact_row ? pass : 0u, pending, rbase, cbase + 32 * ch, xr, ix,
                                       dr, k);
             // keep room for the next chunk: compact approximate lists with
@@ -842,12 +850,16 @@ tc_sweep_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
                     uint64_t* lst = glist + static_cast<size_t>(row0 + src) * kTcListRow;
                     if (approx_compact(sh, lst, row0 + src, kx, c2, sh.c3[row0 + src], sh.c4[row0 + src],
                                        kTcListRow - 32) > kTcListRow - 32) {
-                        to_exact_mode(sh, lst, row0 + src, rbase + row0 + src, xr, ix, dr, k);
-                        exact_any = true;
+                        if (kLose) {
+                            if (lane == src) lost = true;
+                        } else {
+                            to_exact_mode(sh, lst, row0 + src, rbase + row0 + src, xr, ix, dr, k);
+                            exact_any = true;
+                        }
                     }
                 }
                 exact_row = sh.mode[r] == kModeExact;
-                cnt = sh.cnt[r];
+                cnt = lost ? 0 : sh.cnt[r];
             }
             if (changed) set_tau();
         };
@@ -931,10 +943,10 @@ tc_sweep_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
                 process_chunk(ga, ch);
             }
         }
-        if (pending.n > 0) exact_flush(sh, glist, pending, rbase, xr, ix, dr, k);
+        if (!kLose && pending.n > 0) exact_flush(sh, glist, pending, rbase, xr, ix, dr, k);
         TcRow info;
         info.cnt = exact_row ? sh.cnt[r] : cnt;
-        info.mode = exact_row ? kModeExact : kModeApprox;
+        info.mode = lost ? kModeLost : exact_row ? kModeExact : kModeApprox;
         info.c3 = sh.c3[r];
         info.c4 = sh.c4[r];
         row_info[static_cast<size_t>(blockIdx.x) * kRT + r] = info;
@@ -965,7 +977,7 @@ __global__ void __launch_bounds__(32 * kFinWarps)
 tc_final_kernel(const float* __restrict__ xr, const unsigned* __restrict__ ix, int64_t n, int T0, int ntb, int nsplit,
                 int dr, int k, int kx, float c2, const uint64_t* __restrict__ lists, const TcRow* __restrict__ row_info,
                 const uint64_t* __restrict__ seed_keys, int32_t* __restrict__ nbr_idx, float* __restrict__ nbr_d2,
-                float* __restrict__ kdist2) {
+                float* __restrict__ kdist2, int32_t* __restrict__ lost_rows, int* __restrict__ lost_count) {
     __shared__ __align__(16) float row[kFinWarps][kMaxTensorD];
     __shared__ unsigned cand[kFinWarps][kMaxTcSplits * kTcListRow];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -987,6 +999,10 @@ tc_final_kernel(const float* __restrict__ xr, const unsigned* __restrict__ ix, i
         if (s >= nsplit) continue;
         const size_t at = static_cast<size_t>(s) * ntb * kRT + local;
         const TcRow info = row_info[at];
+        if (info.mode == kModeLost) {
+            if (lane == 0) lost_rows[atomicAdd(lost_count, 1)] = static_cast<int32_t>(__ldg(ix + pos));
+            return;
+        }
         c3 = info.c3;
         c4 = info.c4;
         const uint64_t* lst = lists + at * kTcListRow;
@@ -1131,8 +1147,8 @@ TcBuffers tc_prepare(void* buf, const float* xc, const float* norms, int64_t n, 
 
 void tc_sweep(const TcBuffers& b, int64_t n, int nt, int t0, int mt, int nsplit, int d, int k, const unsigned* maxn,
               const unsigned long long* kth_seed, const uint64_t* seed_keys, uint64_t* lists, int* status,
-              int32_t* nbr_idx, float* nbr_d2, float* kdist2, cudaStream_t s, int qs, const uint2* plist,
-              const int* pcount) {
+              int32_t* nbr_idx, float* nbr_d2, float* kdist2, cudaStream_t s, int qs, int32_t* lost_rows,
+              int* lost_count, const uint2* plist, const int* pcount) {
     const bool wide = b.Kp > 128;
     const size_t smem = (wide ? sizeof(TcSmem<4>) : sizeof(TcSmem<2>)) + 1024;
     const auto kernel = wide ? tc_sweep_kernel<4> : tc_sweep_kernel<2>;
@@ -1153,10 +1169,10 @@ void tc_sweep(const TcBuffers& b, int64_t n, int nt, int t0, int mt, int nsplit,
         const unsigned grid = static_cast<unsigned>(ntb) * kRT / kFinWarps;
         if (k <= 32)
             tc_final_kernel<1><<<grid, 32 * kFinWarps, 0, s>>>(b.xr, b.ix, n, T0, ntb, nsplit, b.dr, k, kx, c2, lists, info,
-                                                               seed_keys, nbr_idx, nbr_d2, kdist2);
+                                                               seed_keys, nbr_idx, nbr_d2, kdist2, lost_rows, lost_count);
         else
             tc_final_kernel<2><<<grid, 32 * kFinWarps, 0, s>>>(b.xr, b.ix, n, T0, ntb, nsplit, b.dr, k, kx, c2, lists, info,
-                                                               seed_keys, nbr_idx, nbr_d2, kdist2);
+                                                               seed_keys, nbr_idx, nbr_d2, kdist2, lost_rows, lost_count);
         CG_LAUNCH_CHECK();
     }
 }
