@@ -62,9 +62,9 @@ PATH_NAMES = ["auto", "fast", "general", "tensor"]
 # very workload (dram__bytes_read.sum + dram__bytes_write.sum); other
 # workloads report null.
 MEASURED_SWEEP_TRAFFIC = {
-    ("clusters", 200_000, 8, 20): (16_110_000 + 10_360_000,
-                                   "ncu: 16.11 MB read + 10.36 MB written per sweep_kernel launch at this workload "
-                                   "(the isolated rows' pass beside it: 7.79 MB read)"),
+    ("clusters", 200_000, 8, 20): (32_940_000 + 25_360_000,
+                                   "ncu: 32.94 MB read + 25.36 MB written per small_sweep_kernel launch at this "
+                                   "workload (the pass over the rows that leave it: 8.08 MB read)"),
 }
 
 

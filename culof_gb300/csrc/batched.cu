@@ -10,18 +10,17 @@
 //      same order (chunks of kCenterChunk rows), for every problem at once;
 //   2. a spatial order within each problem (Morton keys over its 8 widest
 //      dimensions, two stable radix sorts);
-//   3. a persistent k-NN kernel: CTAs pull (problem, 128-row tile) work items
-//      from an atomic counter, largest problems first, visit the problem's
-//      column tiles nearest first (spiral from the own tile) and select each row's
-//      exact k nearest among its problem's points (FP32 direct differences,
-//      the oracle's formula, two columns per packed f32x2 instruction) into
-//      per-row lists in shared memory;
+//   3. the exact k-NN of every row among its problem's points: up to 16
+//      features the row-pruned sweep (sweep_rows.cuh) over work items grouped
+//      by list form; above, a persistent kernel whose CTAs pull (problem,
+//      128-row tile) items from an atomic counter, largest problems first,
+//      and visit the problem's column tiles nearest first into per-row lists
+//      in shared memory (FP32 direct differences, the oracle's formula);
 //   4. batched lrd and scores with the reference's FP64 sums.
 // Every problem's scores are bit-identical to a single-problem call. The
 // launch sequence of a given batch layout is captured once as a CUDA graph
 // and replayed; on first sight of a layout a small autotuner times the k-NN
-// kernel's variants (CTAs per SM, one or two column pairs per lane) and
-// keeps the fastest.
+// kernel's variants (CTAs per SM) and keeps the fastest.
 #include <algorithm>
 #include <cstring>
 #include <sstream>
@@ -326,58 +325,6 @@ batched_sweep_kernel(const float* __restrict__ tiles, const float* __restrict__ 
     small::sweep_rows<DP, KR, G, kRowsPer, kWarps, false>(sh, P);
 }
 
-// One warp per (problem, tile of 128 sorted points): the tile's bounding box,
-// tbox[tile_off[p] + t][2][d] (lo, hi).
-__global__ void bm_tilebox_kernel(const float* __restrict__ xs, const int64_t* __restrict__ off, int d,
-                                  const int* __restrict__ tpid, const int64_t* __restrict__ toff, int64_t ntiles,
-                                  float* __restrict__ tbox) {
-    const int lane = threadIdx.x & 31;
-    const int64_t g = static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (g >= ntiles) return;
-    const int p = tpid[g];
-    const int64_t t = g - toff[p];
-    const int64_t b = off[p] + t * kCT;
-    const int64_t e = (b + kCT < off[p + 1]) ? b + kCT : off[p + 1];
-    for (int f = 0; f < d; ++f) {
-        float lo = __int_as_float(0x7f800000), hi = __int_as_float(0xff800000);
-        for (int64_t i = b + lane; i < e; i += 32) {
-            const float v = xs[i * d + f];
-            lo = fminf(lo, v);
-            hi = fmaxf(hi, v);
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
-            hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
-        }
-        if (lane == 0) {
-            tbox[(g * 2) * d + f] = lo;
-            tbox[(g * 2 + 1) * d + f] = hi;
-        }
-    }
-}
-
-// Pruning margin for d <= 64: the float32 direct-difference distance of two
-// points at real squared distance T >= LB is >= T (1 - (d + 2) 2^-24) >
-// LB (1 - 2^-17), so a tile whose rounded-down box gap times (1 - 2^-17)
-// exceeds every row's k-th distance holds no candidate.
-constexpr float kBPruneShrink = 0.9999923706054688f;  // 1 - 2^-17
-
-// Rounded-down squared gap between box a (lo, hi) and box b, lanes over
-// dimensions, round-down sums; the result is warp-uniform.
-__device__ __forceinline__ float gap2_rd(const float* a_lo, const float* a_hi, const float* b_lo, const float* b_hi,
-                                         int d) {
-    const int lane = threadIdx.x & 31;
-    float g = 0.0f;
-    for (int f = lane; f < d; f += 32) {
-        const float gap = fmaxf(0.0f, fmaxf(__fsub_rd(b_lo[f], a_hi[f]), __fsub_rd(a_lo[f], b_hi[f])));
-        g = __fadd_rd(g, __fmul_rd(gap, gap));
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) g = __fadd_rd(g, __shfl_xor_sync(0xffffffffu, g, o));
-    return g;
-}
-
 // ---- persistent k-NN ---------------------------------------------------------
 
 template <int DP>
@@ -385,10 +332,6 @@ struct BatchSmem {
     RowLists<kBM> L;
     uint64_t rows2[kRT][DP];         // this item's rows, each coordinate duplicated into both halves
     uint64_t cols2[kCT / 2][DP + 1];  // one column tile as packed column pairs (odd stride)
-    float wbox[kWarps][2][DP];        // each warp's row box
-    float cbox[2][DP];                // the item's row box
-    float tb[2][2][DP];               // column tile box, by tile parity (warp 0 runs at most one tile ahead)
-    int skip_tile[2];
     int item;
 };
 
@@ -412,36 +355,30 @@ __device__ __forceinline__ void offer(RowLists<kBM>& L, int r, uint64_t key, int
     __syncwarp();
 }
 
-// Offer a row's 2 * CP keys (one warp-uniform test first).
-template <int CP>
-__device__ __forceinline__ void offer_row(RowLists<kBM>& L, int r, const uint64_t (&key)[2 * CP], int k) {
-    uint64_t mn = key[0];
-#pragma unroll
-    for (int q = 1; q < 2 * CP; ++q) mn = key[q] < mn ? key[q] : mn;
+// Offer a row's two keys (one warp-uniform test first).
+__device__ __forceinline__ void offer_row(RowLists<kBM>& L, int r, const uint64_t (&key)[2], int k) {
+    const uint64_t mn = key[1] < key[0] ? key[1] : key[0];
     if (!__any_sync(0xffffffffu, mn < L.kth[r])) return;
-#pragma unroll
-    for (int q = 0; q < 2 * CP; ++q) offer(L, r, key[q], k);
+    offer(L, r, key[0], k);
+    offer(L, r, key[1], k);
 }
 
 // Each warp owns 16 rows of the item. The CTA stages the problem's columns
 // in tiles of 128 (packed column pairs in shared memory); per pass a lane
-// holds CP column pairs in registers (packed f32x2 per dimension), so two
-// rows x CP pairs give 2 * CP independent packed FMA chains. Distances are
+// holds a column pair in registers (packed f32x2 per dimension) and takes two
+// rows at a time: two independent packed FMA chains. Distances are
 // the oracle's direct-difference chain, exactly (per-lane IEEE sub.rn /
 // fma.rn).
-// Two CTAs per SM (what the shared memory allows up to DP = 32); without the
-// minimum, the compiler gives the DP = 8 forms 64 registers and spills.
-template <int DP, int CP>
+template <int DP>
 __global__ void __launch_bounds__(kThreads, DP <= 32 ? 2 : 1)
 batched_knn_kernel(const float* __restrict__ xc, const unsigned* __restrict__ lidx, const int64_t* __restrict__ off,
                    const int* __restrict__ ks, const int64_t* __restrict__ nkoff, const uint2* __restrict__ items,
                    int nitems, int d, unsigned* __restrict__ counter, int32_t* __restrict__ nbr_idx,
-                   float* __restrict__ nbr_d2, float* __restrict__ kdist2, const float* __restrict__ tbox,
-                   const int64_t* __restrict__ toff) {
+                   float* __restrict__ nbr_d2, float* __restrict__ kdist2) {
     extern __shared__ __align__(16) unsigned char braw[];
     BatchSmem<DP>& sh = *reinterpret_cast<BatchSmem<DP>*>(braw);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    constexpr int kTile = 64 * CP;
+    constexpr int kTile = 64;
     for (;;) {
         if (tid == 0) sh.item = static_cast<int>(atomicAdd(counter, 1u));
         __syncthreads();
@@ -466,34 +403,6 @@ batched_knn_kernel(const float* __restrict__ xc, const unsigned* __restrict__ li
         }
         __syncthreads();
         const int rw = warp * kRowsPerWarp;
-        // row boxes: this warp's 16 rows and (warp 0, after the barrier) the item's
-        {
-            const int r = rw + (lane & 15);
-            const bool rv = r0 + r < n;
-            for (int f = 0; f < d; ++f) {
-                const float v = lo_f(sh.rows2[r][f]);
-                float lo = rv ? v : __int_as_float(0x7f800000), hi = rv ? v : __int_as_float(0xff800000);
-#pragma unroll
-                for (int o = 8; o > 0; o >>= 1) {
-                    lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
-                    hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
-                }
-                if (lane == 0) {
-                    sh.wbox[warp][0][f] = lo;
-                    sh.wbox[warp][1][f] = hi;
-                }
-            }
-        }
-        __syncthreads();
-        if (tid < d) {
-            float lo = __int_as_float(0x7f800000), hi = __int_as_float(0xff800000);
-            for (int w = 0; w < kWarps; ++w) {
-                lo = fminf(lo, sh.wbox[w][0][tid]);
-                hi = fmaxf(hi, sh.wbox[w][1][tid]);
-            }
-            sh.cbox[0][tid] = lo;
-            sh.cbox[1][tid] = hi;
-        }
         const unsigned* li = lidx + base;  // original index of each sorted position
         const int ntp = (n + kCT - 1) / kCT;
         // column tiles in spiral order from the item's own tile: near points
@@ -502,45 +411,6 @@ batched_knn_kernel(const float* __restrict__ xc, const unsigned* __restrict__ li
         for (int qt = 0; qt < ntp; ++qt) {
             const int ct = spiral_tile(T, qt, ntp);
             const int c0 = ct * kCT;
-            // prune (warp 0): the tile is farther than every row's k-th distance
-            // (bounding boxes only pay in low dimensions: DP <= 8)
-            const int par = qt & 1;
-            if (DP <= 8 && warp == 0) {
-                const float* g = tbox + (toff[p] + ct) * 2 * d;
-                for (int f = lane; f < d; f += 32) {
-                    sh.tb[par][0][f] = g[f];
-                    sh.tb[par][1][f] = g[d + f];
-                }
-                float km = __int_as_float(0xff800000);
-                for (int r = lane; r < kRT; r += 32) {
-                    if (r0 + r < n) {
-                        const uint64_t kk = sh.L.kth[r];
-                        km = fmaxf(km, kk == kKeyMax ? __int_as_float(0x7f800000) : __uint_as_float(key_bits(kk)));
-                    }
-                }
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) km = fmaxf(km, __shfl_xor_sync(0xffffffffu, km, o));
-                __syncwarp();
-                const float g2 = gap2_rd(sh.cbox[0], sh.cbox[1], sh.tb[par][0], sh.tb[par][1], d);
-                if (lane == 0) sh.skip_tile[par] = __fmul_rd(g2, kBPruneShrink) > km ? 1 : 0;
-            }
-            if (DP <= 8) {
-                __syncthreads();
-                if (sh.skip_tile[par]) continue;
-            }
-            // this warp's rows may all be beyond the tile
-            bool wskip = false;
-            if (DP <= 8) {
-                float wk = __int_as_float(0xff800000);
-                if (lane < kRowsPerWarp && r0 + rw + lane < n) {
-                    const uint64_t kk = sh.L.kth[rw + lane];
-                    wk = kk == kKeyMax ? __int_as_float(0x7f800000) : __uint_as_float(key_bits(kk));
-                }
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) wk = fmaxf(wk, __shfl_xor_sync(0xffffffffu, wk, o));
-                wskip = __fmul_rd(gap2_rd(sh.wbox[warp][0], sh.wbox[warp][1], sh.tb[par][0], sh.tb[par][1], d),
-                                  kBPruneShrink) > wk;
-            }
             // the CTA stages 128 columns (coalesced) as packed pairs
             for (int i = tid; i < kCT * DP; i += kThreads) {
                 const int c = i / DP, f = i % DP;
@@ -549,45 +419,33 @@ batched_knn_kernel(const float* __restrict__ xc, const unsigned* __restrict__ li
             }
             __syncthreads();
 #pragma unroll 1
-            for (int sub = 0; sub < (wskip ? 0 : kCT); sub += kTile) {
-            uint64_t cp[CP][DP];
-            int cc[CP];
+            for (int sub = 0; sub < kCT; sub += kTile) {
+            uint64_t cp[DP];
+            const int pr = (sub >> 1) + lane;  // column pair index in the tile
+            const int cc = c0 + 2 * pr;
+#pragma unroll
+            for (int f = 0; f < DP; ++f) cp[f] = sh.cols2[pr][f];
             // per column: its original index in the key's low half, or all
             // ones (a key of kKeyMax) for columns beyond the problem
-            uint64_t cidx[2 * CP];
-#pragma unroll
-            for (int q = 0; q < CP; ++q) {
-                const int pr = (sub >> 1) + 32 * q + lane;  // column pair index in the tile
-                cc[q] = c0 + 2 * pr;
-#pragma unroll
-                for (int f = 0; f < DP; ++f) cp[q][f] = sh.cols2[pr][f];
-                cidx[2 * q] = cc[q] < n ? static_cast<uint64_t>(li[cc[q]]) : kKeyMax;
-                cidx[2 * q + 1] = cc[q] + 1 < n ? static_cast<uint64_t>(li[cc[q] + 1]) : kKeyMax;
-            }
+            const uint64_t cidx[2] = {cc < n ? static_cast<uint64_t>(li[cc]) : kKeyMax,
+                                      cc + 1 < n ? static_cast<uint64_t>(li[cc + 1]) : kKeyMax};
             const bool own = c0 == r0;  // the only tile holding the rows' own points
 #pragma unroll 1
             for (int rr = 0; rr < kRowsPerWarp; rr += 2) {
                 const int r = rw + rr;
                 if (r0 + r >= n) break;  // warp-uniform: rows beyond the problem
-                uint64_t s[2][CP];
-#pragma unroll
-                for (int h = 0; h < 2; ++h)
-#pragma unroll
-                    for (int q = 0; q < CP; ++q) s[h][q] = 0;
+                uint64_t s[2] = {0, 0};
                 // dimensions past d are zero in both operands: each adds
                 // fma(0, 0, s) = s, so the chain over all DP equals the
                 // oracle's chain over d
 #pragma unroll
                 for (int f = 0; f < DP; ++f) {
                     const uint64_t a0 = sh.rows2[r][f], a1 = sh.rows2[r + 1][f];
-#pragma unroll
-                    for (int q = 0; q < CP; ++q) {
-                        uint64_t t0, t1;
-                        asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(t0) : "l"(a0), "l"(cp[q][f]));
-                        asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(t1) : "l"(a1), "l"(cp[q][f]));
-                        s[0][q] = fma2(t0, t0, s[0][q]);
-                        s[1][q] = fma2(t1, t1, s[1][q]);
-                    }
+                    uint64_t t0, t1;
+                    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(t0) : "l"(a0), "l"(cp[f]));
+                    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(t1) : "l"(a1), "l"(cp[f]));
+                    s[0] = fma2(t0, t0, s[0]);
+                    s[1] = fma2(t1, t1, s[1]);
                 }
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
@@ -597,21 +455,14 @@ batched_knn_kernel(const float* __restrict__ xc, const unsigned* __restrict__ li
                     // is at most the k-th distance: test the distances first
                     const uint64_t kk = sh.L.kth[r + h];
                     const float kd = kk == kKeyMax ? __int_as_float(0x7f800000) : __uint_as_float(key_bits(kk));
-                    bool maybe = false;
-#pragma unroll
-                    for (int q = 0; q < CP; ++q) maybe |= (lo_f(s[h][q]) <= kd) | (hi_f(s[h][q]) <= kd);
-                    if (!__any_sync(0xffffffffu, maybe)) continue;
-                    uint64_t key[2 * CP];
-#pragma unroll
-                    for (int q = 0; q < CP; ++q) {
-                        key[2 * q] = (static_cast<uint64_t>(__float_as_uint(lo_f(s[h][q]))) << 32) | cidx[2 * q];
-                        key[2 * q + 1] = (static_cast<uint64_t>(__float_as_uint(hi_f(s[h][q]))) << 32) | cidx[2 * q + 1];
-                        if (own) {  // a row is not its own neighbour
-                            if (cc[q] == gr) key[2 * q] = kKeyMax;
-                            if (cc[q] + 1 == gr) key[2 * q + 1] = kKeyMax;
-                        }
+                    if (!__any_sync(0xffffffffu, (lo_f(s[h]) <= kd) | (hi_f(s[h]) <= kd))) continue;
+                    uint64_t key[2] = {(static_cast<uint64_t>(__float_as_uint(lo_f(s[h]))) << 32) | cidx[0],
+                                       (static_cast<uint64_t>(__float_as_uint(hi_f(s[h]))) << 32) | cidx[1]};
+                    if (own) {  // a row is not its own neighbour
+                        if (cc == gr) key[0] = kKeyMax;
+                        if (cc + 1 == gr) key[1] = kKeyMax;
                     }
-                    offer_row<CP>(sh.L, r + h, key, k);
+                    offer_row(sh.L, r + h, key, k);
                 }
             }
             }
@@ -708,27 +559,15 @@ __global__ void pid_kernel(const int64_t* __restrict__ off, int num, int* __rest
         for (int64_t i = off[p] + threadIdx.x; i < off[p + 1]; i += blockDim.x) pid[i] = p;
 }
 
-int dp_for(int d) { return d <= 4 ? 4 : d <= 8 ? 8 : d <= 16 ? 16 : d <= 32 ? 32 : 64; }
+int dp_for(int d) { return d <= 32 ? 32 : 64; }  // (up to 16 features: the sweep)
 
-template <int DP, int CP>
-void launch_knn_t(int grid, const BatchDev& b, cudaStream_t s) {
+template <int DP>
+void launch_knn(int grid, const BatchDev& b, cudaStream_t s) {
     const size_t smem = sizeof(BatchSmem<DP>);
-    set_max_dynamic_smem(reinterpret_cast<const void*>(batched_knn_kernel<DP, CP>), static_cast<int>(smem));
-    batched_knn_kernel<DP, CP><<<grid, kThreads, smem, s>>>(b.xs, b.lidx, b.off, b.ks, b.nkoff, b.items, b.nitems,
-                                                           b.d, b.counter, b.nbr, b.d2, b.kd, b.tbox, b.toff);
+    set_max_dynamic_smem(reinterpret_cast<const void*>(batched_knn_kernel<DP>), static_cast<int>(smem));
+    batched_knn_kernel<DP><<<grid, kThreads, smem, s>>>(b.xs, b.lidx, b.off, b.ks, b.nkoff, b.items, b.nitems, b.d,
+                                                       b.counter, b.nbr, b.d2, b.kd);
     CG_LAUNCH_CHECK();
-}
-
-// cp2: two column pairs per lane (d <= 16), else one.
-void launch_knn(int dp, bool cp2, int grid, const BatchDev& b, cudaStream_t s) {
-    switch (dp) {
-        case 4: cp2 ? launch_knn_t<4, 2>(grid, b, s) : launch_knn_t<4, 1>(grid, b, s); break;
-        case 8: cp2 ? launch_knn_t<8, 2>(grid, b, s) : launch_knn_t<8, 1>(grid, b, s); break;
-        case 16: cp2 ? launch_knn_t<16, 2>(grid, b, s) : launch_knn_t<16, 1>(grid, b, s); break;
-        case 32: launch_knn_t<32, 1>(grid, b, s); break;
-        case 64: launch_knn_t<64, 1>(grid, b, s); break;
-        default: throw Error(kInternal, "bad padded dimension");
-    }
 }
 
 constexpr int kSweepMaxD = 16;  // more features take batched_knn_kernel
@@ -757,18 +596,6 @@ void launch_tiles(const BatchDev& b, const unsigned* perm, cudaStream_t s) {
     bm_tile_kernel<DP><<<static_cast<unsigned>(b.ntiles), kCT, 0, s>>>(b.xc, b.d, perm, b.off, b.tpid, b.toff, b.tiles,
                                                                        b.tbox);
     CG_LAUNCH_CHECK();
-}
-
-template <int DP>
-size_t knn_smem() { return sizeof(BatchSmem<DP>); }
-size_t knn_smem_for(int dp) {
-    switch (dp) {
-        case 4: return knn_smem<4>();
-        case 8: return knn_smem<8>();
-        case 16: return knn_smem<16>();
-        case 32: return knn_smem<32>();
-        default: return knn_smem<64>();
-    }
 }
 
 int grid_cap(int64_t items) {
@@ -944,11 +771,9 @@ void Engine::batch_launch(const float* d_x, float* d_scores) {
     } else {
         bm_gather_kernel<<<grid_cap(P.ntot * d), 256, 0, s>>>(b.xc, P.ntot, d, perm, b.pid, b.off, b.xs, b.lidx);
         CG_LAUNCH_CHECK();
-        bm_tilebox_kernel<<<static_cast<unsigned>(ceil_div(b.ntiles, 8)), 256, 0, s>>>(b.xs, b.off, d, b.tpid, b.toff,
-                                                                                       b.ntiles, b.tbox);
-        CG_LAUNCH_CHECK();
         CG_CUDA(cudaMemsetAsync(b.counter, 0, sizeof(unsigned), s));
-        launch_knn(dp_for(d), btune_packed_, btune_grid_, b, s);
+        if (dp_for(d) == 32) launch_knn<32>(btune_grid_, b, s);
+        else launch_knn<64>(btune_grid_, b, s);
     }
     bl_lrd_kernel<<<static_cast<unsigned>(ceil_div(P.ntot, 256)), 256, 0, s>>>(P.ntot, b.pid, b.off, b.ks, b.nkoff,
                                                                                b.nbr, b.d2, b.kd, b.lrd);
@@ -962,8 +787,7 @@ void Engine::batch_launch(const float* d_x, float* d_scores) {
 void Engine::batch_autotune(const float* d_x, float* d_scores) {
     int sms = 152;
     CG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device_));
-    const int dp = dp_for(bplan_.d);
-    const size_t smem = knn_smem_for(dp);
+    const size_t smem = dp_for(bplan_.d) == 32 ? sizeof(BatchSmem<32>) : sizeof(BatchSmem<64>);
     int max_per_sm = static_cast<int>(227 * 1024 / (smem + 1024));
     if (max_per_sm < 1) max_per_sm = 1;
     if (max_per_sm > 2) max_per_sm = 2;
@@ -976,28 +800,23 @@ void Engine::batch_autotune(const float* d_x, float* d_scores) {
     float best = 1e30f;
     for (float& t : btune_ms_) t = -1.0f;
     for (int per = 1; per <= max_per_sm; ++per) {
-        for (int packed = 0; packed <= (!sweep && dp <= 16 ? 1 : 0); ++packed) {
-            btune_grid_ = per * sms;
-            btune_packed_ = packed != 0;
-            batch_launch(d_x, d_scores);  // warm (first use configures the kernel)
-            CG_CUDA(cudaEventRecord(e0, stream_));
-            batch_launch(d_x, d_scores);
-            CG_CUDA(cudaEventRecord(e1, stream_));
-            CG_CUDA(cudaEventSynchronize(e1));
-            float ms = 0.0f;
-            CG_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-            btune_ms_[2 * (per - 1) + packed] = ms;
-            if (ms < best) {
-                best = ms;
-                bbest_grid_ = btune_grid_;
-                bbest_packed_ = btune_packed_;
-            }
+        btune_grid_ = per * sms;
+        batch_launch(d_x, d_scores);  // warm (first use configures the kernel)
+        CG_CUDA(cudaEventRecord(e0, stream_));
+        batch_launch(d_x, d_scores);
+        CG_CUDA(cudaEventRecord(e1, stream_));
+        CG_CUDA(cudaEventSynchronize(e1));
+        float ms = 0.0f;
+        CG_CUDA(cudaEventElapsedTime(&ms, e0, e1));
+        btune_ms_[2 * (per - 1)] = ms;
+        if (ms < best) {
+            best = ms;
+            bbest_grid_ = btune_grid_;
         }
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     btune_grid_ = bbest_grid_;
-    btune_packed_ = bbest_packed_;
     btuned_ = true;
 }
 
@@ -1072,6 +891,6 @@ void Engine::batched_tuning(float* ms4, int* per_sm, int* pairs_per_lane) const 
     int dev_sms = 152;
     cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, device_);
     *per_sm = btuned_ ? sms / (dev_sms > 0 ? dev_sms : 1) : 0;
-    *pairs_per_lane = btuned_ ? (bbest_packed_ ? 2 : 1) : 0;
+    *pairs_per_lane = btuned_ ? 1 : 0;
 }
 }  // namespace culof_gb300

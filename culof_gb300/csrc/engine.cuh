@@ -119,7 +119,7 @@ public:
     // The batched autotuner's measurements for the current layout (times of
     // the whole batched call): ms4[2 (c - 1) + (p - 1)] for the k-NN kernel at
     // c CTAs per SM (the sweep of up to 16 features: 1, or 2 for as many as fit)
-    // and p column pairs per lane (-1: not tried), and its
+    // and p column pairs per lane (-1: not tried; only one pair is), and its
     // choice (0 before the first batched call).
     void batched_tuning(float* ms4, int* per_sm, int* pairs_per_lane) const;
     // Pairs the last FP32 small-d sweep evaluated and the pairs of an
@@ -164,7 +164,7 @@ private:
     DevBuf bxs_, blidx_, bpmm_, bpdims_, bskeys_, bsvals_, bscounts_;
     DevBuf bplan_toff_, bplan_tpid_, btbox_, btiles_;
     bool use_graphs_ = true;
-    bool btuned_ = false, btune_packed_ = true, bbest_packed_ = true;
+    bool btuned_ = false;
     int btune_grid_ = 152, bbest_grid_ = 152, bsms_ = 152;
     float btune_ms_[4] = {-1.0f, -1.0f, -1.0f, -1.0f};  // (CTAs per SM 1..2) x (column pairs 1..2)
     cudaGraphExec_t bgraph_exec_ = nullptr;

@@ -9,17 +9,16 @@
 //     with a stable LSD radix sort; tiles of 128 consecutive sorted points
 //     are spatially compact.
 //  2. d <= 8: one kernel per row tile (small.cu) with per-row pruning.
-//     Wider points: a seed (per row, the exact k best over its own tile; its
-//     k-th key bounds the row's true k-th key), then a sweep over the other
-//     tiles (tc_sweep.cu on the tensor cores, wide.cu in FP32): a filter value
-//     per pair is compared with a per-row threshold, a rigorous error bound
-//     over the row's current k-th key, so every column that can still enter
-//     the k best passes and is rescored exactly. The k-th key is shared across
-//     the column splits of a row tile through global memory (atomicMin), so
-//     later splits start from earlier ones'.
-//  3. merge (wider points): the seed list and the S column-split lists give
-//     the k best keys; slots are written in the reference's order (keys below
-//     the k-th by ascending index, then the ties, knn.cu:190-224).
+//     Wider points: a sweep over the column tiles on the tensor cores
+//     (tc_sweep.cu) or in FP32 (wide.cu, started from a seed: per row, the
+//     exact k best over its own tile): a filter value per pair is compared
+//     with a per-row threshold, a rigorous error bound over the row's current
+//     k-th key, so every column that can still enter the k best passes and is
+//     rescored exactly.
+//  3. the tensor path's final kernel, or the FP32 path's merge of its seed and
+//     S column-split lists, gives the k best keys; slots are written in the
+//     reference's order (keys below the k-th by ascending index, then the
+//     ties, knn.cu:190-224).
 //
 // Exactness: the selection key is (exact float32 distance bits, original
 // index), identical to the general path and the oracle; the filter only
