@@ -13,8 +13,8 @@ pytestmark = pytest.mark.gpu
 
 CASES = [
     # one tile, two tiles, a last tile of one point; k at the list registers'
-    # and the group minima's limits (63 + the row itself fill the 64 groups, 64
-    # takes no scan); d at the operand boxes' limits
+    # and the group minima's limits (63 + the row itself fill the 64 groups; the
+    # scan has two halves above 55); d at the operand boxes' limits
     (100, 16, 20), (129, 42, 32), (256, 43, 33), (1000, 64, 63), (1000, 65, 64), (3001, 128, 50), (20000, 24, 1),
 ]
 
