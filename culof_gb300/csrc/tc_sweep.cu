@@ -563,6 +563,20 @@ __noinline__ __device__ bool exact_chunk(TcRows& sh, uint64_t* __restrict__ glis
     bool compacted = false;
     const int64_t own = rbase + row0 + lane - cbase;  // not the row itself
     if (own >= 0 && own < 32) pass &= ~(1u << static_cast<int>(own));
+    // a row that most columns pass: the lanes are its columns, consecutive in
+    // memory (20,000 equal points of 32 features: 38 ms for 42)
+    unsigned dense = __ballot_sync(0xffffffffu, __popc(pass) >= 16);
+    while (dense) {
+        const int src = __ffs(dense) - 1;
+        dense &= dense - 1;
+        const unsigned cols = __shfl_sync(0xffffffffu, pass, src);
+        ExactPending q;
+        q.row = row0 + src;
+        q.col = cbase + __fns(cols, 0, lane + 1);
+        q.n = __popc(cols);
+        compacted |= exact_flush(sh, glist, q, rbase, xr, ix, dr, k);
+        if (lane == src) pass = 0u;
+    }
     while (__any_sync(0xffffffffu, pass != 0u)) {
         // every row with candidates left gives one to the next free lanes
         const unsigned rows = __ballot_sync(0xffffffffu, pass != 0u);
@@ -570,7 +584,7 @@ __noinline__ __device__ bool exact_chunk(TcRows& sh, uint64_t* __restrict__ glis
         const int mine = __popc(rows & ((1u << lane) - 1u));  // my place among the givers
         const int b = pass != 0u ? __ffs(pass) - 1 : 0;
         const int want = lane - p.n;  // which giver this lane takes
-        const int src = want >= 0 && want < take ? static_cast<int>(__fns(rows, 0, want + 1)) : 0;
+        const int src = want < 0 || want >= take ? 0 : give == 32 ? want : static_cast<int>(__fns(rows, 0, want + 1));
         const int gb = __shfl_sync(0xffffffffu, b, src);
         if (want >= 0 && want < take) {
             p.row = row0 + src;

@@ -42,3 +42,14 @@ def test_small_sweep_bit_exact(monkeypatch, n, d, k, iso):
     np.testing.assert_array_equal(kd.cpu().numpy().view(np.uint32), o_kd.view(np.uint32))
     np.testing.assert_array_equal(idx.cpu().numpy(), o_idx)
     np.testing.assert_array_equal(d2.cpu().numpy().view(np.uint32), o_d2.view(np.uint32))
+
+
+@pytest.mark.parametrize("n,d,k", [(8000, 1, 20), (9000, 3, 32), (17000, 8, 33)])
+def test_ties_enter_by_index_only(n, d, k):
+    # a few distinct points: most distances tie with the k-th
+    rng = np.random.default_rng(n)
+    X = np.round(rng.random((n, d)) * 2).astype(np.float32)
+    with _culof.Context() as ctx:
+        ctx.set_path(_culof.PATH_FAST)
+        got = ctx.lof(X, k)
+    np.testing.assert_array_equal(got.view(np.uint32), oracle.lof(X, k).view(np.uint32))
