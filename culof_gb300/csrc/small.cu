@@ -36,6 +36,7 @@
 #include "row_list.cuh"
 #include "small.cuh"
 #include "sweep_rows.cuh"
+#include "tile_order.cuh"
 #include "warp_sort.cuh"
 
 namespace culof_gb300 {
@@ -221,16 +222,19 @@ __device__ __forceinline__ float box_extent(const float* __restrict__ b, int dp)
 // Launch order of the sweep's row tiles [t0, t0 + mt): widest boxes first
 // (their rows lie in sparse regions, have far neighbours and take the
 // longest), so that no long CTA starts last. The rank is counted against
-// every other tile (mt^2 comparisons).
+// every other tile (mt^2 comparisons) in a total order (tile_order.cuh), so
+// every place of order is written once, whatever the points hold.
 __global__ void __launch_bounds__(256) tile_order_kernel(const float* __restrict__ boxes, int dp, int t0, int mt,
                                                          int* __restrict__ order) {
     // 32 tiles per block, eight threads per tile for an eighth of the others each
-    __shared__ float other[256];
+    __shared__ unsigned other[256];
     __shared__ int ranks[32];
-    const auto extent = [&](int t) { return box_extent(boxes + static_cast<int64_t>(t0 + t) * 2 * dp, dp); };
+    const auto extent = [&](int t) {
+        return extent_key(__float_as_uint(box_extent(boxes + static_cast<int64_t>(t0 + t) * 2 * dp, dp)));
+    };
     const int lane = threadIdx.x & 31, part = threadIdx.x >> 5;
     const int t = blockIdx.x * 32 + lane;
-    const float mine = t < mt ? extent(t) : 0.0f;
+    const unsigned mine = t < mt ? extent(t) : 0u;
     if (part == 0) ranks[lane] = 0;
     int rank = 0;
     for (int c0 = 0; c0 < mt; c0 += 256) {
@@ -238,10 +242,7 @@ __global__ void __launch_bounds__(256) tile_order_kernel(const float* __restrict
         if (c0 + static_cast<int>(threadIdx.x) < mt) other[threadIdx.x] = extent(c0 + threadIdx.x);
         __syncthreads();
         const int c1 = min(32 * (part + 1), mt - c0);
-        for (int i = 32 * part; i < c1; ++i) {
-            const float v = other[i];
-            rank += (v > mine || (v == mine && c0 + i < t)) ? 1 : 0;
-        }
+        for (int i = 32 * part; i < c1; ++i) rank += starts_before(other[i], c0 + i, mine, t) ? 1 : 0;
     }
     __syncthreads();
     atomicAdd(&ranks[lane], rank);
@@ -260,13 +261,18 @@ small_sweep_kernel(SweepRows P, int64_t row0, const int* __restrict__ order, int
     // first row position; the tiles' CTAs start in the given order
     constexpr int kPerTile = kCT / Smem::kRows;
     const int tile_i = static_cast<int>(blockIdx.x) / kPerTile;
-    P.base = row0 + static_cast<int64_t>(order ? order[tile_i] : tile_i) * kCT +
-             static_cast<int>(blockIdx.x) % kPerTile * Smem::kRows;
+    const int tile = order ? order[tile_i] : tile_i;
+    if (static_cast<unsigned>(tile) >= static_cast<unsigned>(mt)) {  // never: order is a permutation
+        if (threadIdx.x == 0) atomicExch(P.status, 2);
+        return;
+    }
+    P.base = row0 + static_cast<int64_t>(tile) * kCT + static_cast<int>(blockIdx.x) % kPerTile * Smem::kRows;
     if (P.base >= P.n) return;
     if (defer_rows) {
+        const int median = static_cast<int>(min(static_cast<unsigned>(order[mt / 2]), static_cast<unsigned>(mt - 1)));
         P.sparse = defer_rows == 2 && tile_i < mt / 32 &&
                    box_extent(P.boxes + P.base / kCT * 2 * DP, DP) >
-                       kSparseRatio * box_extent(P.boxes + (row0 / kCT + order[mt / 2]) * 2 * DP, DP);
+                       kSparseRatio * box_extent(P.boxes + (row0 / kCT + median) * 2 * DP, DP);
         sweep_rows<DP, KR, G, RW, W, true>(sh, P);
     } else {
         sweep_rows<DP, KR, G, RW, W, false>(sh, P);
