@@ -194,6 +194,12 @@ bm_minmax_kernel(const float* __restrict__ xc, const int64_t* __restrict__ off, 
                     best = f;
                 }
             }
+            // (ranges that are not numbers: the first feature not yet taken)
+            for (int f = 0; best < 0; ++f) {
+                bool taken = false;
+                for (int q = 0; q < j; ++q) taken |= chosen[q] == f;
+                if (!taken) best = f;
+            }
             chosen[j] = best;
             pdims[p * kMortonDimsB + j] = best;
         }

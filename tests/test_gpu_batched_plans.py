@@ -1,0 +1,46 @@
+"""Batched LOF: every list form, padded width and kernel of the batched path,
+values that are not finite, and plans that are refused."""
+
+import numpy as np
+import pytest
+
+import oracle
+from culof_gb300 import _culof, synthetic
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+
+class Batch:
+    def __init__(self, problems, ks):
+        self.ks = list(ks)
+        self.d = problems[0].shape[1]
+        self.off = np.zeros(len(problems) + 1, np.int64)
+        self.off[1:] = np.cumsum([len(p) for p in problems])
+        self.x = torch.from_numpy(np.concatenate(problems).astype(np.float32)).cuda()
+        self.out = torch.zeros(int(self.off[-1]), device="cuda")
+
+    def run(self, ctx, ks=None, normalize=False):
+        ctx.lof_batched_device(self.off, self.ks if ks is None else ks, self.x.data_ptr(), self.d, normalize,
+                               self.out.data_ptr())
+        ctx.synchronize()
+        s = self.out.cpu().numpy()
+        return [s[self.off[i]:self.off[i + 1]] for i in range(len(self.ks))]
+
+
+def _same(got, problem, k):
+    np.testing.assert_array_equal(got.view(np.uint32), oracle.lof(problem, k).view(np.uint32))
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+@pytest.mark.parametrize("d", [1, 3, 16, 24])
+def test_values_that_are_not_finite_stay_in_their_problem(d, bad):
+    probs = [synthetic.clusters_with_outliers(n, d, seed=n) for n in (300, 900, 2000)]
+    spoilt = [p.copy() for p in probs]
+    spoilt[0][5, 0] = bad  # the first problem: nothing lies before its ranges
+    spoilt[1][:, :] = bad
+    with _culof.Context() as ctx:
+        got = Batch(spoilt, [10, 30, 20]).run(ctx)
+        _same(got[2], probs[2], 20)
+        for g, p, k in zip(Batch(probs, [10, 30, 20]).run(ctx), probs, [10, 30, 20]):
+            _same(g, p, k)
