@@ -824,7 +824,7 @@ void Engine::knn_fast(const float* xc, const float* norms, int64_t n, int d, int
     float* tiles = nullptr;
     TcBuffers tcb{};
     float* boxes = nullptr;
-    if (tensor) tcb = tc_prepare(cols_.get(tc_buffer_bytes(padded, d)), xc, norms, n, d, perm, nt, mm, s);
+    if (tensor) tcb = tc_prepare(cols_.get(tc_buffer_bytes(padded, d)), xc, norms, n, d, perm, nt, mm, max_norm_word(), s);
     if (wide) {
         tiles = cols_.as<float>(wide_tiles_floats(d, nt));
         wide_build_tiles(xc, norms, n, d, perm, nt, tiles, s);

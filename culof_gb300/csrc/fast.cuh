@@ -65,9 +65,10 @@ struct TcBuffers {
     int ksteps;
 };
 size_t tc_buffer_bytes(int64_t padded, int d);
-// minmax: the per-dimension (min, max) keys of the spatial-order pass.
+// minmax: the per-dimension (min, max) keys of the spatial-order pass; maxn:
+// the largest norm (float bits).
 TcBuffers tc_prepare(void* buf, const float* xc, const float* norms, int64_t n, int d, const unsigned* perm, int nt,
-                     const unsigned* minmax, cudaStream_t s);
+                     const unsigned* minmax, const unsigned* maxn, cudaStream_t s);
 int tc_max_splits();
 constexpr int kMaxTensorD = 256;
 constexpr int kTcSplitD = 42;  // split operands up to here (3d <= 128)

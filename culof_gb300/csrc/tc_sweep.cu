@@ -43,8 +43,9 @@
 // of the tensor core (taken as K * 2^-20 relative), the float32 norms and
 // the float32 evaluation of f, so no column that belongs to a row's k
 // nearest is ever dropped. Data whose scale cannot be brought into the f16
-// range (|S| > 62, or non-finite values) disable the filter: every pair is
-// then rescored exactly.
+// range (|S| > 62, or non-finite values) or whose squared norms come near the
+// largest float (above 2^124: f would overflow) disable the filter: every pair
+// is then rescored exactly.
 #include <cuda_fp16.h>
 
 #include <cmath>
@@ -84,10 +85,15 @@ __device__ __forceinline__ float unflip(unsigned k) {
     return __uint_as_float((k & 0x80000000u) ? (k & 0x7FFFFFFFu) : ~k);
 }
 
-// One warp: the scale exponent from the features' ranges.
-__global__ void tc_scale_kernel(const unsigned* __restrict__ mm, int d, TcScale* __restrict__ out) {
+// One warp: the scale exponent from the features' ranges. The filter is off if
+// f = |b|^2 - 2 a.b could overflow: |f| <= 3 nmax (1 + 2^-8) and the bounds add
+// 2 m0 + slack, less than nmax, which together stay below 2^127 up to nmax =
+// 2^124 (the comparison also catches a norm that is not a number).
+constexpr float kMaxNorm = 21267647932558653966460912964485513216.0f;  // 2^124
+__global__ void tc_scale_kernel(const unsigned* __restrict__ mm, int d, const unsigned* __restrict__ max_norm_bits,
+                                TcScale* __restrict__ out) {
     float mx = 0.0f;
-    bool finite = true;
+    bool finite = __uint_as_float(*max_norm_bits) <= kMaxNorm;
     for (int f = threadIdx.x; f < d; f += 32) {
         const float lo = range_lo(mm, f), hi = range_hi(mm, f);
         finite = finite && isfinite(lo) && isfinite(hi);
@@ -1114,7 +1120,7 @@ size_t tc_list_bytes(int nt, int nsplit) {
 }
 
 TcBuffers tc_prepare(void* buf, const float* xc, const float* norms, int64_t n, int d, const unsigned* perm, int nt,
-                     const unsigned* minmax, cudaStream_t s) {
+                     const unsigned* minmax, const unsigned* maxn, cudaStream_t s) {
     const int64_t padded = static_cast<int64_t>(nt) * kCT;
     const auto up = [](size_t x) { return (x + 255) & ~static_cast<size_t>(255); };
     TcBuffers b;
@@ -1140,7 +1146,7 @@ TcBuffers tc_prepare(void* buf, const float* xc, const float* norms, int64_t n, 
     b.ix = reinterpret_cast<unsigned*>(p);
     p += up(sizeof(unsigned) * padded);
     b.scale = p;
-    tc_scale_kernel<<<1, 32, 0, s>>>(minmax, d, reinterpret_cast<TcScale*>(b.scale));
+    tc_scale_kernel<<<1, 32, 0, s>>>(minmax, d, maxn, reinterpret_cast<TcScale*>(b.scale));
     CG_LAUNCH_CHECK();
     int64_t g = ceil_div(padded * b.Kp, 256);
     if (g > 152 * 16) g = 152 * 16;
