@@ -24,6 +24,7 @@
 #include <algorithm>
 #include <cstring>
 #include <sstream>
+#include <utility>
 #include <vector>
 
 #include "common.cuh"
@@ -619,7 +620,7 @@ void Engine::batch_plan(int num, const int64_t* offsets, const int* ks, int d, b
     if (!offsets || !ks) throw Error(kInvalidArgument, "offsets and ks must not be null");
     if (d < 1 || d > kBMaxD) throw Error(kInvalidArgument, "the batched path takes 1 <= n_dims <= 64");
     if (offsets[0] != 0) throw Error(kInvalidArgument, "offsets[0] must be 0");
-    BatchPlan& P = bplan_;
+    BatchPlan P;  // (a refused layout leaves the planned one as it was)
     P.num = num;
     P.d = d;
     P.normalize = normalize;
@@ -668,6 +669,11 @@ void Engine::batch_plan(int num, const int64_t* offsets, const int* ks, int d, b
     if (d <= kSweepMaxD)
         std::stable_sort(items.begin(), items.end(),
                          [&](const std::pair<int64_t, uint2>& a, const std::pair<int64_t, uint2>& b) { return form(a) < form(b); });
+    // From here to the end no layout is planned: a call that runs out of memory
+    // leaves nothing that a later one could match.
+    bgraph_valid_ = false;
+    btuned_ = false;
+    bplan_.num = 0;
     for (int& g : bdev_.group) g = 0;
     for (const auto& it : items) ++bdev_.group[form(it)];
     P.items.resize(items.size());
@@ -721,8 +727,7 @@ void Engine::batch_plan(int num, const int64_t* offsets, const int* ks, int d, b
     pid_kernel<<<num < 4096 ? num : 4096, 256, 0, s>>>(b.off, num, b.pid);
     CG_LAUNCH_CHECK();
     CG_CUDA(cudaStreamSynchronize(s));
-    bgraph_valid_ = false;
-    btuned_ = false;
+    bplan_ = std::move(P);
 }
 
 void Engine::batch_launch(const float* d_x, float* d_scores) {
@@ -836,6 +841,7 @@ bool Engine::batch_same_plan(int num, const int64_t* offsets, const int* ks, int
 void Engine::lof_batched_device(int num, const int64_t* offsets, const int* ks, const float* d_x, int d,
                                 bool normalize, float* d_scores) {
     if (!d_x || !d_scores) throw Error(kInvalidArgument, "device pointers must not be null");
+    if (!offsets || !ks) throw Error(kInvalidArgument, "offsets and ks must not be null");
     CG_CUDA(cudaSetDevice(device_));
     if (!(bplan_.num > 0 && batch_same_plan(num, offsets, ks, d, normalize))) batch_plan(num, offsets, ks, d, normalize);
     if (!btuned_) batch_autotune(d_x, d_scores);
@@ -848,6 +854,7 @@ void Engine::lof_batched_device(int num, const int64_t* offsets, const int* ks, 
             cudaGraphExecDestroy(bgraph_exec_);
             bgraph_exec_ = nullptr;
         }
+        bgraph_valid_ = false;
         cudaGraph_t g = nullptr;
         const unsigned long long before = launch_count();
         CG_CUDA(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));

@@ -44,3 +44,23 @@ def test_values_that_are_not_finite_stay_in_their_problem(d, bad):
         _same(got[2], probs[2], 20)
         for g, p, k in zip(Batch(probs, [10, 30, 20]).run(ctx), probs, [10, 30, 20]):
             _same(g, p, k)
+
+
+def test_a_refused_layout_is_refused_again():
+    # after a valid batch, with the same buffers: neither its graph nor its
+    # plan may answer for the layout that was refused
+    probs = [synthetic.clusters_with_outliers(n, 4, seed=n) for n in (50, 60, 300)]
+    ks = [5, 10, 20]
+    with _culof.Context() as ctx:
+        b = Batch(probs, ks)
+        b.run(ctx)
+        for bad in ([50, 10, 20], [5, 10, 49], [5, 0, 20]):
+            for _ in range(2):
+                b.out.fill_(-1.0)
+                with pytest.raises(ValueError, match="k must satisfy"):
+                    b.run(ctx, ks=bad)
+                assert bool((b.out == -1.0).all())
+        for _ in range(2):
+            for got, p, k in zip(b.run(ctx), probs, ks):
+                _same(got, p, k)
+        assert ctx.batched_tuning()["ctas_per_sm"] > 0
