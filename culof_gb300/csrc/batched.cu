@@ -541,21 +541,12 @@ __global__ void bl_score_kernel(int64_t ntot, const int* __restrict__ pid, const
     const int64_t n = off[p + 1] - base, i = g - base;
     const int k = ks[p];
     const int32_t* ni = nbr_idx + nkoff[p];
-    // the quotients from one reciprocal (lof.cu: score_kernel has the proof)
     const double self = widen(lrd[g]), y = __ddiv_rn(1.0, self);
-    const bool quick = fabs(y) < __longlong_as_double(0x7ff0000000000000ll) && y != 0.0;
+    const bool quick = quotient_quick(y);
     double sum = 0.0;
     for (int t = 0; t < k; ++t) {
         const int32_t j = ni[static_cast<int64_t>(t) * n + i];
-        const double lj = (j >= 0 && j < n) ? widen(lrd[base + j]) : __longlong_as_double(0x7ff8000000000000ll);
-        double q;
-        if (quick) {
-            const double q0 = __dmul_rn(lj, y);
-            q = __fma_rn(__fma_rn(-q0, self, lj), y, q0);
-        } else {
-            q = __ddiv_rn(lj, self);
-        }
-        sum = __dadd_rn(sum, q);
+        sum = __dadd_rn(sum, quotient((j >= 0 && j < n) ? lrd[base + j] : __int_as_float(0x7fc00000), self, y, quick));
     }
     scores[g] = __double2float_rn(__ddiv_rn(sum, static_cast<double>(k)));
 }

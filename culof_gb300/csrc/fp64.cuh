@@ -34,4 +34,27 @@ __device__ __forceinline__ float narrow(double x) {
     return __double2float_rn(x);
 }
 
+// RN(a / b) of two floats, from y = RN(1 / b), once per b: q0 = RN(a y), r = a
+// - q0 b, q = RN(q0 + r y), the correction of a quotient by one residual (P.
+// Markstein, "Computation of elementary functions on the IBM RISC System/6000
+// processor", IBM J. Res. Dev. 34, 1990). With 24-bit significands q is the
+// correctly rounded quotient: q0 is off by at most 1.5 ulp, so r has at most 25
+// significant bits above ulp(q0) ulp(b) and is exact, and q0 + r y before its
+// rounding is off from a / b by at most 2^-104 of it, while a / b, not a
+// midpoint of two neighbouring doubles (a 54-bit midpoint M times b has more
+// than 24 bits), is at least 2^-78 away from one. `quick`: y is neither zero
+// nor infinite nor not a number (b is none of infinite, zero, not a number); an
+// infinite a would leave r = inf - inf. The rest takes the division itself.
+__device__ __forceinline__ bool quotient_quick(double y) {
+    return fabs(y) < __longlong_as_double(0x7ff0000000000000ll) && y != 0.0;
+}
+__device__ __forceinline__ double quotient(float a, double b, double y, bool quick) {
+    const double x = widen(a);
+    if (quick && (__float_as_uint(a) & 0x7FFFFFFFu) < 0x7F800000u) {
+        const double q0 = __dmul_rn(x, y);
+        return __fma_rn(__fma_rn(-q0, b, x), y, q0);
+    }
+    return __ddiv_rn(x, b);
+}
+
 }  // namespace culof_gb300

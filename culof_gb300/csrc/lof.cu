@@ -12,6 +12,7 @@
 
 #include "block.cuh"
 #include "common.cuh"
+#include "fp64.cuh"
 #include "prep.cuh"
 
 namespace culof_gb300 {
@@ -82,14 +83,7 @@ __global__ void __launch_bounds__(kBlock) lrd_kernel(const int32_t* __restrict__
 }
 
 // The slot terms are the correctly rounded quotients lrd_j / lrd_i, from one
-// reciprocal y = RN(1 / lrd_i) per point: q0 = RN(a y), r = a - q0 b, q =
-// RN(q0 + r y). For a, b with 24-bit significands this is RN(a / b): q0 is off
-// by at most 1.5 ulp, so r has at most 25 significant bits above ulp(q0)
-// ulp(b) and is exact, and q0 + r y before its rounding is off from a / b by
-// at most 2^-104 of it, while a / b, not a midpoint of two neighbouring
-// doubles (a 54-bit midpoint M times b has more than 24 bits), is at least
-// 2^-78 away from one. A reciprocal that is zero or not finite (lrd_i infinite,
-// zero or not a number) takes the division itself.
+// reciprocal per point (quotient(), fp64.cuh).
 __global__ void __launch_bounds__(kBlock) score_kernel(const int32_t* __restrict__ nbr_idx,
                                                        const float* __restrict__ lrd, int64_t n, int k,
                                                        const int32_t* __restrict__ rows, int64_t m,
@@ -107,7 +101,7 @@ __global__ void __launch_bounds__(kBlock) score_kernel(const int32_t* __restrict
     }
     __syncthreads();
     const double y = recip[lane];
-    const bool quick = fabs(y) < __longlong_as_double(0x7ff0000000000000ll) && y != 0.0;
+    const bool quick = quotient_quick(y);
     double sum = 0.0;
     for (int c0 = 0; c0 < k; c0 += kTermSlots) {
         const int c1 = k - c0 < kTermSlots ? k - c0 : kTermSlots;
@@ -118,13 +112,7 @@ __global__ void __launch_bounds__(kBlock) score_kernel(const int32_t* __restrict
                 if (j < 0 || j >= n) {
                     bad[lane] = 1;
                 } else {
-                    const double a = static_cast<double>(lrd[j]);
-                    if (quick) {
-                        const double q0 = __dmul_rn(a, y);
-                        v = __fma_rn(__fma_rn(-q0, self, a), y, q0);
-                    } else {
-                        v = __ddiv_rn(a, self);
-                    }
+                    v = quotient(lrd[j], self, y, quick);
                 }
             }
             term[t][lane] = v;
