@@ -269,7 +269,7 @@ __global__ void __launch_bounds__(kOffThreads)
 offset_cluster_kernel(const float* __restrict__ nof, int64_t n, int64_t lo, int use_upper, float w,
                       double* __restrict__ out, int64_t* __restrict__ labels) {
     namespace cg = cooperative_groups;
-    __shared__ int hist[3][kOffsetHistBins];
+    __shared__ __align__(8) int hist[3][kOffsetHistBins];  // read two bins at a time
     __shared__ int warp_sums[kOffThreads / 32];
     __shared__ int found_bin, found_acc, found_eq;
     __shared__ unsigned mn_s;
