@@ -26,18 +26,13 @@ namespace {
 
 using sweep::fma2;
 using sweep::dup2;
+using sweep::sub2;
 
 constexpr int kDirWarps = 8;
 constexpr int kDirThreads = 32 * kDirWarps;
 constexpr int kDirCols = 512;            // columns staged at a time
 constexpr int kDirLd = kDirCols + 4;     // row stride: the d values of a point fall in different banks
 constexpr int kDirBuf = 64;              // gathered keys per row before they are merged
-
-__device__ __forceinline__ uint64_t dsub2(uint64_t a, uint64_t b) {
-    uint64_t d;
-    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
 
 // KR: list registers (k <= 32 KR); G: groups of columns per lane.
 template <int DP, int KR, int G, int R>
@@ -71,7 +66,7 @@ direct_knn_kernel(const float* __restrict__ xc, int n, int d, int row_begin, int
         uint64_t s = 0;
 #pragma unroll
         for (int f = 0; f < DP; ++f) {
-            const uint64_t t = dsub2(a[r][f], x[f]);
+            const uint64_t t = sub2(a[r][f], x[f]);
             s = fma2(t, t, s);
         }
         u[0] = static_cast<unsigned>(s);

@@ -50,12 +50,6 @@ constexpr int kSeedWindow = 5;  // tiles of the seed: T, T+1, T-1, T+2, T-2
 constexpr int kMaxWideD = 128;
 constexpr int kMortonDims = 8;  // Morton key over (up to) the 8 widest dimensions
 
-__device__ __forceinline__ uint64_t sub2(uint64_t a, uint64_t b) {
-    uint64_t d;
-    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-
 // ---------------------------------------------------------------- spatial order
 
 // 32-bit Morton key: 32/m bits for each of the (up to) kMortonDims features of

@@ -20,11 +20,6 @@ constexpr float kDeferRatio = 4.0f;  // a row leaves when its squared k-th dista
 // of the packed f32x2 instructions), k-th distance, own index.
 __host__ __device__ constexpr int row_stride(int dp) { return 2 * dp + 4; }
 
-__device__ __forceinline__ uint64_t sub2(uint64_t a, uint64_t b) {
-    uint64_t d;
-    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
 __device__ __forceinline__ uint64_t add2_rd(uint64_t a, uint64_t b) {
     uint64_t d;
     asm("add.rm.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
