@@ -7,6 +7,10 @@
 // the k-th smallest of them bounds the row's k-th distance. The second pass
 // computes the distances again and gathers the columns within the bound (about
 // 31 at k = 20), which are sorted and written in the reference's slot order.
+// Columns come in ascending index order, so one that only ties with the k-th
+// of a full list cannot enter it: equal points stop gathering once they have
+// k neighbours (6,000 equal points, d = 8: 221 us per scores call, 764 with every tie
+// sorted in).
 //
 // What bounds it: the packed FP32 distances, 2 x 2d per 64 pairs and pass. The
 // distance tile and radix select that it replaces here write and read every
@@ -101,12 +105,13 @@ direct_knn_kernel(const float* __restrict__ xc, int n, int d, int row_begin, int
             }
         }
     }
-    unsigned bound[R];
+    unsigned limit[R];  // distance bits of the columns still to be gathered lie below
     uint64_t b[R][KR];
     int pending[R];
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-        bound[r] = warp_rank_value<G>(g[r], k - 1);
+        const unsigned bound = warp_rank_value<G>(g[r], k - 1);  // (all ones: fewer than k groups)
+        limit[r] = bound == 0xFFFFFFFFu ? bound : bound + 1u;
         pending[r] = 0;
 #pragma unroll
         for (int j = 0; j < KR; ++j) b[r][j] = kKeyMax;
@@ -124,14 +129,14 @@ direct_knn_kernel(const float* __restrict__ xc, int n, int d, int row_begin, int
 #pragma unroll
             for (int r = 0; r < R; ++r) {
                 distances(x, r, c, u[r]);
-                any |= min(u[r][0], u[r][1]) <= bound[r];
+                any |= min(u[r][0], u[r][1]) < limit[r];
             }
             if (!__any_sync(kFullMask, any)) continue;
 #pragma unroll
             for (int r = 0; r < R; ++r) {
 #pragma unroll
                 for (int e = 0; e < 2; ++e) {
-                    const bool in = u[r][e] <= bound[r] && u[r][e] != 0xFFFFFFFFu;
+                    const bool in = u[r][e] < limit[r];
                     const unsigned m = __ballot_sync(kFullMask, in);
                     if (!m) continue;
                     if (pending[r] + __popc(m) > kDirBuf) {  // merge what is gathered
@@ -139,11 +144,13 @@ direct_knn_kernel(const float* __restrict__ xc, int n, int d, int row_begin, int
                         for (int e0 = 0; e0 < pending[r]; e0 += 32)
                             list_merge<KR>(b[r], e0 + lane < pending[r] ? buf[warp][r][e0 + lane] : kKeyMax);
                         pending[r] = 0;
-                        const unsigned kb = list_kth_bits<KR>(b[r], k);
-                        bound[r] = min(bound[r], kb);
+                        // (strict: what is tested from here on lies above every
+                        // merged index; this step's first columns are merged in
+                        // only after its second ones were tested)
+                        limit[r] = min(limit[r], list_kth_bits<KR>(b[r], k));
                         __syncwarp();
                     }
-                    // (keys past a bound that has just tightened are kept: the list drops them)
+                    // (keys past a limit that has just tightened are kept: the list drops them)
                     if (in) buf[warp][r][pending[r] + __popc(m & ((1u << lane) - 1u))] = make_key(u[r][e], c + e);
                     pending[r] += __popc(m);
                 }
