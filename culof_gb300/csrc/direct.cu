@@ -180,12 +180,11 @@ void launch_direct(const float* xc, int n, int d, int row_begin, int row_end, in
 template <int DP>
 void dispatch_direct(const float* xc, int n, int d, int row_begin, int row_end, int k, int32_t* idx, float* d2,
                      float* kd, cudaStream_t s) {
-    // more rows per warp share each staged column once there are enough rows
-    // to fill the SMs
+    // two rows per warp share each staged column once there are enough rows
+    // to fill the SMs (16 per SM: two CTAs of 8 warps)
     const int rows = row_end - row_begin;
     if (DP > 8 || rows <= 2432) launch_direct<DP, 1>(xc, n, d, row_begin, row_end, k, idx, d2, kd, s);
-    else if (DP > 4 || rows <= 9728) launch_direct<DP, 2>(xc, n, d, row_begin, row_end, k, idx, d2, kd, s);
-    else launch_direct<DP, 4>(xc, n, d, row_begin, row_end, k, idx, d2, kd, s);
+    else launch_direct<DP, 2>(xc, n, d, row_begin, row_end, k, idx, d2, kd, s);
 }
 
 }  // namespace
