@@ -838,9 +838,9 @@ void Engine::knn_fast(const float* xc, const float* norms, int64_t n, int d, int
             // CULOF_PRUNE_LISTS=0 lists the column tiles in short segments, as
             // inputs of many segments do (the same results)
             const char* env = std::getenv("CULOF_PRUNE_LISTS");
-            small_knn(tiles, boxes, qbox, perm, n, d, nt, t0, mt, k, sms, iso_rows_enabled(n),
-                      env && env[0] == '0' ? 8 : kSegTiles, iso_.get(small_iso_bytes(mt, k)), iso_count_word(), nbr_idx, nbr_d2, kdist2,
-                      status_ptr(), ev, s);
+            const bool defer = small_defers(iso_rows_enabled(n), nt, mt);
+            small_knn(tiles, boxes, qbox, perm, n, d, nt, t0, mt, k, sms, defer, env && env[0] == '0' ? 8 : kSegTiles,
+                      iso_.get(small_iso_bytes(mt, k, defer)), iso_count_word(), nbr_idx, nbr_d2, kdist2, status_ptr(), ev, s);
             mark(4);
             return;
         }

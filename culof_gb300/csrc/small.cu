@@ -508,7 +508,10 @@ void dispatch_small(const SmallArgs& A) {
 }
 
 constexpr int kOrderMaxTiles = 16384;
-int64_t iso_capacity(int mt) { return static_cast<int64_t>(mt) * kCT / 4 + static_cast<int64_t>(mt / 32) * kCT; }
+// Most rows that can leave (none without the pass of their own).
+int64_t iso_capacity(int mt, bool defer) {
+    return defer ? static_cast<int64_t>(mt) * kCT / 4 + static_cast<int64_t>(mt / 32) * kCT : 0;
+}
 
 }  // namespace
 
@@ -537,29 +540,30 @@ void small_build_tiles(const float* xc, int64_t n, int d, const unsigned* perm, 
     CG_LAUNCH_CHECK();
 }
 
-size_t small_iso_bytes(int mt, int k) {
-    const size_t cap = static_cast<size_t>(iso_capacity(mt));
-    return sizeof(uint64_t) * cap * 32 * (k <= 32 ? 1 : 2) + sizeof(int) * (cap + mt);
+bool small_defers(bool wanted, int nt, int mt) {
+    return wanted && nt > kWindow && nt <= kIsoMaxTiles && mt <= kOrderMaxTiles;
+}
+
+size_t small_iso_bytes(int mt, int k, bool defer) {
+    const size_t cap = static_cast<size_t>(iso_capacity(mt, defer));
+    return sizeof(uint64_t) * cap * 32 * (k <= 32 ? 1 : 2) + sizeof(int) * (cap + (mt <= kOrderMaxTiles ? mt : 0));
 }
 
 void small_knn(const float* tiles, const float* boxes, const void* qbox, const unsigned* perm, int64_t n, int d, int nt,
-               int t0, int mt, int k, int sms, bool defer_rows, int segment, void* iso, int* iso_count, int32_t* nbr_idx, float* nbr_d2,
+               int t0, int mt, int k, int sms, bool defer, int segment, void* iso, int* iso_count, int32_t* nbr_idx, float* nbr_d2,
                float* kdist2, int* status, unsigned long long* evaluated, cudaStream_t s) {
     if (mt <= 0) return;
     SmallArgs A{tiles, boxes, static_cast<const __nv_bfloat16*>(qbox), perm, n, nt, t0, mt, k, sms,
-                segment, defer_rows && nt > kWindow && nt <= kIsoMaxTiles, nullptr, {}, nbr_idx, nbr_d2, kdist2, status,
-                evaluated, s};
+                segment, defer, nullptr, {}, nbr_idx, nbr_d2, kdist2, status, evaluated, s};
     char* w = static_cast<char*>(iso);
     A.iso.count = iso_count;
     A.iso.list = reinterpret_cast<uint64_t*>(w);
-    A.iso.pos = reinterpret_cast<int*>(w + sizeof(uint64_t) * static_cast<size_t>(iso_capacity(mt)) * 32 * (k <= 32 ? 1 : 2));
+    A.iso.pos = reinterpret_cast<int*>(w + sizeof(uint64_t) * static_cast<size_t>(iso_capacity(mt, defer)) * 32 * (k <= 32 ? 1 : 2));
     if (mt <= kOrderMaxTiles) {
-        int* order = A.iso.pos + iso_capacity(mt);
+        int* order = A.iso.pos + iso_capacity(mt, defer);
         tile_order_kernel<<<static_cast<unsigned>(ceil_div(mt, 32)), 256, 0, s>>>(boxes, padded_dims(d), t0, mt, order);
         CG_LAUNCH_CHECK();
         A.order = order;
-    } else {
-        A.defer = false;
     }
     switch (padded_dims(d)) {
         case 2: dispatch_small<2>(A); break;

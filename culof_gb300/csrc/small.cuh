@@ -62,15 +62,17 @@ size_t small_tiles_floats(int dp, int nt);
 void small_build_tiles(const float* xc, int64_t n, int d, const unsigned* perm, int nt, float* tiles, float* boxes,
                        void* qbox, cudaStream_t s);
 
-// Workspace of the rows that leave the sweep for their own pass.
-size_t small_iso_bytes(int mt, int k);
+// Whether rows may leave the sweep for a pass of their own, if that is wanted.
+bool small_defers(bool wanted, int nt, int mt);
+// Workspace of the row tiles' order and, with defer, of the rows that leave.
+size_t small_iso_bytes(int mt, int k, bool defer);
 // Exact k-NN of the rows of row tiles [t0, t0 + mt), written in the
 // reference's slot order. evaluated (nullable) counts (row, half) pairs
-// past the seed window; iso is small_iso_bytes(mt, k) bytes,
-// *iso_count zero; segment (at most
+// past the seed window; defer as small_defers() has it, iso small_iso_bytes(mt,
+// k, defer) bytes, *iso_count zero; segment (at most
 // kSegTiles) column tiles are listed at a time.
 void small_knn(const float* tiles, const float* boxes, const void* qbox, const unsigned* perm, int64_t n, int d, int nt,
-               int t0, int mt, int k, int sms, bool defer_rows, int segment, void* iso, int* iso_count, int32_t* nbr_idx, float* nbr_d2,
+               int t0, int mt, int k, int sms, bool defer, int segment, void* iso, int* iso_count, int32_t* nbr_idx, float* nbr_d2,
                float* kdist2, int* status, unsigned long long* evaluated, cudaStream_t s);
 
 }  // namespace culof_gb300
