@@ -846,12 +846,17 @@ void Engine::knn_fast(const float* xc, const float* norms, int64_t n, int d, int
         }
     }
 
-    // 3. seed lists and the shared k-th keys
-    char* rows = static_cast<char*>(rows_.get(padded * sizeof(uint64_t) * (k + 1) +
-                                              (tensor ? 0 : static_cast<size_t>(nsplit) * padded * k * sizeof(uint64_t)) + 256));
-    uint64_t* seed_keys = reinterpret_cast<uint64_t*>(rows);
-    unsigned long long* kth_shared = reinterpret_cast<unsigned long long*>(seed_keys + padded * k);
-    uint64_t* partial = reinterpret_cast<uint64_t*>(kth_shared + padded);
+    // 3. seed lists and the shared k-th keys (the tensor sweep past 8 features
+    // has no seed)
+    uint64_t* seed_keys = nullptr;
+    unsigned long long* kth_shared = nullptr;
+    uint64_t* partial = nullptr;
+    if (wide || small_tc) {
+        seed_keys = rows_.as<uint64_t>(static_cast<size_t>(padded) * (k + 1) +
+                                       (wide ? static_cast<size_t>(nsplit) * padded * k : 0));
+        kth_shared = reinterpret_cast<unsigned long long*>(seed_keys + padded * k);
+        partial = reinterpret_cast<uint64_t*>(kth_shared + padded);
+    }
     int* status = status_ptr();
     const unsigned* maxn = max_norm_word();
     mark(2);
@@ -889,7 +894,7 @@ void Engine::knn_fast(const float* xc, const float* norms, int64_t n, int d, int
     if (sweep && mt > 0 && tensor) {
         uint64_t* lists = static_cast<uint64_t*>(tc_lists_.get(tc_list_bytes(mt, nsplit)));
         int32_t* lost = d > kMaxWideD ? lost_.as<int32_t>(static_cast<size_t>(mt) * kRT) : nullptr;
-        tc_sweep(tcb, n, nt, t0, mt, nsplit, d, k, maxn, small_tc ? kth_shared : nullptr, small_tc ? seed_keys : nullptr,
+        tc_sweep(tcb, n, nt, t0, mt, nsplit, d, k, maxn, kth_shared, seed_keys,
                  lists, status, nbr_idx, nbr_d2, kdist2, s, qs, lost, lost_count_word(), plist, pcount);
         if (lost) {  // tiles of up to 1 GiB
             const int tile = choose_tile_rows(n, static_cast<size_t>(1) << 30);

@@ -35,3 +35,10 @@ def test_no_lists_for_isolated_rows_that_cannot_leave(monkeypatch):
     off = _kept(n, 2, 8)
     # a list of 32 keys (and its row) for a quarter of the rows and more
     assert on - off > n // 4 * 32 * 8 - (4 << 20)
+
+
+def test_no_seed_lists_without_a_seed():
+    # the tensor path past 8 features starts from none: what it keeps does not
+    # grow with k (the split of the columns is the same)
+    n = 100_000
+    assert abs(_kept(n, 24, 48) - _kept(n, 24, 8)) < 8 << 20
