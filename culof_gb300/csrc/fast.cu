@@ -818,7 +818,11 @@ void Engine::knn_fast(const float* xc, const float* norms, int64_t n, int d, int
     float* tiles = nullptr;
     TcBuffers tcb{};
     float* boxes = nullptr;
-    if (tensor) tcb = tc_prepare(cols_.get(tc_buffer_bytes(padded, d)), xc, norms, n, d, perm, nt, mm, max_norm_word(), s);
+    int32_t* lost = nullptr;
+    if (tensor) {
+        lost = lost_.as<int32_t>(kLostGroups + static_cast<size_t>(mt) * kRT);
+        tcb = tc_prepare(cols_.get(tc_buffer_bytes(padded, d)), xc, norms, n, d, perm, nt, mm, max_norm_word(), lost, s);
+    }
     if (wide) {
         tiles = cols_.as<float>(wide_tiles_floats(d, nt));
         wide_build_tiles(xc, norms, n, d, perm, nt, tiles, s);
@@ -893,19 +897,11 @@ void Engine::knn_fast(const float* xc, const float* norms, int64_t n, int d, int
     // 4. sweep over the other tiles, split S ways
     if (sweep && mt > 0 && tensor) {
         uint64_t* lists = static_cast<uint64_t*>(tc_lists_.get(tc_list_bytes(mt, nsplit)));
-        int32_t* lost = d > kMaxWideD ? lost_.as<int32_t>(static_cast<size_t>(mt) * kRT) : nullptr;
-        tc_sweep(tcb, n, nt, t0, mt, nsplit, d, k, maxn, kth_shared, seed_keys,
-                 lists, status, nbr_idx, nbr_d2, kdist2, s, qs, lost, lost_count_word(), plist, pcount);
-        if (lost) {  // tiles of up to 1 GiB
-            const int tile = choose_tile_rows(n, static_cast<size_t>(1) << 30);
-            float* d_tile = tile_.as<float>(static_cast<size_t>(tile) * n);
-            for (int64_t row0 = 0; row0 < pos1 - pos0; row0 += tile) {
-                const int rows = static_cast<int>(std::min<int64_t>(tile, pos1 - pos0 - row0));
-                distance_tile(xc, n, d, row0, rows, d_tile, s, lost, lost_count_word());
-                select_tile_rows(d_tile, norms, rows, row0, n, k, kSelectDistances, nbr_idx, nbr_d2, kdist2, s, lost,
-                                 lost_count_word());
-            }
-        }
+        int32_t* rows = lost + kLostGroups;
+        tc_sweep(tcb, n, nt, t0, mt, nsplit, d, k, maxn, kth_shared, seed_keys, lists, status, nbr_idx, nbr_d2, kdist2, s,
+                 qs, rows, lost_count_word(), plist, pcount);
+        lost_rows(xc, n, d, k, rows, lost_count_word(), lost_keys_.get(lost_rows_bytes(n, pos1 - pos0, k, sms)), lost,
+                  sms, nbr_idx, nbr_d2, kdist2, s);
         mark(4);
         return;
     } else if (nt > 1 && mt > 0 && wide) {

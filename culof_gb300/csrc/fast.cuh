@@ -66,9 +66,9 @@ struct TcBuffers {
 };
 size_t tc_buffer_bytes(int64_t padded, int d);
 // minmax: the per-dimension (min, max) keys of the spatial-order pass; maxn:
-// the largest norm (float bits).
+// the largest norm (float bits); arrived: what lost_rows() wants zero.
 TcBuffers tc_prepare(void* buf, const float* xc, const float* norms, int64_t n, int d, const unsigned* perm, int nt,
-                     const unsigned* minmax, const unsigned* maxn, cudaStream_t s);
+                     const unsigned* minmax, const unsigned* maxn, int* arrived, cudaStream_t s);
 int tc_max_splits();
 constexpr int kMaxTensorD = 256;
 constexpr int kTcSplitD = 42;  // split operands up to here (3d <= 128)
@@ -81,11 +81,19 @@ size_t tc_list_bytes(int nt, int nsplit);
 // positions 0..qs-1 are the seed's; 0: no seed, kth_seed and seed_keys null);
 // plist / pcount (nullable): per row tile,
 // the column tiles to visit in order (the small-d prune lists); without them
-// every tile past the window is visited. lost_rows / lost_count: d > 128, the
-// original indices of the rows that this path leaves to the general one.
+// every tile past the window is visited. lost_rows / lost_count: the original
+// indices of the rows that it leaves to lost_rows().
 void tc_sweep(const TcBuffers& b, int64_t n, int nt, int t0, int mt, int nsplit, int d, int k, const unsigned* maxn,
               const unsigned long long* kth_seed, const uint64_t* seed_keys, uint64_t* lists, int* status,
               int32_t* nbr_idx, float* nbr_d2, float* kdist2, cudaStream_t s, int qs, int32_t* lost_rows, int* lost_count,
               const uint2* plist = nullptr, const int* pcount = nullptr);
+
+// The exact k nearest of the points rows[0 .. *count) (lost_rows.cu; both on the
+// device, at most max_rows) among all n points, d <= kMaxTensorD. scratch:
+// lost_rows_bytes() bytes; arrived: kLostGroups words, zero (16-byte aligned).
+constexpr int kLostGroups = 512;
+size_t lost_rows_bytes(int64_t n, int64_t max_rows, int k, int sms);
+void lost_rows(const float* xc, int64_t n, int d, int k, const int32_t* rows, const int* count, void* scratch,
+               int* arrived, int sms, int32_t* idx, float* d2, float* kd, cudaStream_t s);
 
 }  // namespace culof_gb300

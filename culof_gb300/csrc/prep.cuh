@@ -32,13 +32,10 @@ enum SelectMode : int {
     kSelectDistances = 0,  // tile holds exact squared distances; self is skipped
     kSelectGram = 1,       // tile holds Gram values (reference contract, knn.cu:136-156)
 };
-// list (nullable): the rows are list[row0, row0 + rows), as far as *count
-// reaches (both on the device), instead of row0 + i.
 void distance_tile(const float* xc, int64_t n, int d, int64_t row0, int rows, float* tile,
-                   cudaStream_t s, const int32_t* list = nullptr, const int* count = nullptr);
+                   cudaStream_t s);
 void select_tile_rows(float* tile, const float* norms, int rows, int64_t row_offset, int64_t n, int k, int mode,
-                      int32_t* nbr_idx, float* nbr_d2, float* kdist2, cudaStream_t s, const int32_t* list = nullptr,
-                      const int* count = nullptr);
+                      int32_t* nbr_idx, float* nbr_d2, float* kdist2, cudaStream_t s);
 int choose_tile_rows(int64_t n_points, size_t budget_bytes);
 // rows[i] = first + i for i < m.
 void iota_rows(int32_t* rows, int64_t first, int64_t m, cudaStream_t s);

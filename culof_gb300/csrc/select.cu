@@ -17,8 +17,6 @@
 //     tile already holds exact distances and the diagonal is skipped.
 // The select itself (row_select_kernel below) is this engine's own design.
 #include "block.cuh"
-#include <algorithm>
-
 #include "common.cuh"
 #include "prep.cuh"
 #include "warp_sort.cuh"
@@ -36,48 +34,46 @@ constexpr int kTileDimChunk = 32; // dims staged per step
 // carried across chunks, which is exactly dist2_direct's operation order.
 __global__ void __launch_bounds__(kTileBlock)
 distance_tile_kernel(const float* __restrict__ xc, int64_t n, int d, int64_t row0, int rows,
-                     float* __restrict__ tile, const int32_t* __restrict__ list, const int* __restrict__ count) {
+                     float* __restrict__ tile) {
     __shared__ float srow[kTileRows][kTileDimChunk];
     __shared__ float scol[kTileBlock][kTileDimChunk + 1];
     const int64_t col0 = static_cast<int64_t>(blockIdx.x) * kTileBlock;
+    const int r0 = blockIdx.y * kTileRows;
     const int tid = threadIdx.x;
-    if (list) rows = static_cast<int>(min(static_cast<int64_t>(rows), *count - row0));
-    for (int r0 = blockIdx.y * kTileRows; r0 < rows; r0 += gridDim.y * kTileRows) {
-        float acc[kTileRows];
+    float acc[kTileRows];
 #pragma unroll
-        for (int r = 0; r < kTileRows; ++r) acc[r] = 0.0f;
+    for (int r = 0; r < kTileRows; ++r) acc[r] = 0.0f;
 
-        for (int f0 = 0; f0 < d; f0 += kTileDimChunk) {
-            const int df = min(kTileDimChunk, d - f0);
-            for (int e = tid; e < kTileRows * kTileDimChunk; e += kTileBlock) {
-                const int r = e / kTileDimChunk, f = e % kTileDimChunk;
-                float v = 0.0f;
-                if (r0 + r < rows && f < df) v = xc[(list ? list[row0 + r0 + r] : row0 + r0 + r) * d + f0 + f];
-                srow[r][f] = v;
-            }
-            for (int e = tid; e < kTileBlock * kTileDimChunk; e += kTileBlock) {
-                const int c = e / kTileDimChunk, f = e % kTileDimChunk;
-                float v = 0.0f;
-                if (col0 + c < n && f < df) v = xc[(col0 + c) * d + f0 + f];
-                scol[c][f] = v;
-            }
-            __syncthreads();
-            for (int f = 0; f < df; ++f) {
-                const float b = scol[tid][f];
-#pragma unroll
-                for (int r = 0; r < kTileRows; ++r) {
-                    const float t = __fsub_rn(srow[r][f], b);
-                    acc[r] = __fmaf_rn(t, t, acc[r]);
-                }
-            }
-            __syncthreads();
+    for (int f0 = 0; f0 < d; f0 += kTileDimChunk) {
+        const int df = min(kTileDimChunk, d - f0);
+        for (int e = tid; e < kTileRows * kTileDimChunk; e += kTileBlock) {
+            const int r = e / kTileDimChunk, f = e % kTileDimChunk;
+            float v = 0.0f;
+            if (r0 + r < rows && f < df) v = xc[(row0 + r0 + r) * d + f0 + f];
+            srow[r][f] = v;
         }
-        const int64_t j = col0 + tid;
-        if (j < n) {
-#pragma unroll
-            for (int r = 0; r < kTileRows; ++r)
-                if (r0 + r < rows) tile[static_cast<int64_t>(r0 + r) * n + j] = acc[r];
+        for (int e = tid; e < kTileBlock * kTileDimChunk; e += kTileBlock) {
+            const int c = e / kTileDimChunk, f = e % kTileDimChunk;
+            float v = 0.0f;
+            if (col0 + c < n && f < df) v = xc[(col0 + c) * d + f0 + f];
+            scol[c][f] = v;
         }
+        __syncthreads();
+        for (int f = 0; f < df; ++f) {
+            const float b = scol[tid][f];
+#pragma unroll
+            for (int r = 0; r < kTileRows; ++r) {
+                const float t = __fsub_rn(srow[r][f], b);
+                acc[r] = __fmaf_rn(t, t, acc[r]);
+            }
+        }
+        __syncthreads();
+    }
+    const int64_t j = col0 + tid;
+    if (j < n) {
+#pragma unroll
+        for (int r = 0; r < kTileRows; ++r)
+            if (r0 + r < rows) tile[static_cast<int64_t>(r0 + r) * n + j] = acc[r];
     }
 }
 
@@ -179,16 +175,16 @@ __device__ __forceinline__ unsigned row_key(const float* row, const unsigned* ca
 __global__ void __launch_bounds__(kSelThreads)
 row_select_kernel(float* __restrict__ tile, const float* __restrict__ norms, int rows, int64_t row_offset,
                   int64_t n, int k, int mode, int32_t* __restrict__ nbr_idx, float* __restrict__ nbr_d2,
-                  float* __restrict__ kdist2, const int32_t* __restrict__ list, const int* __restrict__ count) {
+                  float* __restrict__ kdist2) {
     __shared__ RowSelect sh;
     extern __shared__ unsigned cache[];
     const int r = blockIdx.x;
-    if (r >= rows || (list && row_offset + r >= *count)) return;
+    if (r >= rows) return;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const bool gram = (mode == kSelectGram);
     const bool cached = n <= kRowCache;
     float* row = tile + static_cast<int64_t>(r) * n;
-    const int64_t self = list ? list[row_offset + r] : row_offset + r;
+    const int64_t self = row_offset + r;
     // warp segments: contiguous, a multiple of 32 columns each
     const int64_t seg = ceil_div(ceil_div(n, kSelWarps), 32) * 32;
     const int64_t s0 = static_cast<int64_t>(warp) * seg;
@@ -404,22 +400,19 @@ row_select_kernel(float* __restrict__ tile, const float* __restrict__ norms, int
 }  // namespace
 
 void distance_tile(const float* xc, int64_t n, int d, int64_t row0, int rows, float* tile,
-                   cudaStream_t s, const int32_t* list, const int* count) {
+                   cudaStream_t s) {
     dim3 grid(static_cast<unsigned>(ceil_div(n, kTileBlock)), static_cast<unsigned>(ceil_div(rows, kTileRows)));
-    // a list is usually short: about 16 CTAs per SM that walk it
-    if (list) grid.y = std::min(grid.y, static_cast<unsigned>(ceil_div(152 * 16, grid.x)));
-    distance_tile_kernel<<<grid, kTileBlock, 0, s>>>(xc, n, d, row0, rows, tile, list, count);
+    distance_tile_kernel<<<grid, kTileBlock, 0, s>>>(xc, n, d, row0, rows, tile);
     CG_LAUNCH_CHECK();
 }
 
 void select_tile_rows(float* tile, const float* norms, int rows, int64_t row_offset, int64_t n, int k, int mode,
-                      int32_t* nbr_idx, float* nbr_d2, float* kdist2, cudaStream_t s, const int32_t* list,
-                      const int* count) {
+                      int32_t* nbr_idx, float* nbr_d2, float* kdist2, cudaStream_t s) {
     if (rows <= 0) return;
     set_max_dynamic_smem(reinterpret_cast<const void*>(row_select_kernel), kRowCache * sizeof(unsigned));
     const int smem = n <= kRowCache ? static_cast<int>(n * sizeof(unsigned)) : 0;
     row_select_kernel<<<rows, kSelThreads, smem, s>>>(tile, norms, rows, row_offset, n, k, mode, nbr_idx, nbr_d2,
-                                                      kdist2, list, count);
+                                                      kdist2);
     CG_LAUNCH_CHECK();
 }
 

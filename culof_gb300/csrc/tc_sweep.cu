@@ -26,8 +26,10 @@
 //   * a second kernel rescores each row's surviving entries (about k) exactly
 //     from FP32 row-major coordinates (the oracle's direct-difference chain)
 //     and writes the k best in the reference's slot order. A row whose list
-//     would overflow with entries inside the margin (heavy duplicates)
-//     switches to exact lists: its candidates are then rescored as they pass.
+//     would overflow with entries inside the margin (a wide margin, duplicates)
+//     switches to an exact list: its candidates are then rescored as they pass.
+//     A row that rescores more than a pass over all points would cost leaves
+//     this path for that pass (lost_rows.cu).
 //
 // What bounds it: the MMAs and their operand copies alone take 7.6 ms at
 // n = 200,000, d = 128 (72% of the measured f16 rate); reading the
@@ -44,8 +46,8 @@
 // the float32 evaluation of f, so no column that belongs to a row's k
 // nearest is ever dropped. Data whose scale cannot be brought into the f16
 // range (|S| > 62, or non-finite values) or whose squared norms come near the
-// largest float (above 2^124: f would overflow) disable the filter: every pair
-// is then rescored exactly.
+// largest float (above 2^124: f would overflow) disable the filter: every row
+// then leaves.
 #include <cuda_fp16.h>
 
 #include <cmath>
@@ -88,10 +90,12 @@ __device__ __forceinline__ float unflip(unsigned k) {
 // One warp: the scale exponent from the features' ranges. The filter is off if
 // f = |b|^2 - 2 a.b could overflow: |f| <= 3 nmax (1 + 2^-8) and the bounds add
 // 2 m0 + slack, less than nmax, which together stay below 2^127 up to nmax =
-// 2^124 (the comparison also catches a norm that is not a number).
+// 2^124 (the comparison also catches a norm that is not a number). It also zeroes
+// the counts that lost_rows() starts from.
 constexpr float kMaxNorm = 21267647932558653966460912964485513216.0f;  // 2^124
 __global__ void tc_scale_kernel(const unsigned* __restrict__ mm, int d, const unsigned* __restrict__ max_norm_bits,
-                                TcScale* __restrict__ out) {
+                                TcScale* __restrict__ out, int4* __restrict__ arrived) {
+    for (int i = threadIdx.x; i < kLostGroups / 4; i += 32) arrived[i] = make_int4(0, 0, 0, 0);
     float mx = 0.0f;
     bool finite = __uint_as_float(*max_norm_bits) <= kMaxNorm;
     for (int f = threadIdx.x; f < d; f += 32) {
@@ -288,12 +292,20 @@ __device__ __forceinline__ uint32_t flip_bits(float f) {
 // exact lists hold the usual (distance bits << 32 | original index).
 constexpr int kModeApprox = 0;
 constexpr int kModeExact = 1;
-// More than 128 features: a row whose list overflows leaves the path, and the
-// distance tile and select of the general path take it afterwards. Rescoring
-// its candidates one by one reads two rows of coordinates per pair, which past
-// a tenth of the pairs costs more than the whole tile (clusters, d = 256, n =
-// 8,000, k = 20: 7.5 ms, this way 2.1; the tile and select of all rows 2.7).
+// Rows that lost_rows() takes afterwards. Rescoring a pair reads two rows of
+// coordinates and costs 10 to 18 times a pair there (92 against 5.2 ps, d = 32,
+// n = 20,000 equal points; 273 against 25, d = 128). So an exact row leaves once
+// it has rescored kExactPerTile pairs per column tile of its share: with 8, a
+// few rows of clusters (d = 128, n = 50,000, k = 50) left that are cheaper to
+// keep (12.6 ms for 10.7), with 16 Cauchy data (d = 32, n = 20,000) take 7.4 ms
+// for 5.2 (36.4 when no row left). Rows leave as soon as their list overflows
+// (kLose) where a CTA's share of the columns is short, so that the budget would
+// not cover the rescoring of the list itself (kShortShare tiles: 5,000 clustered
+// points of 64 features 414 us for 726, 8,000 were slower that way, 959 for 739),
+// and past 128 features, where a pair costs the most.
 constexpr int kModeLost = 2;
+constexpr int kExactPerTile = 16;
+constexpr int kShortShare = 12;
 
 // Per-row lists live in global memory (L2-resident while their CTA runs):
 // kTcM keys per row, 128 rows per CTA. Keeping them out of shared memory
@@ -612,7 +624,7 @@ __noinline__ __device__ bool exact_chunk(TcRows& sh, uint64_t* __restrict__ glis
 constexpr int kHalvesK = 56;
 __device__ __forceinline__ int bound_tiles(int count) { return min(count, max(128, count / 4)); }
 
-template <int NB>
+template <int NB, bool kLose>
 __global__ void __launch_bounds__(kTcThreads, NB == 2 ? 2 : 1)
 tc_sweep_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ CUtensorMap tmapb,
                 const float* __restrict__ xr,
@@ -623,7 +635,6 @@ tc_sweep_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
                 const uint2* __restrict__ plist, const int* __restrict__ pcount) {
     extern __shared__ uint8_t tc_raw[];
     TcSmem<NB>& sh = *reinterpret_cast<TcSmem<NB>*>((reinterpret_cast<uintptr_t>(tc_raw) + 1023) & ~uintptr_t(1023));
-    constexpr bool kLose = NB > 2;  // overflowing rows leave (kModeLost)
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int T = T0 + static_cast<int>(blockIdx.x) % ntb;
     const int split = static_cast<int>(blockIdx.x) / ntb;
@@ -634,13 +645,14 @@ tc_sweep_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
     const int q0 = qs + split * per;
     const int q1 = min(nt, q0 + per);
     const int lcount = plist ? pcount[T] : 0;
-    const int count = plist ? (lcount > split ? (lcount - split + nsplit - 1) / nsplit : 0) : (q1 > q0 ? q1 - q0 : 0);
+    const bool off = scale->all != 0.0f;  // the f values carry no information: every row leaves
+    const int count = off ? 0 : plist ? (lcount > split ? (lcount - split + nsplit - 1) / nsplit : 0) : (q1 > q0 ? q1 - q0 : 0);
     const uint2* tlist = plist ? plist + static_cast<int64_t>(T) * nt : nullptr;
     // without a seed window the row itself is among the columns: its list holds
     // one entry more
     const int kx = qs == 0 ? k + 1 : k;
     // tiles 0 .. scan - 1 are read twice: first for the rows' bounds (below)
-    const int scan = scale->all != 0.0f ? 0 : bound_tiles(count);
+    const int scan = bound_tiles(count);
     const int total = scan + count;
     const int halves = kx > kHalvesK && scan > 1 ? 2 : 1;
     auto col_tile = [&](int jj) -> int {
@@ -675,8 +687,7 @@ tc_sweep_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
         sh.cnt[r] = 0;
         sh.sorted[r] = 0;
         sh.athr[r] = __int_as_float(0x7f800000);
-        // with the filter disabled the f values carry no information: exact lists
-        sh.mode[r] = scale->all == 0.0f ? kModeApprox : kLose ? kModeLost : kModeExact;
+        sh.mode[r] = off ? kModeLost : kModeApprox;
         const RowBounds rb = row_bounds(cn[rbase + r], nmax, Kp, split_ops ? 0.0f : rn[rbase + r],
                                         __uint_as_float(scale->resmax), scale->eta, split_ops ? d : 0, 16 * ksteps);
         sh.c0[r] = rb.c0;
@@ -748,11 +759,15 @@ tc_sweep_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
         const int r = row0 + lane;
         uint64_t* const mylist = glist + static_cast<size_t>(r) * kTcListRow;
         const TcScale sc = *scale;
-        const bool all = !kLose && sc.all != 0.0f;
         const bool row_valid = __ldg(ix + rbase + r) != kNoIndex;
-        bool exact_any = all;  // some list of the warp is exact
-        bool exact_row = all;
-        bool lost = kLose && sc.all != 0.0f;
+        bool exact_any = false;  // some list of the warp is exact
+        bool exact_row = false;
+        bool lost = off;
+        int exact_left = kExactPerTile * count;  // pairs that this row may rescore
+        // (from k = 48 on, a list that keeps much more than k by the wide margin of
+        // single operands is compacted again every few entries: clusters of d = 140,
+        // n = 4,100, k = 64 1.31 ms for 1.73; of d = 100 1.47 for 1.85)
+        const int most_kept = kLose && !split_ops && kx > 48 ? min(kx + 12, kTcListRow - 32) : kTcListRow - 32;
         ExactPending pending;
         int cnt = 0;  // entries of this thread's list while it is approximate (sh.cnt while compacting)
         float tau = 0.0f;  // the list's threshold, and as a packed pair
@@ -817,25 +832,20 @@ tc_sweep_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
                 lo[0] = fminf(fminf(lo[0], lo_f(f[2 * q])), hi_f(f[2 * q]));
                 lo[1] = fminf(fminf(lo[1], lo_f(f[2 * q + 1])), hi_f(f[2 * q + 1]));
             }
-            if (!__any_sync(0xffffffffu, fminf(lo[0], lo[1]) <= tau || all)) return;
-            unsigned pass = 0;
-            if (all) {
-                pass = row_valid ? 0xFFFFFFFFu : 0u;
-            } else {
-                // the signs of f - tq (tq the next float above the threshold),
-                // in four independent chains of shifts
-                unsigned part[4] = {0, 0, 0, 0};
+            if (!__any_sync(0xffffffffu, fminf(lo[0], lo[1]) <= tau)) return;
+            // the signs of f - tq (tq the next float above the threshold), in
+            // four independent chains of shifts
+            unsigned part[4] = {0, 0, 0, 0};
 #pragma unroll
-                for (int q = 3; q >= 0; --q) {
+            for (int q = 3; q >= 0; --q) {
 #pragma unroll
-                    for (int c = 0; c < 4; ++c) {
-                        const uint64_t dl = sub2(f[4 * c + q], tq);
-                        part[c] = __funnelshift_l(static_cast<unsigned>(dl >> 32), part[c], 1);
-                        part[c] = __funnelshift_l(static_cast<unsigned>(dl), part[c], 1);
-                    }
+                for (int c = 0; c < 4; ++c) {
+                    const uint64_t dl = sub2(f[4 * c + q], tq);
+                    part[c] = __funnelshift_l(static_cast<unsigned>(dl >> 32), part[c], 1);
+                    part[c] = __funnelshift_l(static_cast<unsigned>(dl), part[c], 1);
                 }
-                pass = part[0] | part[1] << 8 | part[2] << 16 | part[3] << 24;
             }
+            const unsigned pass = part[0] | part[1] << 8 | part[2] << 16 | part[3] << 24;
             if (!exact_row) {
                 // approximate keys straight into the thread's own list (f
                 // recomputed exactly as the packed filter did)
@@ -849,9 +859,21 @@ tc_sweep_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
             }
             bool changed = false;
             __syncwarp();
-            if (!kLose && exact_any)
+            if (!kLose && exact_any) {
                 changed = exact_chunk(sh, glist, row0, exact_row ? pass : 0u, pending, rbase, cbase + 32 * ch, xr, ix,
                                       dr, k);
+                if (exact_row) exact_left -= __popc(pass);
+                if (__any_sync(0xffffffffu, exact_row && exact_left < 0)) {
+                    if (exact_row && exact_left < 0) {
+                        sh.mode[r] = kModeLost;
+                        lost = true;
+                        exact_row = false;
+                        cnt = 0;
+                    }
+                    exact_any = __any_sync(0xffffffffu, exact_row);
+                    changed = true;
+                }
+            }
             // keep room for the next chunk: compact approximate lists with
             // less than 32 free slots
             unsigned full = __ballot_sync(0xffffffffu, !exact_row && cnt > kTcListRow - 32);
@@ -863,14 +885,14 @@ tc_sweep_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
                     const int src = __ffs(full) - 1;
                     full &= full - 1;
                     uint64_t* lst = glist + static_cast<size_t>(row0 + src) * kTcListRow;
-                    if (approx_compact(sh, lst, row0 + src, kx, c2, sh.c3[row0 + src], sh.c4[row0 + src],
-                                       kTcListRow - 32) > kTcListRow - 32) {
-                        if (kLose) {
-                            if (lane == src) lost = true;
-                        } else {
-                            to_exact_mode(sh, lst, row0 + src, rbase + row0 + src, xr, ix, dr, k);
-                            exact_any = true;
-                        }
+                    const int kept = approx_compact(sh, lst, row0 + src, kx, c2, sh.c3[row0 + src], sh.c4[row0 + src],
+                                                    kTcListRow - 32);
+                    if (kept <= most_kept) continue;
+                    if (kLose) {
+                        if (lane == src) lost = true;
+                    } else {
+                        to_exact_mode(sh, lst, row0 + src, rbase + row0 + src, xr, ix, dr, k);
+                        exact_any = true;
                     }
                 }
                 exact_row = sh.mode[r] == kModeExact;
@@ -889,7 +911,7 @@ tc_sweep_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
             // scanned columns below it (102 at k = 51, all at 64), the halves
             // together -128 ln(1 - k / 128) (65 and 89).
             float gm[64];
-            float B = __int_as_float(0xff800000);
+            float B = __int_as_float(0xff800000), top = B;
 #pragma unroll 1
             for (int part = 0; part < halves && alive; ++part) {
                 const int need = halves == 1 ? kx : part == 0 ? (kx + 1) / 2 : kx / 2;
@@ -928,6 +950,10 @@ tc_sweep_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
                         }
                     }
                 }
+                if (kLose) {
+#pragma unroll
+                    for (int q = 0; q < 64; ++q) top = fmaxf(top, gm[q]);
+                }
                 // the need-th smallest of the 64, by bisection over the ordered bits
                 uint32_t at = 0;
 #pragma unroll 1
@@ -944,7 +970,14 @@ tc_sweep_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
                 const float bound = need <= 64 ? unflip(at) : __int_as_float(0x7f800000);
                 B = bound == bound ? fmaxf(B, bound) : __int_as_float(0x7f800000);
             }
-            if (row_valid && B < __int_as_float(0x7f800000)) sh.athr[r] = approx_thr(B, c2, sh.c3[r], sh.c4[r]);
+            if (row_valid && B < __int_as_float(0x7f800000)) {
+                const float athr = approx_thr(B, c2, sh.c3[r], sh.c4[r]);
+                sh.athr[r] = athr;
+                // a threshold over every group's minimum takes in more columns
+                // than the list holds (for k up to 31 the bound it starts from
+                // is close to the row's k-th f)
+                if (kLose) lost = kx <= 32 && top <= athr;
+            }
             set_tau();
         }
         for (int j = scan; alive && j < total; ++j) {
@@ -1115,7 +1148,7 @@ size_t tc_list_bytes(int nt, int nsplit) {
 }
 
 TcBuffers tc_prepare(void* buf, const float* xc, const float* norms, int64_t n, int d, const unsigned* perm, int nt,
-                     const unsigned* minmax, const unsigned* maxn, cudaStream_t s) {
+                     const unsigned* minmax, const unsigned* maxn, int* arrived, cudaStream_t s) {
     const int64_t padded = static_cast<int64_t>(nt) * kCT;
     const auto up = [](size_t x) { return (x + 255) & ~static_cast<size_t>(255); };
     TcBuffers b;
@@ -1141,7 +1174,7 @@ TcBuffers tc_prepare(void* buf, const float* xc, const float* norms, int64_t n, 
     b.ix = reinterpret_cast<unsigned*>(p);
     p += up(sizeof(unsigned) * padded);
     b.scale = p;
-    tc_scale_kernel<<<1, 32, 0, s>>>(minmax, d, maxn, reinterpret_cast<TcScale*>(b.scale));
+    tc_scale_kernel<<<1, 32, 0, s>>>(minmax, d, maxn, reinterpret_cast<TcScale*>(b.scale), reinterpret_cast<int4*>(arrived));
     CG_LAUNCH_CHECK();
     int64_t g = ceil_div(padded * b.Kp, 256);
     if (g > 152 * 16) g = 152 * 16;
@@ -1166,7 +1199,8 @@ void tc_sweep(const TcBuffers& b, int64_t n, int nt, int t0, int mt, int nsplit,
               int* lost_count, const uint2* plist, const int* pcount) {
     const bool wide = b.Kp > 128;
     const size_t smem = (wide ? sizeof(TcSmem<4>) : sizeof(TcSmem<2>)) + 1024;
-    const auto kernel = wide ? tc_sweep_kernel<4> : tc_sweep_kernel<2>;
+    const bool lose = wide || (nt - qs + nsplit - 1) / nsplit <= kShortShare;
+    const auto kernel = wide ? tc_sweep_kernel<4, true> : lose ? tc_sweep_kernel<2, true> : tc_sweep_kernel<2, false>;
     set_max_dynamic_smem(reinterpret_cast<const void*>(kernel), static_cast<int>(smem));
     const CUtensorMap map = tc::make_kmajor_map(b.xh, static_cast<int64_t>(nt) * kCT, b.Kp, true);
     const CUtensorMap mapb = tc::make_kmajor_map(b.xb, static_cast<int64_t>(nt) * kCT, b.Kp, true);
