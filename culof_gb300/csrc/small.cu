@@ -46,7 +46,12 @@ namespace {
 using namespace small;
 
 constexpr float kSparseRatio = 4.0f;  // a tile is sparse when its squared diagonal exceeds 4x the median tile's
-constexpr int kSparseWaves = 4;       // sparse tiles leave whole up to 4 row tiles per SM (see launch_small)
+// Sparse tiles leave whole up to 4 row tiles per SM; with more only those a
+// thousand times as wide as the median tile (heavy tails: 1-d Cauchy data, n =
+// 100,000 and 200,000, 0.77 and 0.80 ms for 1.21 and 1.58; with kSparseRatio at
+// any size, clusters with uniform outliers, d = 1, n = 200,000, 0.93 for 0.78).
+constexpr int kSparseWaves = 4;
+constexpr float kVerySparseRatio = 1e6f;
 
 // ---------------------------------------------------------------- tiles
 
@@ -270,9 +275,9 @@ small_sweep_kernel(SweepRows P, int64_t row0, const int* __restrict__ order, int
     if (P.base >= P.n) return;
     if (defer_rows) {
         const int median = static_cast<int>(min(static_cast<unsigned>(order[mt / 2]), static_cast<unsigned>(mt - 1)));
-        P.sparse = defer_rows == 2 && tile_i < mt / 32 &&
-                   box_extent(P.boxes + P.base / kCT * 2 * DP, DP) >
-                       kSparseRatio * box_extent(P.boxes + (row0 / kCT + median) * 2 * DP, DP);
+        const float usual = box_extent(P.boxes + (row0 / kCT + median) * 2 * DP, DP);
+        P.sparse = tile_i < mt / 32 && (defer_rows == 2 || usual > 0.0f) &&
+                   box_extent(P.boxes + P.base / kCT * 2 * DP, DP) > (defer_rows == 2 ? kSparseRatio : kVerySparseRatio) * usual;
         sweep_rows<DP, KR, G, RW, W, true>(sh, P);
     } else {
         sweep_rows<DP, KR, G, RW, W, false>(sh, P);

@@ -64,3 +64,21 @@ def test_a_refused_layout_is_refused_again():
             for got, p, k in zip(b.run(ctx), probs, ks):
                 _same(got, p, k)
         assert ctx.batched_tuning()["ctas_per_sm"] > 0
+
+
+@pytest.mark.parametrize("normalize", [False, True])
+@pytest.mark.parametrize("d", [2, 4, 5, 8, 9, 12, 13, 16, 17, 32, 33])
+def test_every_list_form_in_every_padded_width(d, normalize):
+    # the lists' limits in one batch (groups of one launch each), sizes at the
+    # tiles' and the window's edges, duplicates more than the gathered buffer holds
+    sizes = (25, 64, 65, 128, 129, 640, 641, 900, 2000)
+    ks = (24, 25, 32, 33, 48, 1, 24, 33, 20)
+    probs = [synthetic.clusters_with_outliers(n, d, seed=n + d) for n in sizes]
+    for p in probs:
+        p[len(p) // 2:] = p[: len(p) - len(p) // 2] if len(p) < 200 else p[len(p) // 2:]
+    probs[7][100:300] = probs[7][7]
+    probs[8][::5] = probs[8][3]
+    with _culof.Context() as ctx:
+        for got, p, k in zip(Batch(probs, ks).run(ctx, normalize=normalize), probs, ks):
+            want = oracle.lof(p, k, normalize)
+            np.testing.assert_array_equal(got.view(np.uint32), want.view(np.uint32))
