@@ -759,21 +759,28 @@ void Engine::knn_fast(const float* xc, const float* norms, int64_t n, int d, int
     int sms = 152;
     CG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device_));
     // The tensor sweep: every split of a row tile scans for its own bounds and
-    // keeps its own lists (together about 64 tile visits), so it takes the
-    // split that needs the least rounds of CTAs times their length (n = 30,011,
-    // d = 100, k = 30: 1.42 ms per fit_predict with one split, 1.50 with two,
-    // 1.53 with three; n = 50,000, d = 32, k = 20, forward and backward: 4.18,
-    // 4.06, 4.08 ms).
+    // keeps its own lists, so it takes the split that needs the least rounds of
+    // CTAs times their length. Up to 128 features two CTAs share an SM and a
+    // split costs about 64 tile visits (n = 30,011, d = 100, k = 30: 1.42 ms per
+    // fit_predict with one split, 1.50 with two, 1.53 with three, when a pass
+    // took twice what it does now; n = 50,000, d = 32, k = 20, forward and
+    // backward: 4.18, 4.06, 4.08 ms). Above, one CTA takes an SM and 30 fit
+    // (scores, factor model, d = 200, k = 20, splits 1 to 4: n = 5,000 309, 259,
+    // 245, 283 us; 8,000 381, 305, 357, 332; 12,000 472, 505, 436, 479; 20,000
+    // 993, 915, 889, 888; 30,000 1275, 1528, 1404, 1506; k = 64: 8,000 829, 801,
+    // 854, 857; 12,000 1086, 1239, 1316, 1485).
     int nsplit = 1;
     if (nt > 1) {
         if (wide) {
             nsplit = choose_splits(mt, sms);
             if (nsplit > nt - 1) nsplit = nt - 1;
         } else if (tensor) {
-            const int64_t slots = 2 * sms;  // CTAs at a time
+            const bool one = d > kMaxWideD;            // CTA per SM
+            const int64_t slots = one ? sms : 2 * sms;  // CTAs at a time
             // (k > 56 leaves a list little room for the filter's margin: most
-            // rows rescore candidates exactly, and every split pays that anew)
-            const int64_t own = k > 56 ? 256 : 64;
+            // rows rescore candidates exactly, or leave, and every split pays
+            // that anew)
+            const int64_t own = k > 56 ? (one ? 64 : 256) : one ? 30 : 64;
             int64_t best = -1;
             // (past two rounds the list entries that every split repeats cost
             // more than the last round's idle SMs: n = 200,000, d = 128, k = 50,
