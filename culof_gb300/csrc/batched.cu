@@ -126,14 +126,6 @@ bc_apply_kernel(const float* __restrict__ x, int64_t ntot, int d, const int* __r
 
 // ---- spatial order within each problem -----------------------------------------
 
-__device__ __forceinline__ unsigned flip_f(float f) {
-    const unsigned u = __float_as_uint(f);
-    return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-}
-__device__ __forceinline__ float unflip_f(unsigned k) {
-    return __uint_as_float((k & 0x80000000u) ? (k & 0x7FFFFFFFu) : ~k);
-}
-
 constexpr int kMortonDimsB = 8;
 
 // One block per problem: per-dimension range of its centred points, then
@@ -167,7 +159,7 @@ bm_minmax_kernel(const float* __restrict__ xc, const int64_t* __restrict__ off, 
             }
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
-                const unsigned k = flip_f(v[j]);
+                const unsigned k = order_bits(v[j]);
                 mn = min(mn, k);
                 mx = max(mx, k);
             }
@@ -177,8 +169,8 @@ bm_minmax_kernel(const float* __restrict__ xc, const int64_t* __restrict__ off, 
     }
     __syncthreads();
     for (int f = threadIdx.x; f < d; f += blockDim.x) {
-        pmm[(static_cast<int64_t>(p) * d + f) * 2] = unflip_f(lo[f]);
-        pmm[(static_cast<int64_t>(p) * d + f) * 2 + 1] = unflip_f(hi[f]);
+        pmm[(static_cast<int64_t>(p) * d + f) * 2] = order_value(lo[f]);
+        pmm[(static_cast<int64_t>(p) * d + f) * 2 + 1] = order_value(hi[f]);
     }
     if (threadIdx.x == 0) {
         const int m = d < kMortonDimsB ? d : kMortonDimsB;
@@ -189,7 +181,7 @@ bm_minmax_kernel(const float* __restrict__ xc, const int64_t* __restrict__ off, 
             for (int f = 0; f < d; ++f) {
                 bool taken = false;
                 for (int q = 0; q < j; ++q) taken |= chosen[q] == f;
-                const float sp = unflip_f(hi[f]) - unflip_f(lo[f]);
+                const float sp = order_value(hi[f]) - order_value(lo[f]);
                 if (!taken && sp > span) {
                     span = sp;
                     best = f;

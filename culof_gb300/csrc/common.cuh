@@ -63,6 +63,16 @@ __host__ __device__ __forceinline__ uint32_t key_index(uint64_t key) {
 
 constexpr uint64_t kKeyMax = ~0ull;
 
+// Bits whose unsigned order is the order of the floats (negative ones flipped),
+// and the float of such bits.
+__device__ __forceinline__ uint32_t order_bits(float f) {
+    const uint32_t u = __float_as_uint(f);
+    return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+}
+__device__ __forceinline__ float order_value(uint32_t k) {
+    return __uint_as_float((k & 0x80000000u) ? (k & 0x7FFFFFFFu) : ~k);
+}
+
 // Rows per partial sum of the centring reduction (the CPU oracle uses the same
 // order, so the FP64 means agree bit for bit).
 constexpr int kCenterChunk = 256;

@@ -134,16 +134,6 @@ __global__ void __launch_bounds__(kBlock) score_kernel(const int32_t* __restrict
 
 // ---- contamination offset --------------------------------------------------
 
-// Float -> uint32 whose unsigned order is the float order (negatives flipped).
-__device__ __forceinline__ unsigned int order_key(float f) {
-    const unsigned int u = __float_as_uint(f);
-    return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-}
-__device__ __forceinline__ float from_order_key(unsigned int k) {
-    const unsigned int u = (k & 0x80000000u) ? (k & 0x7FFFFFFFu) : ~k;
-    return __uint_as_float(u);
-}
-
 __global__ void offset_init_kernel(int* __restrict__ hist, OffsetState* __restrict__ st) {
     for (int b = threadIdx.x; b < kOffsetHistBins; b += blockDim.x) hist[b] = 0;
     if (threadIdx.x == 0) {
@@ -169,7 +159,7 @@ __global__ void offset_hist_kernel(const float* __restrict__ nof, int64_t n, int
     const unsigned int prefix = st->prefix;
     for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
          i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-        const unsigned int key = order_key(nof[i]);
+        const unsigned int key = order_bits(nof[i]);
         if ((key & hi_mask) == (prefix & hi_mask)) atomicAdd(&sh[(key >> shift) & (bins - 1)], 1);
     }
     __syncthreads();
@@ -217,7 +207,7 @@ __global__ void offset_next_kernel(const float* __restrict__ nof, int64_t n, Off
     unsigned int mn = 0xFFFFFFFFu;
     for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
          i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-        const unsigned int key = order_key(nof[i]);
+        const unsigned int key = order_bits(nof[i]);
         if (key <= a) ++cnt;
         else mn = min(mn, key);
     }
@@ -233,8 +223,8 @@ __global__ void offset_next_kernel(const float* __restrict__ nof, int64_t n, Off
 
 __global__ void offset_finalize_kernel(int64_t n, int64_t lo, int use_upper, float w, OffsetState* __restrict__ st,
                                        double* __restrict__ out) {
-    const float a = from_order_key(st->prefix);
-    const float b = (static_cast<int64_t>(st->count_le) >= lo + 2 || lo >= n - 1) ? a : from_order_key(st->min_gt);
+    const float a = order_value(st->prefix);
+    const float b = (static_cast<int64_t>(st->count_le) >= lo + 2 || lo >= n - 1) ? a : order_value(st->min_gt);
     const float diff = __fsub_rn(b, a);
     const float r = use_upper ? __fsub_rn(b, __fmul_rn(diff, w)) : __fadd_rn(a, __fmul_rn(diff, w));
     st->a_key = st->prefix;
@@ -289,7 +279,7 @@ offset_cluster_kernel(const float* __restrict__ nof, int64_t n, int64_t lo, int 
         const unsigned hi_mask = p == 0 ? 0u : 0xFFFFFFFFu << (shift + width);
         for (int64_t i0 = base; i0 < n; i0 += stride) {
             const int64_t i = i0 + tid;
-            const unsigned key = i < n ? order_key(nof[i]) : 0u;
+            const unsigned key = i < n ? order_bits(nof[i]) : 0u;
             const bool in = i < n && ((key ^ prefix) & hi_mask) == 0u;
             // lanes of the same bin elect one adder (scores share few bins)
             const unsigned active = __ballot_sync(0xffffffffu, in);
@@ -324,7 +314,7 @@ offset_cluster_kernel(const float* __restrict__ nof, int64_t n, int64_t lo, int 
     // the smallest key above the order statistic
     unsigned mn = 0xFFFFFFFFu;
     for (int64_t i = base + tid; i < n; i += stride) {
-        const unsigned key = order_key(nof[i]);
+        const unsigned key = order_bits(nof[i]);
         if (key > prefix) mn = min(mn, key);
     }
     mn = __reduce_min_sync(0xffffffffu, mn);
@@ -332,8 +322,8 @@ offset_cluster_kernel(const float* __restrict__ nof, int64_t n, int64_t lo, int 
     cl.sync();
     mn = 0xFFFFFFFFu;
     for (int r = 0; r < nctas; ++r) mn = min(mn, *cl.map_shared_rank(&mn_s, r));
-    const float a = from_order_key(prefix);
-    const float b = (static_cast<int64_t>(below) + eq >= lo + 2 || lo >= n - 1) ? a : from_order_key(mn);
+    const float a = order_value(prefix);
+    const float b = (static_cast<int64_t>(below) + eq >= lo + 2 || lo >= n - 1) ? a : order_value(mn);
     const float diff = __fsub_rn(b, a);
     const float res = use_upper ? __fsub_rn(b, __fmul_rn(diff, w)) : __fadd_rn(a, __fmul_rn(diff, w));
     if (rank == 0 && tid == 0) *out = static_cast<double>(res);

@@ -147,8 +147,8 @@ center_apply_kernel(const float* __restrict__ x, int64_t n, int d, const double*
                     if (kScale) w = __dmul_rn(w, inv);
                     const float c = narrow(w);
                     xc[t + j * stride] = c;
-                    lo = max(lo, ~range_key(c));
-                    hi = max(hi, range_key(c));
+                    lo = max(lo, ~order_bits(c));
+                    hi = max(hi, order_bits(c));
                 }
             }
             if (mm != nullptr) {
@@ -247,8 +247,8 @@ center_small_kernel(const float* __restrict__ x, int n, int d, int normalize, do
         if (normalize) w = __dmul_rn(w, v);
         const float c = narrow(w);
         xc[static_cast<int64_t>(i) * d + f] = c;
-        lo = max(lo, ~range_key(c));
-        hi = max(hi, range_key(c));
+        lo = max(lo, ~order_bits(c));
+        hi = max(hi, order_bits(c));
     }
     if (mm != nullptr) {
         lo = __reduce_max_sync(0xffffffffu, lo);

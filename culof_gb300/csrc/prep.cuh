@@ -4,25 +4,20 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "common.cuh"
+
 namespace culof_gb300 {
 
 // ---- prep.cu -------------------------------------------------------------
 size_t center_partial_count(int64_t n, int d);
 // mm (nullable; zeroed by the caller, unused above kMaxRangeDims features):
-// the range of every centred feature, mm[2 f] = the largest ~range_key, mm[2 f
-// + 1] = the largest range_key.
+// the range of every centred feature, mm[2 f] = the largest ~order_bits, mm[2 f
+// + 1] = the largest order_bits.
 constexpr int kMaxRangeDims = 256;
 void center(const float* x, int64_t n, int d, bool normalize, float* xc, double* partial,
             double* mean, double* inv_std, cudaStream_t s, unsigned* mm = nullptr);
-__device__ __forceinline__ unsigned range_key(float f) {  // order-preserving bits
-    const unsigned u = __float_as_uint(f);
-    return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-}
-__device__ __forceinline__ float range_value(unsigned k) {
-    return __uint_as_float((k & 0x80000000u) ? (k & 0x7FFFFFFFu) : ~k);
-}
-__device__ __forceinline__ float range_lo(const unsigned* mm, int f) { return range_value(~mm[2 * f]); }
-__device__ __forceinline__ float range_hi(const unsigned* mm, int f) { return range_value(mm[2 * f + 1]); }
+__device__ __forceinline__ float range_lo(const unsigned* mm, int f) { return order_value(~mm[2 * f]); }
+__device__ __forceinline__ float range_hi(const unsigned* mm, int f) { return order_value(mm[2 * f + 1]); }
 // max_norm_bits: zeroed by the caller.
 void squared_norms(const float* xc, int64_t n, int d, float* norms, unsigned int* max_norm_bits,
                    cudaStream_t s);

@@ -83,10 +83,6 @@ struct TcScale {
     unsigned resmax;  // float bits
 };
 
-__device__ __forceinline__ float unflip(unsigned k) {
-    return __uint_as_float((k & 0x80000000u) ? (k & 0x7FFFFFFFu) : ~k);
-}
-
 // One warp: the scale exponent from the features' ranges. The filter is off if
 // f = |b|^2 - 2 a.b could overflow: |f| <= 3 nmax (1 + 2^-8) and the bounds add
 // 2 m0 + slack, less than nmax, which together stay below 2^127 up to nmax =
@@ -282,13 +278,7 @@ __device__ __forceinline__ uint64_t pack2(float lo, float hi) {
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
-// Order-preserving bits of a float (negative values included).
-__device__ __forceinline__ uint32_t flip_bits(float f) {
-    const uint32_t u = __float_as_uint(f);
-    return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-}
-
-// Row modes: approximate lists hold (flip(f) << 32 | sorted column position);
+// Row modes: approximate lists hold (order_bits(f) << 32 | sorted column position);
 // exact lists hold the usual (distance bits << 32 | original index).
 constexpr int kModeApprox = 0;
 constexpr int kModeExact = 1;
@@ -451,8 +441,8 @@ __noinline__ __device__ int approx_compact(TcRows& sh, uint64_t* __restrict__ ls
                 lst, s, c, kTcListRow, k - 1,
                 [&](uint64_t key) -> uint64_t {
                     if (key == kKeyMax) return kKeyMax;
-                    thr = approx_thr(unflip(key_bits(key)), c2, c3, c4);
-                    return (static_cast<uint64_t>(flip_bits(thr)) << 32) | 0xFFFFFFFFull;
+                    thr = approx_thr(order_value(key_bits(key)), c2, c3, c4);
+                    return (static_cast<uint64_t>(order_bits(thr)) << 32) | 0xFFFFFFFFull;
                 },
                 &fk);
             if (lane == 0) {
@@ -480,12 +470,12 @@ __noinline__ __device__ int approx_compact(TcRows& sh, uint64_t* __restrict__ ls
             const uint64_t t = __shfl_sync(0xffffffffu, v[j], owner);
             if (j == oreg) kk = t;
         }
-        thr = approx_thr(unflip(key_bits(kk)), c2, c3, c4);
+        thr = approx_thr(order_value(key_bits(kk)), c2, c3, c4);
     }
     int keep = 0;
 #pragma unroll
     for (int j = 0; j < kListE; ++j) {
-        const bool in = v[j] != kKeyMax && unflip(key_bits(v[j])) <= thr;
+        const bool in = v[j] != kKeyMax && order_value(key_bits(v[j])) <= thr;
         keep += __popc(__ballot_sync(0xffffffffu, in));
     }
     if (keep <= cap) {
@@ -854,7 +844,7 @@ tc_sweep_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
                     const int b = __ffs(pp) - 1;
                     pp &= pp - 1;
                     const float fb = __fmaf_rn(__uint_as_float(select32(gr, b)), sc.k2, nbj[32 * ch + b]);
-                    mylist[cnt++] = make_key(flip_bits(fb), static_cast<uint32_t>(cbase + 32 * ch + b));
+                    mylist[cnt++] = make_key(order_bits(fb), static_cast<uint32_t>(cbase + 32 * ch + b));
                 }
             }
             bool changed = false;
@@ -958,7 +948,7 @@ tc_sweep_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
                 uint32_t at = 0;
 #pragma unroll 1
                 for (int bit = 31; bit >= 0; --bit) {
-                    const float probe = unflip(at | ((1u << bit) - 1u));  // every value with this bit clear
+                    const float probe = order_value(at | ((1u << bit) - 1u));  // every value with this bit clear
                     int below = 0;
 #pragma unroll
                     for (int q = 0; q < 64; ++q) below += gm[q] <= probe ? 1 : 0;
@@ -967,7 +957,7 @@ tc_sweep_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
                     if (probe != probe) below = bit == 31 || (at >> 31) ? 64 : 0;
                     if (below < need) at |= 1u << bit;
                 }
-                const float bound = need <= 64 ? unflip(at) : __int_as_float(0x7f800000);
+                const float bound = need <= 64 ? order_value(at) : __int_as_float(0x7f800000);
                 B = bound == bound ? fmaxf(B, bound) : __int_as_float(0x7f800000);
             }
             if (row_valid && B < __int_as_float(0x7f800000)) {
@@ -1074,7 +1064,7 @@ tc_final_kernel(const float* __restrict__ xr, const unsigned* __restrict__ ix, i
             for (int j = 0; j < 4 * kMaxTcSplits; ++j) below += key_bits(v[j]) <= probe ? 1 : 0;
             if (__reduce_add_sync(0xffffffffu, below) < kx) at |= 1u << bit;
         }
-        keep = flip_bits(approx_thr(unflip(at), c2, c3, c4));
+        keep = order_bits(approx_thr(order_value(at), c2, c3, c4));
     }
     __syncwarp();
     int P = 0;
