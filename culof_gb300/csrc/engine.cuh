@@ -177,7 +177,7 @@ private:
     DevBuf morton_, perm_, sort_tmp_, cols_, rows_, tc_lists_, tiles_;
     // tile boxes; the tensor path's tile lists over d <= 8 points
     DevBuf boxes_, plist_, pcount_;
-    DevBuf lost_, lost_keys_;  // rows that leave the tensor path (after their groups' arrival counts), their lists
+    DevBuf lost_, lost_keys_;  // the tensor path's start record and the rows that leave it; their lists
     DevBuf iso_;  // rows that leave the small-d sweep for their own pass
     double stat_total_pairs_ = 0.0;  // pairs the small-d sweep would evaluate without pruning
     // Words that every k-NN call starts from zero: the device status word

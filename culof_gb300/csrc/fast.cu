@@ -38,6 +38,7 @@
 #include "prep.cuh"
 #include "small.cuh"
 #include "sweep_common.cuh"
+#include "tc_scale.cuh"
 #include "warp_sort.cuh"
 
 namespace culof_gb300 {
@@ -55,13 +56,17 @@ constexpr int kMortonDims = 8;  // Morton key over (up to) the 8 widest dimensio
 // 32-bit Morton key: 32/m bits for each of the (up to) kMortonDims features of
 // the widest range, widest first (ties by index), interleaved from the most
 // significant bit, over the bounding box of the centred data (mm, see
-// center()). Every block picks the features itself, with one warp.
+// center()). Every block picks the features itself, with one warp. With tc, a
+// warp of the last block also writes what the tensor path starts from (in a
+// launch of its own it took 3.3 us).
 __global__ void morton_kernel(const float* __restrict__ xc, int64_t n, int d, const unsigned* __restrict__ mm,
-                              unsigned* __restrict__ keys, unsigned* __restrict__ vals) {
+                              unsigned* __restrict__ keys, unsigned* __restrict__ vals,
+                              const unsigned* __restrict__ max_norm_bits, TcStart* __restrict__ tc) {
     __shared__ int dims[kMortonDims];
     __shared__ float dlo[kMortonDims], dspan[kMortonDims];
     const int md = d < kMortonDims ? d : kMortonDims;
     const int bits = (32 / md) < 30 ? (32 / md) : 30;
+    if (tc != nullptr && blockIdx.x == gridDim.x - 1 && threadIdx.x / 32 == 1) tc_start(mm, d, max_norm_bits, tc);
     if (threadIdx.x < 32) {
         const int lane = threadIdx.x;
         float span[kMaxTensorD / 32];
@@ -809,7 +814,9 @@ void Engine::knn_fast(const float* xc, const float* norms, int64_t n, int d, int
     const unsigned* mm = range_words();  // from the centring
     unsigned* keys = morton_.as<unsigned>(2 * static_cast<size_t>(n));
     unsigned* vals = perm_.as<unsigned>(2 * static_cast<size_t>(n));
-    morton_kernel<<<grid_for(n, 256), 256, 0, s>>>(xc, n, d, mm, keys, vals);
+    TcStart* start = tensor ? static_cast<TcStart*>(lost_.get(sizeof(TcStart) + sizeof(int32_t) * static_cast<size_t>(mt) * kRT))
+                            : nullptr;
+    morton_kernel<<<grid_for(n, 256), 256, 0, s>>>(xc, n, d, mm, keys, vals, max_norm_word(), start);
     CG_LAUNCH_CHECK();
     unsigned* vin = nullptr;  // after 4 passes: back in the first half
     sort_pairs_stable(keys, vals, keys + n, vals + n, n, 32, sort_tmp_.as<unsigned>(sort_pairs_counts(n)), s, &vin);
@@ -825,11 +832,7 @@ void Engine::knn_fast(const float* xc, const float* norms, int64_t n, int d, int
     float* tiles = nullptr;
     TcBuffers tcb{};
     float* boxes = nullptr;
-    int32_t* lost = nullptr;
-    if (tensor) {
-        lost = lost_.as<int32_t>(kLostGroups + static_cast<size_t>(mt) * kRT);
-        tcb = tc_prepare(cols_.get(tc_buffer_bytes(padded, d)), xc, norms, n, d, perm, nt, mm, max_norm_word(), lost, s);
-    }
+    if (tensor) tcb = tc_prepare(cols_.get(tc_buffer_bytes(padded, d)), xc, norms, n, d, perm, nt, &start->scale, s);
     if (wide) {
         tiles = cols_.as<float>(wide_tiles_floats(d, nt));
         wide_build_tiles(xc, norms, n, d, perm, nt, tiles, s);
@@ -904,11 +907,11 @@ void Engine::knn_fast(const float* xc, const float* norms, int64_t n, int d, int
     // 4. sweep over the other tiles, split S ways
     if (sweep && mt > 0 && tensor) {
         uint64_t* lists = static_cast<uint64_t*>(tc_lists_.get(tc_list_bytes(mt, nsplit)));
-        int32_t* rows = lost + kLostGroups;
+        int32_t* lost = reinterpret_cast<int32_t*>(start + 1);
         tc_sweep(tcb, n, nt, t0, mt, nsplit, d, k, maxn, kth_shared, seed_keys, lists, status, nbr_idx, nbr_d2, kdist2, s,
-                 qs, rows, lost_count_word(), plist, pcount);
-        lost_rows(xc, n, d, k, rows, lost_count_word(), lost_keys_.get(lost_rows_bytes(n, pos1 - pos0, k, sms)), lost,
-                  sms, nbr_idx, nbr_d2, kdist2, s);
+                 qs, lost, lost_count_word(), plist, pcount);
+        lost_rows(xc, n, d, k, lost, lost_count_word(), lost_keys_.get(lost_rows_bytes(n, pos1 - pos0, k, sms)),
+                  start->arrived, sms, nbr_idx, nbr_d2, kdist2, s);
         mark(4);
         return;
     } else if (nt > 1 && mt > 0 && wide) {

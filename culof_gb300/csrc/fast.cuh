@@ -65,10 +65,9 @@ struct TcBuffers {
     int ksteps;
 };
 size_t tc_buffer_bytes(int64_t padded, int d);
-// minmax: the per-dimension (min, max) keys of the spatial-order pass; maxn:
-// the largest norm (float bits); arrived: what lost_rows() wants zero.
+// scale: the call's scale record (tc_scale.cuh).
 TcBuffers tc_prepare(void* buf, const float* xc, const float* norms, int64_t n, int d, const unsigned* perm, int nt,
-                     const unsigned* minmax, const unsigned* maxn, int* arrived, cudaStream_t s);
+                     void* scale, cudaStream_t s);
 int tc_max_splits();
 constexpr int kMaxTensorD = 256;
 constexpr int kTcSplitD = 42;  // split operands up to here (3d <= 128)
@@ -90,7 +89,7 @@ void tc_sweep(const TcBuffers& b, int64_t n, int nt, int t0, int mt, int nsplit,
 
 // The exact k nearest of the points rows[0 .. *count) (lost_rows.cu; both on the
 // device, at most max_rows) among all n points, d <= kMaxTensorD. scratch:
-// lost_rows_bytes() bytes; arrived: kLostGroups words, zero (16-byte aligned).
+// lost_rows_bytes() bytes; arrived: kLostGroups words, zero.
 constexpr int kLostGroups = 512;
 size_t lost_rows_bytes(int64_t n, int64_t max_rows, int k, int sms);
 void lost_rows(const float* xc, int64_t n, int d, int k, const int32_t* rows, const int* count, void* scratch,

@@ -60,6 +60,7 @@
 #include "row_list.cuh"
 #include "sweep_common.cuh"
 #include "tc.cuh"
+#include "tc_scale.cuh"
 
 namespace culof_gb300 {
 
@@ -73,50 +74,6 @@ constexpr int kTcThreads = 32 * (2 + kEpiWarps);  // producer, MMA, epilogue war
 constexpr int kTmemCols = 256;                    // two 128-column f32 accumulators
 constexpr int kTcM = 128;                         // list capacity per row (k <= 64)
 constexpr int kBox = 128 * 128;                   // bytes of one TMA box: 128 rows x 64 f16
-
-// Scale record on the device: sc = 2^S, k2 = -2 * 2^-2S (undoes the scale of
-// a Gram value and doubles it), eta = 2^-14 * 2^-S (absolute f16 rounding
-// bound in unscaled units), all = 1 when the filter is disabled, resmax the
-// largest residual norm (tc_resid_kernel).
-struct TcScale {
-    float sc, k2, eta, all;
-    unsigned resmax;  // float bits
-};
-
-// One warp: the scale exponent from the features' ranges. The filter is off if
-// f = |b|^2 - 2 a.b could overflow: |f| <= 3 nmax (1 + 2^-8) and the bounds add
-// 2 m0 + slack, less than nmax, which together stay below 2^127 up to nmax =
-// 2^124 (the comparison also catches a norm that is not a number). It also zeroes
-// the counts that lost_rows() starts from.
-constexpr float kMaxNorm = 21267647932558653966460912964485513216.0f;  // 2^124
-__global__ void tc_scale_kernel(const unsigned* __restrict__ mm, int d, const unsigned* __restrict__ max_norm_bits,
-                                TcScale* __restrict__ out, int4* __restrict__ arrived) {
-    for (int i = threadIdx.x; i < kLostGroups / 4; i += 32) arrived[i] = make_int4(0, 0, 0, 0);
-    float mx = 0.0f;
-    bool finite = __uint_as_float(*max_norm_bits) <= kMaxNorm;
-    for (int f = threadIdx.x; f < d; f += 32) {
-        const float lo = range_lo(mm, f), hi = range_hi(mm, f);
-        finite = finite && isfinite(lo) && isfinite(hi);
-        mx = fmaxf(mx, fmaxf(fabsf(lo), fabsf(hi)));
-    }
-    mx = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(mx)));
-    finite = __all_sync(0xffffffffu, finite);
-    if (threadIdx.x != 0) return;
-    int S = 0;
-    bool all = !finite;
-    if (finite && mx > 0.0f) {
-        S = 14 - ilogbf(mx);
-        if (S > 62 || S < -62) all = true;
-    }
-    if (all) S = 0;
-    TcScale r;
-    r.sc = ldexpf(1.0f, S);
-    r.k2 = -ldexpf(1.0f, 1 - 2 * S);
-    r.eta = ldexpf(1.0f, -14 - S);
-    r.all = all ? 1.0f : 0.0f;
-    r.resmax = 0u;
-    *out = r;
-}
 
 // Sorted position p: f16 operand row (scaled), FP32 coordinates (row-major,
 // dr = d rounded up to 4, zero padded), norm (+inf for padding) and original
@@ -1124,7 +1081,7 @@ size_t tc_buffer_bytes(int64_t padded, int d) {
     const int dr = (d + 3) & ~3;
     const auto up = [](size_t x) { return (x + 255) & ~static_cast<size_t>(255); };
     return up(sizeof(__half) * padded * Kp) * (split ? 2 : 1) + up(sizeof(float) * padded * dr) +
-           2 * up(sizeof(float) * padded) + up(sizeof(unsigned) * padded) + up(sizeof(TcScale));
+           2 * up(sizeof(float) * padded) + up(sizeof(unsigned) * padded);
 }
 
 int tc_max_splits() { return kMaxTcSplits; }
@@ -1138,7 +1095,7 @@ size_t tc_list_bytes(int nt, int nsplit) {
 }
 
 TcBuffers tc_prepare(void* buf, const float* xc, const float* norms, int64_t n, int d, const unsigned* perm, int nt,
-                     const unsigned* minmax, const unsigned* maxn, int* arrived, cudaStream_t s) {
+                     void* scale, cudaStream_t s) {
     const int64_t padded = static_cast<int64_t>(nt) * kCT;
     const auto up = [](size_t x) { return (x + 255) & ~static_cast<size_t>(255); };
     TcBuffers b;
@@ -1162,10 +1119,7 @@ TcBuffers tc_prepare(void* buf, const float* xc, const float* norms, int64_t n, 
     b.rn = reinterpret_cast<float*>(p);
     p += up(sizeof(float) * padded);
     b.ix = reinterpret_cast<unsigned*>(p);
-    p += up(sizeof(unsigned) * padded);
-    b.scale = p;
-    tc_scale_kernel<<<1, 32, 0, s>>>(minmax, d, maxn, reinterpret_cast<TcScale*>(b.scale), reinterpret_cast<int4*>(arrived));
-    CG_LAUNCH_CHECK();
+    b.scale = scale;
     int64_t g = ceil_div(padded * b.Kp, 256);
     if (g > 152 * 16) g = 152 * 16;
     tc_build_kernel<<<static_cast<unsigned>(g), 256, 0, s>>>(xc, norms, n, d, b.Kp, b.dr, b.split, perm, padded,
