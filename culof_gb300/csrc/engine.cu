@@ -132,24 +132,25 @@ int Engine::tile_rows_for(int64_t n) {
 // AUTO, with the direct two-pass kernel (direct.cu) wherever it is fastest; all
 // give the same bits. k-NN on clusters (d = 128: factor model), one call, in us:
 //   d     n   k   direct  small-d   tensor   tile + select
-//   3   7168  20     155      226
-//   8   7168  20     242      273             (at 8000 direct 329, small-d 267)
-//  12   4096  20     179               157
-//  12   7168  20     376               194
-//  16   3000  20     178               148             203
-//  16   5000  20     363               168
-//  16   7000  64     548              1300
-//  24   2560  20                       143             180
-//  24   3000  64                       776             237
-//  43   3000  20                       602             264
-// 128   3000  20                       168             384
+//   3   7168  20     140      212
+//   8   7168  20     234      265             (at 8000 direct 329, small-d 263)
+//  12   4096  20     180               146
+//  12   7168  20     376               188
+//  16   3000  20     165               134             195
+//  16   5000  20     363               165
+//  16   7000  64     539              1183
+//  24   2560  20                       135             168
+//  24   3000  64                       815             198
+//  43   3000  20                       156             222
+// 128   3000  20                       157             317
 // - n <= 4096: the general path, which takes the direct kernel for d <= 16 and
 //   k <= 64. From 2561 points the tensor path for split f16 operands (16 < d
-//   <= 42) and k <= 48: with single operands its time depends on the data's
-//   spread (43 and 128 features above), and past k = 48 its lists have little
-//   room for the filter's margin. Also for d > 128, where the tile costs most
-//   (d = 200, n = 4,100, k = 20: factor model 205 us for 741, clusters 311 for
-//   721; the worst measured, clusters at k = 64: 2,182 for 727).
+//   <= 42) and k <= 48, past which its lists have little room for the filter's
+//   margin, and for d > 128, where the tile costs most (d = 200, n = 4,100,
+//   k = 20: factor model 186 us for 723, clusters 452 for 710; k = 64: 561 for
+//   725, clusters, the worst measured, 1,461 for 714). 42 < d <= 128 was drawn
+//   when rows that the filter decides little about stayed in the sweep (d = 43
+//   took 602); they now cost it less.
 // - d <= 8: the FP32 path (direct up to 7168 points, then the small-d sweep).
 // - 8 < d <= 16: the direct kernel as far as it wins, 7168 points past k = 48
 //   and 4096 for d > 12 else; for d <= 12 up to 6144, where the tensor path

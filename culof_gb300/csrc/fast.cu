@@ -237,13 +237,6 @@ __device__ __forceinline__ void pair_dist2(const float* tile, int p, const uint6
     d1 = hi_f(s);
 }
 
-// Per row of tile T: the exact k best keys over the seed window (sorted,
-// kKeyMax padded) and its k-th key, the starting point of the row's shared
-// k-th key (kth_shared) that the sweep CTAs tighten with atomicMin. The
-// window is the first qs spiral positions: tile T itself and its Morton
-// neighbours T+1, T-1, T+2 and T-2, whose points start the k-th distances much closer
-// to their final values than tile T alone (fewer candidates reach the
-// sweep's lists); the sweep covers the spiral from position qs on.
 // Per row tile T (one block): the column tiles that can hold a candidate for
 // any of its rows under the seed's k-th distances, in visiting order (the
 // tensor sweep over d <= 8 points visits only those), each with its
@@ -308,6 +301,13 @@ __global__ void __launch_bounds__(256) prune_list_kernel(const float* __restrict
     if (threadIdx.x == 0) pcount[T] = base_s;
 }
 
+// (The tensor path over d <= 8 points.) Per row of tile T: the exact k best keys
+// over the seed window (sorted, kKeyMax padded) and its k-th key, from which the
+// sweep's thresholds start (kth_shared). The window is the first qs spiral
+// positions: tile T itself and its Morton neighbours T+1, T-1, T+2 and T-2, whose
+// points start the k-th distances much closer to their final values than tile T
+// alone (fewer candidates reach the sweep's lists); the sweep covers the spiral
+// from position qs on.
 template <int DP>
 __global__ void __launch_bounds__(kThreads) seed_kernel(const float* __restrict__ tiles, int nt, int t0, int64_t n,
                                                         int k, int qs, uint64_t* __restrict__ seed_keys,

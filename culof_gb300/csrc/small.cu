@@ -108,7 +108,7 @@ __global__ void __launch_bounds__(kCT) small_tile_kernel(const float* __restrict
 // Refines the Morton order: every chunk of 1024 sorted points becomes a
 // balanced k-d order (halved along the dimension of largest variance down to
 // 16 points), which makes tiles, halves and the 16-row groups more compact:
-// the sweep evaluates 138 instead of 192 halves per row (n = 200,000, d = 8,
+// the sweep evaluates 145 instead of 192 halves per row (n = 200,000, d = 8,
 // k = 20; larger chunks gain little more). One CTA per chunk, one thread per
 // point; a point's sort key is its coordinate's order-preserving bits with
 // the low 10 replaced by its place in the chunk (the order is a heuristic, no

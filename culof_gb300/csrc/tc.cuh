@@ -89,9 +89,6 @@ __device__ __forceinline__ void mma_commit(uint64_t* bar) {
                  : "memory");
 }
 
-// Asynchronous form: issue the load; the registers are valid only after
-// tmem_wait32 on the same array (which takes them as read-write operands, so
-// no use can be scheduled above the wait).
 // 32 columns, waited for in the same statement (a separate wait that ties the
 // registers costs a move per register).
 __device__ __forceinline__ void tmem_ld32_bits(uint32_t taddr, uint32_t (&r)[32]) {

@@ -1,5 +1,6 @@
 // The fused distance + filtered exact select for wider points (8 < d <= 128),
-// FP32 on the CUDA cores.
+// FP32 on the CUDA cores: the FAST path past 8 features when it is asked for
+// (AUTO takes the direct kernel or the tensor path there).
 //
 // Same algorithm as the small-d sweep (fast.cu): rows of a 128-point tile
 // against column tiles in Morton order, e = |b|^2 - 2 a.b evaluated once per

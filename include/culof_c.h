@@ -37,10 +37,14 @@ extern "C" {
 #define CULOF_ERR_KERNEL 5 /* a kernel reported an error status word (e.g. a bounded wait expired) */
 
 /* Path selection for culof_context_set_path. */
-/* AUTO: GENERAL for n <= 4096 (2560 for d > 16), past k = 64 or past d = 256;
- * FAST for d <= 8, and for d <= 16 up to n = 7168; TENSOR otherwise. Inputs
- * of up to 7168 points and 16 features (k <= 64) then run one direct kernel
- * instead of the FAST or GENERAL path's own. */
+/* AUTO:
+ *   GENERAL past k = 64 or past d = 256; for n <= 4096; but only for n <= 2560
+ *           where 17 <= d <= 42 and k <= 48, and where d > 128;
+ *   FAST    otherwise for d <= 8, and for 9 <= d <= 16 up to n = 7168 (k > 48),
+ *           n = 6144 (k <= 48, d <= 12) or n = 4096 (k <= 48, d > 12);
+ *   TENSOR  otherwise.
+ * For d <= 16 and k <= 64, GENERAL up to n = 4096 and FAST up to the sizes above
+ * (7168 for d <= 8) run one direct kernel instead of their own. */
 #define CULOF_PATH_AUTO 0
 #define CULOF_PATH_FAST 1    /* fused FP32 distance + select (d <= 128, k <= 64)          */
 #define CULOF_PATH_GENERAL 2 /* exact distance tile + radix select (any d, any k)        */
@@ -68,10 +72,7 @@ CULOF_API int culof_device_info(char* buf, size_t cap);
  * The context binds to the device current at creation. */
 CULOF_API int culof_context_create(culof_context** out);
 CULOF_API void culof_context_destroy(culof_context* ctx);
-/* Run on a caller's cudaStream_t (NULL: the context's own stream). Part of a
- * call may run on two streams of the context forked from that stream by an
- * event and joined back to it before the call's later work: everything a
- * call writes is ordered on the call's stream as if it ran there alone. */
+/* Run on a caller's cudaStream_t (NULL: the context's own stream). */
 CULOF_API int culof_context_set_stream(culof_context* ctx, void* cuda_stream);
 CULOF_API int culof_context_synchronize(culof_context* ctx);
 /* CULOF_PATH_* (default AUTO). Every path returns bit-identical results. */
