@@ -20,6 +20,9 @@ constexpr int kRowsPerWarp = kRT / kWarps;  // 16 rows owned by each warp
 constexpr int kMaxK = 64;
 constexpr int kQueueCap = 32 + 8 * 32;      // one rescoring chunk + one step's worth of candidates
 constexpr unsigned kNoIndex = 0xFFFFFFFFu;
+// Filters of the form |b|^2 - 2 a.b are off where the largest squared norm passes
+// 2^124 (or is not a number): their values could overflow.
+constexpr float kMaxFilterNorm = 21267647932558653966460912964485513216.0f;
 constexpr long long kSpinLimit = 1ll << 24;  // bounded mbarrier waits (~1-2 s with backoff)
 
 // Column-tile visiting order of row tile T: T, T+1, T-1, T+2, T-2, ... mod nt

@@ -7,6 +7,7 @@
 
 #include "fast.cuh"
 #include "prep.cuh"
+#include "sweep_common.cuh"
 
 namespace culof_gb300 {
 
@@ -22,13 +23,12 @@ struct TcScale {
 // One warp: the scale exponent from the features' ranges. The filter is off if
 // f = |b|^2 - 2 a.b could overflow: |f| <= 3 nmax (1 + 2^-8) and the bounds add
 // 2 m0 + slack, less than nmax, which together stay below 2^127 up to nmax =
-// 2^124 (the comparison also catches a norm that is not a number).
-constexpr float kMaxTcNorm = 21267647932558653966460912964485513216.0f;  // 2^124
+// 2^124 = kMaxFilterNorm (the comparison also catches a norm that is not a number).
 __device__ __forceinline__ void tc_scale_record(const unsigned* __restrict__ mm, int d,
                                                 const unsigned* __restrict__ max_norm_bits, TcScale* __restrict__ out) {
     const int lane = threadIdx.x & 31;
     float mx = 0.0f;
-    bool finite = __uint_as_float(*max_norm_bits) <= kMaxTcNorm;
+    bool finite = __uint_as_float(*max_norm_bits) <= sweep::kMaxFilterNorm;
     for (int f = lane; f < d; f += 32) {
         const float lo = range_lo(mm, f), hi = range_hi(mm, f);
         finite = finite && isfinite(lo) && isfinite(hi);

@@ -162,6 +162,7 @@ wide_sweep_kernel(const float* __restrict__ tiles, int nt, int t0, int mt, int n
     const int split = static_cast<int>(blockIdx.x) / mt;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const float nmax = __uint_as_float(*max_norm_bits);
+    const bool off = !(nmax <= kMaxFilterNorm);  // every pair is rescored
     const int64_t tfl = wide_tile_floats(dpw);
     const float* own = tiles + static_cast<int64_t>(T) * tfl;
     const int per = (nt - 1 + nsplit - 1) / nsplit;
@@ -269,20 +270,26 @@ wide_sweep_kernel(const float* __restrict__ tiles, int nt, int t0, int mt, int n
                     asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(dlt) : "l"(acc[ip][c]), "l"(tau2p[ip]));
                     signs |= static_cast<unsigned>(dlt) | static_cast<unsigned>(dlt >> 32);
                 }
-                if (__any_sync(0xffffffffu, static_cast<int>(signs) < 0)) {
+                if (off || __any_sync(0xffffffffu, static_cast<int>(signs) < 0)) {
                     unsigned pass = 0;
+                    const int col = block_col(tx, c);
 #pragma unroll
                     for (int ip = 0; ip < 4; ++ip) {
                         pass |= (lo_f(acc[ip][c]) <= tau_r[2 * ip] ? 1u : 0u) << (2 * ip);
                         pass |= (hi_f(acc[ip][c]) <= tau_r[2 * ip + 1] ? 1u : 0u) << (2 * ip + 1);
                     }
+                    if (off) {  // (rows and columns of the padding aside)
+                        pass = 0;
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) pass |= (tau_r[i] != __int_as_float(0xff800000) ? 1u : 0u) << i;
+                        if (H.bi[hb][col] == kNoIndex) pass = 0;
+                    }
                     int tot;
-                    int off = warp_prefix_offset(__popc(pass), tot);
-                    const int col = block_col(tx, c);
+                    int at = warp_prefix_offset(__popc(pass), tot);
                     while (pass) {
                         const int b = __ffs(pass) - 1;
                         pass &= pass - 1;
-                        H.queue[warp][qc + off++] = static_cast<uint16_t>(((r0 + b) << 8) | col);
+                        H.queue[warp][qc + at++] = static_cast<uint16_t>(((r0 + b) << 8) | col);
                     }
                     qc += tot;
                     __syncwarp();
