@@ -147,8 +147,8 @@ int Engine::tile_rows_for(int64_t n) {
 //   k <= 64. From 2561 points the tensor path for split f16 operands (16 < d
 //   <= 42) and k <= 48, past which its lists have little room for the filter's
 //   margin, and for d > 128, where the tile costs most (d = 200, n = 4,100,
-//   k = 20: factor model 186 us for 723, clusters 452 for 710; k = 64: 561 for
-//   725, clusters, the worst measured, 1,461 for 714). 42 < d <= 128 was drawn
+//   k = 20: factor model 186 us for 723, clusters 452 for 710; k = 64, scores:
+//   682 for 767, clusters, the worst measured, 1,215 for 756). 42 < d <= 128 was drawn
 //   when rows that the filter decides little about stayed in the sweep (d = 43
 //   took 602); they now cost it less.
 // - d <= 8: the FP32 path (direct up to 7168 points, then the small-d sweep).

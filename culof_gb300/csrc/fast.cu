@@ -772,8 +772,11 @@ void Engine::knn_fast(const float* xc, const float* norms, int64_t n, int d, int
     // backward: 4.18, 4.06, 4.08 ms). Above, one CTA takes an SM and 30 fit
     // (scores, factor model, d = 200, k = 20, splits 1 to 4: n = 5,000 309, 259,
     // 245, 283 us; 8,000 381, 305, 357, 332; 12,000 472, 505, 436, 479; 20,000
-    // 993, 915, 889, 888; 30,000 1275, 1528, 1404, 1506; k = 64: 8,000 829, 801,
-    // 854, 857; 12,000 1086, 1239, 1316, 1485).
+    // 993, 915, 889, 888; 30,000 1275, 1528, 1404, 1506). Past k = 56 there one
+    // split: a list of a share starts from a looser bound, and clusters fill it
+    // (d = 200, k = 64, n = 4,100, one split against the three of that rule: 1,227
+    // for 1,500 us, factor model 688 for 601; n = 8,000 2,726 for 2,948 and 822
+    // for 788; the general path takes 767 and 2,412).
     int nsplit = 1;
     if (nt > 1) {
         if (wide) {
@@ -783,14 +786,14 @@ void Engine::knn_fast(const float* xc, const float* norms, int64_t n, int d, int
             const bool one = d > kMaxWideD;            // CTA per SM
             const int64_t slots = one ? sms : 2 * sms;  // CTAs at a time
             // (k > 56 leaves a list little room for the filter's margin: most
-            // rows rescore candidates exactly, or leave, and every split pays
-            // that anew)
-            const int64_t own = k > 56 ? (one ? 64 : 256) : one ? 30 : 64;
+            // rows rescore candidates exactly, and every split pays that anew)
+            const int64_t own = one ? 30 : k > 56 ? 256 : 64;
             int64_t best = -1;
             // (past two rounds the list entries that every split repeats cost
             // more than the last round's idle SMs: n = 200,000, d = 128, k = 50,
             // 24.2 ms with one split, 31.0 with two)
-            for (int v = 1; v <= (mt >= 2 * slots ? 1 : tc_max_splits()) && v < nt; ++v) {
+            const int most = mt >= 2 * slots || (one && k > 56) ? 1 : tc_max_splits();
+            for (int v = 1; v <= most && v < nt; ++v) {
                 const int64_t cost = ceil_div(static_cast<int64_t>(mt) * v, slots) * (nt / v + own);
                 if (best < 0 || cost < best) {
                     best = cost;
