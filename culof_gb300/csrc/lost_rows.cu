@@ -13,9 +13,9 @@
 // item of a group to finish merges the group's lists.
 //
 // What bounds it: the packed FP32 distances, 9/8 x 4d instructions per 128 columns
-// and row. The FMA pipe is busy 45% of the time (barriers, list merges and the
-// last round of CTAs take the rest). 20,000 Cauchy points of 32 features, which
-// all leave, take 2.1 ms here (7.5 ms the call, 36.4 when their pairs were
+// and row. The FMA pipe is busy half of the time (barriers, list merges and a
+// partly empty last wave take the rest). 20,000 Cauchy points of 32 features,
+// which all leave, take 2.2 ms here (7.5 ms the call, 36.4 when their pairs were
 // rescored one by one in the sweep, 19.4 when that had seven splits of the
 // columns); 8,000 of 200 features 1.8 ms (2.0 the call; 2.9 when the distance
 // tile and select took them).
